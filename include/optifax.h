@@ -231,9 +231,9 @@ int optifax_opo_run(optifax_handle h, const optifax_opo* cavities, int32_t n_cav
  *
  * The caller passes the pulse's inputs and outputs (device pointers, as for
  * optifax_propagate, validated by the same rules; stats optional) and no
- * handle.  The descriptor, twiddle tables and cluster exchange buffer live in
- * one static device array of 350,720 bytes (about 0.35 MB) that each GPU
- * loading the library reserves until the process exits.  n_points must be 8192
+ * handle.  The descriptor and twiddle tables live in one static device array of
+ * 18,944 bytes that each GPU loading the library reserves until the process
+ * exits (the cluster exchange runs through shared memory).  n_points must be 8192
  * or 16384 (clusters of 2 or 4 CTAs of 4096 points); other sizes, including
  * anything above 16384, return OPTIFAX_ERR_UNSUPPORTED.  Variants BATCH_XTAL,
  * BATCH_OP, NO_BC and HARD_BC are accepted.

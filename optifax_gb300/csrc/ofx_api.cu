@@ -29,8 +29,8 @@ struct optifax_context {
     std::map<int, Twiddle*> passtw;      // M -> pass-1 table [16][M/16] then pass-2 [16][M/256]
     PulseDev* d_desc = nullptr;
     size_t desc_cap = 0;
-    float2* d_xch = nullptr;             // cluster exchange scratch
-    size_t xch_cap = 0;                  // in complex values
+    float2* d_xs = nullptr;              // cavities' trip-output scratch
+    size_t xs_cap = 0;                   // in complex values
     std::vector<cudaStream_t> side;      // streams for concurrent launch groups
     std::vector<cudaEvent_t> ev;         // fork/join events
     int* d_grid_flags = nullptr;
@@ -47,7 +47,7 @@ namespace {
 
 // out[e] = W_n^e = exp(-2 pi i e / n) for e < count, rounded to FP32, with
 // d = 1/|w|^2 - 1 in FP64.  The cluster exchange's tables: the quarter period of
-// W_M (count M/4) and W_N^i for i < 64.
+// W_M (count M/4) and W_N^i for i < 64 (also the source of the crystal pass's FFT tables).
 __global__ void twiddle_kernel(Twiddle* out, int n, int count) {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count) return;
@@ -208,8 +208,8 @@ int ensure_sync_objects(optifax_context* h, size_t n_streams) {
 // Order the groups for launch (longest work first within a group; groups in order
 // of their longest pulse, longest first: the block scheduler serves earlier
 // launches first, so the critical path starts at once and large clusters find
-// whole GPCs free only at the start) and return the exchange scratch they need
-// (complex values).
+// whole GPCs free only at the start) and return the scratch that their cavities need
+// (complex values: the trip's crystal output of each).
 size_t order_groups(std::vector<Group>& groups) {
     for (auto& g : groups) {
         std::stable_sort(g.d.begin(), g.d.end(),
@@ -218,23 +218,20 @@ size_t order_groups(std::vector<Group>& groups) {
     auto group_key = [](const Group& g) { return g.d.empty() ? 0.0 : pulse_cost(g.d.front()); };
     std::stable_sort(groups.begin(), groups.end(),
                      [&](const Group& x, const Group& y) { return group_key(x) > group_key(y); });
-    size_t need_xch = 0;
-    for (auto& g : groups) {
-        if (g.C > 1) need_xch += g.d.size() * 2 * (size_t)g.M * g.C;
+    size_t need_xs = 0;
+    for (auto& g : groups)
         for (const auto& d : g.d)
-            if (d.fb) need_xch += (size_t)g.M * g.C;    // OPO: the trip's crystal output (cavity scratch)
-    }
-    return need_xch;
+            if (d.fb) need_xs += (size_t)g.M * g.C;
+    return need_xs;
 }
 
-// Descriptors in launch order with their exchange scratch carved from xch.
-std::vector<PulseDev> place_descriptors(std::vector<Group>& groups, float2* xch) {
+// Descriptors in launch order with their cavity scratch carved from xs.
+std::vector<PulseDev> place_descriptors(std::vector<Group>& groups, float2* xs) {
     std::vector<PulseDev> all;
     size_t xoff = 0;
     for (auto& g : groups)
         for (auto& d : g.d) {
-            if (g.C > 1) { d.xch = xch + xoff; xoff += 2 * (size_t)g.M * g.C; }
-            if (d.fb) { d.xs = xch + xoff; xoff += (size_t)g.M * g.C; }
+            if (d.fb) { d.xs = xs + xoff; xoff += (size_t)g.M * g.C; }
             all.push_back(d);
         }
     return all;
@@ -247,10 +244,6 @@ int group_tables(optifax_context* h, const std::vector<Group>& groups, cudaStrea
     tabv->assign(groups.size(), FftTables{});
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const int M = groups[gi].M;
-        const Twiddle* twp = get_pass_twiddles(h, M, st, &rc);
-        if (!twp) return rc;
-        (*tabv)[gi].tw1 = twp;
-        (*tabv)[gi].tw2 = twp + M;
         (*tabv)[gi].quad = get_table(h, h->quadtw, M, M / 4, st, &rc);       // quarter period of W_M
         if (!(*tabv)[gi].quad) return rc;
         (*tabv)[gi].low = get_table(h, h->tw, M * groups[gi].C, 64, st, &rc);  // W_N^i, i < 64
@@ -310,7 +303,7 @@ int enqueue_groups(optifax_context* h, const std::vector<Group>& groups, int met
         }
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3((unsigned)(g.d.size() * C), 1, 1);
-        lc.blockDim = dim3(M / 16, 1, 1);
+        lc.blockDim = dim3((unsigned)ke->threads, 1, 1);
         lc.dynamicSmemBytes = ke->smem;
         lc.stream = ls;
         cudaLaunchAttribute attrs[2];
@@ -341,15 +334,15 @@ int enqueue_groups(optifax_context* h, const std::vector<Group>& groups, int met
 // Stage every group's descriptors into the handle's scratch and launch the groups.
 int launch_groups(optifax_context* h, std::vector<Group>& groups, int method, const VariantCfg& vc,
                   bool shared, cudaStream_t st) {
-    const size_t need_xch = order_groups(groups);
-    if (need_xch > h->xch_cap) {
-        size_t cap = h->xch_cap * sizeof(float2);
-        int grc = grow_scratch(h, (void**)&h->d_xch, &cap, need_xch * sizeof(float2), st,
-                               "cudaMallocAsync(exchange scratch)");
-        h->xch_cap = cap / sizeof(float2);
+    const size_t need_xs = order_groups(groups);
+    if (need_xs > h->xs_cap) {
+        size_t cap = h->xs_cap * sizeof(float2);
+        int grc = grow_scratch(h, (void**)&h->d_xs, &cap, need_xs * sizeof(float2), st,
+                               "cudaMallocAsync(cavity scratch)");
+        h->xs_cap = cap / sizeof(float2);
         if (grc) return grc;
     }
-    std::vector<PulseDev> all = place_descriptors(groups, h->d_xch);
+    std::vector<PulseDev> all = place_descriptors(groups, h->d_xs);
     size_t nb = all.size() * sizeof(PulseDev);
     if (nb > h->desc_cap) {
         int grc = grow_scratch(h, (void**)&h->d_desc, &h->desc_cap, nb < 4096 ? 4096 : nb * 2, st,
@@ -425,7 +418,7 @@ int optifax_destroy(optifax_handle h) {
     for (auto& kv : h->quadtw) cudaFree(kv.second);
     if (h->d_desc) cudaFree(h->d_desc);
     if (h->d_grid_flags) cudaFree(h->d_grid_flags);
-    if (h->d_xch) cudaFree(h->d_xch);
+    if (h->d_xs) cudaFree(h->d_xs);
     if (h->d_gnlse_desc) cudaFree(h->d_gnlse_desc);
     if (h->d_gnlse_k) cudaFree(h->d_gnlse_k);
     for (auto s_ : h->side) cudaStreamDestroy(s_);
@@ -494,7 +487,6 @@ struct optifax_graph_s {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     PulseDev* d_desc = nullptr;
-    float2* d_xch = nullptr;
     int kernels = 0;
 };
 
@@ -519,7 +511,6 @@ int optifax_graph_destroy(optifax_graph g) {
     if (g->exec) cudaGraphExecDestroy(g->exec);
     if (g->graph) cudaGraphDestroy(g->graph);
     if (g->d_desc) cudaFree(g->d_desc);       // synchronises with any launch still running
-    if (g->d_xch) cudaFree(g->d_xch);
     delete g;
     return OPTIFAX_OK;
 }
@@ -539,9 +530,9 @@ int optifax_propagate_graph(optifax_handle h, const optifax_pulse* pulses, int32
     optifax_graph g = new (std::nothrow) optifax_graph_s();
     if (!g) return fail(h, OPTIFAX_ERR_NO_MEMORY, "graph object");
     g->device = h->device;
-    // the graph owns its descriptors and exchange scratch: later calls on the handle
-    // neither move nor overwrite them
-    const size_t need_xch = order_groups(gv);
+    // the graph owns its descriptors: later calls on the handle neither move nor
+    // overwrite them (passes without a cavity need no scratch)
+    order_groups(gv);
     std::vector<PulseDev> all;
     cudaStream_t s0 = nullptr;
     std::vector<cudaStream_t> side;
@@ -554,9 +545,7 @@ int optifax_propagate_graph(optifax_handle h, const optifax_pulse* pulses, int32
         if (code) optifax_graph_destroy(g);
         return code;
     };
-    if ((e = cudaMalloc(&g->d_xch, (need_xch ? need_xch : 1) * sizeof(float2))) != cudaSuccess)
-        return cleanup(cuda_fail(h, e, "cudaMalloc(graph exchange scratch)"));
-    all = place_descriptors(gv, g->d_xch);
+    all = place_descriptors(gv, nullptr);
     if ((e = cudaMalloc(&g->d_desc, all.size() * sizeof(PulseDev))) != cudaSuccess)
         return cleanup(cuda_fail(h, e, "cudaMalloc(graph descriptors)"));
     if ((e = cudaMemcpy(g->d_desc, all.data(), all.size() * sizeof(PulseDev), cudaMemcpyHostToDevice)) != cudaSuccess)

@@ -9,11 +9,11 @@ namespace ofx {
 
 typedef void (*KernelFn)(const PulseDev*, FftTables, KernelCfg);
 
-struct KernelEntry { KernelFn fn; size_t smem; int M, C, method; };
+struct KernelEntry { KernelFn fn; size_t smem; int threads, M, C, method; };
 
 template <int M, int C, int METH>
 KernelEntry kernel_entry() {
-    return KernelEntry{&pass_kernel<M, C, METH>, Smem<M, METH, C>::bytes, M, C, METH};
+    return KernelEntry{&pass_kernel<M, C, METH>, Smem<M, METH, C>::bytes, M / kPoints<M>, M, C, METH};
 }
 
 void register_kernels_heun_large(std::vector<KernelEntry>& v);

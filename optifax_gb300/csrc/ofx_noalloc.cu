@@ -6,10 +6,10 @@
 // allocator up front, and a latency-critical loop cannot afford cudaMalloc /
 // cudaFree, which may synchronise the whole device.  optifax_propagate_noalloc
 // serves them.  The caller still passes every input and output; everything else
-// the pass needs -- the pulse descriptor, the FFT twiddle tables and the
-// cluster exchange buffer -- lives in one file-scope static device array of
-// fixed size (g_noalloc_scratch, 350,720 bytes, about 0.35 MB), which every GPU
-// that loads this library reserves until the process exits.
+// the pass needs -- the pulse descriptor and the twiddle tables -- lives in one
+// file-scope static device array of fixed size (g_noalloc_scratch, 18,944 bytes),
+// which every GPU that loads this library reserves until the process exits.  The
+// cluster exchange runs through the CTAs' shared memory.
 //
 // The kernel is the clustered Heun crystal pass (4096 points per CTA, clusters
 // of 2 or 4 CTAs), so n_points must be 8192 or 16384; anything else, in
@@ -22,9 +22,7 @@
 // twiddle tables of both sizes.  That call must come before any stream capture;
 // made while its stream captures, it returns OPTIFAX_ERR_UNSUPPORTED and sets
 // nothing up.  Each call writes its descriptor with a one-thread kernel that
-// receives it as a kernel parameter (no host staging buffer), and every
-// exchange value is written before it is read, so nothing in the array has to
-// start at zero.  All calls share the array and it keeps the last call's
+// receives it as a kernel parameter (no host staging buffer).  All calls share the array and it keeps the last call's
 // contents: calls that overlap on the GPU (other streams, other host threads)
 // race on it and must be serialised by the caller.
 #include <cmath>
@@ -44,18 +42,14 @@ namespace {
 constexpr int kM = 4096;                 // points per CTA
 constexpr int kMaxN = 16384;             // cluster of 4
 constexpr size_t kDescBytes = 512;
-constexpr size_t kPassTw = kM + 16 * (kM / 256);          // pass-1 + pass-2 outer twiddles
 constexpr size_t kQuadTw = kM / 4;                         // W_M^y, y < M/4 (cluster exchange)
 constexpr size_t kLowTw = 64;                              // W_N^i, i < 64 (cluster exchange), per N
-constexpr size_t kXch = 2 * (size_t)kMaxN;                 // exchange buffer (complex)
-constexpr size_t kOffPass = kDescBytes;
-constexpr size_t kOffQuad = kOffPass + sizeof(Twiddle) * kPassTw;
+constexpr size_t kOffQuad = kDescBytes;
 constexpr size_t kOffLow8k = kOffQuad + sizeof(Twiddle) * kQuadTw;     // W_8192^i
 constexpr size_t kOffLow16k = kOffLow8k + sizeof(Twiddle) * kLowTw;    // W_16384^i
-constexpr size_t kOffXch = kOffLow16k + sizeof(Twiddle) * kLowTw;
-constexpr size_t kBytes = kOffXch + sizeof(float2) * kXch;
+constexpr size_t kBytes = kOffLow16k + sizeof(Twiddle) * kLowTw;
 static_assert(sizeof(PulseDev) <= kDescBytes, "descriptor slot too small");
-static_assert(kBytes == 350720, "the documented size of the static array");
+static_assert(kBytes == 18944, "the documented size of the static array");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kBytes];
 
@@ -94,18 +88,6 @@ bool current_context_id(unsigned long long* id) {
     return get_current && get_id && get_current(&ctx) == 0 && ctx && get_id(ctx, id) == 0;
 }
 
-__global__ void noalloc_pass_twiddles(Twiddle* out, int L) {
-    int lr = L / 16;
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 16 * lr) return;
-    int r = idx / lr, off = idx - r * lr;
-    double s, c;
-    sincospi(-2.0 * (double)(off * r) / (double)L, &s, &c);
-    float cf = (float)c, sf = (float)s;
-    double m2 = (double)cf * (double)cf + (double)sf * (double)sf;
-    out[idx] = Twiddle{cf, sf, (float)(1.0 / m2 - 1.0), 0.f};
-}
-
 // out[e] = W_n^e for e < count (FP32, d = 1/|w|^2 - 1 in FP64)
 __global__ void noalloc_twiddles(Twiddle* out, int n, int count) {
     int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -122,9 +104,6 @@ __global__ void noalloc_twiddles(Twiddle* out, int n, int count) {
 __global__ void noalloc_put_desc(PulseDev* slot, PulseDev d) { *slot = d; }
 
 int setup_tables(unsigned char* base, cudaStream_t st) {
-    Twiddle* tw = reinterpret_cast<Twiddle*>(base + kOffPass);
-    noalloc_pass_twiddles<<<(kM + 255) / 256, 256, 0, st>>>(tw, kM);
-    noalloc_pass_twiddles<<<1, 256, 0, st>>>(tw + kM, kM / 16);
     noalloc_twiddles<<<(int)((kQuadTw + 255) / 256), 256, 0, st>>>(
         reinterpret_cast<Twiddle*>(base + kOffQuad), kM, (int)kQuadTw);
     noalloc_twiddles<<<1, 64, 0, st>>>(reinterpret_cast<Twiddle*>(base + kOffLow8k), 8192, (int)kLowTw);
@@ -183,7 +162,6 @@ extern "C" int optifax_propagate_noalloc(const optifax_pulse* pulse, int32_t var
         }
     }
 
-    d.xch = reinterpret_cast<float2*>(base + kOffXch);
     PulseDev* slot = reinterpret_cast<PulseDev*>(base);
     noalloc_put_desc<<<1, 1, 0, st>>>(slot, d);
     if (cudaGetLastError() != cudaSuccess) return OPTIFAX_ERR_CUDA;
@@ -199,13 +177,11 @@ extern "C" int optifax_propagate_noalloc(const optifax_pulse* pulse, int32_t var
     cfg.max_attempts_mul = 64;
     cfg.grid_flags = nullptr;
     FftTables tabs;
-    tabs.tw1 = reinterpret_cast<const Twiddle*>(base + kOffPass);
-    tabs.tw2 = tabs.tw1 + kM;
     tabs.quad = reinterpret_cast<const Twiddle*>(base + kOffQuad);
     tabs.low = reinterpret_cast<const Twiddle*>(base + (N == 8192 ? kOffLow8k : kOffLow16k));
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)C, 1, 1);
-    lc.blockDim = dim3(kM / 16, 1, 1);
+    lc.blockDim = dim3((unsigned)ke->threads, 1, 1);
     lc.dynamicSmemBytes = ke->smem;
     lc.stream = st;
     cudaLaunchAttribute attr;

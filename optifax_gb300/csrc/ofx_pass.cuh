@@ -4,18 +4,17 @@
 // through the whole crystal in a single launch.  CTA rank c holds time points
 // [c M, (c+1) M) for the nonlinear sub-steps and, after the forward
 // transform, the spectral modes k = c + C k2 (k2 = 0..M-1).  Thread t owns
-// time points 16t .. 16t+15 of its CTA (held in registers across steps) and
-// spectral slots 16t .. 16t+15 (mode k2 = bitrev(slot)).
+// time points P t .. P t + P-1 of its CTA (held in registers across steps) and
+// spectral slots P t .. P t + P-1 (mode k2 = bitrev(slot)).
 //
 // Per step attempt (reference: OPO_CUDA_BATCH_XTAL.cu:432-506, Heun;
 // ode23/OPO_CUDA_ODE23.cu:446-538, RK23):
 //   RK stages: NL drive (A^2 e^{i phi} + 2|A|^2 e^{-i phi}, phi = w0 t - bdiffw0 z),
 //   shock-term central difference, stage combine -- all in registers, with
-//   the +-1 neighbours exchanged through shared memory (and distributed
-//   shared memory across the cluster).  Error classification (max-norm,
-//   percent) is an OR-reduction over the pulse (or over the batch when the
-//   reference's shared schedule is requested).  Accepted steps run the
-//   absorber, the forward FFT, the dispersion multiply, the inverse FFT and
+//   the +-1 neighbours exchanged by shuffles and shared memory.  Error
+//   classification (max-norm, percent) is an OR-reduction over the pulse (or over
+//   the batch when the reference's shared schedule is requested).  Accepted steps
+//   run the absorber, the forward FFT, the dispersion multiply, the inverse FFT and
 //   the 1/N scale without leaving the SM (cluster exchange for C > 1).
 //
 // Precision: FP32 field and FFT; phases exact in 64-bit fixed point (time
@@ -23,12 +22,17 @@
 // linear sub-step is applied as an increment, A_new = E + IFFT((D-1) FFT(E))/N,
 // with D - 1 = -2 sin^2(beta s/2) - i sin(beta s) evaluated without
 // cancellation, so transform rounding scales with |D - 1| rather than |E|; the
-// per-mode phase actually applied is tracked in fixed point and its FP32
-// rounding fed back into the next step (no drift of the accumulated phase);
-// the inverse FFT applies the exact reciprocal of each forward twiddle.
+// per-mode phase of every step is the exact fixed-point one of its position (no
+// drift of the accumulated phase); the inverse FFT applies the exact reciprocal of
+// each forward twiddle.
+//
+// What bounds it: instruction issue and latency on one SM per 4096 points; HBM is
+// idle by design.  Hence packed FP32 pairs, eight points per thread (four below 2048
+// points per CTA) for 16 warps where 2048 or more points share a CTA, every table in
+// shared memory, and square roots off the common path of the error class.
 #pragma once
 #include <cooperative_groups.h>
-#include "ofx_fft.cuh"
+#include "ofx_fftp.cuh"
 #include "../../include/optifax.h"
 
 namespace cg = cooperative_groups;
@@ -66,15 +70,12 @@ struct PulseDev {
     float* esd;
     int n_esd;
     float* smt;              // optional per-trip stepmods records (n_trips x S)
-    float2* xs;              // trip-output scratch (N) for the ESD sums when hist is not given
-    // cluster (C > 1) exchange scratch in global memory: 2 N complex
-    float2* xch;
+    float2* xs;              // cavities: the trip's crystal output (N), scratch of the cavity step
 };
 
+// Global tables from which every CTA fills its shared-memory ones:
+// W_M^x from the quarter period, W_N^e = W_M^{(64/C)(e >> 6)} W_N^{e & 63}
 struct FftTables {
-    const Twiddle* tw1;      // pass-1 outer twiddles [16][M/16]: W_M^{off r}
-    const Twiddle* tw2;      // pass-2 outer twiddles [16][M/256]: W_{M/16}^{off r}
-    // cluster exchange (copied to shared memory): W_N^e = W_M^{(64/C)(e >> 6)} W_N^{e & 63}
     const Twiddle* quad;     // W_M^y, y in [0, M/4)
     const Twiddle* low;      // W_N^i, i in [0, 64)
 };
@@ -96,21 +97,57 @@ constexpr int kHeunNee = 2;
 // ---------------------------------------------------------------------------
 // pointwise physics
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 nl_eval(float2 a, float2 cph, float2 z) {
-    float2 e = cmul(cph, z);
-    float ax2 = a.x * a.x, ay2 = a.y * a.y;
-    float2 a2 = make_float2(ax2 - ay2, 2.f * a.x * a.y);
-    float m2 = 2.f * (ax2 + ay2);
-    return make_float2(fmaf(a2.x, e.x, fmaf(-a2.y, e.y, m2 * e.x)),
-                       fmaf(a2.x, e.y, fmaf(a2.y, e.x, -m2 * e.y)));
+// Pairs of points (j, j + P/2) of one thread in structure-of-arrays form: `re` and
+// `im` hold the two points' parts, so that every operation of the stages is packed.
+struct Pair { float2 re, im; };
+
+__device__ __forceinline__ Pair pair_add(const Pair& a, const Pair& b) { return Pair{add2(a.re, b.re), add2(a.im, b.im)}; }
+__device__ __forceinline__ Pair pair_sub(const Pair& a, const Pair& b) { return Pair{sub2(a.re, b.re), sub2(a.im, b.im)}; }
+// a s + b
+__device__ __forceinline__ Pair pair_fma(const Pair& a, float s, const Pair& b) {
+    return Pair{cfma1(a.re, s, b.re), cfma1(a.im, s, b.im)};
+}
+
+// NL = a^2 e + 2 |a|^2 conj(e) with e = carrier z; with w = a e this is
+// a (3 Re w - i Im w), 14 packed operations for two points.
+__device__ __forceinline__ Pair nl_eval(const Pair& a, const Pair& cph, float2 z) {
+    const float2 zx = dup2(z.x), zy = dup2(z.y), nzx = dup2(-z.x), nzy = dup2(-z.y);
+    const float2 ex = fma2(cph.re, zx, mul2(cph.im, nzy));
+    const float2 ney = fma2(cph.re, nzy, mul2(cph.im, nzx));
+    const float2 nax = mul2(a.re, dup2(-1.f));
+    const float2 wx = fma2(a.im, ney, mul2(a.re, ex));
+    const float2 wy = fma2(nax, ney, mul2(a.im, ex));
+    const float2 w3 = mul2(wx, dup2(3.f));
+    return Pair{fma2(a.im, wy, mul2(a.re, w3)), fma2(nax, wy, mul2(a.im, w3))};
 }
 
 // K = -i hG (NL - i cs (NL[+1] - NL[-1]))
-__device__ __forceinline__ float2 k_eval(float2 nlm, float2 nl0, float2 nlp, float hg, float cs) {
-    float2 d = csub(nlp, nlm);
-    float inx = fmaf(cs, d.y, nl0.x);
-    float iny = fmaf(-cs, d.x, nl0.y);
-    return make_float2(hg * iny, -hg * inx);
+__device__ __forceinline__ Pair k_eval(const Pair& nlm, const Pair& nl0, const Pair& nlp, float hg, float cs) {
+    const Pair d = pair_sub(nlp, nlm);
+    return Pair{mul2(cfma1(d.re, -cs, nl0.im), dup2(hg)), mul2(cfma1(d.im, cs, nl0.re), dup2(-hg))};
+}
+// the same for one point
+__device__ __forceinline__ float2 nl_one(float2 a, float2 cph, float2 z) {
+    const Pair p = nl_eval(Pair{dup2(a.x), dup2(a.y)}, Pair{dup2(cph.x), dup2(cph.y)}, z);
+    return make_float2(p.re.x, p.im.x);
+}
+__device__ __forceinline__ float2 k_one(float2 nlm, float2 nl0, float2 nlp, float hg, float cs) {
+    const Pair p = k_eval(Pair{dup2(nlm.x), dup2(nlm.y)}, Pair{dup2(nl0.x), dup2(nl0.y)},
+                          Pair{dup2(nlp.x), dup2(nlp.y)}, hg, cs);
+    return make_float2(p.re.x, p.im.x);
+}
+
+// K of all H pairs of a thread from its drive and the neighbours' values L and R
+template <int H>
+__device__ __forceinline__ void k_all(const Pair (&nl)[H], float2 L, float2 R, float hg, float cs, Pair (&k)[H]) {
+#pragma unroll
+    for (int j = 0; j < H; ++j) {
+        const Pair m = j > 0 ? nl[j - 1]
+                             : Pair{make_float2(L.x, nl[H - 1].re.x), make_float2(L.y, nl[H - 1].im.x)};
+        const Pair p = j < H - 1 ? nl[j + 1]
+                                 : Pair{make_float2(nl[0].re.y, R.x), make_float2(nl[0].im.y, R.y)};
+        k[j] = k_eval(m, nl[j], p, hg, cs);
+    }
 }
 
 __device__ __forceinline__ int time_index(int i, int n, int mode) {
@@ -169,6 +206,74 @@ __device__ __forceinline__ int classify_nee(float scale, float2 d, float2 e, flo
     return bits;
 }
 
+__device__ __forceinline__ float sqrt_fast(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// OR of the error classes of a thread's points, from E and d (pct = scale |d| / (|E| + 1)).
+// The common case takes the largest q = |d|^2 / (|E| + 1)^2 by approximate square roots
+// and reciprocals (relative error below 1e-6) and decides where q is more than 1e-5
+// from both thresholds and below the upper one; everything else -- a point near or
+// above a threshold, a non-finite, huge or vanishing field, non-positive bounds --
+// goes through the exact classes, so every decision is theirs.  The exact class's IEEE
+// square root costs more than the rest of a point's stage arithmetic.
+struct Bounds {
+    float scale, maxE, minE, qhi, qlo0, qlo1;
+    __device__ Bounds(float sc, float hi, float lo) : scale(sc), maxE(hi), minE(lo) {
+        const float is2 = 1.f / (sc * sc), l = lo > 0.f ? lo * lo * is2 : -1.f;
+        qhi = hi > 0.f && lo > 0.f ? hi * hi * is2 * (1.f - 1e-5f) : -1.f;      // -1: always the exact classes
+        qlo0 = l * (1.f - 1e-5f);
+        qlo1 = l * (1.f + 1e-5f);
+    }
+};
+
+template <int H, bool NEE>
+__device__ __forceinline__ int classify_all(const Bounds& B, const Pair (&d)[H], const Pair (&e)[H]) {
+    float qmax = 0.f, emin = 3e38f;
+    float2 sum = dup2(0.f);
+#pragma unroll
+    for (int j = 0; j < H; ++j) {
+        const float2 e2 = fma2(e[j].re, e[j].re, mul2(e[j].im, e[j].im));
+        const float2 d2 = fma2(d[j].re, d[j].re, mul2(d[j].im, d[j].im));
+        const float2 den = add2(make_float2(sqrt_fast(e2.x), sqrt_fast(e2.y)), dup2(1.f));
+        const float2 r = make_float2(rcp_fast(den.x), rcp_fast(den.y));
+        const float2 q = mul2(mul2(d2, r), r);
+        qmax = fmaxf(qmax, fmaxf(q.x, q.y));
+        emin = fminf(emin, fminf(e2.x, e2.y));
+        sum = add2(sum, e2);
+    }
+    const float s = sum.x + sum.y;
+    const bool low = qmax < B.qlo0, high = qmax > B.qlo1;
+    if (s < 1e30f && qmax < B.qhi && (low || (high && (NEE || emin > 1e-30f)))) return high ? 2 : 0;
+    int bits = 0;
+#pragma unroll
+    for (int j = 0; j < H; ++j) {
+        const float2 d0 = make_float2(d[j].re.x, d[j].im.x), d1 = make_float2(d[j].re.y, d[j].im.y);
+        const float2 e0 = make_float2(e[j].re.x, e[j].im.x), e1 = make_float2(e[j].re.y, e[j].im.y);
+        bits |= NEE ? classify_nee(B.scale, d0, e0, B.maxE, B.minE) : classify(B.scale, d0, e0, B.maxE, B.minE);
+        bits |= NEE ? classify_nee(B.scale, d1, e1, B.maxE, B.minE) : classify(B.scale, d1, e1, B.maxE, B.minE);
+    }
+    return bits;
+}
+
+// Phase rate beta (radians per step) as a 64-bit fixed-point fraction of a turn
+__device__ __forceinline__ uint64_t phase_rate(float beta) {
+    constexpr double kTwoPi = 6.283185307179586476925286766559, kTwoPiLo = 2.4492935982947064e-16;
+    constexpr double kTurnScale = 18446744073709551616.0 / kTwoPi;   // 2^64 / (2 pi)
+    const double b = (double)beta, n = rint(b * (1.0 / kTwoPi));
+    double x = fma(-n, kTwoPiLo, fma(-n, kTwoPi, b)) * kTurnScale;
+    if (x >= 9.2233720368547758e18) x -= 1.8446744073709552e19;
+    if (x < -9.2233720368547758e18) x += 1.8446744073709552e19;
+    return (uint64_t)(long long)llrint(x);
+}
+
 // D - 1 = alpha^s exp(-i th) - 1 for the phase increment d32 (units of 2^-32
 // turn; converted to FP32, *dapplied receives the integer actually used) and
 // log2 alpha l2 (-inf: alpha = 0).
@@ -199,42 +304,60 @@ __device__ __forceinline__ float2 dispersion_dm1(int d32, float l2, int s, int* 
     return dm1;
 }
 
-// 16-byte stores of consecutive complex pairs to global memory (L2 only)
-__device__ __forceinline__ void store_pair(float2* base, int j, float2 v, float2& prev) {
-    if (j & 1) __stcg(reinterpret_cast<float4*>(base) + (j >> 1), make_float4(prev.x, prev.y, v.x, v.y));
-    else prev = v;
-}
-
 __device__ __forceinline__ float2 zphase(uint64_t tau_z4, float pos) {
     uint64_t p4 = (uint64_t)(uint32_t)(4.0f * pos);
     return turn_to_unit((uint64_t)0 - tau_z4 * p4);
 }
 
+// The z-phasors of up to three positions, one lane evaluating each
+__device__ __forceinline__ void zphases(uint64_t tau_z4, int t, float p0, float p1, float p2, float2& z0, float2& z1,
+                                        float2& z2) {
+    const int l = t & 31;
+    const float2 z = zphase(tau_z4, l == 0 ? p0 : (l == 1 ? p1 : p2));
+    z0 = make_float2(__shfl_sync(0xffffffffu, z.x, 0), __shfl_sync(0xffffffffu, z.y, 0));
+    z1 = make_float2(__shfl_sync(0xffffffffu, z.x, 1), __shfl_sync(0xffffffffu, z.y, 1));
+    z2 = make_float2(__shfl_sync(0xffffffffu, z.x, 2), __shfl_sync(0xffffffffu, z.y, 2));
+}
+
 // ---------------------------------------------------------------------------
 // shared-memory layout
 // ---------------------------------------------------------------------------
+// Points per thread
+template <int M>
+constexpr int kPoints = (M >= 2048) ? 8 : 4;
+
+// Cluster exchange: CTA c takes the n2 columns [c M/C, (c+1) M/C) of the C blocks, PER
+// consecutive columns to each of XT threads.
+template <int M, int C>
+struct Xch {
+    static constexpr int T = M / kPoints<M>;
+    static constexpr int COLS = M / C;
+    static constexpr int XT = COLS < T ? COLS : T;
+    static constexpr int PER = COLS / XT;
+};
+
 template <int M, int METHOD, int C>
 struct Smem {
-    static constexpr int T = M / 16;
-    static constexpr int PADM = M + M / 16;
-    static constexpr int NBUF = (METHOD == OPTIFAX_RK23) ? 3 : 2;   // E, X (+K1 for RK23)
-    static constexpr size_t off_buf = 0;
-    static constexpr size_t off_tau = off_buf + sizeof(float2) * PADM * NBUF;
-    static constexpr size_t off_l2a = off_tau + sizeof(uint64_t) * M;
-    static constexpr size_t off_papp = off_l2a + sizeof(float) * M;
-    static constexpr size_t off_abc = off_papp + sizeof(uint32_t) * M;
-    // Heun: per-mode D - 1 and its fixed-point phase increment for the cached stepmod
-    static constexpr int NCACHE = (METHOD != OPTIFAX_RK23) ? M : 0;
-    static constexpr size_t off_dmc = off_abc + sizeof(float) * M;
-    static constexpr size_t off_dfc = off_dmc + sizeof(float2) * NCACHE;
-    static constexpr size_t off_edge = off_dfc + sizeof(int) * NCACHE;
-    static constexpr size_t off_red = off_edge + sizeof(float2) * 4 * T;
-    static constexpr size_t off_dred = off_red + 256;               // FP64 reduction slots
-    // exchange twiddle tables (16-byte entries, clusters only): quarter-period W_M,
-    // W_N^i for i < 64
-    static constexpr size_t off_quad = (off_dred + sizeof(double) * (8 * 4 + 2 * 16 * 4 + 4) + 15) & ~size_t(15);
-    static constexpr size_t off_low = off_quad + (C > 1 ? sizeof(Twiddle) * (M / 4) : 0);
-    static constexpr size_t bytes = off_low + (C > 1 ? sizeof(Twiddle) * 64 : 0);
+    static constexpr int P = kPoints<M>;
+    static constexpr int T = M / P, NW = T / 32;
+    using F = FftPlan<M, P>;
+    using XC = Xch<M, C>;
+    static constexpr size_t off_x = 0;                                               // stage output, FFT buffer
+    static constexpr size_t off_g = off_x + sizeof(float2) * M;                      // clusters: gathered columns
+    static constexpr size_t off_dm = off_g + (C > 1 ? sizeof(float2) * M : 0);       // per-mode D - 1
+    static constexpr size_t off_tlo = off_dm + sizeof(float2) * M;                   // phase rates, low words
+    static constexpr size_t off_abc = off_tlo + sizeof(uint32_t) * M;
+    static constexpr size_t off_tw = off_abc + sizeof(float) * M;
+    static constexpr size_t off_td = (off_tw + sizeof(float2) * F::TW + 15) & ~size_t(15);
+    // exchange twiddles W_N^{n2 k1} and their d: [u (C-1) + r - 1][XT]
+    static constexpr size_t off_xtw = (off_td + sizeof(float) * F::TD + 15) & ~size_t(15);
+    static constexpr size_t off_xtd = off_xtw + (C > 1 ? sizeof(float2) * XC::PER * (C - 1) * XC::XT : 0);
+    static constexpr size_t off_edge = (off_xtd + (C > 1 ? sizeof(float) * XC::PER * (C - 1) * XC::XT : 0) + 15) & ~size_t(15);
+    static constexpr size_t off_halo = off_edge + sizeof(float2) * 4 * NW;           // [parity][first, last][warp]
+    static constexpr size_t off_red = off_halo + sizeof(float2) * 8;                 // E and increment of 4 halo points
+    static constexpr size_t off_dred = off_red + sizeof(int) * (2 * NW + 2 * 16 + 4);
+    static constexpr size_t bytes = ((off_dred + 15) & ~size_t(15)) + sizeof(double) * (NW * 4 + 2 * 16 * 4);
+    static_assert(bytes <= 232448 - 512, "shared memory of one CTA");
 };
 
 // ---------------------------------------------------------------------------
@@ -263,35 +386,41 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
     return r;
 }
-__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
-    return v;
-}
 __device__ __forceinline__ void st_cluster_f2(uint32_t addr, float2 v) {
     asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
 }
+__device__ __forceinline__ void st_cluster_f4(uint32_t addr, float2 v, float2 w) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(w.x), "f"(w.y)
+                 : "memory");
+}
+__device__ __forceinline__ void st_cluster_i32(uint32_t addr, int v) {
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 
-// Publish this thread's first/last stencil values and fetch the neighbours'.
-template <int M, int C>
-__device__ __forceinline__ void exchange_edges(float2* edge, int& par, int t, int c, float2 first,
-                                               float2 last, float2& left, float2& right) {
-    constexpr int T = M / 16;
-    float2* e = edge + par * 2 * T;
-    e[2 * t] = first;
-    e[2 * t + 1] = last;
-    csync<C>();
-    if (t > 0) left = e[2 * t - 1];
-    else left = remote<C>(e, (c + C - 1) % C)[2 * T - 1];
-    if (t < T - 1) right = e[2 * t + 2];
-    else right = remote<C>(e, (c + 1) % C)[0];
+// The neighbours' adjacent drive values: shuffles inside a warp, one shared-memory slot
+// per warp edge.  REMOTE: the CTA's own ends come from the neighbouring CTAs (clusters),
+// else they wrap around (one CTA) or are replaced by the caller.
+template <int M, int C, bool REMOTE>
+__device__ __forceinline__ void exchange_edges(float2* edge, int& par, int t, int c, float2 first, float2 last,
+                                               float2& left, float2& right) {
+    constexpr int NW = M / kPoints<M> / 32;
+    const int w = t >> 5, lane = t & 31;
+    float2* e = edge + par * 2 * NW;
+    if (lane == 0) e[w] = first;
+    if (lane == 31) e[NW + w] = last;
+    left = make_float2(__shfl_up_sync(0xffffffffu, last.x, 1), __shfl_up_sync(0xffffffffu, last.y, 1));
+    right = make_float2(__shfl_down_sync(0xffffffffu, first.x, 1), __shfl_down_sync(0xffffffffu, first.y, 1));
+    if constexpr (REMOTE && C > 1) csync<C>();
+    else __syncthreads();
+    if (lane == 0) left = (w > 0) ? e[NW + w - 1] : ((REMOTE ? remote<C>(e, (c + C - 1) % C) : e)[2 * NW - 1]);
+    if (lane == 31) right = (w < NW - 1) ? e[w + 1] : ((REMOTE ? remote<C>(e, (c + 1) % C) : e)[0]);
     par ^= 1;
 }
 
-// N-point twiddle W_N^e, 0 <= e < N = C M, from the two shared-memory tables:
-// W_M^{(64/C)(e >> 6)} (quarter table, exact) times W_N^{e & 63}.  The product is
-// rounded once; the inverse multiplies by its exact reciprocal conj(w)(1 + d),
-// d = 1/|w|^2 - 1 formed from w itself, so forward + inverse carry no gain.
+// N-point twiddle W_N^e, 0 <= e < N = C M, from the two tables: W_M^{(64/C)(e >> 6)}
+// (quarter table, exact) times W_N^{e & 63}.  The product is rounded once; the inverse
+// multiplies by its exact reciprocal conj(w)(1 + d), d = 1/|w|^2 - 1 formed from w
+// itself, so forward + inverse carry no gain.
 template <int M, int C>
 __device__ __forceinline__ float2 twn_val(const Twiddle* quad, const Twiddle* low, int e) {
     static_assert(64 % C == 0, "cluster size must divide 64");
@@ -299,102 +428,165 @@ __device__ __forceinline__ float2 twn_val(const Twiddle* quad, const Twiddle* lo
     const Twiddle b = low[e & 63];
     return cmul(make_float2(a.c, a.s), make_float2(b.c, b.s));
 }
+
+// Four-step split of the N = C M transform across a cluster, all of it through
+// distributed shared memory.  Every value is pushed into the shared memory of the CTA
+// that uses it next, so that each of the four steps of an accepted step is one wave of
+// remote stores and one cluster barrier, and no transfer waits on L2:
+//   push_columns   own time points -> the owners of their n2 columns (buffer g)
+//   exchange_fwd   C-point DFTs of the own columns, twiddle -> the blocks' owners (x)
+//   (local transforms, dispersion; the last inverse pass pushes into the columns' g)
+//   exchange_inv   inverse twiddle and C-point DFTs, 1/N -> the blocks' owners (x)
+// Ordering comes from the cluster barriers between the steps: a buffer is written only
+// after the barrier that follows its last read.
 template <int M, int C>
-__device__ __forceinline__ float2 twn_fwd(float2 v, const Twiddle* quad, const Twiddle* low, int e) {
-    return cmul(v, twn_val<M, C>(quad, low, e));
-}
-template <int M, int C>
-__device__ __forceinline__ float2 twn_inv(float2 v, const Twiddle* quad, const Twiddle* low, int e) {
-    const float2 w = twn_val<M, C>(quad, low, e);
-    const float2 t = cmulc(v, w);
-    const float d = inv_norm2_m1(w);
-    return make_float2(fmaf(t.x, d, t.x), fmaf(t.y, d, t.y));
+__device__ __forceinline__ void push_columns(uint32_t g, const float2 (&v)[kPoints<M>], int t, int c) {
+    using XC = Xch<M, C>;
+    constexpr int P = kPoints<M>;
+    static_assert(XC::COLS % P == 0, "a thread's points belong to one column owner");
+    const uint32_t dst = cluster_addr(g, (P * t) / XC::COLS);
+    const int s0 = swz(c * XC::COLS + (P * t) % XC::COLS);
+#pragma unroll
+    for (int j = 0; j < P; j += 2) st_cluster_f4(dst + 8 * (s0 ^ j), v[j], v[j + 1]);
 }
 
-// Exchange results go straight into their owners' shared memory for clusters of
-// up to 8 CTAs; 16-CTA clusters keep them in global memory (L2), where their
-// wider fan-out measured faster (and the kernel stays free of spills).
-template <int C>
-constexpr bool kPushExchange = (C <= 8);
-// The forward gather reads the C blocks' stage outputs straight from their CTAs'
-// shared memory (ld.shared::cluster) for clusters of up to 4; larger clusters
-// gather them from global memory (measured: 4 CTAs 13.9 -> 13.6 us per attempt,
-// 8 CTAs 14.9 -> 15.0).
-template <int C>
-constexpr bool kPullGather = (C <= 4);
+// Store `v` (PER consecutive columns n2 of block k) into the FFT buffer of CTA k
+template <int PER>
+__device__ __forceinline__ void push_block(uint32_t x, int k, int n2, const float2 (&v)[PER]) {
+    const uint32_t dst = cluster_addr(x, k);
+    const int s0 = swz(n2);
+    if constexpr (PER == 1) {
+        st_cluster_f2(dst + 8 * s0, v[0]);
+    } else {
+#pragma unroll
+        for (int u = 0; u < PER; u += 2) st_cluster_f4(dst + 8 * (s0 ^ u), v[u], v[u + 1]);
+    }
+}
 
-// Four-step split of the N = C M transform: forward step 1 (C-point DFTs over
-// CTAs, twiddle W_N^{n2 k1}).  Each CTA gathers its n2 slice of the C blocks --
-// from the blocks' stage outputs in their CTAs' shared memory (`bufe`, clusters
-// of up to 4) or from global memory (`xx`, all loads in flight) -- computes the
-// C-point DFTs and stores the results in their owners' shared memory (`buf`, the
-// owner's FFT buffer, at phys(n2)) or, for 16-CTA clusters, in their blocks of
-// `yy` (global).  Ordering comes from the cluster barriers around the calls
-// (release/acquire at cluster scope covers global and distributed shared memory):
-// the stage outputs are complete at the error-flag barrier before the call, and no
-// CTA reads its FFT buffer again until the barrier after it.  Global accesses
-// bypass L1.
 template <int M, int C>
-__device__ __forceinline__ void exchange_forward_g(const float2* __restrict__ xx, const float2* bufe,
-                                                   float2* buf, float2* yy,
-                                                   const Twiddle* quad, const Twiddle* low, int t, int c) {
-    if constexpr (C > 1) {
-        constexpr int T = M / 16, PER = 16 / C, LOGC = (C == 2) ? 1 : (C == 4) ? 2 : (C == 8) ? 3 : 4;
-        float2 v[PER][C];
+__device__ __forceinline__ void load_columns(const float2* g, int t, float2 (&v)[Xch<M, C>::PER][C]) {
+    using XC = Xch<M, C>;
 #pragma unroll
-        for (int u = 0; u < PER; ++u)          // every load in flight before any use
+    for (int n1 = 0; n1 < C; ++n1) {
+        const int s0 = swz(n1 * XC::COLS + t * XC::PER);
 #pragma unroll
-            for (int n1 = 0; n1 < C; ++n1) {
-                if constexpr (kPullGather<C>)
-                    v[u][n1] = ld_cluster_f2(cluster_addr(smem_u32(bufe + phys(c * (M / C) + t + T * u)), n1));
-                else v[u][n1] = __ldcg(xx + n1 * M + c * (M / C) + t + T * u);
-            }
+        for (int u = 0; u < XC::PER; ++u) v[u][n1] = g[s0 ^ u];
+    }
+}
+
+template <int M, int C>
+__device__ __forceinline__ void exchange_fwd(const float2* g, uint32_t x, const float2* xtw, int t, int c) {
+    using XC = Xch<M, C>;
+    if (t >= XC::XT) return;
+    float2 v[XC::PER][C];
+    load_columns<M, C>(g, t, v);
+    const int n2 = c * XC::COLS + t * XC::PER;
 #pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            int n2 = c * (M / C) + t + T * u;
-            dft_dif<C>(v[u]);
+    for (int u = 0; u < XC::PER; ++u) {
+        dftp<C>(v[u]);
 #pragma unroll
-            for (int r = 0; r < C; ++r) {
-                int k1 = bitrev(r, LOGC);
-                const float2 y = k1 == 0 ? v[u][r] : twn_fwd<M, C>(v[u][r], quad, low, n2 * k1);
-                if constexpr (kPullGather<C>) st_cluster_f2(cluster_addr(smem_u32(buf + phys(n2)), k1), y);
-                else if constexpr (kPushExchange<C>) remote<C>(buf, k1)[phys(n2)] = y;
-                else __stcg(yy + k1 * M + n2, y);
+        for (int r = 1; r < C; ++r) v[u][r] = cmul(v[u][r], xtw[(u * (C - 1) + r - 1) * XC::XT + t]);
+    }
+#pragma unroll
+    for (int r = 0; r < C; ++r) {
+        float2 o[XC::PER];
+#pragma unroll
+        for (int u = 0; u < XC::PER; ++u) o[u] = v[u][r];
+        push_block<XC::PER>(x, brev4(r, ilog2(C)), n2, o);
+    }
+}
+
+// g holds the inverse-transformed blocks' columns at [k1 COLS + column].  Block-edge
+// increments also go to the neighbouring CTAs' halo slots: halo[0..1] hold the points
+// -2, -1 and halo[2..3] the points M, M + 1 of the owner.
+template <int M, int C, bool HALO>
+__device__ __forceinline__ void exchange_inv(const float2* g, uint32_t x, uint32_t halo, const float2* xtw,
+                                             const float* xtd, int t, int c, float invN) {
+    using XC = Xch<M, C>;
+    if (t >= XC::XT) return;
+    float2 v[XC::PER][C];
+    load_columns<M, C>(g, t, v);
+    const int n2 = c * XC::COLS + t * XC::PER;
+#pragma unroll
+    for (int u = 0; u < XC::PER; ++u) {
+        float2 w[C];
+        w[0] = v[u][0];
+#pragma unroll
+        for (int r = 1; r < C; ++r) {                   // register r of the inverse DFT holds k1 = bitrev(r)
+            const int i = (u * (C - 1) + r - 1) * XC::XT + t;
+            w[r] = mul_recip(v[u][brev4(r, ilog2(C))], xtw[i], xtd[i]);
+        }
+        dftp_inv<C>(w);
+#pragma unroll
+        for (int n1 = 0; n1 < C; ++n1) v[u][n1] = mul2(w[n1], dup2(invN));
+    }
+#pragma unroll
+    for (int n1 = 0; n1 < C; ++n1) {
+        float2 o[XC::PER];
+#pragma unroll
+        for (int u = 0; u < XC::PER; ++u) o[u] = v[u][n1];
+        push_block<XC::PER>(x, n1, n2, o);
+        if constexpr (HALO) {
+#pragma unroll
+            for (int u = 0; u < XC::PER; ++u) {
+                if (n2 + u < 2) st_cluster_f2(cluster_addr(halo, (n1 + C - 1) % C) + 8 * (2 + n2 + u), o[u]);
+                if (n2 + u >= M - 2) st_cluster_f2(cluster_addr(halo, (n1 + 1) % C) + 8 * (n2 + u - (M - 2)), o[u]);
             }
         }
     }
 }
 
-// Inverse step: gather the n2 slice of the C inverse-transformed blocks from
-// global memory, undo the twiddles, C-point inverse DFTs, scale by 1/N and store
-// each result in its owner's shared memory (`buf` at phys(n2)) or, for 16-CTA
-// clusters, in its block of `xx` (global).
+// The last inverse pass's outputs (points t + q M/P of this CTA's block) into the g
+// buffers of their columns' owners.
 template <int M, int C>
-__device__ __forceinline__ void exchange_inverse_g(const float2* __restrict__ yy, float2* buf, float2* xx,
-                                                   const Twiddle* quad, const Twiddle* low, int t, int c,
-                                                   float invN) {
-    if constexpr (C > 1) {
-        constexpr int T = M / 16, PER = 16 / C, LOGC = (C == 2) ? 1 : (C == 4) ? 2 : (C == 8) ? 3 : 4;
-        float2 v[PER][C];
+__device__ __forceinline__ void push_inverse(uint32_t g, const float2 (&v)[kPoints<M>], int t, int c) {
+    using XC = Xch<M, C>;
+    constexpr int P = kPoints<M>;
 #pragma unroll
-        for (int u = 0; u < PER; ++u)          // every load in flight before any use
-#pragma unroll
-            for (int r = 0; r < C; ++r) v[u][r] = __ldcg(yy + bitrev(r, LOGC) * M + c * (M / C) + t + T * u);
-#pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            int n2 = c * (M / C) + t + T * u;
-#pragma unroll
-            for (int r = 1; r < C; ++r) v[u][r] = twn_inv<M, C>(v[u][r], quad, low, n2 * bitrev(r, LOGC));
-            dft_dit_inv<C>(v[u]);
-#pragma unroll
-            for (int n1 = 0; n1 < C; ++n1) {
-                if constexpr (kPullGather<C>)
-                    st_cluster_f2(cluster_addr(smem_u32(buf + phys(n2)), n1), cscale(v[u][n1], invN));
-                else if constexpr (kPushExchange<C>) remote<C>(buf, n1)[phys(n2)] = cscale(v[u][n1], invN);
-                else __stcg(xx + n1 * M + n2, cscale(v[u][n1], invN));
-            }
-        }
+    for (int q = 0; q < P; ++q) {
+        const int m = t + q * (M / P);
+        st_cluster_f2(cluster_addr(g, m / XC::COLS) + 8 * swz(c * XC::COLS + m % XC::COLS), v[q]);
     }
+}
+
+// OR of the error flags over the pulse: one slot per warp, then (clusters) one per CTA.
+// Double buffered by attempt.  The barrier inside also publishes what the threads
+// stored before it (stage output, pushed columns).
+template <int M, int C>
+__device__ __forceinline__ int combine_flags(int bits, int* red, int attempt, int t, int c, const KernelCfg& cfg) {
+    constexpr int NW = M / kPoints<M> / 32;
+    const int par = attempt & 1;
+    int* wf = red + par * NW;
+    const int w = __reduce_or_sync(0xffffffffu, bits);
+    if ((t & 31) == 0) wf[t >> 5] = w;
+    __syncthreads();
+    int f = 0;
+    if constexpr (NW >= 4) {
+#pragma unroll
+        for (int i = 0; i < NW; i += 4) {
+            const int4 q = *reinterpret_cast<const int4*>(wf + i);
+            f |= q.x | q.y | q.z | q.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < NW; ++i) f |= wf[i];
+    }
+    if constexpr (C > 1) {
+        int* cl = red + 2 * NW + par * 16;
+        if (t < C) st_cluster_i32(cluster_addr(smem_u32(cl + c), t), f);
+        cg::this_cluster().sync();
+        f = 0;
+#pragma unroll
+        for (int r = 0; r < C; ++r) f |= cl[r];
+    }
+    if (cfg.shared_sched) {
+        const int gslot = attempt % 3;
+        if (t == 0 && c == 0 && f) atomicOr(&cfg.grid_flags[gslot], f);
+        cg::this_grid().sync();
+        f = *((volatile int*)&cfg.grid_flags[gslot]);
+        if (blockIdx.x == 0 && t == 0) cfg.grid_flags[(attempt + 2) % 3] = 0;
+    }
+    return f;
 }
 
 // OR of per-thread flag bits over the CTA, the cluster and (shared schedule)
@@ -437,7 +629,7 @@ __device__ __forceinline__ int reduce_flags(int bits, int* red, int attempt, int
 template <int M, int C>
 __device__ __forceinline__ void reduce_tallies(const float (&part)[4], double (&out)[4], double* dred,
                                                int t, int c, int parity) {
-    constexpr int T = M / 16, NW = T / 32;
+    constexpr int T = M / kPoints<M>, NW = T / 32;
     double v[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -450,7 +642,7 @@ __device__ __forceinline__ void reduce_tallies(const float (&part)[4], double (&
         for (int i = 0; i < 4; ++i) dred[(t >> 5) * 4 + i] = v[i];
     }
     __syncthreads();
-    double* cl = dred + 8 * 4 + parity * 16 * 4;
+    double* cl = dred + NW * 4 + parity * 16 * 4;
     if (t == 0) {
         double s[4] = {0, 0, 0, 0};
         for (int w = 0; w < NW; ++w)
@@ -480,29 +672,33 @@ __device__ __forceinline__ void reduce_tallies(const float (&part)[4], double (&
 // delay and the pump injection are all per-mode products folded into fb and
 // pump by the host.  Per-trip energy tallies sum tally_w |X|^2 in FP64.
 template <int M, int C, int METHOD>
-__global__ void __launch_bounds__(M / 16, 1)
+__global__ void __launch_bounds__(M / kPoints<M>, 1)
 pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) {
-    constexpr int T = M / 16;
+    constexpr int P = kPoints<M>, H = P / 2;
+    constexpr int T = M / P;
     constexpr int N = M * C;
-    constexpr int LOG2M = FftShape<M>::LOG2M;
+    constexpr int LOG2M = ilog2(M);
+    constexpr bool nee = (METHOD == kHeunNee);   // NEE_CPU.m: k is 1-based, no chunk clamp
+    constexpr bool heun = (METHOD != OPTIFAX_RK23);
+    // clusters, Heun: the two points beyond each end of the CTA's block are carried
+    // along by the end threads, so the stages need no exchange between CTAs
+    constexpr bool HALO = heun && C > 1;
     using SM = Smem<M, METHOD, C>;
     extern __shared__ __align__(16) unsigned char smem[];
-    float2* bufE = reinterpret_cast<float2*>(smem + SM::off_buf);
-    float2* bufX = bufE + SM::PADM;
-    float2* bufK = bufX + SM::PADM;   // RK23 only: FSAL K1 (own points)
-    uint64_t* tau_s = reinterpret_cast<uint64_t*>(smem + SM::off_tau);
-    float* l2a_s = reinterpret_cast<float*>(smem + SM::off_l2a);
-    uint32_t* papp_s = reinterpret_cast<uint32_t*>(smem + SM::off_papp);
+    float2* bufX = reinterpret_cast<float2*>(smem + SM::off_x);
+    float2* bufG = reinterpret_cast<float2*>(smem + SM::off_g);
+    float2* dm_s = reinterpret_cast<float2*>(smem + SM::off_dm);
+    uint32_t* tlo_s = reinterpret_cast<uint32_t*>(smem + SM::off_tlo);
     float* abc_s = reinterpret_cast<float*>(smem + SM::off_abc);
-    float2* dmc_s = reinterpret_cast<float2*>(smem + SM::off_dmc);
-    int* dfc_s = reinterpret_cast<int*>(smem + SM::off_dfc);
-    const Twiddle* __restrict__ tw1 = tabs.tw1;
-    const Twiddle* __restrict__ tw2 = tabs.tw2;
-    Twiddle* quad_s = reinterpret_cast<Twiddle*>(smem + SM::off_quad);
-    Twiddle* low_s = reinterpret_cast<Twiddle*>(smem + SM::off_low);
+    float2* tw_s = reinterpret_cast<float2*>(smem + SM::off_tw);
+    float* td_s = reinterpret_cast<float*>(smem + SM::off_td);
+    float2* xtw_s = reinterpret_cast<float2*>(smem + SM::off_xtw);
+    float* xtd_s = reinterpret_cast<float*>(smem + SM::off_xtd);
     float2* edge = reinterpret_cast<float2*>(smem + SM::off_edge);
+    float2* halo_e = reinterpret_cast<float2*>(smem + SM::off_halo);      // E of points -2, -1, M, M + 1
+    float2* halo_d = halo_e + 4;                                          // their increments
     int* red = reinterpret_cast<int*>(smem + SM::off_red);
-    double* dred = reinterpret_cast<double*>(smem + SM::off_dred);
+    double* dred = reinterpret_cast<double*>(smem + ((SM::off_dred + 15) & ~size_t(15)));
 
     const int t = threadIdx.x;
     const int c = (C > 1) ? (int)cg::this_cluster().block_rank() : 0;
@@ -513,80 +709,117 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     __shared__ PulseDev sP;
     if (t == 0) sP = pulses[p];
     __syncthreads();
-    const PulseDev& P = sP;
+    const PulseDev& P_ = sP;
 
     // ---- prologue -------------------------------------------------------
-    for (int i = t; i < 64; i += T) red[i] = 0;
+    fft_tables<M, P>(tw_s, td_s, tabs.quad, t);
     if constexpr (C > 1) {
-        for (int i = t; i < M / 4; i += T) quad_s[i] = tabs.quad[i];
-        for (int i = t; i < 64; i += T) low_s[i] = tabs.low[i];
+        using XC = Xch<M, C>;
+        if (t < XC::XT) {
+#pragma unroll 1
+            for (int u = 0; u < XC::PER; ++u)
+#pragma unroll 1
+                for (int r = 1; r < C; ++r) {
+                    const float2 w = twn_val<M, C>(tabs.quad, tabs.low,
+                                                   (c * XC::COLS + t * XC::PER + u) * bitrev(r, ilog2(C)));
+                    const int i = (u * (C - 1) + r - 1) * XC::XT + t;
+                    xtw_s[i] = w;
+                    xtd_s[i] = inv_norm2_m1(w);
+                }
+        }
     }
-    float2 cph[16], a[16];
+    // per-thread tables as vectors of four (or two) values: [j / 4][t][j % 4]
+    auto at4 = [&](int j) { return ((j >> 2) * T + t) * 4 + (j & 3); };
+    auto at2 = [&](int j) { return ((j >> 1) * T + t) * 2 + (j & 1); };
+    auto carrier = [&](int i) { return turn_to_unit(P_.tau_theta * (uint64_t)time_index(i, N, cfg.time_mode)); };
+    Pair a[H], cph[H];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        int i = c * M + 16 * t + j;
-        uint64_t jt = (uint64_t)time_index(i, N, cfg.time_mode);
-        cph[j] = turn_to_unit(P.tau_theta * jt);
-        a[j] = P.E_in[i];
-        abc_s[j * T + t] = abc_factor(i, N, cfg.abc_mode);
+    for (int j = 0; j < H; ++j) {
+        const int i = c * M + P * t + j;
+        const float2 c0 = carrier(i), c1 = carrier(i + H), e0 = P_.E_in[i], e1 = P_.E_in[i + H];
+        cph[j] = Pair{make_float2(c0.x, c1.x), make_float2(c0.y, c1.y)};
+        a[j] = Pair{make_float2(e0.x, e1.x), make_float2(e0.y, e1.y)};
+        abc_s[at4(j)] = abc_factor(i, N, cfg.abc_mode);
+        abc_s[at4(j + H)] = abc_factor(i + H, N, cfg.abc_mode);
+    }
+    // end threads: the adjacent (h1) and the outer (h2) point beyond the block's end
+    const bool lend = HALO && t == 0, rend = HALO && t == T - 1;
+    float2 h1 = make_float2(0.f, 0.f), h2 = h1, hc1 = h1, hc2 = h1;
+    if (lend || rend) {
+        const int i1 = lend ? (c * M + N - 1) % N : (c * M + M) % N;
+        const int i2 = lend ? (c * M + N - 2) % N : (c * M + M + 1) % N;
+        h1 = P_.E_in[i1]; h2 = P_.E_in[i2];
+        hc1 = carrier(i1); hc2 = carrier(i2);
     }
 #pragma unroll 1
-    for (int j = 0; j < 16; ++j) {
-        int slot = 16 * t + j;
-        int k = c + C * bitrev(slot, LOG2M);
-        double b = (double)P.beta[k];
-        constexpr double kTwoPi = 6.283185307179586476925286766559;
-        constexpr double kTurnScale = 18446744073709551616.0 / kTwoPi;   // 2^64 / (2 pi)
-        double r = b - kTwoPi * rint(b / kTwoPi);
-        double x = r * kTurnScale;
-        if (x >= 9.2233720368547758e18) x -= 1.8446744073709552e19;
-        if (x < -9.2233720368547758e18) x += 1.8446744073709552e19;
-        tau_s[j * T + t] = (uint64_t)(long long)llrint(x);
-        l2a_s[j * T + t] = log2f(P.alpha[k]);
+    for (int j = 0; j < P; ++j) {
+        const int k = c + C * bitrev(P * t + j, LOG2M);
+        const uint64_t tau = phase_rate(P_.beta[k]);
+        tlo_s[at4(j)] = (uint32_t)tau;
     }
     if constexpr (C > 1) cg::this_cluster().sync(); else __syncthreads();
 
-    const float* G = P.G;
-    const float h = P.h, sel = P.sel, cs = P.c_shock, Sf = (float)P.S;
-    const float maxE = P.max_err, minE = P.min_err;
+    const float* G = P_.G;
+    const float h = P_.h, sel = P_.sel, cs = P_.c_shock, Sf = (float)P_.S;
+    const Bounds bounds(heun ? 50.f : 200.f, P_.max_err, P_.min_err);
+    // what the caller asked for beyond the field, as one register (tested per attempt)
+    constexpr int kForced = 1, kTrace = 2, kSteps = 4, kAp = 8;
+    const int opts = (P_.forced && P_.n_forced > 0 ? kForced : 0) | (P_.trace ? kTrace : 0) |
+                     (!nee && (P_.stepmods || P_.smt) ? kSteps : 0) | (P_.Ap ? kAp : 0);
     const float invN = 1.0f / (float)N;
     const int guard = cfg.guard;
-    const long long max_attempts = (long long)cfg.max_attempts_mul * (long long)(P.S + 16) + 64;
-    const int nchunks = P.nchunks;
+    const long long max_attempts = (long long)cfg.max_attempts_mul * (long long)(P_.S + 16) + 64;
+    const int nchunks = P_.nchunks;
     const float pass_end = (float)nchunks * sel;
-    const bool opo = P.fb != nullptr;
-    const int n_trips = P.n_trips > 0 ? P.n_trips : 1;
+    const bool opo = P_.fb != nullptr;
+    const int n_trips = P_.n_trips > 0 ? P_.n_trips : 1;
     const bool rec = (c == 0 && t == 0);
+    const uint32_t x_addr = smem_u32(bufX), g_addr = smem_u32(bufG);
 
-    constexpr bool nee = (METHOD == kHeunNee);   // NEE_CPU.m: k is 1-based, no chunk clamp
-    constexpr bool heun = (METHOD != OPTIFAX_RK23);
     float k = nee ? 1.f : 0.f, stepprev = 4.f, stepmod = 4.f;
     unsigned q = 0;                          // accumulated dispersion position (sum of stepmod)
-    int s_cached = -1;                       // stepmod of the cached per-mode D - 1 (Heun)
+    int s_cached = -1;                       // stepmod of the cached per-mode D - 1
     int attempt = 0, n_acc = 0, n_rej = 0, status = 0, par = 0, trip = 0, trips_done = 0;
     int gatt = 0, tot_att = 0, tot_acc = 0, tot_rej = 0, steady_count = 0;
     double prev_tally = 0.0;
 
-    float2 k1r[16];   // RK23: K1 (first stage, FSAL) between attempts
+    // neighbours' drive values at the thread's ends; hv: the halo point's drive (end threads)
+    auto edges = [&](const Pair (&nl)[H], float2 hv, float2& L, float2& R) {
+        exchange_edges<M, C, !HALO>(edge, par, t, c, make_float2(nl[0].re.x, nl[0].im.x),
+                                    make_float2(nl[H - 1].re.y, nl[H - 1].im.y), L, R);
+        if constexpr (HALO) {
+            if (t == 0) L = hv;
+            if (t == T - 1) R = hv;
+        }
+    };
+
+    // z-phasors of an attempt's stages and its G sample, made ahead (before the
+    // transforms of the previous step) and keyed by the position and the step
+    float zk = -1.f, zs = -1.f, gval = 0.f;
+    float2 z0 = make_float2(0.f, 0.f), z1 = z0, z2 = z0;
+    auto prepare = [&](float kp, float sm) {
+        if constexpr (heun) zphases(P_.tau_z4, t, kp, kp + sm, 0.f, z0, z1, z2);
+        else zphases(P_.tau_z4, t, kp + 0.5f * sm, kp + 0.75f * sm, kp + sm, z0, z1, z2);
+        gval = G[(int)kp];
+        zk = kp; zs = sm;
+    };
+
+    Pair k1r[H];      // RK23: K1 (first stage, FSAL) between attempts
     for (trip = 0; trip < n_trips; ++trip) {
         k = nee ? 1.f : 0.f; stepprev = 4.f; stepmod = 4.f; q = 0;
         attempt = 0; n_acc = 0; n_rej = 0;
         int trip_status = 0;
         double tally[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 1
-        for (int j = 0; j < 16; ++j) papp_s[j * T + t] = 0;
-        if constexpr (METHOD == OPTIFAX_RK23) {
+        if constexpr (!heun) {
             // initial K1 at k = 0 with stepmod = 4 (OPO_CUDA_ODE23.cu:432-438)
-            float hg = (stepmod * h) * G[0];
-            float2 z = zphase(P.tau_z4, 0.f);
-            float2 nl[16];
+            const float hg = (stepmod * h) * G[0];
+            const float2 z = zphase(P_.tau_z4, 0.f);
+            Pair nl[H];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) nl[j] = nl_eval(a[j], cph[j], z);
+            for (int j = 0; j < H; ++j) nl[j] = nl_eval(a[j], cph[j], z);
             float2 L, R;
-            exchange_edges<M, C>(edge, par, t, c, nl[0], nl[15], L, R);
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                k1r[j] = k_eval(j == 0 ? L : nl[j - 1], nl[j], j == 15 ? R : nl[j + 1], hg, cs);
+            edges(nl, h1, L, R);
+            k_all<H>(nl, L, R, hg, cs, k1r);
         }
 
         for (int chunk = 0; chunk < nchunks; ++chunk) {
@@ -594,124 +827,145 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
             const float cend = (float)(chunk + 1) * sel;
             while (k < cend && (nee ? k <= Sf : (!guard || k < Sf))) {
                 if (attempt >= max_attempts) { status |= OPTIFAX_PULSE_ATTEMPT_LIMIT; goto done; }
-                const int kidx = nee ? (int)k - 1 : (int)k;   // G33(k) is 1-based in NEE_CPU.m
                 const int krec = (int)k;
-                const float kpos = nee ? k - 1.f : k;          // z of the first stage, in steps
+                // z of the first stage in steps and index of G (G33(k) is 1-based in NEE_CPU.m)
+                const float kpos = nee ? k - 1.f : k;
                 bool accepted = false;
-                const float hmod = stepmod * h;
-                const float hg = hmod * G[kidx];
-                int bits = 0;
+                if (kpos != zk || stepmod != zs) prepare(kpos, stepmod);
+                const float hg = (stepmod * h) * gval;
+                Pair ev[H];                                    // E, then E behind the absorber
+                Pair dv[H];                                    // its error difference
+                Pair k4[H];                                    // RK23: FSAL candidate
                 if constexpr (heun) {
                     // ---- stage 1: K1 = f(A0) at z = k ----
-                    float2 nl[16], k1[16], L, R;
-                    float2 z = zphase(P.tau_z4, kpos);
+                    Pair nl[H], k1[H], k2[H];
+                    float2 L, R, zu = make_float2(0.f, 0.f);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) nl[j] = nl_eval(a[j], cph[j], z);
-                    exchange_edges<M, C>(edge, par, t, c, nl[0], nl[15], L, R);
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        k1[j] = k_eval(j == 0 ? L : nl[j - 1], nl[j], j == 15 ? R : nl[j + 1], hg, cs);
+                    for (int j = 0; j < H; ++j) nl[j] = nl_eval(a[j], cph[j], z0);
+                    float2 hn = make_float2(0.f, 0.f);
+                    if (lend || rend) {
+                        // drive and A1 of the adjacent halo point
+                        const float2 n1 = nl_one(h1, hc1, z0), n2 = nl_one(h2, hc2, z0);
+                        const float2 in = lend ? make_float2(nl[0].re.x, nl[0].im.x)
+                                               : make_float2(nl[H - 1].re.y, nl[H - 1].im.y);
+                        const float2 kh = lend ? k_one(n2, n1, in, hg, cs) : k_one(in, n1, n2, hg, cs);
+                        hn = n1;
+                        zu = nl_one(cadd(h1, kh), hc1, z1);
+                    }
+                    edges(nl, hn, L, R);
+                    k_all<H>(nl, L, R, hg, cs, k1);
                     // ---- stage 2: K2 = f(A0 + K1) at z = k + stepmod ----
-                    z = zphase(P.tau_z4, kpos + stepmod);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) nl[j] = nl_eval(cadd(a[j], k1[j]), cph[j], z);
-                    exchange_edges<M, C>(edge, par, t, c, nl[0], nl[15], L, R);
-                    float2 prev;
+                    for (int j = 0; j < H; ++j) nl[j] = nl_eval(pair_add(a[j], k1[j]), cph[j], z1);
+                    edges(nl, zu, L, R);
+                    k_all<H>(nl, L, R, hg, cs, k2);
+                    // E = A0 + (K2/2 + K1/2) (MEX) or (A0 + K1/2) + K2/2 (NEE_CPU.m:75)
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        float2 k2 = k_eval(j == 0 ? L : nl[j - 1], nl[j], j == 15 ? R : nl[j + 1], hg, cs);
-                        // E = A0 + (K2/2 + K1/2) (MEX) or (A0 + K1/2) + K2/2 (NEE_CPU.m:75)
-                        float2 e = nee ? cadd(cadd(a[j], cscale(k1[j], 0.5f)), cscale(k2, 0.5f))
-                                       : cadd(a[j], cadd(cscale(k2, 0.5f), cscale(k1[j], 0.5f)));
-                        float2 d = csub(k2, k1[j]);                        // = 2 (E - A1)
-                        bits |= nee ? classify_nee(50.f, d, e, maxE, minE) : classify(50.f, d, e, maxE, minE);
-                        float2 ea = cscale(e, abc_s[j * T + t]);
-                        bufE[phys(16 * t + j)] = ea;
-                        if constexpr (C == 1) bufX[phys(16 * t + j)] = ea;
-                        else if constexpr (!kPullGather<C>) store_pair(P.xch + c * M + 16 * t, j, ea, prev);
+                    for (int j = 0; j < H; ++j) {
+                        ev[j] = nee ? pair_fma(k2[j], 0.5f, pair_fma(k1[j], 0.5f, a[j]))
+                                    : pair_fma(pair_add(k2[j], k1[j]), 0.5f, a[j]);
+                        dv[j] = pair_sub(k2[j], k1[j]);                        // = 2 (E - A1)
                     }
                 } else {
                     // ---- RK23: K2 at k + s/2, K3 at k + 3s/4, K4 at k + s (FSAL) ----
-                    float2 nl[16], k2[16], pp[16], L, R;
-                    float2 z = zphase(P.tau_z4, k + 0.5f * stepmod);
+                    Pair nl[H], k2[H], pp[H];
+                    float2 L, R;
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) nl[j] = nl_eval(cadd(a[j], cscale(k1r[j], 0.5f)), cph[j], z);
-                    exchange_edges<M, C>(edge, par, t, c, nl[0], nl[15], L, R);
+                    for (int j = 0; j < H; ++j) nl[j] = nl_eval(pair_fma(k1r[j], 0.5f, a[j]), cph[j], z0);
+                    edges(nl, h1, L, R);
+                    k_all<H>(nl, L, R, hg, cs, k2);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        k2[j] = k_eval(j == 0 ? L : nl[j - 1], nl[j], j == 15 ? R : nl[j + 1], hg, cs);
-                    z = zphase(P.tau_z4, k + 0.75f * stepmod);
+                    for (int j = 0; j < H; ++j) nl[j] = nl_eval(pair_fma(k2[j], 0.75f, a[j]), cph[j], z1);
+                    edges(nl, h1, L, R);
+                    k_all<H>(nl, L, R, hg, cs, pp);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) nl[j] = nl_eval(cadd(a[j], cscale(k2[j], 0.75f)), cph[j], z);
-                    exchange_edges<M, C>(edge, par, t, c, nl[0], nl[15], L, R);
-                    float2 ev[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        float2 k3 = k_eval(j == 0 ? L : nl[j - 1], nl[j], j == 15 ? R : nl[j + 1], hg, cs);
-                        float2 e = cadd(a[j], cadd(cscale(k3, 4.f / 9.f), cscale(k2[j], 1.f / 3.f)));
-                        ev[j] = cadd(e, cscale(k1r[j], 2.f / 9.f));
+                    for (int j = 0; j < H; ++j) {
+                        const Pair k3 = pp[j];
+                        const float2 b1 = fma2(k2[j].re, dup2(1.f / 3.f), mul2(k3.re, dup2(4.f / 9.f)));
+                        const float2 b2 = fma2(k2[j].im, dup2(1.f / 3.f), mul2(k3.im, dup2(4.f / 9.f)));
+                        ev[j] = pair_fma(k1r[j], 2.f / 9.f, pair_add(a[j], Pair{b1, b2}));
                         // E - A1 without K4: (4/9-1/3) K3 + (1/3-1/4) K2 + (2/9-7/24) K1
-                        pp[j] = cadd(cadd(cscale(k3, 1.f / 9.f), cscale(k2[j], 1.f / 12.f)),
-                                     cscale(k1r[j], -5.f / 72.f));
+                        const float2 c1 = fma2(k2[j].re, dup2(1.f / 12.f), mul2(k3.re, dup2(1.f / 9.f)));
+                        const float2 c2 = fma2(k2[j].im, dup2(1.f / 12.f), mul2(k3.im, dup2(1.f / 9.f)));
+                        pp[j] = pair_fma(k1r[j], -5.f / 72.f, Pair{c1, c2});
                     }
-                    z = zphase(P.tau_z4, k + stepmod);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) nl[j] = nl_eval(ev[j], cph[j], z);
-                    exchange_edges<M, C>(edge, par, t, c, nl[0], nl[15], L, R);
-                    float2 prev;
+                    for (int j = 0; j < H; ++j) nl[j] = nl_eval(ev[j], cph[j], z2);
+                    edges(nl, h1, L, R);
+                    k_all<H>(nl, L, R, hg, cs, k4);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        float2 k4 = k_eval(j == 0 ? L : nl[j - 1], nl[j], j == 15 ? R : nl[j + 1], hg, cs);
-                        float2 d = csub(pp[j], cscale(k4, 1.f / 8.f));  // = E - A1
-                        bits |= classify(200.f, d, ev[j], maxE, minE);
-                        float2 ea = cscale(ev[j], abc_s[j * T + t]);
-                        bufE[phys(16 * t + j)] = ea;
-                        if constexpr (C == 1) bufX[phys(16 * t + j)] = ea;
-                        else if constexpr (!kPullGather<C>) store_pair(P.xch + c * M + 16 * t, j, ea, prev);
-                        bufK[phys(16 * t + j)] = k4;   // FSAL candidate (own points)
+                    for (int j = 0; j < H; ++j) dv[j] = pair_fma(k4[j], -1.f / 8.f, pp[j]);   // = E - A1
+                }
+                const int bits = classify_all<H, nee>(bounds, dv, ev);
+                // E behind the absorber: into the FFT buffer, or its columns' owners
+                {
+                    float2 o[P];
+                    float ab[P];
+#pragma unroll
+                    for (int j = 0; j < P; j += 4) {
+                        const float4 w = *reinterpret_cast<const float4*>(abc_s + at4(j));
+                        ab[j] = w.x; ab[j + 1] = w.y; ab[j + 2] = w.z; ab[j + 3] = w.w;
+                    }
+#pragma unroll
+                    for (int j = 0; j < H; ++j) {
+                        const float2 f = make_float2(ab[j], ab[j + H]);
+                        ev[j] = Pair{mul2(ev[j].re, f), mul2(ev[j].im, f)};
+                        o[j] = make_float2(ev[j].re.x, ev[j].im.x);
+                        o[j + H] = make_float2(ev[j].re.y, ev[j].im.y);
+                    }
+                    if constexpr (C > 1) push_columns<M, C>(g_addr, o, t, c);
+                    else store_own<P>(bufX, t, o);
+                    if (lend) {          // E of this block's first points: the left neighbour's right halo
+                        const uint32_t dst = cluster_addr(smem_u32(halo_e), (c + C - 1) % C);
+                        st_cluster_f2(dst + 16, o[0]);
+                        st_cluster_f2(dst + 24, o[1]);
+                    }
+                    if (rend) {
+                        const uint32_t dst = cluster_addr(smem_u32(halo_e), (c + 1) % C);
+                        st_cluster_f2(dst, o[P - 2]);
+                        st_cluster_f2(dst + 8, o[P - 1]);
                     }
                 }
 
-                int fl = reduce_flags<M, C>(bits, red, gatt, t, c, cfg);
-                if (P.forced && gatt < P.n_forced) fl = (P.forced[gatt] & 3) | (fl & 4);
+                int fl = combine_flags<M, C>(bits, red, gatt, t, c, cfg);
+                if ((opts & kForced) && gatt < P_.n_forced) fl = (P_.forced[gatt] & 3) | (fl & 4);
                 if (fl & 4) trip_status |= OPTIFAX_PULSE_NAN;
 
                 if ((fl & 1) && stepmod > 1.f && (nee || (k - stepmod) > 0.f)) {
                     // ---- reject: A0 unchanged; MEX: k moves back by one in net (the loop
                     // adds the new stepmod); NEE: k stays (NEE_CPU.m:68-70)
-                    if (rec && P.trace && gatt < P.trace_cap) {
-                        P.trace[3 * gatt] = krec; P.trace[3 * gatt + 1] = (int)stepmod;
-                        P.trace[3 * gatt + 2] = fl & 7;
+                    if ((opts & kTrace) && rec && gatt < P_.trace_cap) {
+                        P_.trace[3 * gatt] = krec; P_.trace[3 * gatt + 1] = (int)stepmod;
+                        P_.trace[3 * gatt + 2] = fl & 7;
                     }
                     ++n_rej;
                     if (!nee) k = k - stepmod;
                     stepmod = stepmod - 1.f;
                     stepprev = stepmod;
-                    if constexpr (METHOD == OPTIFAX_RK23) {
+                    if constexpr (!heun) {
                         // K1 recomputed at z = k + stepmod with G[k] (OPO_CUDA_ODE23.cu:484-487)
-                        float hg1 = (stepmod * h) * G[(int)k];
-                        float2 z = zphase(P.tau_z4, k + stepmod);
-                        float2 nl[16], L, R;
+                        const float hg1 = (stepmod * h) * G[(int)k];
+                        const float2 z = zphase(P_.tau_z4, k + stepmod);
+                        Pair nl[H];
+                        float2 L, R;
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) nl[j] = nl_eval(a[j], cph[j], z);
-                        exchange_edges<M, C>(edge, par, t, c, nl[0], nl[15], L, R);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            k1r[j] = k_eval(j == 0 ? L : nl[j - 1], nl[j], j == 15 ? R : nl[j + 1], hg1, cs);
+                        for (int j = 0; j < H; ++j) nl[j] = nl_eval(a[j], cph[j], z);
+                        edges(nl, h1, L, R);
+                        k_all<H>(nl, L, R, hg1, cs, k1r);
                     }
                 } else {
                     // ---- accept ----
-                    if (rec && P.trace && gatt < P.trace_cap) {
-                        P.trace[3 * gatt] = krec; P.trace[3 * gatt + 1] = (int)stepmod;
-                        P.trace[3 * gatt + 2] = (fl & 7) | 8;
+                    if ((opts & kTrace) && rec && gatt < P_.trace_cap) {
+                        P_.trace[3 * gatt] = krec; P_.trace[3 * gatt + 1] = (int)stepmod;
+                        P_.trace[3 * gatt + 2] = (fl & 7) | 8;
                     }
                     ++n_acc;
                     accepted = true;
                     const int s_used = (int)stepmod;
-                    if (!nee && rec && P.stepmods && kidx < P.stepmods_limit && kidx < P.S)
-                        P.stepmods[kidx] = (float)s_used;
-                    if (!nee && rec && P.smt && kidx < P.stepmods_limit && kidx < P.S)
-                        P.smt[(size_t)trip * P.S + kidx] = (float)s_used;
+                    if ((opts & kSteps) && rec && krec < P_.stepmods_limit && krec < P_.S) {
+                        if (P_.stepmods) P_.stepmods[krec] = (float)s_used;
+                        if (P_.smt) P_.smt[(size_t)trip * P_.S + krec] = (float)s_used;
+                    }
                     // step control (OPO_CUDA_BATCH_XTAL.cu:487-506; ODE23 :519-538 doubles;
                     // NEE_CPU.m:77-83: grow below minErr, clamp only at the crystal end)
                     if (nee) {
@@ -734,136 +988,125 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     const bool pass_ends = !(knext < pass_end && (nee ? knext <= Sf : (!guard || knext < Sf)));
                     const bool cav = opo && pass_ends;
                     const unsigned qn = q + (unsigned)s_used;
+                    if (!pass_ends) {
+                        const float kn = nee ? knext - 1.f : knext;
+                        prepare(kn, (!nee && last_in_chunk) ? stepprev : stepmod);
+                    }
 
                     // ---- linear sub-step ----
                     // Incremental form: A_new = E + IFFT((D - 1) FFT(E)) / N with
                     // D = alpha^s exp(-i beta s): transform rounding then scales with
                     // |D - 1| instead of |E|.  At the end of an OPO pass the full
                     // spectrum goes through the cavity instead: A_new = IFFT(D FFT(E) fb + pump) / N.
-                    // clusters: the exchanged block lands in bufX (the FFT buffer; bufE keeps E),
-                    // or in ybuf (global) for 16-CTA clusters
-                    float2* fbuf = (C > 1) ? bufX : bufE;
-                    float2* ybuf = (C > 1) ? P.xch + N + c * M : nullptr;
+                    float2 he1 = h1, he2 = h1;
                     if constexpr (C > 1) {
-                        exchange_forward_g<M, C>(P.xch, bufE, bufX, P.xch + N, quad_s, low_s, t, c);
-                        cg::this_cluster().sync();
-                    } else {
-                        __syncthreads();
+                        if (lend) { he1 = halo_e[1]; he2 = halo_e[0]; }
+                        if (rend) { he1 = halo_e[2]; he2 = halo_e[3]; }
+                        exchange_fwd<M, C>(bufG, x_addr, xtw_s, t, c);
                     }
-                    if constexpr (heun) {
-                        // refresh the per-mode D - 1 cache when the step size changed (a
-                        // compact loop: kept out of the unrolled mode loop below)
-                        if (s_used != s_cached) {
+                    // refresh the per-mode D - 1 when the step size changed (a compact loop:
+                    // kept out of the unrolled mode loop below), for the exact fixed-point
+                    // increment beta s: the FP32 rounding of its angle is applied as a
+                    // first-order rotation, D e^{-i eps} - 1 ~ (D - 1) - i eps D
+                    constexpr float kUnit = 1.4629180792671596e-09f;     // 2 pi 2^-32
+                    if (s_used != s_cached) {
 #pragma unroll 1
-                            for (int j = 0; j < 16; ++j) {
-                                const int idx = j * T + t;
-                                int dc;
-                                const uint64_t inc = tau_s[idx] * (uint64_t)(unsigned)s_used;
-                                dmc_s[idx] = dispersion_dm1((int)((long long)inc >> 32), l2a_s[idx], s_used, &dc);
-                                dfc_s[idx] = dc;
-                            }
+                        for (int j = 0; j < P; ++j) {
+                            const int kk = c + C * bitrev(P * t + j, LOG2M);
+                            const uint64_t tau = phase_rate(P_.beta[kk]);
+                            const uint64_t inc = tau * (uint64_t)(unsigned)s_used;
+                            const int d32 = (int)((long long)inc >> 32);
+                            int dc;
+                            const float l2 = log2f(P_.alpha[kk]);
+                            const float2 m = dispersion_dm1(d32, l2, s_used, &dc);
+                            const float e = (float)(int)((unsigned)d32 - (unsigned)dc) * kUnit;
+                            dm_s[at2(j)] = make_float2(fmaf(e, m.y, m.x), fmaf(-e, 1.f + m.x, m.y));
                         }
+                        s_cached = s_used;
                     }
-                    float2 v[16];
-                    fft_forward_to_regs<M>(fbuf, tw1, tw2, t, v, kPushExchange<C> ? nullptr : ybuf);
-                    float2* apc = (last_in_chunk && P.Ap) ? P.Ap + (size_t)chunk * N : nullptr;
+                    if constexpr (C > 1) cg::this_cluster().sync();
+                    float2 v[P];
+                    fftp_forward<M, P>(bufX, tw_s, t, v);
+                    float2* apc = (last_in_chunk && (opts & kAp)) ? P_.Ap + (size_t)chunk * N : nullptr;
                     float part[4] = {0.f, 0.f, 0.f, 0.f};
                     // the trip's crystal output goes to the cavity scratch; the cavity
                     // work (tallies, ESD sums, history, transfer) runs after the loop
-                    float2* const xsp = cav ? P.xs : nullptr;
+                    float2* const xsp = cav ? P_.xs : nullptr;
+                    uint32_t lo_[P];
+                    float2 dm_[P];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        // phase increment beta*s from the exact fixed-point target minus the
-                        // phase applied so far (error feedback: FP32 rounding of the
-                        // increment is carried into the next step instead of accumulating)
-                        // increment beta*s: exact fixed-point target minus the phase applied
-                        // so far (error feedback: nothing accumulates from FP32 rounding)
-                        const int idx = j * T + t;
-                        uint64_t target = tau_s[idx] * (uint64_t)qn;
-                        uint32_t ph = papp_s[idx];
-                        int d32 = (int)((long long)(target - ((uint64_t)ph << 32)) >> 32);
-                        float2 dm1;
-                        int dused;
-                        if constexpr (heun) {
-                            // D - 1 cached per mode for the current stepmod; the small
-                            // difference eps between the wanted and the cached increment
-                            // is applied to first order: D e^{-i eps} - 1 ~ (D - 1) - i eps D
-                            float2 dc1 = dmc_s[idx];
-                            int eps = d32 - dfc_s[idx];
-                            dm1 = dc1;
-                            if (eps != 0) {
-                                float e = (float)eps * 1.4629180792671596e-09f;
-                                float2 D = make_float2(1.f + dc1.x, dc1.y);
-                                dm1 = make_float2(fmaf(e, D.y, dc1.x), fmaf(-e, D.x, dc1.y));
-                            }
-                            dused = d32;
-                        } else {
-                            dm1 = dispersion_dm1(d32, l2a_s[idx], s_used, &dused);
-                        }
-                        papp_s[idx] = ph + (uint32_t)dused;
-                        float2 eh = v[j];
-                        int kk = c + C * bitrev(16 * t + j, LOG2M);
-                        if (apc) apc[kk] = cadd(eh, cmul(eh, dm1));
-                        if (cav) xsp[kk] = cadd(eh, cmul(eh, dm1));
-                        else v[j] = cmul(eh, dm1);
+                    for (int j = 0; j < P; j += 4) {
+                        const uint4 w = *reinterpret_cast<const uint4*>(tlo_s + at4(j));
+                        lo_[j] = w.x; lo_[j + 1] = w.y; lo_[j + 2] = w.z; lo_[j + 3] = w.w;
                     }
-                    s_cached = s_used;
+#pragma unroll
+                    for (int j = 0; j < P; j += 2) {
+                        const float4 w = *reinterpret_cast<const float4*>(dm_s + at2(j));
+                        dm_[j] = make_float2(w.x, w.y);
+                        dm_[j + 1] = make_float2(w.z, w.w);
+                    }
+#pragma unroll
+                    for (int j = 0; j < P; ++j) {
+                        // The step's phase is the difference of the two positions' exact
+                        // fixed-point phases in units of 2^-32 turn: the cached increment's
+                        // high word plus the carry of the low words' sum, tau qn = tau q + tau s.
+                        const float e = (lo_[j] * qn < lo_[j] * (unsigned)s_used) ? kUnit : 0.f;
+                        const float2 dm1 = make_float2(fmaf(e, dm_[j].y, dm_[j].x), fmaf(-e, 1.f + dm_[j].x, dm_[j].y));
+                        const float2 eh = v[j];
+                        if (apc || cav) {
+                            const int kk = c + C * bitrev(P * t + j, LOG2M);
+                            const float2 o = cadd(eh, cmul(eh, dm1));
+                            if (apc) apc[kk] = o;
+                            if (cav) xsp[kk] = o;
+                        }
+                        v[j] = cmul(eh, dm1);
+                    }
                     if (cav) {
-                        // once per round trip, outside the unrolled mode loop (code size is
-                        // this kernel's bound): energy tallies, ESD sums and history of the
-                        // crystal output X, then Y = X fb + pump; every mode has one owner
-                        // thread, which reads back only what it wrote
+                        // once per round trip, outside the unrolled mode loop (code size):
+                        // energy tallies, ESD sums and history of the crystal output X,
+                        // then Y = X fb + pump; every mode has one owner thread, which
+                        // reads back only what it wrote
 #pragma unroll 1
-                        for (int j = 0; j < 16; ++j) {
-                            const int kk = c + C * bitrev(16 * t + j, LOG2M);
+                        for (int j = 0; j < P; ++j) {
+                            const int kk = c + C * bitrev(P * t + j, LOG2M);
                             const float2 X = xsp[kk];
                             const float x2 = X.x * X.x + X.y * X.y;
 #pragma unroll
                             for (int i = 0; i < 4; ++i)
-                                if (i < P.n_tally) part[i] = fmaf(P.tally_w[(size_t)i * N + kk], x2, part[i]);
+                                if (i < P_.n_tally) part[i] = fmaf(P_.tally_w[(size_t)i * N + kk], x2, part[i]);
 #pragma unroll 1
-                            for (int i = 0; i < P.n_esd; ++i)
-                                P.esd[(size_t)i * N + kk] += P.esd_w[(size_t)i * N + kk] * x2;
-                            if (P.hist) P.hist[(size_t)trip * N + kk] = X;
-                            xsp[kk] = cadd(cmul(X, P.fb[kk]), P.pump[kk]);
+                            for (int i = 0; i < P_.n_esd; ++i)
+                                P_.esd[(size_t)i * N + kk] += P_.esd_w[(size_t)i * N + kk] * x2;
+                            if (P_.hist) P_.hist[(size_t)trip * N + kk] = X;
+                            xsp[kk] = cadd(cmul(X, P_.fb[kk]), P_.pump[kk]);
                         }
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] = xsp[c + C * bitrev(16 * t + j, LOG2M)];
+                        for (int j = 0; j < P; ++j) v[j] = xsp[c + C * bitrev(P * t + j, LOG2M)];
                     }
-                    fft_inverse_from_regs<M>(fbuf, tw1, tw2, t, v, ybuf);
+                    fftp_inverse<M, P>(bufX, tw_s, td_s, t, v);
                     if constexpr (C > 1) {
+                        push_inverse<M, C>(g_addr, v, t, c);
                         cg::this_cluster().sync();
-                        exchange_inverse_g<M, C>(P.xch + N, bufX, P.xch, quad_s, low_s, t, c, invN);
+                        exchange_inv<M, C, HALO>(bufG, x_addr, smem_u32(halo_d), xtw_s, xtd_s, t, c, invN);
                         cg::this_cluster().sync();
-                        if constexpr (kPushExchange<C>) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const float2 d = bufX[phys(16 * t + j)];
-                                a[j] = cav ? d : cadd(bufE[phys(16 * t + j)], d);
-                            }
-                        } else {
-                            const float4* src = reinterpret_cast<const float4*>(P.xch + c * M + 16 * t);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                float4 w = __ldcg(src + j);
-                                float2 d0 = make_float2(w.x, w.y), d1 = make_float2(w.z, w.w);
-                                a[2 * j] = cav ? d0 : cadd(bufE[phys(16 * t + 2 * j)], d0);
-                                a[2 * j + 1] = cav ? d1 : cadd(bufE[phys(16 * t + 2 * j + 1)], d1);
-                            }
+                        if (lend || rend) {
+                            const float2 d1 = halo_d[lend ? 1 : 2], d2 = halo_d[lend ? 0 : 3];
+                            h1 = cav ? d1 : cadd(he1, d1);
+                            h2 = cav ? d2 : cadd(he2, d2);
                         }
                     } else {
-                        if (cav) {
+                        const int s0 = swz(t);
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) a[j] = cscale(bufE[phys(16 * t + j)], invN);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                a[j] = cadd(bufX[phys(16 * t + j)], cscale(bufE[phys(16 * t + j)], invN));
-                        }
+                        for (int i = 0; i < P; ++i) bufX[swz_at(s0, i * (M / P))] = v[i];
+                        __syncthreads();
                     }
-                    if constexpr (METHOD == OPTIFAX_RK23) {
+                    load_own<P>(bufX, t, v);
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) k1r[j] = bufK[phys(16 * t + j)];
+                    for (int j = 0; j < H; ++j) {
+                        const Pair d{make_float2(v[j].x, v[j + H].x), make_float2(v[j].y, v[j + H].y)};
+                        if constexpr (C > 1) a[j] = cav ? d : pair_add(ev[j], d);
+                        else a[j] = cav ? Pair{mul2(d.re, dup2(invN)), mul2(d.im, dup2(invN))} : pair_fma(d, invN, ev[j]);
+                        if constexpr (!heun) k1r[j] = k4[j];
                     }
                     if (cav) reduce_tallies<M, C>(part, tally, dred, t, c, trip & 1);
                     q = qn;
@@ -877,31 +1120,35 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
         tot_att += attempt; tot_acc += n_acc; tot_rej += n_rej;
         trips_done = trip + 1;
         if (opo) {
-            if (rec && P.trips) {
+            if (rec && P_.trips) {
                 optifax_trip_record tr;
                 tr.attempts = attempt; tr.accepted = n_acc; tr.rejected = n_rej; tr.status = trip_status;
                 for (int i = 0; i < 4; ++i) tr.tally[i] = tally[i];
-                P.trips[trip] = tr;
+                P_.trips[trip] = tr;
             }
-            if (P.steady_trips > 0) {
-                double cur = tally[P.steady_tally & 3];
-                bool flat = trip > 0 && cur != 0.0 && fabs(cur - prev_tally) <= (double)P.steady_tol * fabs(cur);
+            if (P_.steady_trips > 0) {
+                double cur = tally[P_.steady_tally & 3];
+                bool flat = trip > 0 && cur != 0.0 && fabs(cur - prev_tally) <= (double)P_.steady_tol * fabs(cur);
                 steady_count = flat ? steady_count + 1 : 0;
                 prev_tally = cur;
-                if (steady_count >= P.steady_trips) break;
+                if (steady_count >= P_.steady_trips) break;
             }
         }
     }
 done:
 #pragma unroll
-    for (int j = 0; j < 16; ++j) P.A_out[c * M + 16 * t + j] = a[j];
-    if (rec && P.stats) {
+    for (int j = 0; j < H; ++j) {
+        P_.A_out[c * M + P * t + j] = make_float2(a[j].re.x, a[j].im.x);
+        P_.A_out[c * M + P * t + j + H] = make_float2(a[j].re.y, a[j].im.y);
+    }
+    if (rec && P_.stats) {
         optifax_pulse_stats st;
         st.attempts = tot_att; st.accepted = tot_acc; st.rejected = tot_rej; st.status = status;
         st.z_steps = (long long)q; st.k_final = k; st.stepmod_final = stepmod; st.n_chunks = nchunks;
         st.reserved[0] = trips_done; st.reserved[1] = st.reserved[2] = 0;
-        *P.stats = st;
+        *P_.stats = st;
     }
+    if constexpr (C > 1) cg::this_cluster().sync();      // no CTA leaves while a peer may still read its memory
 }
 
 }  // namespace ofx
