@@ -38,6 +38,7 @@ struct optifax_context {
     size_t gnlse_desc_cap = 0;
     float2* d_gnlse_k = nullptr;
     size_t gnlse_k_cap = 0;                  // complex values
+    std::map<const void*, int> resident;     // kernel -> clusters that fit the GPU at once
     cudaEvent_t done_ev = nullptr;           // end of the last call's work on the GPU
     bool done_pending = false;               // done_ev has been recorded
     std::string last_error;
@@ -175,15 +176,108 @@ const KernelEntry* find_kernel(int M, int C, int method) {
     return nullptr;
 }
 
-int choose_M(int N, int cta_points) {
-    if (cta_points > 0) return cta_points;
-    return N <= 4096 ? N : 4096;
-}
-
 struct Group {
     int M, C;
     std::vector<PulseDev> d;
 };
+
+// Kernel attributes (dynamic shared memory, 16-CTA clusters): not stream work, so set
+// before the launches (and outside any capture).
+cudaError_t set_attributes(const KernelEntry& ke) {
+    cudaError_t e = cudaFuncSetAttribute(ke.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ke.smem);
+    if (e == cudaSuccess && ke.C > 8) e = cudaFuncSetAttribute(ke.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+
+// How many clusters of a kernel the GPU holds at once
+int resident_clusters(optifax_context* h, const KernelEntry& ke) {
+    auto it = h->resident.find((const void*)ke.fn);
+    if (it != h->resident.end()) return it->second;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)ke.C, 1, 1);
+    lc.blockDim = dim3((unsigned)ke.threads, 1, 1);
+    lc.dynamicSmemBytes = ke.smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ke.C; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    lc.attrs = &attr;
+    lc.numAttrs = 1;
+    int n = 0;
+    if (set_attributes(ke) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, ke.fn, &lc) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    h->resident[(const void*)ke.fn] = n;
+    return n;
+}
+
+// Points per CTA of a grid of N points that carries no choice of the caller, by spread:
+//   0  the shortest time per attempt of one pulse
+//   1  half the CTAs
+//   2  4096 points per CTA (one CTA up to 4096 points): the least SM time per attempt
+// One pulse, us per attempt (GB300, 2 W, 30 um poling), at spread 2 -> 1 -> 0:
+//   4096: 6.4 -> 5.2 -> 4.6   8192: 10.7 -> 7.0 -> 5.6   16384: 11.4 -> 7.7 -> 7.0
+// SM time per attempt goes the other way (4096: 6.4, 21, 37 SM us), so the wider
+// spreads serve calls that leave SMs idle otherwise.
+int spread_points(int N, int spread) {
+    const int narrow = N <= 4096 ? N : 4096;
+    if (N <= 2048 || N > 32768 || spread >= 2) return narrow;
+    const int wide = N == 4096 ? 512 : N == 32768 ? 2048 : 1024;
+    return spread == 0 ? wide : (2 * wide < narrow ? 2 * wide : narrow);
+}
+
+// One pulse of a call before its group is known
+struct Placed {
+    PulseDev d;
+    int want;        // points per CTA asked for, 0: the rule's choice
+};
+
+int no_kernel(optifax_context* h, int M, int C) {
+    return fail(h, OPTIFAX_ERR_UNSUPPORTED,
+                "no kernel for cta_points=" + std::to_string(M) + " cluster=" + std::to_string(C));
+}
+
+// Groups the pulses by (cta_points, cluster).  Pulses without a choice of the caller
+// take the widest spread at which every cluster of the call is resident at once (each
+// kernel's clusters as a share of what the GPU holds of it), else the narrow one.
+int group_pulses(optifax_context* h, std::vector<Placed>& pulses, int method, std::vector<Group>* gv) {
+    auto points = [&](const Placed& p, int spread) {
+        const int narrow = p.d.N <= 4096 ? p.d.N : 4096;
+        if (p.want > 0) return p.want < p.d.N ? p.want : p.d.N;
+        const int M = spread_points(p.d.N, spread);
+        // sizes without a kernel at 4096 points per CTA stay refused
+        return find_kernel(narrow, p.d.N / narrow, method) && find_kernel(M, p.d.N / M, method) ? M : narrow;
+    };
+    for (const Placed& p : pulses) {
+        const int M = points(p, 2), C = p.d.N / M;
+        if (C > 16) return fail(h, OPTIFAX_ERR_UNSUPPORTED, "n_points / cta_points exceeds 16");
+        const KernelEntry* ke = find_kernel(M, C, method);
+        if (!ke || (p.want > 0 && ke->rule_only)) return no_kernel(h, M, C);
+    }
+    int spread = 0;
+    for (; spread < 2; ++spread) {
+        std::map<std::pair<int, int>, int> count;
+        for (const Placed& p : pulses) {
+            const int M = points(p, spread);
+            ++count[{M, p.d.N / M}];
+        }
+        double share = 0.0;
+        for (const auto& g : count) {
+            const KernelEntry* ke = find_kernel(g.first.first, g.first.second, method);
+            const int n = ke ? resident_clusters(h, *ke) : 0;
+            share += n > 0 ? (double)g.second / n : 2.0;
+        }
+        if (share <= 1.0) break;
+    }
+    std::map<std::pair<int, int>, std::vector<PulseDev>> groups;
+    for (const Placed& p : pulses) {
+        const int M = points(p, spread);
+        groups[{M, p.d.N / M}].push_back(p.d);
+    }
+    gv->clear();
+    for (auto& g : groups) gv->push_back(Group{g.first.first, g.first.second, std::move(g.second)});
+    return OPTIFAX_OK;
+}
 
 double pulse_cost(const PulseDev& d) {
     return (double)d.N * std::log2((double)d.N) * (double)d.S;
@@ -252,19 +346,12 @@ int group_tables(optifax_context* h, const std::vector<Group>& groups, cudaStrea
     return rc;
 }
 
-// Kernel attributes of every group's kernel (dynamic shared memory, 16-CTA clusters);
-// not stream work, so set before the launches (and outside any capture).
 int group_attributes(optifax_context* h, const std::vector<Group>& groups, int method, const VariantCfg& vc) {
     for (const auto& g : groups) {
         const KernelEntry* ke = find_kernel(g.M, g.C, vc.nee ? kHeunNee : method);
-        if (!ke) return fail(h, OPTIFAX_ERR_UNSUPPORTED,
-                             "no kernel for cta_points=" + std::to_string(g.M) + " cluster=" + std::to_string(g.C));
-        cudaError_t e = cudaFuncSetAttribute(ke->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ke->smem);
-        if (e != cudaSuccess) return cuda_fail(h, e, "cudaFuncSetAttribute(smem)");
-        if (g.C > 8) {
-            e = cudaFuncSetAttribute(ke->fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            if (e != cudaSuccess) return cuda_fail(h, e, "cudaFuncSetAttribute(cluster 16)");
-        }
+        if (!ke) return no_kernel(h, g.M, g.C);
+        cudaError_t e = set_attributes(*ke);
+        if (e != cudaSuccess) return cuda_fail(h, e, "cudaFuncSetAttribute");
     }
     return OPTIFAX_OK;
 }
@@ -285,8 +372,7 @@ int enqueue_groups(optifax_context* h, const std::vector<Group>& groups, int met
         const Group& g = groups[gi];
         const int M = g.M, C = g.C;
         const KernelEntry* ke = find_kernel(M, C, vc.nee ? kHeunNee : method);
-        if (!ke) return fail(h, OPTIFAX_ERR_UNSUPPORTED,
-                             "no kernel for cta_points=" + std::to_string(M) + " cluster=" + std::to_string(C));
+        if (!ke) return no_kernel(h, M, C);
         const FftTables tabs = tabv[gi];
         KernelCfg cfg;
         cfg.time_mode = vc.time_mode;
@@ -367,15 +453,6 @@ int launch_groups(optifax_context* h, std::vector<Group>& groups, int method, co
     rc = enqueue_groups(h, groups, method, vc, shared, h->d_desc, tabv, h->d_grid_flags, st, h->side, h->ev);
     if (rc) return rc;
     return mark_done(h, st);
-}
-
-int launch_group(optifax_context* h, const std::vector<PulseDev>& descs, int M, int C, int method,
-                 const VariantCfg& vc, bool shared, cudaStream_t st) {
-    std::vector<Group> groups(1);
-    groups[0].M = M;
-    groups[0].C = C;
-    groups[0].d = descs;
-    return launch_groups(h, groups, method, vc, shared, st);
 }
 
 int fill_desc(optifax_context* h, const optifax_pulse& in, const VariantCfg& vc, PulseDev* d,
@@ -461,23 +538,16 @@ int propagate_groups(optifax_handle h, const optifax_pulse* pulses, int32_t n_pu
         return fail(h, OPTIFAX_ERR_INVALID_ARGUMENT, "the NEE variant is a Heun schedule (NEE_CPU.m)");
     if (cta_points != 0 && (!is_pow2(cta_points) || cta_points < 512 || cta_points > 4096))
         return fail(h, OPTIFAX_ERR_INVALID_ARGUMENT, "cta_points must be 0 or a power of two in [512, 4096]");
-    std::map<std::pair<int, int>, std::vector<PulseDev>> groups;
+    std::vector<Placed> placed((size_t)n_pulses);
     for (int i = 0; i < n_pulses; ++i) {
-        PulseDev d;
-        int rc = fill_desc(h, pulses[i], *vc, &d, stats ? stats + i : nullptr);
+        int rc = fill_desc(h, pulses[i], *vc, &placed[i].d, stats ? stats + i : nullptr);
         if (rc) return rc;
         int want = pulses[i].cta_points > 0 ? pulses[i].cta_points : cta_points;
         if (want != 0 && (!is_pow2(want) || want < 512 || want > 4096))
             return fail(h, OPTIFAX_ERR_INVALID_ARGUMENT, "pulse cta_points must be 0 or a power of two in [512, 4096]");
-        int M = choose_M(pulses[i].n_points, want);
-        if (M > pulses[i].n_points) M = pulses[i].n_points;
-        int C = pulses[i].n_points / M;
-        if (C > 16) return fail(h, OPTIFAX_ERR_UNSUPPORTED, "n_points / cta_points exceeds 16");
-        groups[{M, C}].push_back(d);
+        placed[i].want = want;
     }
-    gv->clear();
-    for (auto& g : groups) gv->push_back(Group{g.first.first, g.first.second, std::move(g.second)});
-    return OPTIFAX_OK;
+    return group_pulses(h, placed, vc->nee ? kHeunNee : method, gv);
 }
 
 }  // namespace
@@ -598,7 +668,7 @@ int optifax_opo_run(optifax_handle h, const optifax_opo* cavities, int32_t n_cav
         return fail(h, OPTIFAX_ERR_INVALID_ARGUMENT, "cta_points must be 0 or a power of two in [512, 4096]");
     cudaError_t e = cudaSetDevice(h->device);
     if (e != cudaSuccess) return cuda_fail(h, e, "cudaSetDevice");
-    std::map<std::pair<int, int>, std::vector<PulseDev>> groups;
+    std::vector<Placed> placed((size_t)n_cavities);
     for (int i = 0; i < n_cavities; ++i) {
         const optifax_opo& cv = cavities[i];
         if (!cv.feedback || !cv.pump) return fail(h, OPTIFAX_ERR_INVALID_ARGUMENT, "feedback and pump are required");
@@ -607,7 +677,8 @@ int optifax_opo_run(optifax_handle h, const optifax_opo* cavities, int32_t n_cav
             return fail(h, OPTIFAX_ERR_INVALID_ARGUMENT, "n_tally must be 0..4 with tally_w");
         if (cv.steady_trips < 0 || cv.steady_tally < 0 || cv.steady_tally >= 4)
             return fail(h, OPTIFAX_ERR_INVALID_ARGUMENT, "bad steady-state settings");
-        PulseDev d;
+        PulseDev& d = placed[i].d;
+        placed[i].want = cta_points;
         int rc = fill_desc(h, cv.pass, vc, &d, stats ? stats + i : nullptr);
         if (rc) return rc;
         d.fb = (const float2*)cv.feedback;
@@ -626,14 +697,10 @@ int optifax_opo_run(optifax_handle h, const optifax_opo* cavities, int32_t n_cav
         d.esd = cv.n_esd > 0 ? cv.esd : nullptr;
         d.n_esd = cv.n_esd;
         d.smt = cv.stepmods_trips;
-        int M = choose_M(cv.pass.n_points, cta_points);
-        if (M > cv.pass.n_points) M = cv.pass.n_points;
-        int C = cv.pass.n_points / M;
-        if (C > 16) return fail(h, OPTIFAX_ERR_UNSUPPORTED, "n_points / cta_points exceeds 16");
-        groups[{M, C}].push_back(d);
     }
     std::vector<Group> gv;
-    for (auto& g : groups) gv.push_back(Group{g.first.first, g.first.second, std::move(g.second)});
+    int rc = group_pulses(h, placed, vc.nee ? kHeunNee : OPTIFAX_HEUN, &gv);
+    if (rc) return rc;
     return launch_groups(h, gv, OPTIFAX_HEUN, vc, false, (cudaStream_t)stream);
 }
 
@@ -668,7 +735,7 @@ int optifax_opo_mex_batch(optifax_handle h,
                             cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess) return cuda_fail(h, e, "copy stepmods");
     }
-    std::vector<PulseDev> descs((size_t)n_pulses);
+    std::vector<Placed> placed((size_t)n_pulses);
     for (int b = 0; b < n_pulses; ++b) {
         optifax_pulse p;
         memset(&p, 0, sizeof(p));
@@ -684,14 +751,17 @@ int optifax_opo_mex_batch(optifax_handle h,
         p.stepmods = stepmods_out;
         p.w0 = w0; p.h = step_h; p.bdiffw0 = bdiffw0; p.dt = dt;
         p.max_err = max_pct_err; p.min_err = min_pct_err; p.sel = sel;
-        int rc = fill_desc(h, p, vc, &descs[b], nullptr);
+        placed[b].want = 0;
+        int rc = fill_desc(h, p, vc, &placed[b].d, nullptr);
         if (rc) return rc;
     }
-    int M = choose_M(n_points, 0);
-    int C = n_points / M;
-    if (n_pulses * C > 148)
+    if (n_pulses * (n_points > 4096 ? n_points / 4096 : 1) > 148)
         return fail(h, OPTIFAX_ERR_UNSUPPORTED, "shared-schedule batch larger than one wave of SMs");
-    return launch_group(h, descs, M, C, method, vc, n_pulses > 1, st);
+    // one size, so one group: every pulse of the shared schedule is in one cooperative grid
+    std::vector<Group> gv;
+    int rc = group_pulses(h, placed, vc.nee ? kHeunNee : method, &gv);
+    if (rc) return rc;
+    return launch_groups(h, gv, method, vc, n_pulses > 1, st);
 }
 
 }  // extern "C"

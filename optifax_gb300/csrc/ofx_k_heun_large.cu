@@ -11,5 +11,6 @@ void register_kernels_heun_large(std::vector<KernelEntry>& v) {
     v.push_back(kernel_entry<2048, 2, OPTIFAX_HEUN>());
     v.push_back(kernel_entry<2048, 4, OPTIFAX_HEUN>());
     v.push_back(kernel_entry<2048, 8, OPTIFAX_HEUN>());
+    v.push_back(kernel_entry<2048, 16, OPTIFAX_HEUN>(true));
 }
 }  // namespace ofx

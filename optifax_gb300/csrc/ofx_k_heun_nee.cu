@@ -10,8 +10,13 @@ void register_kernels_heun_nee(std::vector<KernelEntry>& v) {
     v.push_back(kernel_entry<2048, 2, kHeunNee>());
     v.push_back(kernel_entry<2048, 4, kHeunNee>());
     v.push_back(kernel_entry<1024, 1, kHeunNee>());
+    v.push_back(kernel_entry<2048, 8, kHeunNee>(true));
     v.push_back(kernel_entry<1024, 2, kHeunNee>());
+    v.push_back(kernel_entry<1024, 4, kHeunNee>(true));
+    v.push_back(kernel_entry<1024, 8, kHeunNee>(true));
+    v.push_back(kernel_entry<1024, 16, kHeunNee>(true));
     v.push_back(kernel_entry<512, 1, kHeunNee>());
     v.push_back(kernel_entry<512, 2, kHeunNee>());
+    v.push_back(kernel_entry<512, 8, kHeunNee>(true));
 }
 }  // namespace ofx

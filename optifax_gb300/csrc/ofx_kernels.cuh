@@ -9,11 +9,13 @@ namespace ofx {
 
 typedef void (*KernelFn)(const PulseDev*, FftTables, KernelCfg);
 
-struct KernelEntry { KernelFn fn; size_t smem; int threads, M, C, method; };
+// rule_only: a shape that the library's own choice of points per CTA may take, not one
+// that a caller may ask for.
+struct KernelEntry { KernelFn fn; size_t smem; int threads, M, C, method; bool rule_only; };
 
 template <int M, int C, int METH>
-KernelEntry kernel_entry() {
-    return KernelEntry{&pass_kernel<M, C, METH>, Smem<M, METH, C>::bytes, M / kPoints<M>, M, C, METH};
+KernelEntry kernel_entry(bool rule_only = false) {
+    return KernelEntry{&pass_kernel<M, C, METH>, Smem<M, METH, C>::bytes, M / kPoints<M>, M, C, METH, rule_only};
 }
 
 void register_kernels_heun_large(std::vector<KernelEntry>& v);
