@@ -64,6 +64,7 @@ typedef enum {
 /* Per-pulse status bits returned in optifax_pulse_stats.status. */
 #define OPTIFAX_PULSE_NAN           0x1  /* a non-finite field value was produced */
 #define OPTIFAX_PULSE_ATTEMPT_LIMIT 0x2  /* the step-attempt safety limit was reached */
+#define OPTIFAX_PULSE_TIMEOUT       0x4  /* a wait inside a cluster ran out (about 2 s); the field is not valid */
 
 typedef struct {
     int32_t attempts;       /* step attempts (accepted + rejected) */

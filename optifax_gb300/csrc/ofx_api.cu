@@ -216,13 +216,14 @@ int resident_clusters(optifax_context* h, const KernelEntry& ke) {
 //   1  half the CTAs
 //   2  4096 points per CTA (one CTA up to 4096 points): the least SM time per attempt
 // One pulse, us per attempt (GB300, 2 W, 30 um poling), at spread 2 -> 1 -> 0:
-//   4096: 6.4 -> 5.2 -> 4.6   8192: 10.7 -> 7.0 -> 5.6   16384: 11.4 -> 7.7 -> 7.0
-// SM time per attempt goes the other way (4096: 6.4, 21, 37 SM us), so the wider
+//   2048: 4.2 -> 4.2 -> 3.3    4096: 6.5 -> 4.2 -> 3.5    8192: 9.4 -> 6.1 -> 4.4
+//   16384: 9.8 -> 5.9 -> 5.0   32768: 10.5 -> 10.5 -> (2048 points per CTA)
+// SM time per attempt goes the other way (4096: 6.5, 17, 28 SM us), so the wider
 // spreads serve calls that leave SMs idle otherwise.
 int spread_points(int N, int spread) {
     const int narrow = N <= 4096 ? N : 4096;
-    if (N <= 2048 || N > 32768 || spread >= 2) return narrow;
-    const int wide = N == 4096 ? 512 : N == 32768 ? 2048 : 1024;
+    if (N <= 1024 || N > 32768 || spread >= 2) return narrow;
+    const int wide = N <= 4096 ? 512 : N == 32768 ? 2048 : 1024;
     return spread == 0 ? wide : (2 * wide < narrow ? 2 * wide : narrow);
 }
 

@@ -17,6 +17,7 @@ void register_kernels_heun_nee(std::vector<KernelEntry>& v) {
     v.push_back(kernel_entry<1024, 16, kHeunNee>(true));
     v.push_back(kernel_entry<512, 1, kHeunNee>());
     v.push_back(kernel_entry<512, 2, kHeunNee>());
+    v.push_back(kernel_entry<512, 4, kHeunNee>(true));
     v.push_back(kernel_entry<512, 8, kHeunNee>(true));
 }
 }  // namespace ofx

@@ -16,6 +16,7 @@ void register_kernels_rk23(std::vector<KernelEntry>& v) {
     v.push_back(kernel_entry<1024, 16, OPTIFAX_RK23>(true));
     v.push_back(kernel_entry<512, 1, OPTIFAX_RK23>());
     v.push_back(kernel_entry<512, 2, OPTIFAX_RK23>());
+    v.push_back(kernel_entry<512, 4, OPTIFAX_RK23>(true));
     v.push_back(kernel_entry<512, 8, OPTIFAX_RK23>(true));
 }
 }  // namespace ofx

@@ -2,9 +2,13 @@
 //
 // One thread-block cluster of C CTAs propagates one pulse of N = C * M points
 // through the whole crystal in a single launch.  CTA rank c holds time points
-// [c M, (c+1) M) for the nonlinear sub-steps and, after the forward
-// transform, the spectral modes k = c + C k2 (k2 = 0..M-1).  Thread t owns
-// time points P t .. P t + P-1 of its CTA (held in registers across steps) and
+// n1 M + n2, n1 < C, for the M/C values n2 of its columns [c M/C, (c+1) M/C): C
+// segments of M/C consecutive points.  So the C-point DFTs over n1, the first step of
+// the four-step transform, are local, the inverse ends where the next step begins, and
+// only the two middle exchanges of a transform pair cross the cluster; the stencil pays
+// for it with a halo at both ends of every segment.  After the forward transform the
+// CTA holds the spectral modes k = c + C k2 (k2 = 0..M-1).  Thread t owns P consecutive
+// time points, the local ones P t .. P t + P-1 (held in registers across steps), and
 // spectral slots P t .. P t + P-1 (mode k2 = bitrev(slot)).
 //
 // Per step attempt (reference: OPO_CUDA_BATCH_XTAL.cu:432-506, Heun;
@@ -225,9 +229,9 @@ __device__ __forceinline__ float rcp_fast(float x) {
 // goes through the exact classes, so every decision is theirs.  The exact class's IEEE
 // square root costs more than the rest of a point's stage arithmetic.
 struct Bounds {
-    float scale, maxE, minE, qhi, qlo0, qlo1;
-    __device__ Bounds(float sc, float hi, float lo) : scale(sc), maxE(hi), minE(lo) {
-        const float is2 = 1.f / (sc * sc), l = lo > 0.f ? lo * lo * is2 : -1.f;
+    float qhi, qlo0, qlo1;
+    __device__ Bounds(float scale, float hi, float lo) {
+        const float is2 = 1.f / (scale * scale), l = lo > 0.f ? lo * lo * is2 : -1.f;
         qhi = hi > 0.f && lo > 0.f ? hi * hi * is2 * (1.f - 1e-5f) : -1.f;      // -1: always the exact classes
         qlo0 = l * (1.f - 1e-5f);
         qlo1 = l * (1.f + 1e-5f);
@@ -235,7 +239,8 @@ struct Bounds {
 };
 
 template <int H, bool NEE>
-__device__ __forceinline__ int classify_all(const Bounds& B, const Pair (&d)[H], const Pair (&e)[H]) {
+__device__ __forceinline__ int classify_all(const Bounds& B, const PulseDev& P, float scale, const Pair (&d)[H],
+                                            const Pair (&e)[H]) {
     float qmax = 0.f, emin = 3e38f;
     float2 sum = dup2(0.f);
 #pragma unroll
@@ -253,12 +258,13 @@ __device__ __forceinline__ int classify_all(const Bounds& B, const Pair (&d)[H],
     const bool low = qmax < B.qlo0, high = qmax > B.qlo1;
     if (s < 1e30f && qmax < B.qhi && (low || (high && (NEE || emin > 1e-30f)))) return high ? 2 : 0;
     int bits = 0;
+    const float maxE = P.max_err, minE = P.min_err;
 #pragma unroll
     for (int j = 0; j < H; ++j) {
         const float2 d0 = make_float2(d[j].re.x, d[j].im.x), d1 = make_float2(d[j].re.y, d[j].im.y);
         const float2 e0 = make_float2(e[j].re.x, e[j].im.x), e1 = make_float2(e[j].re.y, e[j].im.y);
-        bits |= NEE ? classify_nee(B.scale, d0, e0, B.maxE, B.minE) : classify(B.scale, d0, e0, B.maxE, B.minE);
-        bits |= NEE ? classify_nee(B.scale, d1, e1, B.maxE, B.minE) : classify(B.scale, d1, e1, B.maxE, B.minE);
+        bits |= NEE ? classify_nee(scale, d0, e0, maxE, minE) : classify(scale, d0, e0, maxE, minE);
+        bits |= NEE ? classify_nee(scale, d1, e1, maxE, minE) : classify(scale, d1, e1, maxE, minE);
     }
     return bits;
 }
@@ -326,14 +332,32 @@ __device__ __forceinline__ void zphases(uint64_t tau_z4, int t, float p0, float 
 template <int M>
 constexpr int kPoints = (M >= 2048) ? 8 : 4;
 
-// Cluster exchange: CTA c takes the n2 columns [c M/C, (c+1) M/C) of the C blocks, PER
-// consecutive columns to each of XT threads.
+// Cluster exchange: CTA c holds the n2 columns [c M/C, (c+1) M/C) of the C blocks.
+// A thread takes PER consecutive columns whole, or, where there are fewer columns than
+// threads (SPLIT), LANES consecutive lanes share a column: P values each, the C-point DFT as P-point DFTs in registers and a LANES-point one by
+// shuffles.  (16 CTAs of 1024 points: two warps with 16 values a thread took 800 and
+// 2190 cycles forward and inverse.)
 template <int M, int C>
 struct Xch {
-    static constexpr int T = M / kPoints<M>;
+    static constexpr int P = kPoints<M>, T = M / P;
     static constexpr int COLS = M / C;
-    static constexpr int XT = COLS < T ? COLS : T;
-    static constexpr int PER = COLS / XT;
+    static constexpr bool SPLIT = COLS < T;
+    static constexpr int LANES = SPLIT ? T / COLS : 1;
+    static constexpr int XT = T;                             // every thread takes part
+    static constexpr int PER = SPLIT ? 1 : COLS / T;
+    static constexpr int NV = SPLIT ? P : PER * (C - 1);     // outer twiddles per thread
+    // own parts of the exchange by plain stores and a block barrier (clusters of up to
+    // 4, where they are a quarter or more of it), else through the cluster as the others
+    static constexpr bool LOCAL = C <= 4;
+    static constexpr int SEGT = COLS / P;                    // threads of a segment
+};
+
+// What a pass counts and only its records or the end of a trip need: kept by thread 0 in
+// shared memory (the 4096-point kernels have 128 registers a thread, and spilled values
+// wait on L2 beside 200 KB of shared memory).
+struct RunState {
+    double tally[4], prev_tally;
+    int n_acc, n_rej, tot_att, tot_acc, tot_rej, steady, stop, slots;
 };
 
 template <int M, int METHOD, int C>
@@ -347,17 +371,24 @@ struct Smem {
     static constexpr size_t off_dm = off_g + (C > 1 ? sizeof(float2) * M : 0);       // per-mode D - 1
     static constexpr size_t off_tlo = off_dm + sizeof(float2) * M;                   // phase rates, low words
     static constexpr size_t off_abc = off_tlo + sizeof(uint32_t) * M;
-    static constexpr size_t off_tw = off_abc + sizeof(float) * M;
+    // absorber factors of the threads that have one (a quarter of them: the absorber spans
+    // [6/16, 10/16] of the window in every variant), P each
+    static constexpr size_t off_tw = off_abc + sizeof(float) * P * (T / 4 + 2);
     static constexpr size_t off_td = (off_tw + sizeof(float2) * F::TW + 15) & ~size_t(15);
-    // exchange twiddles W_N^{n2 k1} and their d: [u (C-1) + r - 1][XT]
+    // exchange twiddles W_N^{n2 k1} and their d: [value][XT]
     static constexpr size_t off_xtw = (off_td + sizeof(float) * F::TD + 15) & ~size_t(15);
-    static constexpr size_t off_xtd = off_xtw + (C > 1 ? sizeof(float2) * XC::PER * (C - 1) * XC::XT : 0);
-    static constexpr size_t off_edge = (off_xtd + (C > 1 ? sizeof(float) * XC::PER * (C - 1) * XC::XT : 0) + 15) & ~size_t(15);
+    static constexpr size_t off_xtd = off_xtw + (C > 1 ? sizeof(float2) * XC::NV * XC::XT : 0);
+    static constexpr size_t off_edge = (off_xtd + (C > 1 ? sizeof(float) * XC::NV * XC::XT : 0) + 15) & ~size_t(15);
     static constexpr size_t off_halo = off_edge + sizeof(float2) * 4 * NW;           // [parity][first, last][warp]
-    static constexpr size_t off_red = off_halo + sizeof(float2) * 8;                 // E and increment of 4 halo points
+    // Heun: E and increment of the 4 halo points of every segment; RK23: the neighbours'
+    // end values [parity][segment][left, right]
+    // and, for a segment's two end threads, the field and the carrier of their halo points
+    static constexpr size_t off_bar = off_halo + (C > 1 ? sizeof(float2) * (8 + 8) * C : 0);
+    static constexpr size_t off_red = off_bar + sizeof(uint64_t) * 6;
     static constexpr size_t off_dred = off_red + sizeof(int) * (2 * NW + 2 * 16 + 4);
-    static constexpr size_t bytes = ((off_dred + 15) & ~size_t(15)) + sizeof(double) * (NW * 4 + 2 * 16 * 4);
-    static_assert(bytes <= 232448 - 512, "shared memory of one CTA");
+    static constexpr size_t off_run = ((off_dred + 15) & ~size_t(15)) + sizeof(double) * (NW * 4 + 2 * 16 * 4);
+    static constexpr size_t bytes = off_run + sizeof(RunState);
+    static_assert(bytes <= 232448 - 288, "shared memory of one CTA");
 };
 
 // ---------------------------------------------------------------------------
@@ -386,34 +417,69 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void st_cluster_f2(uint32_t addr, float2 v) {
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
+// ---------------------------------------------------------------------------
+// Stores into a peer's shared memory that count their bytes on the peer's mbarrier
+// (st.async): the receiver waits for exactly the bytes of one step of the exchange, with
+// no fence and no cluster-wide barrier.  (32 KB all-to-all over 16 CTAs: 2370 cycles,
+// against 3320 for plain remote stores and a cluster barrier; 4 KB over 8: 760, 1165.)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void st_async(uint32_t addr, float2 v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr),
+                 "f"(v.x), "f"(v.y), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void st_cluster_f4(uint32_t addr, float2 v, float2 w) {
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(w.x), "f"(w.y)
-                 : "memory");
+__device__ __forceinline__ void st_async(uint32_t addr, float2 v, float2 w, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                     addr), "f"(v.x), "f"(v.y), "f"(w.x), "f"(w.y), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void st_cluster_i32(uint32_t addr, int v) {
-    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+__device__ __forceinline__ void st_async(uint32_t addr, int v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.s32 [%0], %1, [%2];" ::"r"(addr), "r"(v),
+                 "r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_init(uint32_t bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+// the one arrival of a phase, with the bytes that complete it
+__device__ __forceinline__ void bar_arm(uint32_t bar, int bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                 " selp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done != 0;
+}
+// Bounded wait (about 2 s); after a wait that ran out the CTA's flag makes every later
+// one return at once, and the pass ends at its next block barrier.
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, volatile int* dead) {
+    if (bar_try(bar, parity)) return;
+    const long long t0 = clock64();
+    while (!bar_try(bar, parity)) {
+        if (*dead) return;
+        if (clock64() - t0 > 4000000000LL) {
+            *dead = 1;
+            return;
+        }
+    }
 }
 
 // The neighbours' adjacent drive values: shuffles inside a warp, one shared-memory slot
-// per warp edge.  REMOTE: the CTA's own ends come from the neighbouring CTAs (clusters),
-// else they wrap around (one CTA) or are replaced by the caller.
-template <int M, int C, bool REMOTE>
-__device__ __forceinline__ void exchange_edges(float2* edge, int& par, int t, int c, float2 first, float2 last,
-                                               float2& left, float2& right) {
+// per warp edge where a segment is longer than a warp's points.  The ends of a segment
+// wrap around (one CTA) or are replaced by the caller.
+template <int M, int C>
+__device__ __forceinline__ void exchange_edges(float2* edge, int& par, int t, float2 first, float2 last, float2& left,
+                                               float2& right) {
     constexpr int NW = M / kPoints<M> / 32;
     const int w = t >> 5, lane = t & 31;
-    float2* e = edge + par * 2 * NW;
-    if (lane == 0) e[w] = first;
-    if (lane == 31) e[NW + w] = last;
     left = make_float2(__shfl_up_sync(0xffffffffu, last.x, 1), __shfl_up_sync(0xffffffffu, last.y, 1));
     right = make_float2(__shfl_down_sync(0xffffffffu, first.x, 1), __shfl_down_sync(0xffffffffu, first.y, 1));
-    if constexpr (REMOTE && C > 1) csync<C>();
-    else __syncthreads();
-    if (lane == 0) left = (w > 0) ? e[NW + w - 1] : ((REMOTE ? remote<C>(e, (c + C - 1) % C) : e)[2 * NW - 1]);
-    if (lane == 31) right = (w < NW - 1) ? e[w + 1] : ((REMOTE ? remote<C>(e, (c + 1) % C) : e)[0]);
+    if constexpr (Xch<M, C>::SEGT > 32) {
+        float2* e = edge + par * 2 * NW;
+        if (lane == 0) e[w] = first;
+        if (lane == 31) e[NW + w] = last;
+        __syncthreads();
+        if (lane == 0) left = e[NW + (w > 0 ? w - 1 : NW - 1)];
+        if (lane == 31) right = e[w < NW - 1 ? w + 1 : 0];
+    }
     par ^= 1;
 }
 
@@ -429,108 +495,217 @@ __device__ __forceinline__ float2 twn_val(const Twiddle* quad, const Twiddle* lo
     return cmul(make_float2(a.c, a.s), make_float2(b.c, b.s));
 }
 
-// Four-step split of the N = C M transform across a cluster, all of it through
-// distributed shared memory.  Every value is pushed into the shared memory of the CTA
-// that uses it next, so that each of the four steps of an accepted step is one wave of
-// remote stores and one cluster barrier, and no transfer waits on L2:
-//   push_columns   own time points -> the owners of their n2 columns (buffer g)
-//   exchange_fwd   C-point DFTs of the own columns, twiddle -> the blocks' owners (x)
-//   (local transforms, dispersion; the last inverse pass pushes into the columns' g)
-//   exchange_inv   inverse twiddle and C-point DFTs, 1/N -> the blocks' owners (x)
-// Ordering comes from the cluster barriers between the steps: a buffer is written only
-// after the barrier that follows its last read.
-template <int M, int C>
-__device__ __forceinline__ void push_columns(uint32_t g, const float2 (&v)[kPoints<M>], int t, int c) {
-    using XC = Xch<M, C>;
-    constexpr int P = kPoints<M>;
-    static_assert(XC::COLS % P == 0, "a thread's points belong to one column owner");
-    const uint32_t dst = cluster_addr(g, (P * t) / XC::COLS);
-    const int s0 = swz(c * XC::COLS + (P * t) % XC::COLS);
-#pragma unroll
-    for (int j = 0; j < P; j += 2) st_cluster_f4(dst + 8 * (s0 ^ j), v[j], v[j + 1]);
-}
-
+// Four-step split of the N = C M transform across a cluster through distributed shared
+// memory.  Every value is pushed into the shared memory of the CTA that uses it next;
+// each step has one mbarrier per CTA that counts the bytes the CTA gets in it:
+//   A  the error flags and the halo points' E
+//   B  exchange_fwd  C-point DFTs of the own columns (buffer g), twiddle -> the blocks' owners (x)
+//   C  push_inverse  the last inverse pass's outputs -> the columns' owners (g)
+//   D  exchange_inv  inverse twiddle and C-point DFTs, 1/N -> own points (x); the halo
+//                    points' increments
+// No buffer is written before its last read: what a CTA sends in a step carries what all
+// of its threads read before (every thread adds to every peer's bytes of A, through the
+// flags behind a block barrier, and of C; every reader of g to those of B).
 // Store `v` (PER consecutive columns n2 of block k) into the FFT buffer of CTA k
-template <int PER>
-__device__ __forceinline__ void push_block(uint32_t x, int k, int n2, const float2 (&v)[PER]) {
-    const uint32_t dst = cluster_addr(x, k);
+template <int PER, bool LOCAL>
+__device__ __forceinline__ void push_block(float2* bufx, uint32_t x, uint32_t bar, int k, int n2, const float2 (&v)[PER],
+                                           int c) {
     const int s0 = swz(n2);
+    if (LOCAL && k == c) {
+#pragma unroll
+        for (int u = 0; u < PER; ++u) bufx[s0 ^ u] = v[u];
+        return;
+    }
+    const uint32_t dst = cluster_addr(x, k), db = dst + (bar - x);
     if constexpr (PER == 1) {
-        st_cluster_f2(dst + 8 * s0, v[0]);
+        st_async(dst + 8 * s0, v[0], db);
     } else {
 #pragma unroll
-        for (int u = 0; u < PER; u += 2) st_cluster_f4(dst + 8 * (s0 ^ u), v[u], v[u + 1]);
+        for (int u = 0; u < PER; u += 2) st_async(dst + 8 * (s0 ^ u), v[u], v[u + 1], db);
     }
 }
 
-template <int M, int C>
-__device__ __forceinline__ void load_columns(const float2* g, int t, float2 (&v)[Xch<M, C>::PER][C]) {
-    using XC = Xch<M, C>;
-#pragma unroll
-    for (int n1 = 0; n1 < C; ++n1) {
-        const int s0 = swz(n1 * XC::COLS + t * XC::PER);
-#pragma unroll
-        for (int u = 0; u < XC::PER; ++u) v[u][n1] = g[s0 ^ u];
-    }
+__device__ __forceinline__ float2 shfl_xor2(float2 v, int m) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
 }
-
-template <int M, int C>
-__device__ __forceinline__ void exchange_fwd(const float2* g, uint32_t x, const float2* xtw, int t, int c) {
-    using XC = Xch<M, C>;
-    if (t >= XC::XT) return;
-    float2 v[XC::PER][C];
-    load_columns<M, C>(g, t, v);
-    const int n2 = c * XC::COLS + t * XC::PER;
+// LANES-point DFT across the lanes of a column (lane l ends with output bitrev(l)), and
+// its exact reverse; one packed add or subtract per butterfly side.
+template <int LANES, int NV>
+__device__ __forceinline__ void lanes_fwd(float2 (&v)[NV], int l) {
 #pragma unroll
-    for (int u = 0; u < XC::PER; ++u) {
-        dftp<C>(v[u]);
+    for (int hr = LANES / 2; hr >= 1; hr >>= 1) {
+        const bool up = (l & hr) != 0;
+        const bool turn = LANES == 4 && hr == 2 && (l & 1);
 #pragma unroll
-        for (int r = 1; r < C; ++r) v[u][r] = cmul(v[u][r], xtw[(u * (C - 1) + r - 1) * XC::XT + t]);
-    }
-#pragma unroll
-    for (int r = 0; r < C; ++r) {
-        float2 o[XC::PER];
-#pragma unroll
-        for (int u = 0; u < XC::PER; ++u) o[u] = v[u][r];
-        push_block<XC::PER>(x, brev4(r, ilog2(C)), n2, o);
-    }
-}
-
-// g holds the inverse-transformed blocks' columns at [k1 COLS + column].  Block-edge
-// increments also go to the neighbouring CTAs' halo slots: halo[0..1] hold the points
-// -2, -1 and halo[2..3] the points M, M + 1 of the owner.
-template <int M, int C, bool HALO>
-__device__ __forceinline__ void exchange_inv(const float2* g, uint32_t x, uint32_t halo, const float2* xtw,
-                                             const float* xtd, int t, int c, float invN) {
-    using XC = Xch<M, C>;
-    if (t >= XC::XT) return;
-    float2 v[XC::PER][C];
-    load_columns<M, C>(g, t, v);
-    const int n2 = c * XC::COLS + t * XC::PER;
-#pragma unroll
-    for (int u = 0; u < XC::PER; ++u) {
-        float2 w[C];
-        w[0] = v[u][0];
-#pragma unroll
-        for (int r = 1; r < C; ++r) {                   // register r of the inverse DFT holds k1 = bitrev(r)
-            const int i = (u * (C - 1) + r - 1) * XC::XT + t;
-            w[r] = mul_recip(v[u][brev4(r, ilog2(C))], xtw[i], xtd[i]);
+        for (int i = 0; i < NV; ++i) {
+            const float2 o = shfl_xor2(v[i], hr);
+            float2 d = up ? sub2(o, v[i]) : add2(v[i], o);
+            if (up && turn) d = make_float2(d.y, -d.x);
+            v[i] = d;
         }
-        dftp_inv<C>(w);
-#pragma unroll
-        for (int n1 = 0; n1 < C; ++n1) v[u][n1] = mul2(w[n1], dup2(invN));
     }
+}
+template <int LANES, int NV>
+__device__ __forceinline__ void lanes_inv(float2 (&v)[NV], int l) {
 #pragma unroll
-    for (int n1 = 0; n1 < C; ++n1) {
-        float2 o[XC::PER];
+    for (int hr = 1; hr <= LANES / 2; hr <<= 1) {
+        const bool up = (l & hr) != 0;
+        const bool turn = LANES == 4 && hr == 2 && (l & 1);
 #pragma unroll
-        for (int u = 0; u < XC::PER; ++u) o[u] = v[u][n1];
-        push_block<XC::PER>(x, n1, n2, o);
-        if constexpr (HALO) {
+        for (int i = 0; i < NV; ++i) {
+            if (up && turn) v[i] = make_float2(-v[i].y, v[i].x);
+            const float2 o = shfl_xor2(v[i], hr);
+            v[i] = up ? sub2(o, v[i]) : add2(v[i], o);
+        }
+    }
+}
+
+// Inner twiddles W_C^{j ka} of a lane's values (SPLIT), with their reciprocals' d
+template <int M, int C>
+struct Inner {
+    float2 w[Xch<M, C>::SPLIT ? kPoints<M> : 1];
+    float d[Xch<M, C>::SPLIT ? kPoints<M> : 1];
+    __device__ __forceinline__ void fill(const Twiddle* quad, int t) {
+        if constexpr (Xch<M, C>::SPLIT) {
+            constexpr int P = kPoints<M>;
+#pragma unroll
+            for (int r = 0; r < P; ++r) {
+                const Twiddle a = quad_tw<M>(quad, ((t % Xch<M, C>::LANES) * brev4(r, ilog2(P))) * (M / C) % M);
+                w[r] = make_float2(a.c, a.s);
+                d[r] = a.d;
+            }
+        }
+    }
+};
+
+// k1 of outer twiddle i of thread t (register i of the forward DFT)
+template <int M, int C>
+__device__ __forceinline__ int outer_k1(int i, int t) {
+    using XC = Xch<M, C>;
+    if constexpr (XC::SPLIT) return brev4(i, ilog2(XC::P)) + XC::P * brev4(t % XC::LANES, ilog2(XC::LANES));
+    else return brev4(i % (C - 1) + 1, ilog2(C));
+}
+
+template <int M, int C>
+__device__ __forceinline__ void exchange_fwd(const float2* g, float2* bufx, uint32_t x, uint32_t bar, const float2* xtw,
+                                             const Inner<M, C>& in, int t, int c) {
+    using XC = Xch<M, C>;
+    if (t >= XC::XT) return;
+    if constexpr (XC::SPLIT) {
+        constexpr int P = XC::P;
+        const int l = t % XC::LANES, col = t / XC::LANES;
+        float2 v[P];
+#pragma unroll
+        for (int i = 0; i < P; ++i) v[i] = g[swz((i * XC::LANES + l) * XC::COLS + col)];
+        dftp<P>(v);
+#pragma unroll
+        for (int r = 1; r < P; ++r) v[r] = cmul(v[r], in.w[r]);
+        lanes_fwd<XC::LANES, P>(v, l);
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+            const float2 o[1] = {cmul(v[r], xtw[r * XC::XT + t])};
+            push_block<1, XC::LOCAL>(bufx, x, bar, outer_k1<M, C>(r, t), c * XC::COLS + col, o, c);
+        }
+    } else {
+        float2 v[XC::PER][C];
+        const int n2 = c * XC::COLS + t * XC::PER;
+#pragma unroll
+        for (int n1 = 0; n1 < C; ++n1) {
+            const int s0 = swz(n1 * XC::COLS + t * XC::PER);
+#pragma unroll
+            for (int u = 0; u < XC::PER; ++u) v[u][n1] = g[s0 ^ u];
+        }
+#pragma unroll
+        for (int u = 0; u < XC::PER; ++u) {
+            dftp<C>(v[u]);
+#pragma unroll
+            for (int r = 1; r < C; ++r) v[u][r] = cmul(v[u][r], xtw[(u * (C - 1) + r - 1) * XC::XT + t]);
+        }
+#pragma unroll
+        for (int r = 0; r < C; ++r) {
+            float2 o[XC::PER];
+#pragma unroll
+            for (int u = 0; u < XC::PER; ++u) o[u] = v[u][r];
+            push_block<XC::PER, XC::LOCAL>(bufx, x, bar, brev4(r, ilog2(C)), n2, o, c);
+        }
+    }
+}
+
+// The segments next to segment `seg` of CTA c: their CTA, and their index there
+template <int C>
+__device__ __forceinline__ int seg_left(int seg, int c) { return c > 0 ? seg : (seg + C - 1) % C; }
+template <int C>
+__device__ __forceinline__ int seg_right(int seg, int c) { return c < C - 1 ? seg : (seg + 1) % C; }
+
+// Increment of one of a segment's first or last two points for the neighbour's halo:
+// halo[4 seg + 0..1] hold the points -2, -1 and halo[4 seg + 2..3] the points COLS,
+// COLS + 1 of segment seg.
+template <int M, int C>
+__device__ __forceinline__ void push_halo(uint32_t halo, uint32_t bar, int seg, int col, float2 v, int c) {
+    constexpr int COLS = Xch<M, C>::COLS;
+    if (col >= 2 && col < COLS - 2) return;
+    const bool first = col < 2;
+    const uint32_t dst = cluster_addr(halo, first ? (c + C - 1) % C : (c + 1) % C);
+    const int slot = first ? 4 * seg_left<C>(seg, c) + 2 + col : 4 * seg_right<C>(seg, c) + col - (COLS - 2);
+    st_async(dst + 8 * slot, v, dst + (bar - halo));
+}
+
+template <int M, int C, bool HALO>
+__device__ __forceinline__ void exchange_inv(const float2* g, float2* bufx, uint32_t halo, uint32_t bar, const float2* xtw,
+                                             const float* xtd, const Inner<M, C>& in, int t, int c, float invN) {
+    using XC = Xch<M, C>;
+    if (t >= XC::XT) return;
+    if constexpr (XC::SPLIT) {
+        constexpr int P = XC::P;
+        const int l = t % XC::LANES, col = t / XC::LANES;
+        float2 v[P];
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+            v[r] = g[swz(outer_k1<M, C>(r, t) * XC::COLS + col)];
+            v[r] = mul_recip(v[r], xtw[r * XC::XT + t], xtd[r * XC::XT + t]);
+        }
+        lanes_inv<XC::LANES, P>(v, l);
+#pragma unroll
+        for (int r = 1; r < P; ++r) v[r] = mul_recip(v[r], in.w[r], in.d[r]);
+        dftp_inv<P>(v);
+        const bool ends = HALO && (col < 2 || col >= XC::COLS - 2);
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+            const int n1 = i * XC::LANES + l;
+            v[i] = mul2(v[i], dup2(invN));
+            bufx[swz(n1 * XC::COLS + col)] = v[i];
+            if (ends) push_halo<M, C>(halo, bar, n1, col, v[i], c);
+        }
+    } else {
+        float2 v[XC::PER][C];
+        const int col = t * XC::PER;
+#pragma unroll
+        for (int n1 = 0; n1 < C; ++n1) {
+            const int s0 = swz(n1 * XC::COLS + col);
+#pragma unroll
+            for (int u = 0; u < XC::PER; ++u) v[u][n1] = g[s0 ^ u];
+        }
+#pragma unroll
+        for (int u = 0; u < XC::PER; ++u) {
+            float2 w[C];
+            w[0] = v[u][0];
+#pragma unroll
+            for (int r = 1; r < C; ++r) {               // register r of the inverse DFT holds k1 = bitrev(r)
+                const int i = (u * (C - 1) + r - 1) * XC::XT + t;
+                w[r] = mul_recip(v[u][brev4(r, ilog2(C))], xtw[i], xtd[i]);
+            }
+            dftp_inv<C>(w);
+#pragma unroll
+            for (int n1 = 0; n1 < C; ++n1) v[u][n1] = mul2(w[n1], dup2(invN));
+        }
+        const bool ends = HALO && (col < 2 || col + XC::PER > XC::COLS - 2);
+#pragma unroll
+        for (int n1 = 0; n1 < C; ++n1) {
+            const int s0 = swz(n1 * XC::COLS + col);
 #pragma unroll
             for (int u = 0; u < XC::PER; ++u) {
-                if (n2 + u < 2) st_cluster_f2(cluster_addr(halo, (n1 + C - 1) % C) + 8 * (2 + n2 + u), o[u]);
-                if (n2 + u >= M - 2) st_cluster_f2(cluster_addr(halo, (n1 + 1) % C) + 8 * (n2 + u - (M - 2)), o[u]);
+                bufx[s0 ^ u] = v[u][n1];
+                if (ends) push_halo<M, C>(halo, bar, n1, col + u, v[u][n1], c);
             }
         }
     }
@@ -539,21 +714,33 @@ __device__ __forceinline__ void exchange_inv(const float2* g, uint32_t x, uint32
 // The last inverse pass's outputs (points t + q M/P of this CTA's block) into the g
 // buffers of their columns' owners.
 template <int M, int C>
-__device__ __forceinline__ void push_inverse(uint32_t g, const float2 (&v)[kPoints<M>], int t, int c) {
+__device__ __forceinline__ void push_inverse(float2* bufg, uint32_t g, uint32_t bar, const float2 (&v)[kPoints<M>], int t,
+                                             int c) {
     using XC = Xch<M, C>;
     constexpr int P = kPoints<M>;
+    // with more CTAs than points a thread does not add to every peer's bytes, which then
+    // say nothing about its reads of the FFT buffer
+    if constexpr (C > P) __syncthreads();
 #pragma unroll
     for (int q = 0; q < P; ++q) {
-        const int m = t + q * (M / P);
-        st_cluster_f2(cluster_addr(g, m / XC::COLS) + 8 * swz(c * XC::COLS + m % XC::COLS), v[q]);
+        const int m = t + q * (M / P), r = m / XC::COLS, i = swz(c * XC::COLS + m % XC::COLS);
+        if (XC::LOCAL && r == c) {
+            bufg[i] = v[q];
+        } else {
+            const uint32_t dst = cluster_addr(g, r);
+            st_async(dst + 8 * i, v[q], dst + (bar - g));
+        }
     }
 }
 
 // OR of the error flags over the pulse: one slot per warp, then (clusters) one per CTA.
 // Double buffered by attempt.  The barrier inside also publishes what the threads
 // stored before it (stage output, pushed columns).
+constexpr int kDead = 8;          // a bounded wait ran out
+
 template <int M, int C>
-__device__ __forceinline__ int combine_flags(int bits, int* red, int attempt, int t, int c, const KernelCfg& cfg) {
+__device__ __forceinline__ int combine_flags(int bits, int* red, uint32_t bar, uint32_t parity, int bytes, int* dead,
+                                             int attempt, int t, int c, const KernelCfg& cfg) {
     constexpr int NW = M / kPoints<M> / 32;
     const int par = attempt & 1;
     int* wf = red + par * NW;
@@ -572,12 +759,18 @@ __device__ __forceinline__ int combine_flags(int bits, int* red, int attempt, in
         for (int i = 0; i < NW; ++i) f |= wf[i];
     }
     if constexpr (C > 1) {
+        const int lost = *(volatile int*)dead;       // written before the barrier: the same for every thread
         int* cl = red + 2 * NW + par * 16;
-        if (t < C) st_cluster_i32(cluster_addr(smem_u32(cl + c), t), f);
-        cg::this_cluster().sync();
-        f = 0;
+        if (t < C && t != c) {
+            const uint32_t src = smem_u32(cl + c), dst = cluster_addr(src, t);
+            st_async(dst, f, dst + (bar - src));
+        }
+        bar_wait(bar, parity, dead);
+        if (t == 0) bar_arm(bar, bytes);
 #pragma unroll
-        for (int r = 0; r < C; ++r) f |= cl[r];
+        for (int r = 0; r < C; ++r)
+            if (r != c) f |= cl[r];
+        f = lost ? kDead : (f & 7);
     }
     if (cfg.shared_sched) {
         const int gslot = attempt % 3;
@@ -695,10 +888,13 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     float2* xtw_s = reinterpret_cast<float2*>(smem + SM::off_xtw);
     float* xtd_s = reinterpret_cast<float*>(smem + SM::off_xtd);
     float2* edge = reinterpret_cast<float2*>(smem + SM::off_edge);
-    float2* halo_e = reinterpret_cast<float2*>(smem + SM::off_halo);      // E of points -2, -1, M, M + 1
-    float2* halo_d = halo_e + 4;                                          // their increments
+    float2* halo_e = reinterpret_cast<float2*>(smem + SM::off_halo);      // E of every segment's halo points
+    float2* halo_d = halo_e + 4 * C;                                      // their increments
+    float2* ends = halo_e;                                                // RK23: [parity][segment][left, right]
     int* red = reinterpret_cast<int*>(smem + SM::off_red);
+    int* dead = red + 2 * SM::NW + 2 * 16;
     double* dred = reinterpret_cast<double*>(smem + ((SM::off_dred + 15) & ~size_t(15)));
+    RunState* run = reinterpret_cast<RunState*>(smem + SM::off_run);
 
     const int t = threadIdx.x;
     const int c = (C > 1) ? (int)cg::this_cluster().block_rank() : 0;
@@ -707,7 +903,10 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     // those reads off the global path (and out of reach of aliasing with the
     // kernel's global stores).
     __shared__ PulseDev sP;
-    if (t == 0) sP = pulses[p];
+    if (t == 0) {
+        sP = pulses[p];
+        *run = RunState{};
+    }
     __syncthreads();
     const PulseDev& P_ = sP;
 
@@ -717,39 +916,65 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
         using XC = Xch<M, C>;
         if (t < XC::XT) {
 #pragma unroll 1
-            for (int u = 0; u < XC::PER; ++u)
-#pragma unroll 1
-                for (int r = 1; r < C; ++r) {
-                    const float2 w = twn_val<M, C>(tabs.quad, tabs.low,
-                                                   (c * XC::COLS + t * XC::PER + u) * bitrev(r, ilog2(C)));
-                    const int i = (u * (C - 1) + r - 1) * XC::XT + t;
-                    xtw_s[i] = w;
-                    xtd_s[i] = inv_norm2_m1(w);
-                }
+            for (int i = 0; i < XC::NV; ++i) {
+                const int n2 = c * XC::COLS + (XC::SPLIT ? t / XC::LANES : t * XC::PER + i / (C - 1));
+                const float2 w = twn_val<M, C>(tabs.quad, tabs.low, n2 * outer_k1<M, C>(i, t));
+                xtw_s[i * XC::XT + t] = w;
+                xtd_s[i * XC::XT + t] = inv_norm2_m1(w);
+            }
         }
     }
+    Inner<M, C> inner;
+    if constexpr (C > 1) inner.fill(tabs.quad, t);
+    // barriers of the exchange steps A to D, and of RK23's end values [parity]; bytes that
+    // a CTA gets in each
+    using XC_ = Xch<M, C>;
+    constexpr int kAll = 8 * (XC_::LOCAL ? M - XC_::COLS : M);
+    constexpr int kBytesA = 4 * (C - 1) + (HALO ? 32 * C : 0), kBytesD = 32 * C, kBytesE = 16 * C;
+    const uint32_t bars = smem_u32(smem + SM::off_bar);
+    const uint32_t bar_a = bars, bar_b = bars + 8, bar_c = bars + 16, bar_d = bars + 24, bar_e = bars + 32;
+    if (C > 1 && t == 0) {
+        *dead = 0;
+        for (int i = 0; i < 6; ++i) bar_init(bars + 8 * i);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        bar_arm(bar_a, kBytesA);
+        bar_arm(bar_b, kAll);
+        bar_arm(bar_c, kAll);
+        bar_arm(bar_d, kBytesD);
+        bar_arm(bar_e, kBytesE);
+        bar_arm(bar_e + 8, kBytesE);
+    }
+    uint32_t ph_a = 0, ph_x = 0, ph_e = 0;        // phase parities: A, B to D, end values (bit per parity)
     // per-thread tables as vectors of four (or two) values: [j / 4][t][j % 4]
     auto at4 = [&](int j) { return ((j >> 2) * T + t) * 4 + (j & 3); };
     auto at2 = [&](int j) { return ((j >> 1) * T + t) * 2 + (j & 1); };
     auto carrier = [&](int i) { return turn_to_unit(P_.tau_theta * (uint64_t)time_index(i, N, cfg.time_mode)); };
+    // this thread's points: i0 .. i0 + P-1; its place in a segment
+    const int seg = t / XC_::SEGT, tin = t % XC_::SEGT;
+    const int i0 = seg * M + c * XC_::COLS + P * tin;
     Pair a[H], cph[H];
 #pragma unroll
     for (int j = 0; j < H; ++j) {
-        const int i = c * M + P * t + j;
+        const int i = i0 + j;
         const float2 c0 = carrier(i), c1 = carrier(i + H), e0 = P_.E_in[i], e1 = P_.E_in[i + H];
         cph[j] = Pair{make_float2(c0.x, c1.x), make_float2(c0.y, c1.y)};
         a[j] = Pair{make_float2(e0.x, e1.x), make_float2(e0.y, e1.y)};
-        abc_s[at4(j)] = abc_factor(i, N, cfg.abc_mode);
-        abc_s[at4(j + H)] = abc_factor(i + H, N, cfg.abc_mode);
     }
-    // end threads: the adjacent (h1) and the outer (h2) point beyond the block's end
-    const bool lend = HALO && t == 0, rend = HALO && t == T - 1;
-    float2 h1 = make_float2(0.f, 0.f), h2 = h1, hc1 = h1, hc2 = h1;
-    if (lend || rend) {
-        const int i1 = lend ? (c * M + N - 1) % N : (c * M + M) % N;
-        const int i2 = lend ? (c * M + N - 2) % N : (c * M + M + 1) % N;
-        h1 = P_.E_in[i1]; h2 = P_.E_in[i2];
-        hc1 = carrier(i1); hc2 = carrier(i2);
+    float* abc = nullptr;                    // this thread's absorber factors, where it has any
+    if (i0 + P > 6 * (N / 16) && i0 <= 10 * (N / 16) && cfg.abc_mode != ABC_NONE) {
+        abc = abc_s + P * atomicAdd(&run->slots, 1);
+#pragma unroll 1
+        for (int j = 0; j < P; ++j) abc[j] = abc_factor(i0 + j, N, cfg.abc_mode);
+    }
+    // a segment's end threads: the adjacent (h1) and the outer (h2) point beyond its end
+    const bool lend = C > 1 && tin == 0, rend = C > 1 && tin == XC_::SEGT - 1;
+    // (field and carrier of both in shared memory: hs[0..1] and hs[2..3])
+    float2* hs = halo_e + 8 * C + 4 * (2 * seg + (rend ? 1 : 0));
+    if (HALO && (lend || rend)) {
+        const int i1 = lend ? (i0 + N - 1) % N : (i0 + P) % N;
+        const int i2 = lend ? (i0 + N - 2) % N : (i0 + P + 1) % N;
+        hs[0] = P_.E_in[i1]; hs[1] = P_.E_in[i2];
+        hs[2] = carrier(i1); hs[3] = carrier(i2);
     }
 #pragma unroll 1
     for (int j = 0; j < P; ++j) {
@@ -759,19 +984,21 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     }
     if constexpr (C > 1) cg::this_cluster().sync(); else __syncthreads();
 
-    const float* G = P_.G;
-    const float h = P_.h, sel = P_.sel, cs = P_.c_shock, Sf = (float)P_.S;
+    // Values of the descriptor that every attempt uses: in registers, or read from shared
+    // memory at each use where registers are short (4096 points per CTA)
+    constexpr bool tight = T * 128 >= 65536;
+    struct Hot { float h, cs, sel, S; int nchunks; const float* G; bool cavity; };
+    auto load_hot = [&] { return Hot{P_.h, P_.c_shock, P_.sel, (float)P_.S, P_.nchunks, P_.G, P_.fb != nullptr}; };
+    const Hot hot_ = load_hot();
+    auto hot = [&]() -> Hot { if constexpr (tight) return load_hot(); else return hot_; };
+    const int max_attempts = cfg.max_attempts_mul * (P_.S + 16) + 64;
     const Bounds bounds(heun ? 50.f : 200.f, P_.max_err, P_.min_err);
     // what the caller asked for beyond the field, as one register (tested per attempt)
     constexpr int kForced = 1, kTrace = 2, kSteps = 4, kAp = 8;
     const int opts = (P_.forced && P_.n_forced > 0 ? kForced : 0) | (P_.trace ? kTrace : 0) |
                      (!nee && (P_.stepmods || P_.smt) ? kSteps : 0) | (P_.Ap ? kAp : 0);
-    const float invN = 1.0f / (float)N;
+    constexpr float invN = 1.0f / (float)N;
     const int guard = cfg.guard;
-    const long long max_attempts = (long long)cfg.max_attempts_mul * (long long)(P_.S + 16) + 64;
-    const int nchunks = P_.nchunks;
-    const float pass_end = (float)nchunks * sel;
-    const bool opo = P_.fb != nullptr;
     const int n_trips = P_.n_trips > 0 ? P_.n_trips : 1;
     const bool rec = (c == 0 && t == 0);
     const uint32_t x_addr = smem_u32(bufX), g_addr = smem_u32(bufG);
@@ -779,17 +1006,34 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     float k = nee ? 1.f : 0.f, stepprev = 4.f, stepmod = 4.f;
     unsigned q = 0;                          // accumulated dispersion position (sum of stepmod)
     int s_cached = -1;                       // stepmod of the cached per-mode D - 1
-    int attempt = 0, n_acc = 0, n_rej = 0, status = 0, par = 0, trip = 0, trips_done = 0;
-    int gatt = 0, tot_att = 0, tot_acc = 0, tot_rej = 0, steady_count = 0;
-    double prev_tally = 0.0;
+    int attempt = 0, status = 0, par = 0, trip = 0, trips_done = 0, gatt = 0;
 
     // neighbours' drive values at the thread's ends; hv: the halo point's drive (end threads)
     auto edges = [&](const Pair (&nl)[H], float2 hv, float2& L, float2& R) {
-        exchange_edges<M, C, !HALO>(edge, par, t, c, make_float2(nl[0].re.x, nl[0].im.x),
-                                    make_float2(nl[H - 1].re.y, nl[H - 1].im.y), L, R);
+        const float2 first = make_float2(nl[0].re.x, nl[0].im.x), last = make_float2(nl[H - 1].re.y, nl[H - 1].im.y);
+        const int ep = par;
+        if constexpr (C > 1 && !HALO) {
+            // own end values to the neighbours; a slot is used again two exchanges later,
+            // after its reader has sent its next values
+            if (lend || rend) {
+                const uint32_t src = smem_u32(ends + (ep * C + (lend ? seg_left<C>(seg, c) : seg_right<C>(seg, c))) * 2 +
+                                              (lend ? 1 : 0));
+                const uint32_t dst = cluster_addr(src, lend ? (c + C - 1) % C : (c + 1) % C);
+                st_async(dst, lend ? first : last, dst + (bar_e + 8 * ep - src));
+            }
+        }
+        exchange_edges<M, C>(edge, par, t, first, last, L, R);
         if constexpr (HALO) {
-            if (t == 0) L = hv;
-            if (t == T - 1) R = hv;
+            if (lend) L = hv;
+            if (rend) R = hv;
+        } else if constexpr (C > 1) {
+            if (lend || rend) {
+                const uint32_t b = bar_e + 8 * ep;
+                bar_wait(b, (ph_e >> ep) & 1, dead);
+                if (t == 0) bar_arm(b, kBytesE);
+                (lend ? L : R) = ends[(ep * C + seg) * 2 + (lend ? 0 : 1)];
+            }
+            ph_e ^= 1u << ep;
         }
     };
 
@@ -800,39 +1044,43 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     auto prepare = [&](float kp, float sm) {
         if constexpr (heun) zphases(P_.tau_z4, t, kp, kp + sm, 0.f, z0, z1, z2);
         else zphases(P_.tau_z4, t, kp + 0.5f * sm, kp + 0.75f * sm, kp + sm, z0, z1, z2);
-        gval = G[(int)kp];
+        gval = hot().G[(int)kp];
         zk = kp; zs = sm;
     };
 
     Pair k1r[H];      // RK23: K1 (first stage, FSAL) between attempts
     for (trip = 0; trip < n_trips; ++trip) {
         k = nee ? 1.f : 0.f; stepprev = 4.f; stepmod = 4.f; q = 0;
-        attempt = 0; n_acc = 0; n_rej = 0;
+        attempt = 0;
         int trip_status = 0;
-        double tally[4] = {0.0, 0.0, 0.0, 0.0};
         if constexpr (!heun) {
             // initial K1 at k = 0 with stepmod = 4 (OPO_CUDA_ODE23.cu:432-438)
-            const float hg = (stepmod * h) * G[0];
+            const float hg = (stepmod * hot().h) * hot().G[0], cs = hot().cs;
             const float2 z = zphase(P_.tau_z4, 0.f);
             Pair nl[H];
 #pragma unroll
             for (int j = 0; j < H; ++j) nl[j] = nl_eval(a[j], cph[j], z);
             float2 L, R;
-            edges(nl, h1, L, R);
+            edges(nl, make_float2(0.f, 0.f), L, R);
             k_all<H>(nl, L, R, hg, cs, k1r);
         }
 
-        for (int chunk = 0; chunk < nchunks; ++chunk) {
+        // whether the pass goes on at position kk of a chunk that ends at ce
+        auto more = [&](float kk, float ce) {
+            const float Sf = hot().S;
+            return kk < ce && (nee ? kk <= Sf : (!guard || kk < Sf));
+        };
+        for (int chunk = 0; chunk < hot().nchunks; ++chunk) {
             if (!nee) stepmod = stepprev;
-            const float cend = (float)(chunk + 1) * sel;
-            while (k < cend && (nee ? k <= Sf : (!guard || k < Sf))) {
+            const float cend = (float)(chunk + 1) * hot().sel;
+            while (more(k, cend)) {
                 if (attempt >= max_attempts) { status |= OPTIFAX_PULSE_ATTEMPT_LIMIT; goto done; }
                 const int krec = (int)k;
                 // z of the first stage in steps and index of G (G33(k) is 1-based in NEE_CPU.m)
                 const float kpos = nee ? k - 1.f : k;
                 bool accepted = false;
                 if (kpos != zk || stepmod != zs) prepare(kpos, stepmod);
-                const float hg = (stepmod * h) * gval;
+                const float hg = (stepmod * hot().h) * gval, cs = hot().cs;
                 Pair ev[H];                                    // E, then E behind the absorber
                 Pair dv[H];                                    // its error difference
                 Pair k4[H];                                    // RK23: FSAL candidate
@@ -843,9 +1091,10 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
 #pragma unroll
                     for (int j = 0; j < H; ++j) nl[j] = nl_eval(a[j], cph[j], z0);
                     float2 hn = make_float2(0.f, 0.f);
-                    if (lend || rend) {
+                    if (HALO && (lend || rend)) {
                         // drive and A1 of the adjacent halo point
-                        const float2 n1 = nl_one(h1, hc1, z0), n2 = nl_one(h2, hc2, z0);
+                        const float2 h1 = hs[0], hc1 = hs[2];
+                        const float2 n1 = nl_one(h1, hc1, z0), n2 = nl_one(hs[1], hs[3], z0);
                         const float2 in = lend ? make_float2(nl[0].re.x, nl[0].im.x)
                                                : make_float2(nl[H - 1].re.y, nl[H - 1].im.y);
                         const float2 kh = lend ? k_one(n2, n1, in, hg, cs) : k_one(in, n1, n2, hg, cs);
@@ -872,11 +1121,11 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     float2 L, R;
 #pragma unroll
                     for (int j = 0; j < H; ++j) nl[j] = nl_eval(pair_fma(k1r[j], 0.5f, a[j]), cph[j], z0);
-                    edges(nl, h1, L, R);
+                    edges(nl, make_float2(0.f, 0.f), L, R);
                     k_all<H>(nl, L, R, hg, cs, k2);
 #pragma unroll
                     for (int j = 0; j < H; ++j) nl[j] = nl_eval(pair_fma(k2[j], 0.75f, a[j]), cph[j], z1);
-                    edges(nl, h1, L, R);
+                    edges(nl, make_float2(0.f, 0.f), L, R);
                     k_all<H>(nl, L, R, hg, cs, pp);
 #pragma unroll
                     for (int j = 0; j < H; ++j) {
@@ -891,43 +1140,40 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     }
 #pragma unroll
                     for (int j = 0; j < H; ++j) nl[j] = nl_eval(ev[j], cph[j], z2);
-                    edges(nl, h1, L, R);
+                    edges(nl, make_float2(0.f, 0.f), L, R);
                     k_all<H>(nl, L, R, hg, cs, k4);
 #pragma unroll
                     for (int j = 0; j < H; ++j) dv[j] = pair_fma(k4[j], -1.f / 8.f, pp[j]);   // = E - A1
                 }
-                const int bits = classify_all<H, nee>(bounds, dv, ev);
-                // E behind the absorber: into the FFT buffer, or its columns' owners
+                const int bits = classify_all<H, nee>(bounds, P_, heun ? 50.f : 200.f, dv, ev);
+                // E behind the absorber: into the FFT buffer, or the columns' buffer
                 {
                     float2 o[P];
-                    float ab[P];
+                    if (abc) {
 #pragma unroll
-                    for (int j = 0; j < P; j += 4) {
-                        const float4 w = *reinterpret_cast<const float4*>(abc_s + at4(j));
-                        ab[j] = w.x; ab[j + 1] = w.y; ab[j + 2] = w.z; ab[j + 3] = w.w;
+                        for (int j = 0; j < H; ++j) {
+                            const float2 f = make_float2(abc[j], abc[j + H]);
+                            ev[j] = Pair{mul2(ev[j].re, f), mul2(ev[j].im, f)};
+                        }
                     }
 #pragma unroll
                     for (int j = 0; j < H; ++j) {
-                        const float2 f = make_float2(ab[j], ab[j + H]);
-                        ev[j] = Pair{mul2(ev[j].re, f), mul2(ev[j].im, f)};
                         o[j] = make_float2(ev[j].re.x, ev[j].im.x);
                         o[j + H] = make_float2(ev[j].re.y, ev[j].im.y);
                     }
-                    if constexpr (C > 1) push_columns<M, C>(g_addr, o, t, c);
-                    else store_own<P>(bufX, t, o);
-                    if (lend) {          // E of this block's first points: the left neighbour's right halo
-                        const uint32_t dst = cluster_addr(smem_u32(halo_e), (c + C - 1) % C);
-                        st_cluster_f2(dst + 16, o[0]);
-                        st_cluster_f2(dst + 24, o[1]);
-                    }
-                    if (rend) {
-                        const uint32_t dst = cluster_addr(smem_u32(halo_e), (c + 1) % C);
-                        st_cluster_f2(dst, o[P - 2]);
-                        st_cluster_f2(dst + 8, o[P - 1]);
+                    store_own<P>(C > 1 ? bufG : bufX, t, o);
+                    if (HALO && (lend || rend)) {  // E of the end points: the neighbours' halos
+                        const uint32_t src = smem_u32(halo_e + 4 * (lend ? seg_left<C>(seg, c) : seg_right<C>(seg, c)));
+                        const uint32_t dst = cluster_addr(src, lend ? (c + C - 1) % C : (c + 1) % C);
+                        const uint32_t db = dst + (bar_a - src);
+                        if (lend) st_async(dst + 16, o[0], o[1], db);
+                        else st_async(dst, o[P - 2], o[P - 1], db);
                     }
                 }
 
-                int fl = combine_flags<M, C>(bits, red, gatt, t, c, cfg);
+                int fl = combine_flags<M, C>(bits, red, bar_a, ph_a, kBytesA, dead, gatt, t, c, cfg);
+                ph_a ^= 1;
+                if (C > 1 && (fl & kDead)) { status |= OPTIFAX_PULSE_TIMEOUT; goto done; }
                 if ((opts & kForced) && gatt < P_.n_forced) fl = (P_.forced[gatt] & 3) | (fl & 4);
                 if (fl & 4) trip_status |= OPTIFAX_PULSE_NAN;
 
@@ -938,19 +1184,21 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                         P_.trace[3 * gatt] = krec; P_.trace[3 * gatt + 1] = (int)stepmod;
                         P_.trace[3 * gatt + 2] = fl & 7;
                     }
-                    ++n_rej;
+                    if (t == 0) ++run->n_rej;
+                    // the next attempt's flags and halos must not overtake this one's
+                    if constexpr (C > 1) cg::this_cluster().sync();
                     if (!nee) k = k - stepmod;
                     stepmod = stepmod - 1.f;
                     stepprev = stepmod;
                     if constexpr (!heun) {
                         // K1 recomputed at z = k + stepmod with G[k] (OPO_CUDA_ODE23.cu:484-487)
-                        const float hg1 = (stepmod * h) * G[(int)k];
+                        const float hg1 = (stepmod * hot().h) * hot().G[(int)k];
                         const float2 z = zphase(P_.tau_z4, k + stepmod);
                         Pair nl[H];
                         float2 L, R;
 #pragma unroll
                         for (int j = 0; j < H; ++j) nl[j] = nl_eval(a[j], cph[j], z);
-                        edges(nl, h1, L, R);
+                        edges(nl, make_float2(0.f, 0.f), L, R);
                         k_all<H>(nl, L, R, hg1, cs, k1r);
                     }
                 } else {
@@ -959,7 +1207,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                         P_.trace[3 * gatt] = krec; P_.trace[3 * gatt + 1] = (int)stepmod;
                         P_.trace[3 * gatt + 2] = (fl & 7) | 8;
                     }
-                    ++n_acc;
+                    if (t == 0) ++run->n_acc;
                     accepted = true;
                     const int s_used = (int)stepmod;
                     if ((opts & kSteps) && rec && krec < P_.stepmods_limit && krec < P_.S) {
@@ -970,6 +1218,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     // NEE_CPU.m:77-83: grow below minErr, clamp only at the crystal end)
                     if (nee) {
                         if (!(fl & 2)) stepmod = stepmod + 1.f;
+                        const float Sf = hot().S;
                         if (k < Sf && k + stepmod > Sf) stepmod = Sf - k;
                     } else if (k + stepmod >= cend && k < cend - 1.f) {
                         float stepend = (cend - k) - 1.f;
@@ -984,25 +1233,22 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                         stepprev = stepmod;
                     }
                     const float knext = k + stepmod;
-                    const bool last_in_chunk = !(knext < cend && (nee ? knext <= Sf : (!guard || knext < Sf)));
-                    const bool pass_ends = !(knext < pass_end && (nee ? knext <= Sf : (!guard || knext < Sf)));
-                    const bool cav = opo && pass_ends;
+                    const bool last_in_chunk = !more(knext, cend);
+                    const bool pass_ends = !more(knext, (float)hot().nchunks * hot().sel);
+                    const bool cav = pass_ends && hot().cavity;
                     const unsigned qn = q + (unsigned)s_used;
-                    if (!pass_ends) {
-                        const float kn = nee ? knext - 1.f : knext;
-                        prepare(kn, (!nee && last_in_chunk) ? stepprev : stepmod);
-                    }
 
                     // ---- linear sub-step ----
                     // Incremental form: A_new = E + IFFT((D - 1) FFT(E)) / N with
                     // D = alpha^s exp(-i beta s): transform rounding then scales with
                     // |D - 1| instead of |E|.  At the end of an OPO pass the full
                     // spectrum goes through the cavity instead: A_new = IFFT(D FFT(E) fb + pump) / N.
-                    float2 he1 = h1, he2 = h1;
                     if constexpr (C > 1) {
-                        if (lend) { he1 = halo_e[1]; he2 = halo_e[0]; }
-                        if (rend) { he1 = halo_e[2]; he2 = halo_e[3]; }
-                        exchange_fwd<M, C>(bufG, x_addr, xtw_s, t, c);
+                        if (HALO && (lend || rend)) {
+                            hs[0] = halo_e[4 * seg + (lend ? 1 : 2)];
+                            hs[1] = halo_e[4 * seg + (lend ? 0 : 3)];
+                        }
+                        exchange_fwd<M, C>(bufG, bufX, x_addr, bar_b, xtw_s, inner, t, c);
                     }
                     // refresh the per-mode D - 1 when the step size changed (a compact loop:
                     // kept out of the unrolled mode loop below), for the exact fixed-point
@@ -1024,7 +1270,15 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                         }
                         s_cached = s_used;
                     }
-                    if constexpr (C > 1) cg::this_cluster().sync();
+                    if (!pass_ends) {
+                        const float kn = nee ? knext - 1.f : knext;
+                        prepare(kn, (!nee && last_in_chunk) ? stepprev : stepmod);
+                    }
+                    if constexpr (C > 1) {
+                        if constexpr (XC_::LOCAL) __syncthreads();
+                        bar_wait(bar_b, ph_x, dead);
+                        if (t == 0) bar_arm(bar_b, kAll);
+                    }
                     float2 v[P];
                     fftp_forward<M, P>(bufX, tw_s, t, v);
                     float2* apc = (last_in_chunk && (opts & kAp)) ? P_.Ap + (size_t)chunk * N : nullptr;
@@ -1085,15 +1339,21 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     }
                     fftp_inverse<M, P>(bufX, tw_s, td_s, t, v);
                     if constexpr (C > 1) {
-                        push_inverse<M, C>(g_addr, v, t, c);
-                        cg::this_cluster().sync();
-                        exchange_inv<M, C, HALO>(bufG, x_addr, smem_u32(halo_d), xtw_s, xtd_s, t, c, invN);
-                        cg::this_cluster().sync();
-                        if (lend || rend) {
-                            const float2 d1 = halo_d[lend ? 1 : 2], d2 = halo_d[lend ? 0 : 3];
-                            h1 = cav ? d1 : cadd(he1, d1);
-                            h2 = cav ? d2 : cadd(he2, d2);
+                        push_inverse<M, C>(bufG, g_addr, bar_c, v, t, c);
+                        if constexpr (XC_::LOCAL) __syncthreads();
+                        bar_wait(bar_c, ph_x, dead);
+                        if (t == 0) bar_arm(bar_c, kAll);
+                        exchange_inv<M, C, HALO>(bufG, bufX, smem_u32(halo_d), bar_d, xtw_s, xtd_s, inner, t, c, invN);
+                        __syncthreads();
+                        if (HALO && (lend || rend)) {
+                            bar_wait(bar_d, ph_x, dead);
+                            if (t == 0) bar_arm(bar_d, kBytesD);
+                            const float2 d1 = halo_d[4 * seg + (lend ? 1 : 2)];
+                            const float2 d2 = halo_d[4 * seg + (lend ? 0 : 3)];
+                            hs[0] = cav ? d1 : cadd(hs[0], d1);
+                            hs[1] = cav ? d2 : cadd(hs[1], d2);
                         }
+                        ph_x ^= 1;
                     } else {
                         const int s0 = swz(t);
 #pragma unroll
@@ -1108,7 +1368,12 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                         else a[j] = cav ? Pair{mul2(d.re, dup2(invN)), mul2(d.im, dup2(invN))} : pair_fma(d, invN, ev[j]);
                         if constexpr (!heun) k1r[j] = k4[j];
                     }
-                    if (cav) reduce_tallies<M, C>(part, tally, dred, t, c, trip & 1);
+                    if (cav) {
+                        double tally[4];
+                        reduce_tallies<M, C>(part, tally, dred, t, c, trip & 1);
+                        if (t == 0)
+                            for (int i = 0; i < 4; ++i) run->tally[i] = tally[i];
+                    }
                     q = qn;
                 }
                 ++attempt;
@@ -1117,34 +1382,40 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
             }
         }
         status |= trip_status;
-        tot_att += attempt; tot_acc += n_acc; tot_rej += n_rej;
         trips_done = trip + 1;
-        if (opo) {
-            if (rec && P_.trips) {
+        if (t == 0) {
+            if (rec && P_.fb && P_.trips) {
                 optifax_trip_record tr;
-                tr.attempts = attempt; tr.accepted = n_acc; tr.rejected = n_rej; tr.status = trip_status;
-                for (int i = 0; i < 4; ++i) tr.tally[i] = tally[i];
+                tr.attempts = attempt; tr.accepted = run->n_acc; tr.rejected = run->n_rej; tr.status = trip_status;
+                for (int i = 0; i < 4; ++i) tr.tally[i] = run->tally[i];
                 P_.trips[trip] = tr;
             }
-            if (P_.steady_trips > 0) {
-                double cur = tally[P_.steady_tally & 3];
-                bool flat = trip > 0 && cur != 0.0 && fabs(cur - prev_tally) <= (double)P_.steady_tol * fabs(cur);
-                steady_count = flat ? steady_count + 1 : 0;
-                prev_tally = cur;
-                if (steady_count >= P_.steady_trips) break;
-            }
+            run->tot_att += attempt; run->tot_acc += run->n_acc; run->tot_rej += run->n_rej;
+            run->n_acc = run->n_rej = 0;
+            // steady state of a cavity: the totals are the same in every CTA of the cluster
+            const double cur = run->tally[P_.steady_tally & 3];
+            const bool flat = trip > 0 && cur != 0.0 &&
+                              fabs(cur - run->prev_tally) <= (double)P_.steady_tol * fabs(cur);
+            run->steady = flat ? run->steady + 1 : 0;
+            run->prev_tally = cur;
+            run->stop = P_.fb && P_.steady_trips > 0 && run->steady >= P_.steady_trips;
+            for (int i = 0; i < 4; ++i) run->tally[i] = 0.0;
+        }
+        if (n_trips > 1) {
+            __syncthreads();
+            if (run->stop) break;
         }
     }
 done:
 #pragma unroll
     for (int j = 0; j < H; ++j) {
-        P_.A_out[c * M + P * t + j] = make_float2(a[j].re.x, a[j].im.x);
-        P_.A_out[c * M + P * t + j + H] = make_float2(a[j].re.y, a[j].im.y);
+        P_.A_out[i0 + j] = make_float2(a[j].re.x, a[j].im.x);
+        P_.A_out[i0 + j + H] = make_float2(a[j].re.y, a[j].im.y);
     }
     if (rec && P_.stats) {
         optifax_pulse_stats st;
-        st.attempts = tot_att; st.accepted = tot_acc; st.rejected = tot_rej; st.status = status;
-        st.z_steps = (long long)q; st.k_final = k; st.stepmod_final = stepmod; st.n_chunks = nchunks;
+        st.attempts = run->tot_att; st.accepted = run->tot_acc; st.rejected = run->tot_rej; st.status = status;
+        st.z_steps = (long long)q; st.k_final = k; st.stepmod_final = stepmod; st.n_chunks = P_.nchunks;
         st.reserved[0] = trips_done; st.reserved[1] = st.reserved[2] = 0;
         *P_.stats = st;
     }
