@@ -26,7 +26,6 @@ struct optifax_context {
     int device = 0;
     std::map<int, Twiddle*> tw;          // N -> W_N^i, i < 64 (cluster exchange)
     std::map<int, Twiddle*> quadtw;      // M -> W_M^y, y < M/4 (cluster exchange)
-    std::map<int, Twiddle*> passtw;      // M -> pass-1 table [16][M/16] then pass-2 [16][M/256]
     PulseDev* d_desc = nullptr;
     size_t desc_cap = 0;
     float2* d_xs = nullptr;              // cavities' trip-output scratch
@@ -59,22 +58,6 @@ __global__ void twiddle_kernel(Twiddle* out, int n, int count) {
     Twiddle w;
     w.c = cf; w.s = sf; w.d = (float)(1.0 / m2 - 1.0); w.pad = 0.f;
     out[e] = w;
-}
-
-// outer twiddles of one FFT pass over blocks of length L with radix 16:
-// out[r * (L/16) + off] = W_L^{off r}
-__global__ void pass_twiddle_kernel(Twiddle* out, int L) {
-    int lr = L / 16;
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 16 * lr) return;
-    int r = idx / lr, off = idx - r * lr;
-    double s, c;
-    sincospi(-2.0 * (double)(off * r) / (double)L, &s, &c);
-    float cf = (float)c, sf = (float)s;
-    double m2 = (double)cf * (double)cf + (double)sf * (double)sf;
-    Twiddle w;
-    w.c = cf; w.s = sf; w.d = (float)(1.0 / m2 - 1.0); w.pad = 0.f;
-    out[idx] = w;
 }
 
 int fail(optifax_context* h, int code, const std::string& msg) {
@@ -139,22 +122,6 @@ const Twiddle* get_table(optifax_context* h, std::map<int, Twiddle*>& cache, int
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { cudaFree(d); *rc = cuda_fail(h, e, "twiddle_kernel sync"); return nullptr; }
     cache[n] = d;
-    return d;
-}
-
-const Twiddle* get_pass_twiddles(optifax_context* h, int M, cudaStream_t st, int* rc) {
-    auto it = h->passtw.find(M);
-    if (it != h->passtw.end()) return it->second;
-    int n1 = M, n2 = 16 * (M / 256);
-    Twiddle* d = nullptr;
-    cudaError_t e = cudaMalloc(&d, sizeof(Twiddle) * (size_t)(n1 + n2));
-    if (e != cudaSuccess) { *rc = cuda_fail(h, e, "cudaMalloc(pass twiddles)"); return nullptr; }
-    pass_twiddle_kernel<<<(n1 + 255) / 256, 256, 0, st>>>(d, M);
-    pass_twiddle_kernel<<<(n2 + 255) / 256, 256, 0, st>>>(d + n1, M / 16);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) { cudaFree(d); *rc = cuda_fail(h, e, "pass_twiddle_kernel"); return nullptr; }
-    h->passtw[M] = d;
     return d;
 }
 
@@ -492,7 +459,6 @@ int optifax_destroy(optifax_handle h) {
     cudaSetDevice(h->device);
     cudaDeviceSynchronize();
     for (auto& kv : h->tw) cudaFree(kv.second);
-    for (auto& kv : h->passtw) cudaFree(kv.second);
     for (auto& kv : h->quadtw) cudaFree(kv.second);
     if (h->d_desc) cudaFree(h->d_desc);
     if (h->d_grid_flags) cudaFree(h->d_grid_flags);
@@ -804,8 +770,8 @@ extern "C" int optifax_gnlse(optifax_handle h, const optifax_gnlse_pulse* pulses
     cudaError_t de = cudaSetDevice(h->device);
     if (de != cudaSuccess) return cuda_fail(h, de, "cudaSetDevice");
     int rc = OPTIFAX_OK;
-    const Twiddle* twp = get_pass_twiddles(h, M, st, &rc);
-    if (!twp) return rc;
+    const Twiddle* quad = get_table(h, h->quadtw, M, M / 4, st, &rc);
+    if (!quad) return rc;
     const size_t need_k = (size_t)8 * M * n_pulses;
     if (need_k > h->gnlse_k_cap) {
         size_t cap = h->gnlse_k_cap * sizeof(float2);
@@ -827,7 +793,7 @@ extern "C" int optifax_gnlse(optifax_handle h, const optifax_gnlse_pulse* pulses
     cudaError_t e = cudaMemcpyAsync(h->d_gnlse_desc, d.data(), sizeof(GnlseDev) * (size_t)n_pulses,
                                     cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(h, e, "cudaMemcpyAsync(gnlse descriptors)");
-    e = launch_gnlse(M, h->d_gnlse_desc, n_pulses, twp, twp + M, st);
+    e = launch_gnlse(M, h->d_gnlse_desc, n_pulses, quad, st);
     if (e != cudaSuccess) return cuda_fail(h, e, "gnlse_kernel launch");
     return mark_done(h, st);
 }

@@ -64,14 +64,6 @@ __device__ __forceinline__ float2 turn_to_unit(uint64_t u) {
 // plus inverse transform carries no systematic per-mode gain.
 struct __align__(16) Twiddle { float c, s, d, pad; };
 
-__device__ __forceinline__ float2 tw_fwd(float2 v, const Twiddle& w) {
-    return cmul(v, make_float2(w.c, w.s));
-}
-__device__ __forceinline__ float2 tw_inv(float2 v, const Twiddle& w) {
-    float2 t = cmulc(v, make_float2(w.c, w.s));
-    return make_float2(fmaf(t.x, w.d, t.x), fmaf(t.y, w.d, t.y));
-}
-
 // W_M^x for 0 <= x < M from the quarter-period table q[y] = W_M^y, y < M/4
 // (kept in shared memory): x = k M/4 + y gives W_M^y (-i)^k, a swap and sign
 // changes, so the value and its d are those of a full table.
@@ -100,10 +92,5 @@ __device__ __forceinline__ float inv_norm2_m1(float2 w) {
 __device__ __forceinline__ int bitrev(int x, int bits) {
     return bits == 0 ? 0 : (int)(__brev((unsigned)x) >> (32 - bits));
 }
-
-// Shared-memory placement of a complex point: one float2 of padding per 16
-// keeps both the per-thread contiguous (16 points) accesses of the RK stages
-// and the strided FFT-pass accesses free of bank conflicts.
-__device__ __forceinline__ int phys(int m) { return m + (m >> 4); }
 
 }  // namespace ofx

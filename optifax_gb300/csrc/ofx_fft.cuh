@@ -1,37 +1,53 @@
-// ofx_fft.cuh -- in-shared-memory complex FFT of one CTA's M points.
+// ofx_fft.cuh -- in-shared-memory complex FFT of one CTA's M points with P points
+// per thread (P = 4 or 8), for the FP32 crystal pass and the fibre kernel.
 //
-// Decimation in frequency with three register passes of radix 16/16/(M/256):
-// each thread owns one radix-R butterfly group (16 points) per pass.  A pass
-// over blocks of length L computes, for every offset `off` in [0, L/R),
-//     y_r = W_L^{off r} * DFT_R(x[off + q L/R])_r
-// with DFT_R done in registers by radix-2 stages whose twiddles are
-// compile-time constants (bit-reversed output: register q holds r = bitrev(q)),
-// and the outer twiddle W_L^{off r} read from a per-pass table laid out
-// [r][off] so consecutive threads read consecutive entries.  The forward
-// transform therefore leaves the spectrum in bit-reversed slot order; the
-// inverse undoes every multiply with the exact reciprocal (conj(w)(1+d)) and
-// returns natural order.  The last forward pass and the first inverse pass
-// act on the same registers (thread t holds slots 16t .. 16t+15), so per-mode
-// work sits between them without a shared-memory round trip.
+// Decimation in frequency: passes of radix P over blocks of length M, M/P, ...; the
+// last pass has the remaining radix.  In a pass over blocks of length L every thread
+// owns one butterfly: y_q = W_L^{off r} DFT_P(x[off + q L/P])_r with r = bitrev(q), so
+// the forward transform leaves the spectrum in bit-reversed slot order and the inverse
+// undoes it, multiplying by the exact reciprocal conj(w)(1 + d) of every forward
+// twiddle.  The last forward and the first inverse pass act on the same registers
+// (thread t holds slots P t .. P t + P - 1).  Unnormalised: forward then inverse
+// multiplies by M.
 //
-// Unnormalised: forward followed by inverse multiplies by M.
+// The outer twiddles sit in shared memory: (c, s) as [pass][q - 1][off] and the
+// reciprocals' d = 1/|w|^2 - 1 as [pass][off][P], read as vectors.
+//
+// Eight points per thread instead of sixteen: twice the warps hide the latency of the
+// fixed-latency chains and shared-memory round trips that bound the pass (two warps per
+// scheduler issued on half of the cycles), for one more pass through shared memory at
+// 4096 points.
 #pragma once
 #include "ofx_common.cuh"
 
 namespace ofx {
 
+// Points per thread of a CTA with M points
 template <int M>
-struct FftShape {
-    static_assert(M >= 512 && M <= 4096 && (M & (M - 1)) == 0, "M must be 512..4096");
-    static constexpr int T = M / 16;      // threads per CTA
-    static constexpr int L1 = M, R1 = 16;
-    static constexpr int L2 = M / 16, R2 = 16;
-    static constexpr int L3 = M / 256, R3 = M / 256;   // last pass: L == R
-    static constexpr int LOG2M = (M == 512) ? 9 : (M == 1024) ? 10 : (M == 2048) ? 11 : 12;
-    // outer-twiddle tables: pass 1 [16][M/16], pass 2 [16][M/256]
-    static constexpr int TW1 = 16 * (M / 16);
-    static constexpr int TW2 = 16 * (M / 256);
+constexpr int kPoints = (M >= 2048) ? 8 : 4;
+
+__host__ __device__ constexpr int ilog2(int x) { return x <= 1 ? 0 : 1 + ilog2(x / 2); }
+
+template <int M, int P>
+struct FftPlan {
+    static constexpr int T = M / P, RB = ilog2(P), BITS = ilog2(M);
+    static constexpr int NP = (BITS + RB - 1) / RB;                 // passes
+    static constexpr int LAST = 1 << (BITS - (NP - 1) * RB);        // radix of the last pass
+    static constexpr int L(int p) { return M >> (p * RB); }         // block length of pass p
+    static constexpr int tw_off(int p) { return p == 0 ? 0 : tw_off(p - 1) + (P - 1) * (L(p - 1) / P); }
+    static constexpr int td_off(int p) { return p == 0 ? 0 : td_off(p - 1) + L(p - 1); }
+    static constexpr int TW = tw_off(NP - 1);                       // float2 entries
+    static constexpr int TD = td_off(NP - 1);                       // d entries
 };
+
+// Shared-memory placement of point m: 16-byte pairs are permuted inside every 128-byte
+// row by higher bits of m, so that the strided accesses of every pass, the per-thread
+// contiguous accesses (16-byte vectors) and the unit-stride ones are free of bank
+// conflicts without padding.  swz is linear over XOR.
+__host__ __device__ constexpr int swz(int m) { return m ^ (((m >> 4) & 3) << 1) ^ ((m >> 3) & 8); }
+
+// swz(base + k) for s0 = swz(base) where base has zeros in the bits of the constant k
+__device__ __forceinline__ int swz_at(int s0, int k) { return (s0 ^ (swz(k) & 15)) + (k & ~15); }
 
 // W_16^m = exp(-2 pi i m / 16), m = 0..7, rounded to FP32; d = 1/|w|^2 - 1
 __device__ __forceinline__ float w16c(int m) {
@@ -50,54 +66,6 @@ __device__ __forceinline__ float w16d(int m) {
     return d[m];
 }
 
-// v * W_16^m for a compile-time m in 0..7 (trivial cases folded)
-__device__ __forceinline__ float2 mul_w16(float2 v, int m) {
-    if (m == 0) return v;
-    if (m == 4) return make_float2(v.y, -v.x);                 // * (-i)
-    return cmul(v, make_float2(w16c(m), w16s(m)));
-}
-// v / W_16^m = v * conj(W_16^m) (1 + d)
-__device__ __forceinline__ float2 div_w16(float2 v, int m) {
-    if (m == 0) return v;
-    if (m == 4) return make_float2(-v.y, v.x);                 // * i
-    float2 t = cmulc(v, make_float2(w16c(m), w16s(m)));
-    float d = w16d(m);
-    return make_float2(fmaf(t.x, d, t.x), fmaf(t.y, d, t.y));
-}
-
-// DFT_R of v[0..R) by radix-2 DIF stages; register q ends holding output bitrev(q)
-template <int R>
-__device__ __forceinline__ void dft_dif(float2* v) {
-#pragma unroll
-    for (int hr = R / 2; hr >= 1; hr >>= 1) {
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-            if (q & hr) continue;
-            const int m16 = (q & (hr - 1)) * (R / (2 * hr)) * (16 / R);
-            float2 a = v[q], b = v[q + hr];
-            v[q] = cadd(a, b);
-            v[q + hr] = mul_w16(csub(a, b), m16);
-        }
-    }
-}
-
-// exact reverse of dft_dif (unnormalised: each stage doubles)
-template <int R>
-__device__ __forceinline__ void dft_dit_inv(float2* v) {
-#pragma unroll
-    for (int hr = 1; hr <= R / 2; hr <<= 1) {
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-            if (q & hr) continue;
-            const int m16 = (q & (hr - 1)) * (R / (2 * hr)) * (16 / R);
-            float2 a = v[q];
-            float2 t = div_w16(v[q + hr], m16);
-            v[q] = cadd(a, t);
-            v[q + hr] = csub(a, t);
-        }
-    }
-}
-
 __device__ __forceinline__ int brev4(int q, int bits) {
     // bit reversal of q within `bits` (<= 4) bits, compile-time foldable
     int r = 0;
@@ -107,136 +75,215 @@ __device__ __forceinline__ int brev4(int q, int bits) {
     return r;
 }
 
-// element index of (butterfly slot u, leg q) handled by thread t in a pass of
-// radix R over blocks of length L.  LASTMAP assigns each thread contiguous
-// butterflies (slots 16t..16t+15 in the last pass); otherwise consecutive
-// threads take consecutive butterflies (coalesced, conflict-free).
-template <int M, int R, int L, bool LASTMAP>
-__device__ __forceinline__ int pass_index(int t, int u, int q, int& off) {
-    constexpr int T = M / 16, NB = 16 / R, LR = L / R;
-    int beta = LASTMAP ? t * NB + u : t + T * u;
-    int b = beta / LR;
-    off = beta - b * LR;
-    return b * L + off + q * LR;
+// Small DFTs in registers with packed additions: radix-2 stages, forward decimation in
+// frequency (register q ends holding output bitrev(q)), the inverse its exact reverse
+// (every constant's exact reciprocal).  m16: exponent of W_16.
+__device__ __forceinline__ float2 rot_fwd(float2 v, int m16) {
+    if (m16 == 0) return v;
+    if (m16 == 4) return make_float2(v.y, -v.x);
+    if (m16 == 2 || m16 == 6) {                            // c (1 - i), c (-1 - i)
+        const float2 t = mul2(v, dup2(w16c(2)));
+        return m16 == 2 ? make_float2(t.x + t.y, t.y - t.x) : make_float2(t.y - t.x, -(t.x + t.y));
+    }
+    return cmul(v, make_float2(w16c(m16), w16s(m16)));
 }
-
-template <int M, int R, int L, bool LASTMAP>
-__device__ __forceinline__ void pass_load(const float2* buf, int t, float2 (&v)[16], int (&offs)[16 / R]) {
+__device__ __forceinline__ float2 rot_inv(float2 v, int m16) {
+    if (m16 == 0) return v;
+    if (m16 == 4) return make_float2(-v.y, v.x);
+    float2 u;
+    if (m16 == 2 || m16 == 6) {
+        const float2 t = mul2(v, dup2(w16c(2)));
+        u = m16 == 2 ? make_float2(t.x - t.y, t.y + t.x) : make_float2(-(t.x + t.y), t.x - t.y);
+    } else {
+        u = cmulc(v, make_float2(w16c(m16), w16s(m16)));
+    }
+    return cfma1(u, w16d(m16), u);
+}
+template <int R>
+__device__ __forceinline__ void dftp(float2* v) {
 #pragma unroll
-    for (int u = 0; u < 16 / R; ++u)
+    for (int hr = R / 2; hr >= 1; hr >>= 1) {
 #pragma unroll
         for (int q = 0; q < R; ++q) {
-            int off;
-            int m = pass_index<M, R, L, LASTMAP>(t, u, q, off);
-            v[u * R + q] = buf[phys(m)];
-            offs[u] = off;
+            if (q & hr) continue;
+            const float2 a = v[q], b = v[q + hr];
+            v[q] = add2(a, b);
+            v[q + hr] = rot_fwd(sub2(a, b), (q & (hr - 1)) * (R / (2 * hr)) * (16 / R));
         }
+    }
 }
-
-template <int M, int R, int L, bool LASTMAP>
-__device__ __forceinline__ void pass_store(float2* buf, int t, const float2 (&v)[16]) {
+template <int R>
+__device__ __forceinline__ void dftp_inv(float2* v) {
 #pragma unroll
-    for (int u = 0; u < 16 / R; ++u)
+    for (int hr = 1; hr <= R / 2; hr <<= 1) {
 #pragma unroll
         for (int q = 0; q < R; ++q) {
-            int off;
-            int m = pass_index<M, R, L, LASTMAP>(t, u, q, off);
-            buf[phys(m)] = v[u * R + q];
+            if (q & hr) continue;
+            const float2 a = v[q], t = rot_inv(v[q + hr], (q & (hr - 1)) * (R / (2 * hr)) * (16 / R));
+            v[q] = add2(a, t);
+            v[q + hr] = sub2(a, t);
         }
-}
-
-template <int M, int R, int L>
-__device__ __forceinline__ void fwd_pass_smem(float2* buf, const Twiddle* __restrict__ tw, int t,
-                                              const float2* gin = nullptr) {
-    constexpr int LR = L / R, BITS = (R == 16) ? 4 : (R == 8) ? 3 : (R == 4) ? 2 : 1;
-    float2 v[16];
-    int offs[16 / R];
-    if (gin) {
-        // input from global memory (cluster exchange buffer, natural order, L2)
-#pragma unroll
-        for (int u = 0; u < 16 / R; ++u)
-#pragma unroll
-            for (int q = 0; q < R; ++q) {
-                int off;
-                int m = pass_index<M, R, L, false>(t, u, q, off);
-                v[u * R + q] = __ldcg(gin + m);
-                offs[u] = off;
-            }
-    } else {
-        pass_load<M, R, L, false>(buf, t, v, offs);
-    }
-#pragma unroll
-    for (int u = 0; u < 16 / R; ++u) {
-        dft_dif<R>(v + u * R);
-#pragma unroll
-        for (int q = 1; q < R; ++q) v[u * R + q] = tw_fwd(v[u * R + q], tw[brev4(q, BITS) * LR + offs[u]]);
-    }
-    pass_store<M, R, L, false>(buf, t, v);
-}
-
-template <int M, int R, int L>
-__device__ __forceinline__ void inv_pass_smem(float2* buf, const Twiddle* __restrict__ tw, int t,
-                                              float2* gout = nullptr) {
-    constexpr int LR = L / R, BITS = (R == 16) ? 4 : (R == 8) ? 3 : (R == 4) ? 2 : 1;
-    float2 v[16];
-    int offs[16 / R];
-    pass_load<M, R, L, false>(buf, t, v, offs);
-#pragma unroll
-    for (int u = 0; u < 16 / R; ++u) {
-#pragma unroll
-        for (int q = 1; q < R; ++q) v[u * R + q] = tw_inv(v[u * R + q], tw[brev4(q, BITS) * LR + offs[u]]);
-        dft_dit_inv<R>(v + u * R);
-    }
-    if (gout) {
-#pragma unroll
-        for (int u = 0; u < 16 / R; ++u)
-#pragma unroll
-            for (int q = 0; q < R; ++q) {
-                int off;
-                int m = pass_index<M, R, L, false>(t, u, q, off);
-                __stcg(gout + m, v[u * R + q]);
-            }
-    } else {
-        pass_store<M, R, L, false>(buf, t, v);
     }
 }
 
-// Forward passes 1 and 2 in shared memory, then the last pass into registers:
-// on return v[j] holds slot 16t + j.  tw1/tw2: outer-twiddle tables of
-// passes 1 and 2.  Pass 1 reads `gin` (global, natural order) when given,
-// else buf.  The caller synchronises before (input complete).
-template <int M>
-__device__ __forceinline__ void fft_forward_to_regs(float2* buf, const Twiddle* __restrict__ tw1,
-                                                    const Twiddle* __restrict__ tw2, int t, float2 (&v)[16],
-                                                    const float2* gin = nullptr) {
-    using S = FftShape<M>;
-    fwd_pass_smem<M, S::R1, S::L1>(buf, tw1, t, gin);
-    __syncthreads();
-    fwd_pass_smem<M, S::R2, S::L2>(buf, tw2, t);
-    __syncthreads();
-    int offs[16 / S::R3];
-    pass_load<M, S::R3, S::L3, true>(buf, t, v, offs);
+// this thread's P contiguous points (16-byte vectors)
+template <int P>
+__device__ __forceinline__ void load_own(const float2* buf, int t, float2 (&v)[P]) {
+    const int s0 = swz(P * t);
 #pragma unroll
-    for (int u = 0; u < 16 / S::R3; ++u) dft_dif<S::R3>(v + u * S::R3);
+    for (int j = 0; j < P; j += 2) {
+        const float4 w = *reinterpret_cast<const float4*>(buf + (s0 ^ j));
+        v[j] = make_float2(w.x, w.y);
+        v[j + 1] = make_float2(w.z, w.w);
+    }
+}
+template <int P>
+__device__ __forceinline__ void store_own(float2* buf, int t, const float2 (&v)[P]) {
+    const int s0 = swz(P * t);
+#pragma unroll
+    for (int j = 0; j < P; j += 2)
+        *reinterpret_cast<float4*>(buf + (s0 ^ j)) = make_float4(v[j].x, v[j].y, v[j + 1].x, v[j + 1].y);
 }
 
-// Inverse of fft_forward_to_regs: v holds slots 16t+j; on return buf (or
-// `gout`, global, when given) holds the unnormalised inverse transform in
-// natural order.  Each thread only writes its own slots before the first
-// barrier, so no barrier is needed on entry.
-template <int M>
-__device__ __forceinline__ void fft_inverse_from_regs(float2* buf, const Twiddle* __restrict__ tw1,
-                                                      const Twiddle* __restrict__ tw2, int t, float2 (&v)[16],
-                                                      float2* gout = nullptr) {
-    using S = FftShape<M>;
+// v / w for w = (c, s) with reciprocal correction d
+__device__ __forceinline__ float2 mul_recip(float2 v, float2 w, float d) {
+    const float2 t = cmulc(v, w);
+    return cfma1(t, d, t);
+}
+
+// Barrier between two passes whose data stay inside aligned groups of `group` threads
+template <int GROUP>
+__device__ __forceinline__ void pass_sync() {
+    if constexpr (GROUP <= 32) __syncwarp();
+    else __syncthreads();
+}
+
+// Fill the twiddle tables from the quarter-period table of W_M (global memory).
+template <int M, int P>
+__device__ __forceinline__ void fft_tables(float2* tw, float* td, const Twiddle* quad, int t) {
+    using F = FftPlan<M, P>;
+#pragma unroll 1
+    for (int p = 0; p < F::NP - 1; ++p) {
+        const int L = M >> (p * F::RB), LR = L / P;
+        int o = 0, od = 0;
+        for (int i = 0; i < p; ++i) { o += (P - 1) * ((M >> (i * F::RB)) / P); od += M >> (i * F::RB); }
+#pragma unroll 1
+        for (int i = t; i < L; i += F::T) {
+            const int q = i / LR, off = i - q * LR;
+            const int r = bitrev(q, F::RB);
+            const Twiddle w = quad_tw<M>(quad, off * r * (M / L));
+            if (q > 0) tw[o + (q - 1) * LR + off] = make_float2(w.c, w.s);
+            td[od + off * P + q] = w.d;
+        }
+    }
+}
+
+// One forward pass; LOAD: from buf, else v holds points base + q L/P of the block.
+template <int M, int P, int PASS, bool LOAD = true>
+__device__ __forceinline__ void fftp_fwd(float2* buf, const float2* tw, int t, float2 (&v)[P]) {
+    using F = FftPlan<M, P>;
+    constexpr int L = F::L(PASS), LR = L / P;
+    const int off = t & (LR - 1), s0 = swz((t - off) * P + off);
+    if constexpr (LOAD) {
 #pragma unroll
-    for (int u = 0; u < 16 / S::R3; ++u) dft_dit_inv<S::R3>(v + u * S::R3);
-    pass_store<M, S::R3, S::L3, true>(buf, t, v);
-    __syncthreads();
-    inv_pass_smem<M, S::R2, S::L2>(buf, tw2, t);
-    __syncthreads();
-    inv_pass_smem<M, S::R1, S::L1>(buf, tw1, t, gout);
-    __syncthreads();
+        for (int q = 0; q < P; ++q) v[q] = buf[swz_at(s0, q * LR)];
+    }
+    dftp<P>(v);
+#pragma unroll
+    for (int q = 1; q < P; ++q) v[q] = cmul(v[q], tw[F::tw_off(PASS) + (q - 1) * LR + off]);
+#pragma unroll
+    for (int q = 0; q < P; ++q) buf[swz_at(s0, q * LR)] = v[q];
+}
+
+// One inverse pass; on return v[q] holds points base + q L/P of the block.
+template <int M, int P, int PASS>
+__device__ __forceinline__ void fftp_inv(const float2* buf, const float2* tw, const float* td, int t,
+                                         float2 (&v)[P], int& s0) {
+    using F = FftPlan<M, P>;
+    constexpr int L = F::L(PASS), LR = L / P;
+    const int off = t & (LR - 1);
+    s0 = swz((t - off) * P + off);
+    float d[P];
+#pragma unroll
+    for (int q = 0; q < P; q += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(td + F::td_off(PASS) + off * P + q);
+        d[q] = w.x; d[q + 1] = w.y; d[q + 2] = w.z; d[q + 3] = w.w;
+    }
+#pragma unroll
+    for (int q = 0; q < P; ++q) v[q] = buf[swz_at(s0, q * LR)];
+#pragma unroll
+    for (int q = 1; q < P; ++q) v[q] = mul_recip(v[q], tw[F::tw_off(PASS) + (q - 1) * LR + off], d[q]);
+    dftp_inv<P>(v);
+}
+
+template <int M, int P, int PASS>
+__device__ __forceinline__ void fftp_forward_passes(float2* buf, const float2* tw, int t) {
+    using F = FftPlan<M, P>;
+    if constexpr (PASS < F::NP - 1) {
+        float2 v[P];
+        fftp_fwd<M, P, PASS>(buf, tw, t, v);
+        pass_sync<F::L(PASS) / P>();
+        fftp_forward_passes<M, P, PASS + 1>(buf, tw, t);
+    }
+}
+
+// The last forward pass: v[j] returns slot P t + j
+template <int M, int P>
+__device__ __forceinline__ void fftp_forward_last(const float2* buf, int t, float2 (&v)[P]) {
+    using F = FftPlan<M, P>;
+    load_own<P>(buf, t, v);
+#pragma unroll
+    for (int u = 0; u < P / F::LAST; ++u) dftp<F::LAST>(v + u * F::LAST);
+}
+
+// Forward transform of buf (complete and visible); v[j] returns slot P t + j.
+template <int M, int P>
+__device__ __forceinline__ void fftp_forward(float2* buf, const float2* tw, int t, float2 (&v)[P]) {
+    fftp_forward_passes<M, P, 0>(buf, tw, t);
+    fftp_forward_last<M, P>(buf, t, v);
+}
+
+// Forward transform of v[q] = point t + q M/P, as fftp_inverse leaves them: the first
+// pass works on the registers, through which a point-wise step between an inverse and a
+// forward transform costs no shared-memory round trip.  buf is scratch whose previous
+// reads by other threads are ordered before (fftp_inverse of the same buffer is).
+template <int M, int P>
+__device__ __forceinline__ void fftp_forward_regs(float2* buf, const float2* tw, int t, float2 (&v)[P]) {
+    using F = FftPlan<M, P>;
+    fftp_fwd<M, P, 0, false>(buf, tw, t, v);
+    pass_sync<F::L(0) / P>();
+    fftp_forward_passes<M, P, 1>(buf, tw, t);
+    fftp_forward_last<M, P>(buf, t, v);
+}
+
+template <int M, int P, int PASS>
+__device__ __forceinline__ void fftp_inverse_passes(float2* buf, const float2* tw, const float* td, int t) {
+    using F = FftPlan<M, P>;
+    if constexpr (PASS > 0) {
+        float2 v[P];
+        int s0;
+        fftp_inv<M, P, PASS>(buf, tw, td, t, v, s0);
+#pragma unroll
+        for (int q = 0; q < P; ++q) buf[swz_at(s0, q * (F::L(PASS) / P))] = v[q];
+        pass_sync<F::L(PASS - 1) / P>();
+        fftp_inverse_passes<M, P, PASS - 1>(buf, tw, td, t);
+    }
+}
+
+// Inverse of fftp_forward up to its last pass: on return v[q] holds points
+// t + q M/P (q < P) of the unnormalised inverse transform.  Each thread writes only
+// its own slots before the first barrier, so none is needed on entry.
+template <int M, int P>
+__device__ __forceinline__ void fftp_inverse(float2* buf, const float2* tw, const float* td, int t,
+                                             float2 (&v)[P]) {
+    using F = FftPlan<M, P>;
+#pragma unroll
+    for (int u = 0; u < P / F::LAST; ++u) dftp_inv<F::LAST>(v + u * F::LAST);
+    store_own<P>(buf, t, v);
+    pass_sync<F::L(F::NP - 2) / P>();
+    fftp_inverse_passes<M, P, F::NP - 2>(buf, tw, td, t);
+    int s0;
+    fftp_inv<M, P, 0>(buf, tw, td, t, v, s0);
 }
 
 }  // namespace ofx

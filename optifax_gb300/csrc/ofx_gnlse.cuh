@@ -24,8 +24,7 @@ struct GnlseDev {
 };
 
 // Launches one CTA per pulse for M = n points in {512, 1024, 2048, 4096}.
-// tw1/tw2: the pass-twiddle tables of the M-point FFT.
-cudaError_t launch_gnlse(int M, const GnlseDev* d, int n_pulses, const Twiddle* tw1, const Twiddle* tw2,
-                         cudaStream_t st);
+// quad: the quarter period of W_M, from which every CTA fills its FFT tables.
+cudaError_t launch_gnlse(int M, const GnlseDev* d, int n_pulses, const Twiddle* quad, cudaStream_t st);
 
 }  // namespace ofx

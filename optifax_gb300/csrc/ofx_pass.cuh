@@ -36,7 +36,7 @@
 // shared memory, and square roots off the common path of the error class.
 #pragma once
 #include <cooperative_groups.h>
-#include "ofx_fftp.cuh"
+#include "ofx_fft.cuh"
 #include "../../include/optifax.h"
 
 namespace cg = cooperative_groups;
@@ -328,10 +328,6 @@ __device__ __forceinline__ void zphases(uint64_t tau_z4, int t, float p0, float 
 // ---------------------------------------------------------------------------
 // shared-memory layout
 // ---------------------------------------------------------------------------
-// Points per thread
-template <int M>
-constexpr int kPoints = (M >= 2048) ? 8 : 4;
-
 // Cluster exchange: CTA c holds the n2 columns [c M/C, (c+1) M/C) of the C blocks.
 // A thread takes PER consecutive columns whole, or, where there are fewer columns than
 // threads (SPLIT), LANES consecutive lanes share a column: P values each, the C-point DFT as P-point DFTs in registers and a LANES-point one by
