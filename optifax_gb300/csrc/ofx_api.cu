@@ -32,7 +32,7 @@ struct optifax_context {
     size_t xs_cap = 0;                   // in complex values
     std::vector<cudaStream_t> side;      // streams for concurrent launch groups
     std::vector<cudaEvent_t> ev;         // fork/join events
-    int* d_grid_flags = nullptr;
+    unsigned long long* d_grid_sync = nullptr;   // shared schedules: 3 words
     ofx::GnlseDev* d_gnlse_desc = nullptr;   // GNLSE: descriptors and stage scratch
     size_t gnlse_desc_cap = 0;
     float2* d_gnlse_k = nullptr;
@@ -328,7 +328,7 @@ int group_attributes(optifax_context* h, const std::vector<Group>& groups, int m
 // streams forked from and joined back into `st`, so the block scheduler
 // interleaves them: CTAs of a long group fill SMs as short ones end.
 int enqueue_groups(optifax_context* h, const std::vector<Group>& groups, int method, const VariantCfg& vc,
-                   bool shared, const PulseDev* d_desc, const std::vector<FftTables>& tabv, int* grid_flags,
+                   bool shared, const PulseDev* d_desc, const std::vector<FftTables>& tabv, unsigned long long* grid_sync,
                    cudaStream_t st, const std::vector<cudaStream_t>& side, const std::vector<cudaEvent_t>& ev) {
     cudaError_t e;
     if (groups.size() > 1) {
@@ -348,7 +348,9 @@ int enqueue_groups(optifax_context* h, const std::vector<Group>& groups, int met
         cfg.guard = vc.guard;
         cfg.shared_sched = shared ? 1 : 0;
         cfg.max_attempts_mul = 64;
-        cfg.grid_flags = grid_flags;
+        cfg.grid_flags = nullptr;
+        cfg.grid_sync = grid_sync;
+        cfg.clusters = (int)g.d.size();
         cudaStream_t ls = st;
         if (gi > 0) {
             ls = side[gi - 1];
@@ -408,8 +410,8 @@ int launch_groups(optifax_context* h, std::vector<Group>& groups, int method, co
     cudaError_t e = cudaMemcpyAsync(h->d_desc, all.data(), nb, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(h, e, "cudaMemcpyAsync(descriptors)");
     if (shared) {
-        e = cudaMemsetAsync(h->d_grid_flags, 0, 4 * sizeof(int), st);
-        if (e != cudaSuccess) return cuda_fail(h, e, "cudaMemsetAsync(grid flags)");
+        e = cudaMemsetAsync(h->d_grid_sync, 0, 4 * sizeof(unsigned long long), st);
+        if (e != cudaSuccess) return cuda_fail(h, e, "cudaMemsetAsync(grid sync)");
     }
     rc = ensure_sync_objects(h, groups.size());
     if (rc) return rc;
@@ -418,7 +420,7 @@ int launch_groups(optifax_context* h, std::vector<Group>& groups, int method, co
     if (rc) return rc;
     rc = group_attributes(h, groups, method, vc);
     if (rc) return rc;
-    rc = enqueue_groups(h, groups, method, vc, shared, h->d_desc, tabv, h->d_grid_flags, st, h->side, h->ev);
+    rc = enqueue_groups(h, groups, method, vc, shared, h->d_desc, tabv, h->d_grid_sync, st, h->side, h->ev);
     if (rc) return rc;
     return mark_done(h, st);
 }
@@ -446,10 +448,10 @@ int optifax_create(optifax_handle* out, int device) {
     optifax_context* h = new (std::nothrow) optifax_context();
     if (!h) return OPTIFAX_ERR_NO_MEMORY;
     h->device = device;
-    e = cudaMalloc(&h->d_grid_flags, 4 * sizeof(int));
+    e = cudaMalloc(&h->d_grid_sync, 4 * sizeof(unsigned long long));
     if (e != cudaSuccess) { delete h; return OPTIFAX_ERR_CUDA; }
     e = cudaEventCreateWithFlags(&h->done_ev, cudaEventDisableTiming);
-    if (e != cudaSuccess) { cudaFree(h->d_grid_flags); delete h; return OPTIFAX_ERR_CUDA; }
+    if (e != cudaSuccess) { cudaFree(h->d_grid_sync); delete h; return OPTIFAX_ERR_CUDA; }
     *out = h;
     return OPTIFAX_OK;
 }
@@ -461,7 +463,7 @@ int optifax_destroy(optifax_handle h) {
     for (auto& kv : h->tw) cudaFree(kv.second);
     for (auto& kv : h->quadtw) cudaFree(kv.second);
     if (h->d_desc) cudaFree(h->d_desc);
-    if (h->d_grid_flags) cudaFree(h->d_grid_flags);
+    if (h->d_grid_sync) cudaFree(h->d_grid_sync);
     if (h->d_xs) cudaFree(h->d_xs);
     if (h->d_gnlse_desc) cudaFree(h->d_gnlse_desc);
     if (h->d_gnlse_k) cudaFree(h->d_gnlse_k);
@@ -606,7 +608,7 @@ int optifax_propagate_graph(optifax_handle h, const optifax_pulse* pulses, int32
     if ((e = cudaStreamSynchronize(s0)) != cudaSuccess) return cleanup(cuda_fail(h, e, "table build"));
     if ((e = cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
         return cleanup(cuda_fail(h, e, "cudaStreamBeginCapture"));
-    rc = enqueue_groups(h, gv, method, vc, false, g->d_desc, tabv, h->d_grid_flags, s0, side, ev);
+    rc = enqueue_groups(h, gv, method, vc, false, g->d_desc, tabv, h->d_grid_sync, s0, side, ev);
     e = cudaStreamEndCapture(s0, &g->graph);
     if (rc) return cleanup(rc);
     if (e != cudaSuccess) return cleanup(cuda_fail(h, e, "cudaStreamEndCapture"));

@@ -90,7 +90,9 @@ struct KernelCfg {
     int guard;           // XTAL/BATCH_OP: ceil chunk count and k < Nsteps loop guard
     int shared_sched;    // 1: OR the error flags over every pulse of the launch (grid barrier)
     int max_attempts_mul;
-    int* grid_flags;     // 3 ints (shared schedule only)
+    int* grid_flags;     // wide-state pass, shared schedule: 3 ints
+    unsigned long long* grid_sync;   // FP32 pass, shared schedule: 3 words, zero before the launch
+    int clusters;        // of the launch
 };
 
 // Kernel flavours: the MEX Heun and RK23 schedules (OPTIFAX_HEUN, OPTIFAX_RK23) and
@@ -381,7 +383,7 @@ struct Smem {
     // and, for a segment's two end threads, the field and the carrier of their halo points
     static constexpr size_t off_bar = off_halo + (C > 1 ? sizeof(float2) * (8 + 8) * C : 0);
     static constexpr size_t off_red = off_bar + sizeof(uint64_t) * 6;
-    static constexpr size_t off_dred = off_red + sizeof(int) * (2 * NW + 2 * 16 + 4);
+    static constexpr size_t off_dred = off_red + sizeof(int) * (2 * NW + 2 * 16 + 4);   // warp and CTA flags, dead, grid flags
     static constexpr size_t off_run = ((off_dred + 15) & ~size_t(15)) + sizeof(double) * (NW * 4 + 2 * 16 * 4);
     static constexpr size_t bytes = off_run + sizeof(RunState);
     static_assert(bytes <= 232448 - 288, "shared memory of one CTA");
@@ -734,6 +736,39 @@ __device__ __forceinline__ void push_inverse(float2* bufg, uint32_t g, uint32_t 
 // stored before it (stage output, pushed columns).
 constexpr int kDead = 8;          // a bounded wait ran out
 
+// The same over every pulse of a shared schedule (a cooperative launch).  One 64-bit word
+// per attempt counts the clusters that have arrived and, per flag, those that raised it:
+// one atomic add per cluster and one polling thread per CTA (a cooperative-groups grid
+// barrier with a separate flag word took 5 us an attempt, this 1 to 2).  Three words in
+// turn; cluster 0 clears a word once every cluster has arrived at the next.
+__device__ __forceinline__ int combine_grid(int f, int* slot, int* dead, int attempt, int t, int c, const KernelCfg& cfg) {
+    unsigned long long* w = cfg.grid_sync + attempt % 3;
+    if (t == 0) {
+        if (c == 0) {
+            const unsigned long long v = 1ull + ((unsigned long long)(f & 1) << 16) +
+                                         ((unsigned long long)((f >> 1) & 1) << 32) +
+                                         ((unsigned long long)((f >> 2) & 1) << 48);
+            asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(w), "l"(v) : "memory");
+        }
+        const long long t0 = clock64();
+        unsigned long long v;
+        int g = 0;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
+            if ((int)(v & 0xffffu) == cfg.clusters) break;
+            if (clock64() - t0 > 4000000000LL) {
+                g = kDead;
+                break;
+            }
+        }
+        g |= ((v >> 16) & 0xffffu ? 1 : 0) | ((v >> 32) & 0xffffu ? 2 : 0) | ((v >> 48) ? 4 : 0) | (f & kDead);
+        slot[attempt & 1] = g;
+        if (blockIdx.x == 0) cfg.grid_sync[(attempt + 2) % 3] = 0;
+    }
+    __syncthreads();
+    return slot[attempt & 1];
+}
+
 template <int M, int C>
 __device__ __forceinline__ int combine_flags(int bits, int* red, uint32_t bar, uint32_t parity, int bytes, int* dead,
                                              int attempt, int t, int c, const KernelCfg& cfg) {
@@ -768,13 +803,7 @@ __device__ __forceinline__ int combine_flags(int bits, int* red, uint32_t bar, u
             if (r != c) f |= cl[r];
         f = lost ? kDead : (f & 7);
     }
-    if (cfg.shared_sched) {
-        const int gslot = attempt % 3;
-        if (t == 0 && c == 0 && f) atomicOr(&cfg.grid_flags[gslot], f);
-        cg::this_grid().sync();
-        f = *((volatile int*)&cfg.grid_flags[gslot]);
-        if (blockIdx.x == 0 && t == 0) cfg.grid_flags[(attempt + 2) % 3] = 0;
-    }
+    if (cfg.shared_sched) f = combine_grid(f, red + 2 * NW + 2 * 16 + 1, dead, attempt, t, c, cfg);
     return f;
 }
 
@@ -1169,7 +1198,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
 
                 int fl = combine_flags<M, C>(bits, red, bar_a, ph_a, kBytesA, dead, gatt, t, c, cfg);
                 ph_a ^= 1;
-                if (C > 1 && (fl & kDead)) { status |= OPTIFAX_PULSE_TIMEOUT; goto done; }
+                if (fl & kDead) { status |= OPTIFAX_PULSE_TIMEOUT; goto done; }
                 if ((opts & kForced) && gatt < P_.n_forced) fl = (P_.forced[gatt] & 3) | (fl & 4);
                 if (fl & 4) trip_status |= OPTIFAX_PULSE_NAN;
 
