@@ -348,7 +348,6 @@ int enqueue_groups(optifax_context* h, const std::vector<Group>& groups, int met
         cfg.guard = vc.guard;
         cfg.shared_sched = shared ? 1 : 0;
         cfg.max_attempts_mul = 64;
-        cfg.grid_flags = nullptr;
         cfg.grid_sync = grid_sync;
         cfg.clusters = (int)g.d.size();
         cudaStream_t ls = st;

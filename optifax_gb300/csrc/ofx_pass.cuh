@@ -90,8 +90,7 @@ struct KernelCfg {
     int guard;           // XTAL/BATCH_OP: ceil chunk count and k < Nsteps loop guard
     int shared_sched;    // 1: OR the error flags over every pulse of the launch (grid barrier)
     int max_attempts_mul;
-    int* grid_flags;     // wide-state pass, shared schedule: 3 ints
-    unsigned long long* grid_sync;   // FP32 pass, shared schedule: 3 words, zero before the launch
+    unsigned long long* grid_sync;   // shared schedule: 3 words, zero before the launch
     int clusters;        // of the launch
 };
 
@@ -769,10 +768,9 @@ __device__ __forceinline__ int combine_grid(int f, int* slot, int* dead, int att
     return slot[attempt & 1];
 }
 
-template <int M, int C>
+template <int NW, int C>
 __device__ __forceinline__ int combine_flags(int bits, int* red, uint32_t bar, uint32_t parity, int bytes, int* dead,
                                              int attempt, int t, int c, const KernelCfg& cfg) {
-    constexpr int NW = M / kPoints<M> / 32;
     const int par = attempt & 1;
     int* wf = red + par * NW;
     const int w = __reduce_or_sync(0xffffffffu, bits);
@@ -804,39 +802,6 @@ __device__ __forceinline__ int combine_flags(int bits, int* red, uint32_t bar, u
         f = lost ? kDead : (f & 7);
     }
     if (cfg.shared_sched) f = combine_grid(f, red + 2 * NW + 2 * 16 + 1, dead, attempt, t, c, cfg);
-    return f;
-}
-
-// OR of per-thread flag bits over the CTA, the cluster and (shared schedule)
-// the grid.  red[0..2] CTA slots (triple buffered by attempt), red[4..4+2*16)
-// cluster slots (double buffered).
-template <int M, int C>
-__device__ __forceinline__ int reduce_flags(int bits, int* red, int attempt, int t, int c,
-                                            const KernelCfg& cfg) {
-    int w = __reduce_or_sync(0xffffffffu, bits);
-    int slot = attempt % 3;
-    if ((t & 31) == 0 && w) atomicOr(&red[slot], w);
-    __syncthreads();
-    int f = red[slot];
-    if constexpr (C > 1) {
-        int* cl = red + 4 + (attempt & 1) * 16;
-        if (t == 0) {
-#pragma unroll 1
-            for (int r = 0; r < C; ++r) remote<C>(cl, r)[c] = f;
-        }
-        cg::this_cluster().sync();
-        f = 0;
-#pragma unroll 1
-        for (int r = 0; r < C; ++r) f |= cl[r];
-    }
-    if (cfg.shared_sched) {
-        int gslot = attempt % 3;
-        if (t == 0 && c == 0 && f) atomicOr(&cfg.grid_flags[gslot], f);
-        cg::this_grid().sync();
-        f = *((volatile int*)&cfg.grid_flags[gslot]);
-        if (blockIdx.x == 0 && t == 0) cfg.grid_flags[(attempt + 2) % 3] = 0;
-    }
-    if (t == 0) red[(attempt + 2) % 3] = 0;
     return f;
 }
 
@@ -1196,7 +1161,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     }
                 }
 
-                int fl = combine_flags<M, C>(bits, red, bar_a, ph_a, kBytesA, dead, gatt, t, c, cfg);
+                int fl = combine_flags<T / 32, C>(bits, red, bar_a, ph_a, kBytesA, dead, gatt, t, c, cfg);
                 ph_a ^= 1;
                 if (fl & kDead) { status |= OPTIFAX_PULSE_TIMEOUT; goto done; }
                 if ((opts & kForced) && gatt < P_.n_forced) fl = (P_.forced[gatt] & 3) | (fl & 4);

@@ -9,20 +9,17 @@
 //   R = ff      float-float (ofx_num.cuh), ~48-bit significands from FP32
 //               operations, for high-gain passes in which FP32 rounding of the
 //               field, amplified by the parametric gain, dominates the result.
-// One thread-block cluster of C CTAs holds one pulse of N = C M points for the
-// whole pass; each of the 256 threads of a CTA owns P = M / 256 consecutive
-// time points (field A0 in registers).  Per attempt: the NL drive and shock
-// stencil of both Heun stages (neighbour values through shared and distributed
-// shared memory), the stage combine and the error class, an OR over the cluster
-// (and the grid for a shared batch schedule).  Accepted steps: absorber, the
-// N-point transform as C-point DFTs across the cluster (distributed shared
-// memory, twiddles W_N^{n2 k1}) and an M-point Stockham transform in shared
-// memory, the per-mode dispersion factor alpha^s exp(-i beta s), the inverse,
-// 1/N.  Phases (carrier w0 t_i and z-carrier bdiffw0 z) are exact 64-bit
-// fixed-point turns evaluated by FP64 sincospi; the dispersion factor and the
-// absorber are FP64 (then rounded to R), as in the FP64 oracle.
+// Layout, transforms and cluster exchange are pass_kernel's, in R: a cluster of C CTAs
+// holds one pulse of N = C M points for the whole pass, each CTA its columns of every
+// block, P consecutive points per thread (field A0 in registers), two-point halos at the
+// segments' ends, exchanges pushed into the next user's shared memory and counted on its
+// mbarriers.  Phases (carrier w0 t_i and z-carrier bdiffw0 z) are exact 64-bit
+// fixed-point turns evaluated by FP64 sincospi; the dispersion factor and the absorber
+// are FP64 (then rounded to R), as in the FP64 oracle.  The FP64 kernel is bound by
+// GB300's FP64 pipe, the float-float kernel by issue and the cluster's latency.
 #pragma once
 #include <cooperative_groups.h>
+#include <cstring>
 #include <type_traits>
 #include "ofx_num.cuh"
 #include "ofx_pass.cuh"
@@ -37,36 +34,18 @@ struct PulseX {
     const double* beta;      // N, FFT order
     const double* G;         // S
     int* trace;              // 3 ints per attempt (k, stepmod, flags | 8 accepted), or null
-    const int* forced;
     optifax_pulse_stats* stats;
-    void* cph;               // scratch: N carrier phasors exp(i w0 t_i) in R (written by the prologue)
-    double* abc;             // scratch: N absorber factors
     void* ztab;              // scratch: zcap z-carrier phasors exp(-i bdiffw0 h p), p = 0..zcap-1, in R
     int zcap;
     uint64_t tau_theta;      // w0 dt in turns
     uint64_t tau_z;          // bdiffw0 h in turns (per z-sample)
     double w0, h, dt, max_err, min_err, sel, c_shock;
-    int N, S, nchunks, trace_cap, n_forced;
+    int N, S, nchunks, trace_cap;
 };
 
 // W_N^e (N = C M) for e in [0, N), in R; the local transforms use W_M^e = W_N^{C e}.
 template <typename R>
 struct XTables { const typename Num<R>::cplx* wn; };
-
-constexpr int kXThreads = 256;
-
-template <typename R, int M>
-struct SmemX {
-    using cplx = typename Num<R>::cplx;
-    static constexpr int T = kXThreads;
-    static constexpr size_t off_x = 0;                                    // stage output / transform
-    static constexpr size_t off_k = off_x + sizeof(cplx) * M;             // K1 / transform ping-pong
-    static constexpr size_t off_d = off_k + sizeof(cplx) * M;             // per-mode dispersion factor
-    static constexpr size_t off_edge = off_d + sizeof(cplx) * M;          // 2 parities x 2 x T
-    static constexpr size_t off_wc = off_edge + sizeof(cplx) * 4 * T;     // W_C^m, m < 8
-    static constexpr size_t off_red = off_wc + sizeof(cplx) * 8;          // flag slots
-    static constexpr size_t bytes = off_red + 256;
-};
 
 // exp(2 pi i u / 2^64) in FP64: the turn as a signed fraction in half-turns
 __device__ __forceinline__ double2 turn_unit_d(uint64_t u) {
@@ -77,118 +56,205 @@ __device__ __forceinline__ double2 turn_unit_d(uint64_t u) {
 }
 
 // ---------------------------------------------------------------------------
-// C-point DFT in registers by radix-2 DIF stages (bit-reversed output: v[q]
-// holds output bitrev(q)); wc[m] = W_C^m (m < C/2), INV uses the conjugates.
+// Shape of one kernel: P points per thread, exchange columns, transform passes.
 // ---------------------------------------------------------------------------
-template <typename R, int CP, bool INV>
-__device__ __forceinline__ void dft_small(typename Num<R>::cplx* v, const typename Num<R>::cplx* wc) {
+template <int M, int C>
+struct ShapeX {
+    static constexpr int P = M >= 4096 ? 16 : (M >= 2048 ? 8 : 4);
+    static constexpr int T = M / P, NW = T / 32;
+    static constexpr int COLS = M / C, SEGT = COLS / P;      // columns; threads of a segment
+    static constexpr bool SPLIT = COLS < T;
+    static constexpr int LANES = SPLIT ? T / COLS : 1;       // lanes that share a column
+    static constexpr int PER = SPLIT ? 1 : COLS / T;         // columns per thread
+    static constexpr int NV = SPLIT ? P : PER * (C - 1);     // outer twiddles per thread
+    static constexpr bool TABLES = M <= 2048;                // twiddles in shared memory
+    using F = FftPlan<M, P>;
+    static_assert(SEGT >= 2 || C == 1, "a segment spans threads");
+    static_assert(LANES <= 4, "lane transforms of up to 4 points");
+};
+
+// Shared-memory placement of 16-byte element m: permuted inside every 128-byte row by
+// higher bits, for conflict-free strided, unit-stride and per-thread contiguous access
+template <int P>
+__host__ __device__ constexpr int swzx(int m) {
+    return P == 4 ? m ^ ((m >> 3) & 3) ^ ((m >> 2) & 4) : (P == 8 ? m ^ ((m >> 3) & 7) : m ^ ((m >> 4) & 7));
+}
+template <int P>
+__device__ __forceinline__ int swzx_at(int s0, int k) { return (s0 ^ (swzx<P>(k) & 7)) + (k & ~7); }
+
+template <typename R, int M, int C>
+struct SmemX {
+    using cplx = typename Num<R>::cplx;
+    using SH = ShapeX<M, C>;
+    static constexpr size_t off_x = 0;                                          // transform buffer
+    static constexpr size_t off_g = off_x + sizeof(cplx) * M;                   // clusters: columns
+    static constexpr size_t off_d = off_g + (C > 1 ? sizeof(cplx) * M : 0);     // per-mode dispersion factor
+    static constexpr size_t off_tw = off_d + sizeof(cplx) * M;                  // pass twiddles
+    static constexpr size_t off_xtw = off_tw + (SH::TABLES ? sizeof(cplx) * SH::F::TW : 0);   // outer twiddles
+    static constexpr size_t off_edge = off_xtw + (SH::TABLES && C > 1 ? sizeof(cplx) * SH::NV * SH::T : 0);
+    static constexpr size_t off_halo = off_edge + sizeof(cplx) * 4 * SH::NW;    // [parity][first, last][warp]
+    // E and increment of every segment's 4 halo points; field and carrier of the end threads' two
+    static constexpr size_t off_bar = off_halo + (C > 1 ? sizeof(cplx) * 16 * C : 0);
+    static constexpr size_t off_red = off_bar + sizeof(uint64_t) * 4;
+    static constexpr size_t bytes = off_red + sizeof(int) * (2 * SH::NW + 2 * 16 + 4);
+    static_assert(bytes <= 232448 - 288, "shared memory of one CTA");
+};
+
+// ---------------------------------------------------------------------------
+// small DFTs in registers (radix-2 stages, decimation in frequency; register q ends
+// holding output bitrev(q)) and their exact-order reverse; INV: conjugate twiddles.
+// w16: W_16^m, m < 8.
+// ---------------------------------------------------------------------------
+template <typename R>
+__device__ __forceinline__ typename Num<R>::cplx rotx(typename Num<R>::cplx v, int m16, bool inv,
+                                                      const typename Num<R>::cplx* w16) {
+    using X = Num<R>;
+    if (m16 == 0) return v;
+    if (m16 == 4) return inv ? X::mul_i(v) : X::mul_mi(v);
+    return inv ? X::mulc(v, w16[m16]) : X::mul(v, w16[m16]);
+}
+template <typename R, int K>
+__device__ __forceinline__ void dftx(typename Num<R>::cplx* v, const typename Num<R>::cplx* w16) {
     using X = Num<R>;
 #pragma unroll
-    for (int hr = CP / 2; hr >= 1; hr >>= 1) {
+    for (int hr = K / 2; hr >= 1; hr >>= 1) {
 #pragma unroll
-        for (int q = 0; q < CP; ++q) {
+        for (int q = 0; q < K; ++q) {
             if (q & hr) continue;
-            const int m = (q & (hr - 1)) * (CP / (2 * hr));
             const typename X::cplx a = v[q], b = v[q + hr];
             v[q] = X::add(a, b);
-            const typename X::cplx d = X::sub(a, b);
-            if (m == 0) v[q + hr] = d;
-            else if (2 * m == CP / 2) v[q + hr] = INV ? X::mul_i(d) : X::mul_mi(d);    // W_C^{C/4} = -i
-            else v[q + hr] = INV ? X::mulc(d, wc[m]) : X::mul(d, wc[m]);
+            v[q + hr] = rotx<R>(X::sub(a, b), (q & (hr - 1)) * (K / (2 * hr)) * (16 / K), false, w16);
+        }
+    }
+}
+template <typename R, int K>
+__device__ __forceinline__ void dftx_inv(typename Num<R>::cplx* v, const typename Num<R>::cplx* w16) {
+    using X = Num<R>;
+#pragma unroll
+    for (int hr = 1; hr <= K / 2; hr <<= 1) {
+#pragma unroll
+        for (int q = 0; q < K; ++q) {
+            if (q & hr) continue;
+            const typename X::cplx a = v[q];
+            const typename X::cplx b = rotx<R>(v[q + hr], (q & (hr - 1)) * (K / (2 * hr)) * (16 / K), true, w16);
+            v[q] = X::add(a, b);
+            v[q + hr] = X::sub(a, b);
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// M-point Stockham autosort transform in shared memory (radix 4, one radix-2
-// pass when log2 M is odd), ping-pong between a and b; returns the buffer that
-// holds the result (natural order).  Pass over sub-transform length Ls: for
-// j < M/R, k = j mod Ls, x_r = in[j + r M/R] W_{R Ls}^{r k}, y = DFT_R(x),
-// out[(j - k) R + k + s Ls] = y_s.  Unnormalised; INV conjugates every twiddle.
+// M-point transform in shared memory, the scheme of ofx_fft.cuh in R.  The passes are
+// loops over one body each: unrolled, a float-float attempt was over 100 KB of
+// straight-line code and waited on instruction fetch.
 // ---------------------------------------------------------------------------
-template <typename R, int M, int C, bool INV>
-__device__ __forceinline__ typename Num<R>::cplx* stockham(typename Num<R>::cplx* a, typename Num<R>::cplx* b,
-                                                           const typename Num<R>::cplx* __restrict__ wn, int t) {
+template <typename R, int M, int C>
+struct FftX {
     using X = Num<R>;
     using cplx = typename X::cplx;
-    constexpr int T = kXThreads;
-    cplx* in = a;
-    cplx* out = b;
-    int Ls = 1;
+    using SH = ShapeX<M, C>;
+    using F = typename SH::F;
+    static constexpr int P = SH::P;
+    cplx* buf;
+    const cplx* tw;          // shared-memory pass twiddles (TABLES)
+    const cplx* wn;          // W_N, global
+    const cplx* w16;
+    int t;
+
+    // twiddle of register q in pass ps (blocks of M >> (ps RB) points)
+    __device__ __forceinline__ cplx twiddle(int ps, int q, int off) const {
+        const int LR = (M >> (ps * F::RB)) / P;
+        if constexpr (SH::TABLES) {
+            // entries before pass ps: (P - 1)/P (M + M/P + ...) = M - (M >> ps RB)
+            return tw[M - (M >> (ps * F::RB)) + (q - 1) * LR + off];
+        } else {
+            return wn[(size_t)((off * brev4(q, F::RB)) << (ps * F::RB)) * C];
+        }
+    }
+    __device__ __forceinline__ void load_own(cplx (&v)[P]) const {
+        const int s0 = swzx<P>(P * t);
+#pragma unroll
+        for (int j = 0; j < P; ++j) v[j] = buf[swzx_at<P>(s0, j)];
+    }
+    __device__ __forceinline__ void store_own(cplx* b, const cplx (&v)[P]) const {
+        const int s0 = swzx<P>(P * t);
+#pragma unroll
+        for (int j = 0; j < P; ++j) b[swzx_at<P>(s0, j)] = v[j];
+    }
+    static __device__ __forceinline__ void sync(int group) {
+        if (group <= 32) __syncwarp();
+        else __syncthreads();
+    }
+    __device__ __forceinline__ void forward(cplx (&v)[P]) const {
 #pragma unroll 1
-    for (; Ls * 4 <= M; Ls *= 4) {
-        const int stride = M / (4 * Ls);
+        for (int ps = 0; ps < F::NP - 1; ++ps) {
+            const int LR = (M >> (ps * F::RB)) / P, off = t & (LR - 1), base = (t - off) * P + off;
 #pragma unroll
-        for (int u = 0; u < (M / 4 + T - 1) / T; ++u) {
-            const int j = t + u * T;
-            if (j >= M / 4) break;
-            const int k = j & (Ls - 1);
-            cplx x0 = in[j], x1 = in[j + M / 4], x2 = in[j + M / 2], x3 = in[j + 3 * (M / 4)];
-            if (Ls > 1) {
-                const int e = k * stride;
-                const cplx w1 = wn[(size_t)e * C], w2 = wn[(size_t)(2 * e) * C], w3 = wn[(size_t)(3 * e) * C];
-                x1 = INV ? X::mulc(x1, w1) : X::mul(x1, w1);
-                x2 = INV ? X::mulc(x2, w2) : X::mul(x2, w2);
-                x3 = INV ? X::mulc(x3, w3) : X::mul(x3, w3);
+            for (int q = 0; q < P; ++q) v[q] = buf[swzx<P>(base + q * LR)];
+            dftx<R, P>(v, w16);
+#pragma unroll
+            for (int q = 1; q < P; ++q) v[q] = X::mul(v[q], twiddle(ps, q, off));
+#pragma unroll
+            for (int q = 0; q < P; ++q) buf[swzx<P>(base + q * LR)] = v[q];
+            sync(LR);
+        }
+        load_own(v);
+#pragma unroll
+        for (int u = 0; u < P / F::LAST; ++u) dftx<R, F::LAST>(v + u * F::LAST, w16);
+    }
+    // v[q] returns point t + q M/P
+    __device__ __forceinline__ void inverse(cplx (&v)[P]) const {
+#pragma unroll
+        for (int u = 0; u < P / F::LAST; ++u) dftx_inv<R, F::LAST>(v + u * F::LAST, w16);
+        store_own(buf, v);
+        sync(F::L(F::NP - 2) / P);
+#pragma unroll 1
+        for (int ps = F::NP - 2; ps >= 0; --ps) {
+            const int LR = (M >> (ps * F::RB)) / P, off = t & (LR - 1), base = (t - off) * P + off;
+#pragma unroll
+            for (int q = 0; q < P; ++q) v[q] = buf[swzx<P>(base + q * LR)];
+#pragma unroll
+            for (int q = 1; q < P; ++q) v[q] = X::mulc(v[q], twiddle(ps, q, off));
+            dftx_inv<R, P>(v, w16);
+            if (ps > 0) {
+#pragma unroll
+                for (int q = 0; q < P; ++q) buf[swzx<P>(base + q * LR)] = v[q];
+                sync(LR * P);
             }
-            const cplx a0 = X::add(x0, x2), a1 = X::sub(x0, x2);
-            const cplx b0 = X::add(x1, x3);
-            const cplx d13 = X::sub(x1, x3);
-            const cplx b1 = INV ? X::mul_i(d13) : X::mul_mi(d13);
-            const int base = (j - k) * 4 + k;
-            out[base] = X::add(a0, b0);
-            out[base + Ls] = X::add(a1, b1);
-            out[base + 2 * Ls] = X::sub(a0, b0);
-            out[base + 3 * Ls] = X::sub(a1, b1);
         }
-        __syncthreads();
-        cplx* tmp = in; in = out; out = tmp;
     }
-    if (Ls < M) {   // radix-2 pass, Ls = M / 2
+};
+
+// 16-byte values into a peer's shared memory, counted on its mbarrier
+template <typename V>
+__device__ __forceinline__ void st_async16(uint32_t addr, V v, uint32_t bar) {
+    static_assert(sizeof(V) == 16, "16-byte values");
+    uint32_t w[4];
+    memcpy(w, &v, 16);
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                     addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(bar) : "memory");
+}
+template <typename V>
+__device__ __forceinline__ V shfl16(V v, int src, bool up, bool down, int mask) {
+    uint32_t w[4];
+    memcpy(w, &v, 16);
 #pragma unroll
-        for (int u = 0; u < (M / 2 + T - 1) / T; ++u) {
-            const int j = t + u * T;
-            if (j >= M / 2) break;
-            const int k = j;                       // j < Ls
-            const cplx w = wn[(size_t)k * C];
-            const cplx x0 = in[j];
-            const cplx x1 = INV ? X::mulc(in[j + M / 2], w) : X::mul(in[j + M / 2], w);
-            out[k] = X::add(x0, x1);
-            out[k + Ls] = X::sub(x0, x1);
-        }
-        __syncthreads();
-        cplx* tmp = in; in = out; out = tmp;
-    }
-    return in;
+    for (int i = 0; i < 4; ++i)
+        w[i] = up ? __shfl_up_sync(0xffffffffu, w[i], src)
+                  : (down ? __shfl_down_sync(0xffffffffu, w[i], src) : __shfl_xor_sync(0xffffffffu, w[i], mask));
+    memcpy(&v, w, 16);
+    return v;
 }
 
 // Error class of one point from E and E - A1: pct = 100 |E - A1| / (|E| + 1) in
 // FP64 (as the FP64 oracle), MEX rule (points with |E| = 0 skipped; >= maxErr,
-// else >= minErr) or NEE rule (> maxErr; >= minErr).  Float-float first
-// classifies from its FP32 leading parts and recomputes in FP64 only when pct
-// lies within 1e-5 (relative) of a threshold, so decisions are FP64's.
+// else >= minErr) or NEE rule (> maxErr; >= minErr).
 template <typename R, bool NEE>
 __device__ __forceinline__ int classify_x(typename Num<R>::cplx e, typename Num<R>::cplx d, double maxE,
                                           double minE) {
-    double pct, ae;
-    if constexpr (sizeof(R) == sizeof(ff) && !std::is_same<R, double>::value) {
-        const float ae32 = sqrtf(e.rh * e.rh + e.ih * e.ih);
-        const float p32 = 100.f * sqrtf(d.rh * d.rh + d.ih * d.ih) / (ae32 + 1.f);
-        const bool near = fabsf(p32 - (float)maxE) <= 1e-5f * (float)maxE ||
-                          fabsf(p32 - (float)minE) <= 1e-5f * (float)minE;
-        if (!near) {
-            pct = (double)p32;
-            ae = (double)ae32;
-        } else {
-            const double2 ed = Num<R>::to_d(e), dd = Num<R>::to_d(d);
-            ae = hypot(ed.x, ed.y);
-            pct = 100.0 * hypot(dd.x, dd.y) / (ae + 1.0);
-        }
-    } else {
-        const double2 ed = Num<R>::to_d(e), dd = Num<R>::to_d(d);
-        ae = hypot(ed.x, ed.y);
-        pct = 100.0 * hypot(dd.x, dd.y) / (ae + 1.0);
-    }
+    const double2 ed = Num<R>::to_d(e), dd = Num<R>::to_d(d);
+    const double ae = hypot(ed.x, ed.y);
+    const double pct = 100.0 * hypot(dd.x, dd.y) / (ae + 1.0);
     int bits = 0;
     if (NEE) {
         if (pct > maxE) bits |= 1;
@@ -201,115 +267,232 @@ __device__ __forceinline__ int classify_x(typename Num<R>::cplx e, typename Num<
     return bits;
 }
 
+// OR of the classes of a thread's points.  FP32 magnitudes (of E and of K2 - K1, which
+// is 2 (E - A1) to the working precision) decide where the largest error is 1e-5
+// (relative) away from both thresholds and below the upper one; everything else goes
+// through the FP64 classes, so every decision is FP64's.  Two FP64 hypot and a division
+// a point were a third of the FP64 kernel's arithmetic.
+template <typename R, bool NEE, int P>
+__device__ __forceinline__ int classify_points(const typename Num<R>::cplx (&e)[P], const typename Num<R>::cplx (&d2)[P],
+                                               const typename Num<R>::cplx (&a1)[P], const Bounds& B, double maxE,
+                                               double minE) {
+    using X = Num<R>;
+    float qmax = 0.f, emin = 3e38f, sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        const float2 em = X::abs32(e[j]), dm = X::abs32(d2[j]);
+        const float e2 = fmaf(em.x, em.x, em.y * em.y), dd = fmaf(dm.x, dm.x, dm.y * dm.y);
+        const float r = rcp_fast(sqrt_fast(e2) + 1.f);
+        qmax = fmaxf(qmax, dd * r * r);
+        emin = fminf(emin, e2);
+        sum += e2;
+    }
+    const bool low = qmax < B.qlo0, high = qmax > B.qlo1;
+    if (sum < 1e30f && qmax < B.qhi && (low || (high && (NEE || emin > 1e-30f)))) return high ? 2 : 0;
+    int bits = 0;
+#pragma unroll
+    for (int j = 0; j < P; ++j) bits |= classify_x<R, NEE>(e[j], X::sub(e[j], a1[j]), maxE, minE);
+    return bits;
+}
+
 // ---------------------------------------------------------------------------
-// the kernel
+// the kernel: layout, exchange steps A to D and their ordering as pass_kernel
+// (ofx_pass.cuh), in R
 // ---------------------------------------------------------------------------
 template <typename R, int M, int C, bool NEE>
-__global__ void __launch_bounds__(kXThreads, 1)
+__global__ void __launch_bounds__(M / ShapeX<M, C>::P, 1)
 passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) {
     using X = Num<R>;
     using cplx = typename X::cplx;
     using real = typename X::real;
-    constexpr int T = kXThreads;
-    constexpr int P = M / T;
-    constexpr int N = M * C;
-    static_assert(P >= 1 && P <= 16 && M % T == 0, "M must be 256..4096");
-    using SM = SmemX<R, M>;
+    using SH = ShapeX<M, C>;
+    constexpr int T = SH::T, P = SH::P, COLS = SH::COLS, NW = SH::NW;
+    constexpr int N = M * C, LOG2M = ilog2(M);
+    using SM = SmemX<R, M, C>;
     extern __shared__ __align__(16) unsigned char smem[];
     cplx* bufX = reinterpret_cast<cplx*>(smem + SM::off_x);
-    cplx* bufK = reinterpret_cast<cplx*>(smem + SM::off_k);
-    cplx* Dc = reinterpret_cast<cplx*>(smem + SM::off_d);
+    cplx* bufG = reinterpret_cast<cplx*>(smem + SM::off_g);
+    cplx* D_s = reinterpret_cast<cplx*>(smem + SM::off_d);
+    cplx* tw_s = reinterpret_cast<cplx*>(smem + SM::off_tw);
+    cplx* xtw_s = reinterpret_cast<cplx*>(smem + SM::off_xtw);
     cplx* edge = reinterpret_cast<cplx*>(smem + SM::off_edge);
-    cplx* wc = reinterpret_cast<cplx*>(smem + SM::off_wc);
+    cplx* halo_e = reinterpret_cast<cplx*>(smem + SM::off_halo);
+    cplx* halo_d = halo_e + 4 * C;
     int* red = reinterpret_cast<int*>(smem + SM::off_red);
+    int* dead = red + 2 * NW + 2 * 16;
+    __shared__ PulseX sP;
+    __shared__ cplx w16[8];
 
     const int t = threadIdx.x;
     const int c = (C > 1) ? (int)cg::this_cluster().block_rank() : 0;
     const int p = blockIdx.x / C;
-    __shared__ PulseX sP;
-    if (t == 0) sP = pulses[p];
+    const cplx* __restrict__ wn = tabs.wn;
+    if (t == 0) {
+        sP = pulses[p];
+        *dead = 0;
+    }
+    if (t < 8) w16[t] = wn[(size_t)t * (N / 16)];
     __syncthreads();
     const PulseX& Pd = sP;
-    const cplx* __restrict__ wn = tabs.wn;
-    cplx* cph = reinterpret_cast<cplx*>(Pd.cph);
+    const FftX<R, M, C> fft{bufX, tw_s, wn, w16, t};
 
-    // ---- prologue: field, carrier phasors, absorber, small-DFT twiddles ----
-    for (int i = t; i < 64; i += T) red[i] = 0;
-    if (C > 1 && t < C / 2) wc[t] = wn[(size_t)t * (N / C)];
-    cplx a[P];
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-        const int i = c * M + P * t + j;
-        a[j] = X::from(Pd.E_in[i]);
-        const uint64_t jt = (uint64_t)(long long)time_index(i, N, cfg.time_mode);
-        cph[i] = X::from(turn_unit_d(Pd.tau_theta * jt));
-        double f = 1.0;
-        if (cfg.abc_mode == ABC_NEE) {   // NEE_CPU.m:114-121
-            const int it = (i < N / 2) ? i : i - N;
-            const double range = (double)(N - 1) * Pd.dt, a2t = fabs(2.0 * (double)it * Pd.dt);
-            if (range - a2t < 0.25 * range) {
-                const double sh = 1.0 / cosh(24.0 * (1.0 - a2t / range));
-                f = 1.0 - sh * sh;
+    // ---- prologue: twiddle tables, barriers, field, carrier, absorber, z-phasors ----
+    if constexpr (SH::TABLES) {
+        using F = typename SH::F;
+        int o = 0;
+#pragma unroll 1
+        for (int ps = 0; ps < F::NP - 1; ++ps) {
+            const int L = M >> (ps * F::RB), LR = L / P;
+#pragma unroll 1
+            for (int i = t; i < (P - 1) * LR; i += T) {
+                const int q = i / LR + 1, off = i % LR;
+                tw_s[o + i] = wn[(size_t)(off * bitrev(q, F::RB) * (M / L)) * C];
             }
-        } else if (cfg.abc_mode != ABC_NONE) {   // OPO_CUDA_BATCH_XTAL.cu:105-137
-            const int gi1 = 6 * (N / 16), gi2 = 10 * (N / 16);
-            if (i > gi1 && i < gi2) {
-                if (cfg.abc_mode == ABC_HARD) f = 0.0;
-                else {
-                    const double g = cosh((48.0 / (double)N) * fabs((double)i - (double)N / 2.0));
-                    f = 1.0 - 1.0 / (g * g);
-                }
+            o += (P - 1) * LR;
+        }
+    }
+    // outer twiddle i of this thread: W_N^{n2 k1}; k1 of a register of the column DFT
+    auto outer_k = [&](int i) {
+        if constexpr (SH::SPLIT) return brev4(i, ilog2(P)) + P * brev4(t % SH::LANES, ilog2(SH::LANES));
+        else return brev4(i % (C > 1 ? C - 1 : 1) + 1, ilog2(C));
+    };
+    auto outer = [&](int i) -> cplx {
+        if constexpr (SH::TABLES) return xtw_s[i * T + t];
+        const int n2 = c * COLS + (SH::SPLIT ? t / SH::LANES : t * SH::PER + i / (C > 1 ? C - 1 : 1));
+        return wn[(size_t)n2 * outer_k(i)];
+    };
+    cplx inner[SH::SPLIT ? P : 1];            // W_C^{lane ka}
+    if constexpr (C > 1) {
+        if constexpr (SH::TABLES) {
+#pragma unroll 1
+            for (int i = 0; i < SH::NV; ++i) {
+                const int n2 = c * COLS + (SH::SPLIT ? t / SH::LANES : t * SH::PER + i / (C - 1));
+                xtw_s[i * T + t] = wn[(size_t)n2 * outer_k(i)];
             }
         }
-        Pd.abc[i] = f;
+        if constexpr (SH::SPLIT) {
+#pragma unroll
+            for (int r = 0; r < P; ++r)
+                inner[r] = wn[(size_t)((t % SH::LANES) * brev4(r, ilog2(P)) % C) * (N / C)];
+        }
+    }
+    constexpr bool LOCAL = C <= 4;
+    constexpr int kAll = (int)sizeof(cplx) * (LOCAL ? M - COLS : M);
+    constexpr int kBytesA = 4 * (C - 1) + 64 * C, kBytesD = 64 * C;
+    const uint32_t bars = smem_u32(smem + SM::off_bar);
+    const uint32_t bar_a = bars, bar_b = bars + 8, bar_c = bars + 16, bar_d = bars + 24;
+    if (C > 1 && t == 0) {
+        for (int i = 0; i < 4; ++i) bar_init(bars + 8 * i);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        bar_arm(bar_a, kBytesA);
+        bar_arm(bar_b, kAll);
+        bar_arm(bar_c, kAll);
+        bar_arm(bar_d, kBytesD);
+    }
+    uint32_t ph_a = 0, ph_x = 0;
+    const int seg = t / SH::SEGT, tin = t % SH::SEGT;
+    const int i0 = seg * M + c * COLS + P * tin;             // this thread's first point
+    const bool lend = C > 1 && tin == 0, rend = C > 1 && tin == SH::SEGT - 1;
+    auto carrier = [&](int i) {
+        return X::from(turn_unit_d(Pd.tau_theta * (uint64_t)(long long)time_index(i, N, cfg.time_mode)));
+    };
+    auto absorber = [&](int i) {
+        if (cfg.abc_mode == ABC_NEE) {                       // NEE_CPU.m:114-121
+            const int it = (i < N / 2) ? i : i - N;
+            const double range = (double)(N - 1) * Pd.dt, a2t = fabs(2.0 * (double)it * Pd.dt);
+            if (!(range - a2t < 0.25 * range)) return 1.0;
+            const double sh = 1.0 / cosh(24.0 * (1.0 - a2t / range));
+            return 1.0 - sh * sh;
+        }
+        if (cfg.abc_mode == ABC_NONE || !(i > 6 * (N / 16) && i < 10 * (N / 16))) return 1.0;
+        if (cfg.abc_mode == ABC_HARD) return 0.0;            // OPO_CUDA_BATCH_XTAL.cu:105-137
+        const double g = cosh((48.0 / (double)N) * fabs((double)i - (double)N / 2.0));
+        return 1.0 - 1.0 / (g * g);
+    };
+    cplx a[P], cph[P];
+    bool absorbs = false;              // whether a point of this thread lies in the absorber
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        a[j] = X::from(Pd.E_in[i0 + j]);
+        cph[j] = carrier(i0 + j);
+        const double f = absorber(i0 + j);
+        if (f != 1.0) absorbs = true;
+    }
+    // the end threads' two halo points: hs[0..1] field, hs[2..3] carrier
+    cplx* hs = halo_e + 8 * C + 4 * (2 * seg + (rend ? 1 : 0));
+    if (lend || rend) {
+        const int i1 = lend ? (i0 + N - 1) % N : (i0 + P) % N;
+        const int i2 = lend ? (i0 + N - 2) % N : (i0 + P + 1) % N;
+        hs[0] = X::from(Pd.E_in[i1]); hs[1] = X::from(Pd.E_in[i2]);
+        hs[2] = carrier(i1); hs[3] = carrier(i2);
     }
     // z-carrier phasor of every z-sample of the pass, shared by the cluster's CTAs
-    // (the FP64 sincospi leaves the per-stage path)
     cplx* ztab = reinterpret_cast<cplx*>(Pd.ztab);
     for (int pz = c * T + t; pz < Pd.zcap; pz += C * T)
         ztab[pz] = X::from(turn_unit_d((uint64_t)0 - Pd.tau_z * (uint64_t)pz));
     if constexpr (C > 1) cg::this_cluster().sync(); else __syncthreads();
 
-    const double h = Pd.h, sel = Pd.sel, Sd = (double)Pd.S, cs = Pd.c_shock;
+    const double h = Pd.h, sel = Pd.sel, Sd = (double)Pd.S;
     const double maxE = Pd.max_err, minE = Pd.min_err;
-    const double invN = 1.0 / (double)N;
+    const Bounds bounds(50.f, (float)maxE, (float)minE);
+    constexpr double invN = 1.0 / (double)N;
     const int guard = cfg.guard;
-    const long long max_attempts = (long long)cfg.max_attempts_mul * (long long)(Pd.S + 16) + 64;
+    const int max_attempts = cfg.max_attempts_mul * (Pd.S + 16) + 64;
     const int nchunks = Pd.nchunks;
     const bool rec = (c == 0 && t == 0);
+    const real csr = X::rfrom(Pd.c_shock);
 
     double k = NEE ? 1.0 : 0.0, stepprev = 4.0, stepmod = 4.0;
     long long q = 0;
     int s_cached = -1;
     int attempt = 0, n_acc = 0, n_rej = 0, status = 0, par = 0;
 
-    // NL drive of this thread's points at z-phasor zz (into nl), then the
-    // neighbours' edge values through shared / distributed shared memory
-    auto nl_stage = [&](const cplx (&src)[P], cplx zz, cplx (&nl)[P], cplx& L, cplx& Rr) {
-#pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const cplx e = X::mul(cph[c * M + P * t + j], zz);
-            const cplx s = src[j];
-            const real m2 = X::norm2(s);
-            const cplx s2 = X::mul(s, s);
-            // A^2 e + 2 |A|^2 conj(e)
-            nl[j] = X::add(X::mul(s2, e), X::scale(X::pow2(X::conj(e), 2.0), m2));
-        }
-        cplx* eg = edge + par * 2 * T;
-        eg[2 * t] = nl[0];
-        eg[2 * t + 1] = nl[P - 1];
-        csync<C>();
-        if (t > 0) L = eg[2 * t - 1];
-        else L = remote<C>(eg, (c + C - 1) % C)[2 * T - 1];
-        if (t < T - 1) Rr = eg[2 * t + 2];
-        else Rr = remote<C>(eg, (c + 1) % C)[0];
-        par ^= 1;
+    // A^2 e + 2 |A|^2 conj(e) with e = carrier z: A conj(3 Re w + i Im w) with w = A e
+    auto drive = [&](cplx s, cplx car, cplx zz) -> cplx {
+        const cplx w = X::mul(s, X::mul(car, zz));
+        return X::mulc(s, X::make(X::triple(X::re(w)), X::im(w)));
     };
     // K = -i hG (NL - i cs (NL[+1] - NL[-1]))
-    auto k_of = [&](cplx nm, cplx n0, cplx np, real hg, real csr) -> cplx {
-        const cplx d = X::sub(np, nm);
-        const cplx in = X::sub(n0, X::mul_i(X::scale(d, csr)));
-        return X::mul_mi(X::scale(in, hg));
+    auto k_of = [&](cplx nm, cplx n0, cplx np, real hg) -> cplx {
+        return X::mul_mi(X::scale(X::sub_i(n0, X::sub(np, nm), csr), hg));
+    };
+    // the neighbours' adjacent drive values; hv: the halo point's (end threads)
+    auto edges = [&](const cplx (&nl)[P], cplx hv, cplx& L, cplx& Rr) {
+        L = shfl16(nl[P - 1], 1, true, false, 0);
+        Rr = shfl16(nl[0], 1, false, true, 0);
+        if constexpr (SH::SEGT > 32) {
+            const int w = t >> 5, lane = t & 31;
+            cplx* e = edge + par * 2 * NW;
+            if (lane == 0) e[w] = nl[0];
+            if (lane == 31) e[NW + w] = nl[P - 1];
+            __syncthreads();
+            if (lane == 0) L = e[NW + (w > 0 ? w - 1 : NW - 1)];
+            if (lane == 31) Rr = e[w < NW - 1 ? w + 1 : 0];
+        }
+        if (lend) L = hv;
+        if (rend) Rr = hv;
+        par ^= 1;
+    };
+    auto zphasor = [&](long long pz) -> cplx {
+        return pz < Pd.zcap ? ztab[pz] : X::from(turn_unit_d((uint64_t)0 - Pd.tau_z * (uint64_t)pz));
+    };
+    // a value into CTA r's buffer at element i (same place in every CTA)
+    auto push = [&](cplx* b, int r, int i, cplx v, uint32_t bar) {
+        if (LOCAL && r == c) {
+            b[i] = v;
+        } else {
+            const uint32_t src = smem_u32(b), dst = cluster_addr(src, r);
+            st_async16(dst + 16 * i, v, dst + (bar - src));
+        }
+    };
+    // v: point `col` of this CTA's segment sg, if it is one of the segment's two first or
+    // last points, into the neighbours' halo slots
+    auto push_halo_x = [&](cplx* b, int sg, int col, cplx v, uint32_t bar) {
+        if (col >= 2 && col < COLS - 2) return;
+        const bool first = col < 2;
+        const int slot = first ? 4 * seg_left<C>(sg, c) + 2 + col : 4 * seg_right<C>(sg, c) + col - (COLS - 2);
+        const uint32_t src = smem_u32(b), dst = cluster_addr(src, first ? (c + C - 1) % C : (c + 1) % C);
+        st_async16(dst + 16 * slot, v, dst + (bar - src));
     };
 
     for (int chunk = 0; chunk < nchunks; ++chunk) {
@@ -322,47 +505,63 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
             const double kpos = NEE ? k - 1.0 : k;
             bool accepted = false;
             const real hg = X::rfrom((stepmod * h) * Pd.G[kidx]);
-            const real csr = X::rfrom(cs);
-            int bits = 0;
+            cplx e[P];
+            int bits;
             {
-                cplx nl[P], L, Rr;
-                // ---- stage 1: K1 = f(A0) at z = k ----
-                auto zphasor = [&](long long pz) -> cplx {
-                    return pz < Pd.zcap ? ztab[pz] : X::from(turn_unit_d((uint64_t)0 - Pd.tau_z * (uint64_t)pz));
-                };
-                cplx z = zphasor((long long)kpos);
-                nl_stage(a, z, nl, L, Rr);
-                // A1 = A0 + (K1/2 + K1/2) (MEX) or A0 + K1 (NEE_CPU.m:73); K1 kept in
-                // shared memory, A1 formed again where it is needed
-                auto a1_of = [&](int j) -> cplx {
-                    const cplx k1 = bufK[P * t + j];
-                    return NEE ? X::add(a[j], k1) : X::add(a[j], X::add(X::pow2(k1, 0.5), X::pow2(k1, 0.5)));
-                };
+                cplx nl[P], k1[P], a1[P], d2[P], kh = X::zero();
 #pragma unroll
-                for (int j = 0; j < P; ++j)
-                    bufK[P * t + j] = k_of(j == 0 ? L : nl[j - 1], nl[j], j == P - 1 ? Rr : nl[j + 1], hg, csr);
-                // ---- stage 2: K2 = f(A1) at z = k + stepmod ----
-                z = zphasor((long long)(kpos + stepmod));
-                {
-                    cplx a1[P];
+                for (int j = 0; j < P; ++j) { a1[j] = a[j]; k1[j] = X::zero(); }
+                // stage 0: K1 = f(A0) at z = k; stage 1: K2 = f(A1) at z = k + stepmod, with
+                // A1 = A0 + (K1/2 + K1/2) (MEX) or A0 + K1 (NEE_CPU.m:73), the same value.
+                // One body for both (code size).
+#pragma unroll 1
+                for (int st = 0; st < 2; ++st) {
+                    const cplx z = zphasor((long long)(st ? kpos + stepmod : kpos));
 #pragma unroll
-                    for (int j = 0; j < P; ++j) a1[j] = a1_of(j);
-                    nl_stage(a1, z, nl, L, Rr);
+                    for (int j = 0; j < P; ++j) nl[j] = drive(a1[j], cph[j], z);
+                    cplx hv = X::zero(), L, Rr;
+                    if (lend || rend) {      // drive of the adjacent halo point, and its K1
+                        hv = drive(X::add(hs[0], kh), hs[2], z);
+                        if (st == 0) {
+                            const cplx n2 = drive(hs[1], hs[3], z), in = lend ? nl[0] : nl[P - 1];
+                            kh = k_of(lend ? n2 : in, hv, lend ? in : n2, hg);
+                        }
+                    }
+                    edges(nl, hv, L, Rr);
+#pragma unroll
+                    for (int j = 0; j < P; ++j) {
+                        const cplx kk = k_of(j == 0 ? L : nl[j - 1], nl[j], j == P - 1 ? Rr : nl[j + 1], hg);
+                        if (st == 0) {
+                            k1[j] = kk;
+                            a1[j] = X::add(a[j], kk);
+                        } else {
+                            d2[j] = kk;
+                        }
+                    }
                 }
 #pragma unroll
                 for (int j = 0; j < P; ++j) {
-                    const cplx k2 = k_of(j == 0 ? L : nl[j - 1], nl[j], j == P - 1 ? Rr : nl[j + 1], hg, csr);
-                    const cplx k1 = bufK[P * t + j];
                     // E = A0 + (K2/2 + K1/2) (MEX) or (A0 + K1/2) + K2/2 (NEE_CPU.m:75)
-                    const cplx e = NEE ? X::add(X::add(a[j], X::pow2(k1, 0.5)), X::pow2(k2, 0.5))
-                                       : X::add(a[j], X::add(X::pow2(k2, 0.5), X::pow2(k1, 0.5)));
-                    // pct = 100 |E - A1| / (|E| + 1) (OPO_CUDA_BATCH_XTAL.cu:325-349; NEE_CPU.m:73-79)
-                    bits |= classify_x<R, NEE>(e, X::sub(e, a1_of(j)), maxE, minE);
-                    bufX[P * t + j] = X::scale(e, X::rfrom(Pd.abc[c * M + P * t + j]));
+                    e[j] = NEE ? X::add_half(X::add_half(a[j], k1[j]), d2[j]) : X::add_half(a[j], X::add(d2[j], k1[j]));
+                    d2[j] = X::sub(d2[j], k1[j]);
+                }
+                // pct = 100 |E - A1| / (|E| + 1) (OPO_CUDA_BATCH_XTAL.cu:325-349; NEE_CPU.m:73-79)
+                bits = classify_points<R, NEE, P>(e, d2, a1, bounds, maxE, minE);
+            }
+            if (absorbs) {
+#pragma unroll
+                for (int j = 0; j < P; ++j) e[j] = X::scale(e[j], X::rfrom(absorber(i0 + j)));
+            }
+            fft.store_own(C > 1 ? bufG : bufX, e);
+            if constexpr (C > 1) {
+                if (lend || rend || P < 2) {
+#pragma unroll
+                    for (int j = 0; j < P; ++j) push_halo_x(halo_e, seg, P * tin + j, e[j], bar_a);
                 }
             }
-            int fl = reduce_flags<M, C>(bits, red, attempt, t, c, cfg);
-            if (Pd.forced && attempt < Pd.n_forced) fl = (Pd.forced[attempt] & 3) | (fl & 4);
+            int fl = combine_flags<NW, C>(bits, red, bar_a, ph_a, kBytesA, dead, attempt, t, c, cfg);
+            ph_a ^= 1;
+            if (fl & kDead) { status |= OPTIFAX_PULSE_TIMEOUT; goto done; }
             if (fl & 4) status |= OPTIFAX_PULSE_NAN;
 
             if ((fl & 1) && stepmod > 1.0 && (NEE || (k - stepmod) > 0.0)) {
@@ -371,6 +570,8 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
                     Pd.trace[3 * attempt + 2] = fl & 7;
                 }
                 ++n_rej;
+                // the next attempt's flags and halos must not overtake this one's
+                if constexpr (C > 1) cg::this_cluster().sync();
                 if (!NEE) k = k - stepmod;
                 stepmod = stepmod - 1.0;
                 stepprev = stepmod;
@@ -395,96 +596,142 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
                 }
 
                 // ---- linear sub-step: A0 = IFFT(D FFT(E abc)) / N ----
+                cplx v[P];
+                if constexpr (C > 1) {
+                    if (lend || rend) {
+                        hs[0] = halo_e[4 * seg + (lend ? 1 : 2)];
+                        hs[1] = halo_e[4 * seg + (lend ? 0 : 3)];
+                    }
+                    // C-point DFTs of the own columns, twiddle -> the blocks' owners
+                    if constexpr (SH::SPLIT) {
+                        const int l = t % SH::LANES, col = t / SH::LANES;
+#pragma unroll
+                        for (int i = 0; i < P; ++i) v[i] = bufG[swzx<P>((i * SH::LANES + l) * COLS + col)];
+                        dftx<R, P>(v, w16);
+#pragma unroll
+                        for (int r = 1; r < P; ++r) v[r] = X::mul(v[r], inner[r]);
+#pragma unroll
+                        for (int hr = SH::LANES / 2; hr >= 1; hr >>= 1) {
+                            const bool up = (l & hr) != 0, turn = SH::LANES == 4 && hr == 2 && (l & 1);
+#pragma unroll
+                            for (int i = 0; i < P; ++i) {
+                                const cplx o = shfl16(v[i], 0, false, false, hr);
+                                cplx d = up ? X::sub(o, v[i]) : X::add(v[i], o);
+                                v[i] = up && turn ? X::mul_mi(d) : d;
+                            }
+                        }
+#pragma unroll
+                        for (int r = 0; r < P; ++r)
+                            push(bufX, outer_k(r), swzx<P>(c * COLS + col), X::mul(v[r], outer(r)), bar_b);
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < SH::PER; ++u) {
+                            cplx y[C];
+#pragma unroll
+                            for (int n1 = 0; n1 < C; ++n1) y[n1] = bufG[swzx<P>(n1 * COLS + t * SH::PER + u)];
+                            dftx<R, C>(y, w16);
+#pragma unroll
+                            for (int r = 0; r < C; ++r) {
+                                if (r > 0) y[r] = X::mul(y[r], outer(u * (C - 1) + r - 1));
+                                push(bufX, brev4(r, ilog2(C)), swzx<P>(c * COLS + t * SH::PER + u), y[r], bar_b);
+                            }
+                        }
+                    }
+                }
                 if (s_used != s_cached) {
-                    // D_k = alpha_k^s exp(-i beta_k s) in FP64 (OPO_CUDA_BATCH_XTAL.cu:255-305)
+                    // D_k = alpha_k^s exp(-i beta_k s) / N in FP64 (OPO_CUDA_BATCH_XTAL.cu:255-305)
 #pragma unroll 1
-                    for (int m = t; m < M; m += T) {
-                        const int kk = c + C * m;
+                    for (int j = 0; j < P; ++j) {
+                        const int kk = c + C * bitrev(P * t + j, LOG2M);
                         double sn, cn;
                         sincos(-Pd.beta[kk] * (double)s_used, &sn, &cn);
                         const double al = Pd.alpha[kk];
                         const double af = (al == 1.0) ? 1.0 : pow(al, (double)s_used);
-                        Dc[m] = X::from(make_double2(cn * af, sn * af));
+                        D_s[j * T + t] = X::from(make_double2(cn * af * invN, sn * af * invN));   // 1/N: exact
                     }
                     s_cached = s_used;
                 }
-                // forward: C-point DFTs across the cluster (this CTA takes n2 in
-                // [c M/C, (c+1) M/C)), gathered from every CTA's E (complete at the
-                // flag barrier) and stored into the owners' bufK; the barrier after
-                // the stores also ends every gather, so bufX is free for the transform
-                cplx* src = bufX;
-                cplx* oth = bufK;
                 if constexpr (C > 1) {
-                    constexpr int PER = M / C;
-                    constexpr int NPT = PER >= T ? PER / T : 1;
-                    constexpr int LOGC = (C == 2) ? 1 : (C == 4) ? 2 : (C == 8) ? 3 : 4;
-                    if (PER >= T || t < PER) {
-                        cplx v[NPT][C];
+                    if constexpr (LOCAL) __syncthreads();
+                    bar_wait(bar_b, ph_x, dead);
+                    if (t == 0) bar_arm(bar_b, kAll);
+                }
+                fft.forward(v);
 #pragma unroll
-                        for (int u = 0; u < NPT; ++u)
+                for (int j = 0; j < P; ++j) v[j] = X::mul(v[j], D_s[j * T + t]);
+                fft.inverse(v);
+                if constexpr (C > 1) {
+                    // outputs (points t + q M/P of the block) -> their columns' owners; with more
+                    // CTAs than points a thread does not add to every peer's bytes, which then
+                    // say nothing about its reads of the transform buffer
+                    if constexpr (C > P) __syncthreads();
 #pragma unroll
-                            for (int n1 = 0; n1 < C; ++n1) v[u][n1] = remote<C>(bufX, n1)[c * PER + t + u * T];
+                    for (int i = 0; i < P; ++i) {
+                        const int m = t + i * T;
+                        push(bufG, m / COLS, swzx<P>(c * COLS + m % COLS), v[i], bar_c);
+                    }
+                    if constexpr (LOCAL) __syncthreads();
+                    bar_wait(bar_c, ph_x, dead);
+                    if (t == 0) bar_arm(bar_c, kAll);
+                    // undo the twiddles, inverse C-point DFTs -> own points
+                    if constexpr (SH::SPLIT) {
+                        const int l = t % SH::LANES, col = t / SH::LANES;
 #pragma unroll
-                        for (int u = 0; u < NPT; ++u) {
-                            const int n2 = c * PER + t + u * T;
-                            dft_small<R, C, false>(v[u], wc);
+                        for (int r = 0; r < P; ++r)
+                            v[r] = X::mulc(bufG[swzx<P>(outer_k(r) * COLS + col)], outer(r));
+#pragma unroll
+                        for (int hr = 1; hr <= SH::LANES / 2; hr <<= 1) {
+                            const bool up = (l & hr) != 0, turn = SH::LANES == 4 && hr == 2 && (l & 1);
+#pragma unroll
+                            for (int i = 0; i < P; ++i) {
+                                if (up && turn) v[i] = X::mul_i(v[i]);
+                                const cplx o = shfl16(v[i], 0, false, false, hr);
+                                v[i] = up ? X::sub(o, v[i]) : X::add(v[i], o);
+                            }
+                        }
+#pragma unroll
+                        for (int r = 1; r < P; ++r) v[r] = X::mulc(v[r], inner[r]);
+                        dftx_inv<R, P>(v, w16);
+#pragma unroll
+                        for (int i = 0; i < P; ++i) {
+                            const int n1 = i * SH::LANES + l;
+                            bufX[swzx<P>(n1 * COLS + col)] = v[i];
+                            push_halo_x(halo_d, n1, col, v[i], bar_d);
+                        }
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < SH::PER; ++u) {
+                            const int col = t * SH::PER + u;
+                            cplx y[C];
 #pragma unroll
                             for (int r = 0; r < C; ++r) {
-                                const int k1 = bitrev(r, LOGC);
-                                remote<C>(bufK, k1)[n2] = k1 == 0 ? v[u][r] : X::mul(v[u][r], wn[(size_t)n2 * k1]);
+                                y[r] = bufG[swzx<P>(brev4(r, ilog2(C)) * COLS + col)];
+                                if (r > 0) y[r] = X::mulc(y[r], outer(u * (C - 1) + r - 1));
+                            }
+                            dftx_inv<R, C>(y, w16);
+#pragma unroll
+                            for (int n1 = 0; n1 < C; ++n1) {
+                                bufX[swzx<P>(n1 * COLS + col)] = y[n1];
+                                push_halo_x(halo_d, n1, col, y[n1], bar_d);
                             }
                         }
                     }
-                    cg::this_cluster().sync();
-                    src = bufK;
-                    oth = bufX;
+                    __syncthreads();
+                    if (lend || rend) {
+                        bar_wait(bar_d, ph_x, dead);
+                        if (t == 0) bar_arm(bar_d, kBytesD);
+                        hs[0] = halo_d[4 * seg + (lend ? 1 : 2)];
+                        hs[1] = halo_d[4 * seg + (lend ? 0 : 3)];
+                    }
+                    ph_x ^= 1;
                 } else {
+                    const int s0 = swzx<P>(t);
+#pragma unroll
+                    for (int i = 0; i < P; ++i) bufX[swzx_at<P>(s0, i * T)] = v[i];
                     __syncthreads();
                 }
-                cplx* fbuf = stockham<R, M, C, false>(src, oth, wn, t);
-                cplx* obuf = (fbuf == bufX) ? bufK : bufX;
-#pragma unroll 1
-                for (int m = t; m < M; m += T) fbuf[m] = X::mul(fbuf[m], Dc[m]);
-                __syncthreads();
-                cplx* gbuf = stockham<R, M, C, true>(fbuf, obuf, wn, t);
-                cplx* hbuf = (gbuf == bufX) ? bufK : bufX;
-                const real sN = X::rfrom(invN);
-                if constexpr (C > 1) {
-                    // inverse: every CTA's inverse transform is complete at the first
-                    // barrier (and nobody reads hbuf any more); gather the n2 slice,
-                    // undo the twiddles, inverse C-point DFTs, 1/N, store into the owners' hbuf
-                    constexpr int PER = M / C;
-                    constexpr int NPT = PER >= T ? PER / T : 1;
-                    constexpr int LOGC = (C == 2) ? 1 : (C == 4) ? 2 : (C == 8) ? 3 : 4;
-                    cg::this_cluster().sync();
-                    if (PER >= T || t < PER) {
-                        cplx v[NPT][C];
-#pragma unroll
-                        for (int u = 0; u < NPT; ++u) {
-                            const int n2 = c * PER + t + u * T;
-#pragma unroll
-                            for (int k1 = 0; k1 < C; ++k1) {
-                                const cplx y = remote<C>(gbuf, k1)[n2];
-                                v[u][k1] = k1 == 0 ? y : X::mulc(y, wn[(size_t)n2 * k1]);
-                            }
-                        }
-#pragma unroll
-                        for (int u = 0; u < NPT; ++u) {
-                            const int n2 = c * PER + t + u * T;
-                            dft_small<R, C, true>(v[u], wc);
-#pragma unroll
-                            for (int r = 0; r < C; ++r) remote<C>(hbuf, bitrev(r, LOGC))[n2] = X::scale(v[u][r], sN);
-                        }
-                    }
-                    cg::this_cluster().sync();
-#pragma unroll
-                    for (int j = 0; j < P; ++j) a[j] = hbuf[P * t + j];
-                } else {
-#pragma unroll
-                    for (int j = 0; j < P; ++j) a[j] = X::scale(gbuf[P * t + j], sN);
-                }
+                fft.load_own(a);
                 q += s_used;
-                __syncthreads();
             }
             ++attempt;
             if (!NEE || accepted) k = k + stepmod;
@@ -492,7 +739,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
     }
 done:
 #pragma unroll
-    for (int j = 0; j < P; ++j) Pd.A_out[c * M + P * t + j] = X::to_d(a[j]);
+    for (int j = 0; j < P; ++j) Pd.A_out[i0 + j] = X::to_d(a[j]);
     if (rec && Pd.stats) {
         optifax_pulse_stats st;
         st.attempts = attempt; st.accepted = n_acc; st.rejected = n_rej; st.status = status;
@@ -500,6 +747,7 @@ done:
         st.reserved[0] = 1; st.reserved[1] = st.reserved[2] = 0;
         *Pd.stats = st;
     }
+    if constexpr (C > 1) cg::this_cluster().sync();      // no CTA leaves while a peer may still write its memory
 }
 
 }  // namespace ofx

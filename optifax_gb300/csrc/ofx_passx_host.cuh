@@ -25,13 +25,13 @@ template <typename R>
 struct XKernel {
     void (*fn)(const PulseX*, XTables<R>, KernelCfg);
     size_t smem;
-    int M, C;
+    int threads, M, C;
     bool nee;
 };
 
 template <typename R, int M, int C, bool NEE>
 XKernel<R> xkernel() {
-    return XKernel<R>{&passx_kernel<R, M, C, NEE>, SmemX<R, M>::bytes, M, C, NEE};
+    return XKernel<R>{&passx_kernel<R, M, C, NEE>, SmemX<R, M, C>::bytes, ShapeX<M, C>::T, M, C, NEE};
 }
 
 // W_N^e for e < N in FP64, rounded to R
@@ -44,28 +44,59 @@ __global__ void passx_twiddles(typename Num<R>::cplx* out, int n) {
     out[e] = Num<R>::from(make_double2(c, s));
 }
 
-// points per CTA: clusters of up to 16 CTAs, at most 1024 points per CTA below
-// 2^15 points (the FP64 rate bounds this kernel, so more SMs per pulse pay).
-// Float-float spreads further up to 2^12 points, 512 per CTA (GB300, 0.3 mm pass:
-// 2^11 13.6 against 18.6 us per attempt, 2^12 16.3 against 19.3); at 2^13, 16 CTAs
-// of 512 points lose to 8 of 1024 (26.6 against 21.7 us), and 2048 or 4096 points
-// per CTA lose at every size (2^14: 50.1 and 90.6 against 38.6 us).
+// How many clusters of a kernel the GPU holds at once (0 on an error)
 template <typename R>
-inline int passx_cta_points(int n) {
-    int m = n < 1024 ? n : 1024;
-    if (std::is_same<R, ff>::value && n <= 4096) m = n < 512 ? n : 512;
-    if (n / m > 16) m = n / 16;
-    return m;
+inline int xresident(const XKernel<R>& k) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)k.C, 1, 1);
+    lc.blockDim = dim3((unsigned)k.threads, 1, 1);
+    lc.dynamicSmemBytes = k.smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = k.C; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    lc.attrs = &attr;
+    lc.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k.fn, &lc) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+template <typename R>
+inline cudaError_t xattributes(const XKernel<R>& k) {
+    cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+    if (e == cudaSuccess && k.C > 8) e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+
+// The kernel of n points for a call of B pulses.  The FP64 rate and the serial chain
+// bound these kernels, so a pulse takes as many SMs as a cluster allows: 512 points per
+// CTA up to 2^13 points, then n / 16 (one pulse, us per attempt, GB300, FP64 at 1024 and
+// 512 points per CTA: 2^10 38 and 26, 2^12 48 and 30, 2^13 53 and 33; float-float at 2^13
+// 19 and 16).  Several pulses on one schedule run at once, so they take 1024 points per
+// CTA (float-float: 512 up to 2^12 points) where the wider shape's clusters do not all
+// fit the GPU.
+template <typename R>
+inline const XKernel<R>* xchoose(const std::vector<XKernel<R>>& kernels, int n, int B, bool nee) {
+    auto find = [&](int m) -> const XKernel<R>* {
+        if (n / m > 16) m = n / 16;
+        for (const auto& k : kernels)
+            if (k.M == m && k.C == n / m && k.nee == nee) return &k;
+        return nullptr;
+    };
+    const XKernel<R>* narrow = find(n < 1024 || (std::is_same<R, ff>::value && n <= 4096) ? 512 : 1024);
+    const XKernel<R>* wide = find(512);
+    if (!narrow || !wide) return narrow;
+    if (wide != narrow && B > 1 && (xattributes(*wide) != cudaSuccess || B > xresident(*wide))) return narrow;
+    return wide;
 }
 
 template <typename R>
 struct XWork {
     int n_tab = 0;
     typename Num<R>::cplx* tab = nullptr;
-    void* cph = nullptr;
-    size_t cph_bytes = 0;
-    double* abc = nullptr;
-    size_t abc_bytes = 0;
     void* ztab = nullptr;
     size_t ztab_bytes = 0;
     PulseX* desc = nullptr;
@@ -73,7 +104,7 @@ struct XWork {
     int* trace = nullptr;
     size_t trace_n = 0;
     optifax_pulse_stats* stats = nullptr;
-    int* flags = nullptr;
+    unsigned long long* flags = nullptr;
 };
 
 template <typename T>
@@ -97,12 +128,12 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
     if (64LL * (S + 16) + 64 > 0x7fffffffLL) return OPTIFAX_ERR_INVALID_ARGUMENT;
     VariantCfg vc;
     if (variant == OPTIFAX_VARIANT_ODE23 || !variant_cfg(variant, &vc)) return OPTIFAX_ERR_INVALID_ARGUMENT;
-    const int M = passx_cta_points<R>(n), C = n / M;
-    const XKernel<R>* ke = nullptr;
-    for (const auto& k : kernels)
-        if (k.M == M && k.C == C && k.nee == (vc.nee != 0)) ke = &k;
+    const XKernel<R>* ke = xchoose(kernels, n, B, vc.nee != 0);
     if (!ke) return OPTIFAX_ERR_UNSUPPORTED;
-    if (B > 1 && B * C > 148) return OPTIFAX_ERR_UNSUPPORTED;   // one co-resident wave (cooperative launch)
+    const int C = ke->C;
+    // one co-resident wave (cooperative launch), counted in the narrow shape
+    const int narrow = n < 1024 || (std::is_same<R, ff>::value && n <= 4096) ? 512 : 1024;
+    if (B > 1 && B * (n / narrow > 16 ? 16 : n / narrow) > 148) return OPTIFAX_ERR_UNSUPPORTED;
 
     int rc;
     using cplx = typename Num<R>::cplx;
@@ -113,8 +144,6 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
         if (cudaGetLastError() != cudaSuccess) { w.n_tab = 0; return OPTIFAX_ERR_CUDA; }
         w.n_tab = n;
     }
-    if ((rc = grow_dev(&w.cph, &w.cph_bytes, sizeof(cplx) * (size_t)n * B))) return rc;
-    if ((rc = grow_dev(&w.abc, &w.abc_bytes, sizeof(double) * (size_t)n * B))) return rc;
     const int zcap = S + 64;     // z-samples k + stepmod of a pass stay below S + stepmod's clamp
     if ((rc = grow_dev(&w.ztab, &w.ztab_bytes, sizeof(cplx) * (size_t)zcap * B))) return rc;
     size_t dn = w.desc_n * sizeof(PulseX);
@@ -126,8 +155,8 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
     if (tcap) w.trace_n = tn / (3 * sizeof(int));
     size_t sb = w.stats ? sizeof(optifax_pulse_stats) : 0;
     if ((rc = grow_dev(&w.stats, &sb, sizeof(optifax_pulse_stats)))) return rc;
-    size_t fb = w.flags ? 4 * sizeof(int) : 0;
-    if ((rc = grow_dev(&w.flags, &fb, 4 * sizeof(int)))) return rc;
+    size_t fb = w.flags ? 4 * sizeof(*w.flags) : 0;
+    if ((rc = grow_dev(&w.flags, &fb, 4 * sizeof(*w.flags)))) return rc;
 
     std::vector<PulseX> d((size_t)B);
     int nchunks = (int)((double)S / sel);
@@ -143,8 +172,6 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
         x.trace = (b == 0 && tcap) ? w.trace : nullptr;
         x.trace_cap = (b == 0) ? (int)tcap : 0;
         x.stats = (b == 0) ? w.stats : nullptr;
-        x.cph = reinterpret_cast<cplx*>(w.cph) + (size_t)b * n;
-        x.abc = w.abc + (size_t)b * n;
         x.ztab = reinterpret_cast<cplx*>(w.ztab) + (size_t)b * zcap;
         x.zcap = zcap;
         x.tau_theta = turns_fixed((long double)w0 * (long double)dt);
@@ -155,13 +182,10 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
         x.N = n; x.S = S; x.nchunks = nchunks;
     }
     if (cudaMemcpyAsync(w.desc, d.data(), sizeof(PulseX) * (size_t)B, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemsetAsync(w.flags, 0, 4 * sizeof(int), st) != cudaSuccess ||
+        cudaMemsetAsync(w.flags, 0, 4 * sizeof(*w.flags), st) != cudaSuccess ||
         cudaMemsetAsync(w.stats, 0, sizeof(optifax_pulse_stats), st) != cudaSuccess)
         return OPTIFAX_ERR_CUDA;
-    if (cudaFuncSetAttribute(ke->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ke->smem) != cudaSuccess)
-        return OPTIFAX_ERR_CUDA;
-    if (C > 8 && cudaFuncSetAttribute(ke->fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        return OPTIFAX_ERR_CUDA;
+    if (xattributes(*ke) != cudaSuccess) return OPTIFAX_ERR_CUDA;
     KernelCfg cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.time_mode = vc.time_mode;
@@ -169,12 +193,13 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
     cfg.guard = vc.guard;
     cfg.shared_sched = B > 1 ? 1 : 0;
     cfg.max_attempts_mul = 64;
-    cfg.grid_flags = w.flags;
+    cfg.grid_sync = w.flags;
+    cfg.clusters = B;
     XTables<R> tabs;
     tabs.wn = w.tab;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)(B * C), 1, 1);
-    lc.blockDim = dim3(kXThreads, 1, 1);
+    lc.blockDim = dim3((unsigned)ke->threads, 1, 1);
     lc.dynamicSmemBytes = ke->smem;
     lc.stream = st;
     cudaLaunchAttribute attrs[2];
