@@ -9,16 +9,21 @@
 // after the last), projection to 4 channels plus a residual connection to the
 // first 4 input channels: y = x[:4] + Q h + q.
 //
+// A layer's two products with a spatial output -- inverse transform and pointwise mix
+// forward, their transposes backward -- run in one kernel per 128 bins (k_layer), whose
+// epilogue adds them, applies bias and GELU (or its derivative) and writes what the next
+// products read; no FP32 intermediate goes through memory but the kept pre-activation.
+//
 // Data layouts (per batch of B samples): "channel-major" Hc[c][b][x] and
 // "point-major" Ht[b][x][c] copies of every activation, so that every product is
 // an A . B^T GEMM with both operands K-major for the tensor-core kernel
 // (optifax_gemm_bf16):
 //   spectral transform   S[(c,b)][m'] = Hc . F^T         (F: 64 x L, m' = 2m + re/im)
-//   inverse transform    Y1[(o,b)][x] = T . G^T          (G: L x 64)
-//   pointwise mix        Y2[(b,x)][o] = Ht . Wp^T        (Wp: 64 x 64, [o][c])
+//   inverse transform    Y1[x][o] = G . T_b^T            (G: L x 64, T: [b][o][m'])
+//   pointwise mix        Y2[x][o] = Ht_b . Wp^T          (Wp: 64 x 64, [o][c])
 //   weight gradient      dWp[o][c]    = dZc[o][(b,x)] . Hc[c][(b,x)]^T
-//   backward transforms  dT = dZc . GT^T, dHs = dS . FT^T, dHp = dZt . WpT^T
-// The per-mode complex channel mixing T[(o,b)][m] = sum_c S[(c,b)][m] W[c][o][m]
+//   backward transforms  dT = dZc . GT^T, dH = FT . dS_b^T + dZt_b . WpT^T
+// The per-mode complex channel mixing T[b][o][m] = sum_c S[(c,b)][m] W[c][o][m]
 // and the element-wise parts run on the CUDA cores.  GEMM operands and
 // activations are BF16; accumulation, pre-activations, gradients, biases, the
 // master weights and the Adam moments are FP32.
@@ -30,6 +35,8 @@
 #include <cstring>
 
 #include "../../include/optifax.h"
+#include "ofx_tc.cuh"
+#include "ofx_tmap.cuh"
 
 typedef __nv_bfloat16 bf16;
 
@@ -48,8 +55,6 @@ constexpr long long off_ws(int l) { return OFF_L0 + l * LAYER_SIZE; }
 constexpr long long off_wp(int l) { return off_ws(l) + LAYER_WS; }
 constexpr long long off_b(int l) { return off_wp(l) + W * W; }
 static_assert(off_wp(0) % 8 == 0 && LAYER_SIZE % 8 == 0, "BF16 GEMM operands must stay 16-byte aligned");
-
-constexpr int XT = 4;   // 32-point x tiles per block in the transposing kernels
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_d(float z) {
@@ -111,61 +116,227 @@ __global__ void k_lift(const float* __restrict__ x, const bf16* __restrict__ Pw,
     for (int j = 0; j < W / 8; ++j) dst[j] = pack[j];
 }
 
-// T[(o,b)][m] = sum_c S[(c,b)][m] W[c][o][m]   (complex)
-__global__ void k_mix_fwd(const float* __restrict__ S, const bf16* __restrict__ Ws, int B, bf16* __restrict__ T) {
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (idx >= (long long)W * B * MODES) return;
-    const int m = (int)(idx % MODES);
-    const long long t = idx / MODES;
-    const int b = (int)(t % B), o = (int)(t / B);
-    float ar = 0.f, ai = 0.f;
-    for (int c = 0; c < W; ++c) {
-        const float* s = S + ((long long)c * B + b) * SPEC + 2 * m;
-        const __nv_bfloat162 w = *reinterpret_cast<const __nv_bfloat162*>(Ws + (((long long)c * W + o) * MODES + m) * 2);
-        const float wr = __low2float(w), wi = __high2float(w);
-        ar = fmaf(s[0], wr, fmaf(-s[1], wi, ar));
-        ai = fmaf(s[0], wi, fmaf(s[1], wr, ai));
+// Channel mixing per mode: out[b][u][m] = sum_v in[(v,b)][m] w (or conj w) with w =
+// Ws[v][u][m] (forward, u = o) or Ws[u][v][m] conjugated (backward, u = c).  One block
+// per (u, group of samples); its 32 lanes are the modes and its 8 warps take 8 v each, so
+// the weights are read once per sample group in whole rows and a sum is 8 steps deep
+// (a thread per output walked 64 dependent steps: 17 us for one sample or 32).
+constexpr int MIXB = 4;           // samples per block
+template <bool BWD, int U>        // U outputs per block share its reads of `in`
+__global__ void __launch_bounds__(256) k_mix(const float* __restrict__ in, const bf16* __restrict__ Ws, int B,
+                                             bf16* __restrict__ out) {
+    __shared__ float2 red[8][MIXB][MODES];
+    const int m = threadIdx.x & 31, wp = threadIdx.x >> 5, u0 = blockIdx.x * U, b0 = blockIdx.y * MIXB;
+    float ar[U][MIXB] = {}, ai[U][MIXB] = {};
+#pragma unroll
+    for (int i = 0; i < W / 8; ++i) {
+        const int v = wp * (W / 8) + i;
+        float2 s[MIXB];
+#pragma unroll
+        for (int k = 0; k < MIXB; ++k)
+            s[k] = b0 + k < B ? *reinterpret_cast<const float2*>(in + ((long long)v * B + b0 + k) * SPEC + 2 * m)
+                              : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const long long wi = BWD ? ((long long)(u0 + q) * W + v) : ((long long)v * W + u0 + q);
+            const __nv_bfloat162 w = *reinterpret_cast<const __nv_bfloat162*>(Ws + (wi * MODES + m) * 2);
+            const float wr = __low2float(w), wj = BWD ? -__high2float(w) : __high2float(w);
+#pragma unroll
+            for (int k = 0; k < MIXB; ++k) {
+                ar[q][k] = fmaf(s[k].x, wr, fmaf(-s[k].y, wj, ar[q][k]));
+                ai[q][k] = fmaf(s[k].x, wj, fmaf(s[k].y, wr, ai[q][k]));
+            }
+        }
     }
-    bf16* d = T + ((long long)o * B + b) * SPEC + 2 * m;
-    d[0] = __float2bfloat16(ar);
-    d[1] = __float2bfloat16(ai);
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+        if (q) __syncthreads();
+#pragma unroll
+        for (int k = 0; k < MIXB; ++k) red[wp][k][m] = make_float2(ar[q][k], ai[q][k]);
+        __syncthreads();
+        if (wp < MIXB && b0 + wp < B) {
+            float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                s.x += red[i][wp][m].x;
+                s.y += red[i][wp][m].y;
+            }
+            *reinterpret_cast<__nv_bfloat162*>(out + ((long long)(b0 + wp) * W + u0 + q) * SPEC + 2 * m) =
+                __floats2bfloat162_rn(s.x, s.y);
+        }
+    }
+}
+// one output per block up to 8 samples (64 blocks a group), four above, where the groups
+// fill the GPU and reading `in` once per output is what costs
+template <bool BWD>
+void launch_mix(const float* in, const bf16* Ws, int B, bf16* out, cudaStream_t st) {
+    const unsigned groups = (unsigned)((B + MIXB - 1) / MIXB);
+    if (B <= 8) k_mix<BWD, 1><<<dim3(W, groups), 256, 0, st>>>(in, Ws, B, out);
+    else k_mix<BWD, 4><<<dim3(W / 4, groups), 256, 0, st>>>(in, Ws, B, out);
 }
 
-// Z = Y1[c][b][x] + Y2[b][x][c] + bias[c]; h = act(Z) -> Hc, Ht (and Z kept for the backward)
-__global__ void k_combine_fwd(const float* __restrict__ Y1, const float* __restrict__ Y2, const float* __restrict__ bias,
-                              int B, int L, int act, float* __restrict__ Zs, bf16* __restrict__ Hc,
-                              bf16* __restrict__ Ht) {
-    __shared__ float tile[32][W + 1];
-    const int b = blockIdx.y;
-    for (int xt = 0; xt < XT; ++xt) {
-        const int x0 = (blockIdx.x * XT + xt) * 32;
-        if (x0 >= L) break;
-        for (int r = 0; r < 8; ++r) {
-            const int i = threadIdx.x + 256 * r, xi = i / W, c = i % W;
-            tile[xi][c] = Y2[((long long)b * L + x0 + xi) * W + c];
+// ---- one layer's spatial part ---------------------------------------------
+// A CTA takes 128 bins of one sample: D1[x][u] = R . X_b^T (R: G or FT, X: T or dS) and
+// D2[x][u] = H_b . V^T (H: Ht or dZt, V: Wp or its transpose), K = 64 each, two
+// tcgen05 accumulators of 64 columns; thread = bin in the epilogue.  48 KB of operands
+// and 128 TMEM columns, so four CTAs share an SM and their loads, products and epilogues
+// overlap.  Bound by the epilogue's traffic (batch 32, 4096 bins: 84 MB forward).
+enum { LAYER_FWD = 0, LAYER_BWD = 1, LAYER_BWD_IN = 2 };
+struct LayerArgs {
+    const float* bias;      // FWD
+    float* Z;               // FWD: pre-activation out [c][b][x] (or null); BWD: in
+    bf16 *Hc, *Ht;          // FWD: activation; BWD: dZ
+    const float* x;         // BWD_IN: network input [b][CIN][x]
+    float* db;              // BWD: bias gradient; BWD_IN: this launch's partial sums [CTA][W][8]
+    int* err;
+    int B, L, act;
+};
+constexpr int LA = 128 * 64 * 2, LB = 64 * 64 * 2;
+constexpr int LAYER_SMEM = 2 * LA + 2 * LB + 1024;
+
+template <int MODE>
+__global__ void __launch_bounds__(128, 4)
+    k_layer(const __grid_constant__ CUtensorMap tmR, const __grid_constant__ CUtensorMap tmH,
+            const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmV, LayerArgs a) {
+    using namespace ofx_tc;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles =
+        reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ __align__(8) uint64_t full, accum;
+    __shared__ uint32_t tmem_slot;
+    __shared__ float s_bias[W];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = blockIdx.y, x0 = blockIdx.x * 128;
+    if (threadIdx.x == 0) {
+        mbar_init(&full, 1);
+        mbar_init(&accum, 1);
+        fence_barrier_init();
+    }
+    if (MODE == LAYER_FWD && threadIdx.x < W) s_bias[threadIdx.x] = a.bias[threadIdx.x];
+    if (warp == 0) tmem_alloc(&tmem_slot, 128);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    if (threadIdx.x == 0) {
+        mbar_expect_tx(&full, 2 * LA + 2 * LB);
+        tma_load_2d(tiles, &tmR, 0, x0, &full);
+        tma_load_2d(tiles + LA, &tmH, 0, b * a.L + x0, &full);
+        tma_load_2d(tiles + 2 * LA, &tmX, 0, b * W, &full);
+        tma_load_2d(tiles + 2 * LA + LB, &tmV, 0, 0, &full);
+        if (mbar_wait(&full, 0)) {
+            tc_fence_after();
+            constexpr uint32_t idesc = idesc_bf16_f32(128, 64);
+#pragma unroll
+            for (int d = 0; d < 2; ++d)
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    mma_bf16(tmem + 64 * d, desc_kmajor_sw128(smem_u32(tiles + d * LA) + kk * 32),
+                             desc_kmajor_sw128(smem_u32(tiles + 2 * LA + d * LB) + kk * 32), idesc, kk > 0 ? 1u : 0u);
+        }
+        mma_commit(&accum);
+    }
+    __syncwarp();
+    // a load that did not arrive in time leaves `full` in its first phase: every thread sees it
+    const bool ok = mbar_wait(&accum, 0) && mbar_try_wait(&full, 0);
+    __syncwarp();
+    tc_fence_after();
+
+    const int x = x0 + threadIdx.x;
+    const bool live = ok && x < a.L;
+    const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+    float* gt = reinterpret_cast<float*>(tiles);              // BWD: g as [x][u], padded (operands are consumed)
+    constexpr int LDG = W + 1;
+    if (MODE != LAYER_FWD) __syncthreads();
+#pragma unroll 1
+    for (int u0 = 0; u0 < W; u0 += 16) {
+        float d1[16], d2[16];
+        tmem_ld16(taddr + u0, d1);
+        tmem_ld16(taddr + 64 + u0, d2);
+        uint4 pack[2];
+        bf16* hp = reinterpret_cast<bf16*>(pack);
+        if (MODE == LAYER_FWD) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const float z = d1[j] + d2[j] + s_bias[u0 + j];
+                const long long o = ((long long)(u0 + j) * a.B + b) * a.L + x;
+                if (a.Z && live) a.Z[o] = z;
+                hp[j] = __float2bfloat16(a.act ? gelu(z) : z);
+                if (live) a.Hc[o] = hp[j];
+            }
+        } else {
+            float zv[16];                                     // every load in flight before any store
+            if (MODE == LAYER_BWD) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    zv[j] = live ? a.Z[((long long)(u0 + j) * a.B + b) * a.L + x] : 0.f;
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                float g = d1[j] + d2[j];
+                if (MODE == LAYER_BWD) {
+                    g *= gelu_d(zv[j]);
+                    hp[j] = __float2bfloat16(g);
+                    if (live) a.Hc[((long long)(u0 + j) * a.B + b) * a.L + x] = hp[j];
+                }
+                gt[threadIdx.x * LDG + u0 + j] = live ? g : 0.f;
+            }
+        }
+        if (MODE != LAYER_BWD_IN && live) {
+            uint4* dst = reinterpret_cast<uint4*>(a.Ht + ((long long)b * a.L + x) * W + u0);
+            dst[0] = pack[0];
+            dst[1] = pack[1];
+        }
+    }
+    if (MODE == LAYER_BWD) {
+        __syncthreads();
+        const int c = threadIdx.x & 63, h = threadIdx.x >> 6;
+        float s = 0.f;
+#pragma unroll 8
+        for (int r = 0; r < 64; ++r) s += gt[(h * 64 + r) * LDG + c];
+        __syncthreads();
+        if (h) gt[c] = s;
+        __syncthreads();
+        if (!h) atomicAdd(&a.db[c], s + gt[c]);
+    }
+    if (MODE == LAYER_BWD_IN) {
+        // dP[c][i] = sum_x g[x][c] x_i, dp[c] = sum_x g[x][c]
+        float* xs = gt + 128 * LDG;                           // [x][8]: the inputs and a one
+        for (int i = 0; i < 8; ++i)
+            xs[threadIdx.x * 8 + i] =
+                i < CIN ? (live ? a.x[((long long)b * CIN + i) * a.L + x] : 0.f) : (i == CIN ? 1.f : 0.f);
+        __syncthreads();
+        const int c = threadIdx.x & 63, h = threadIdx.x >> 6;
+        float s[CIN + 1] = {};
+#pragma unroll 4
+        for (int r = 0; r < 64; ++r) {
+            const float g = gt[(h * 64 + r) * LDG + c];
+            const float4 p = *reinterpret_cast<const float4*>(xs + (h * 64 + r) * 8);
+            const float4 q = *reinterpret_cast<const float4*>(xs + (h * 64 + r) * 8 + 4);
+            s[0] = fmaf(g, p.x, s[0]); s[1] = fmaf(g, p.y, s[1]); s[2] = fmaf(g, p.z, s[2]); s[3] = fmaf(g, p.w, s[3]);
+            s[4] = fmaf(g, q.x, s[4]); s[5] = fmaf(g, q.y, s[5]); s[6] += g;
         }
         __syncthreads();
-        float hv[8];
-        for (int r = 0; r < 8; ++r) {
-            const int i = threadIdx.x + 256 * r, c = i / 32, xi = i % 32;
-            const long long o = ((long long)c * B + b) * L + x0 + xi;
-            const float z = Y1[o] + tile[xi][c] + bias[c];
-            if (Zs) Zs[o] = z;
-            const float h = act ? gelu(z) : z;
-            Hc[o] = __float2bfloat16(h);
-            hv[r] = h;
-        }
+        if (h)
+            for (int i = 0; i <= CIN; ++i) gt[c * 8 + i] = s[i];
         __syncthreads();
-        for (int r = 0; r < 8; ++r) {
-            const int i = threadIdx.x + 256 * r, c = i / 32, xi = i % 32;
-            tile[xi][c] = hv[r];
+        // partial sums to memory, one row per CTA: 448 atomics from each of 1024 CTAs queued on
+        // the same few sectors for 50 us
+        if (!h) {
+            float4* row = reinterpret_cast<float4*>(a.db + ((long long)b * gridDim.x + blockIdx.x) * W * 8 + c * 8);
+            row[0] = make_float4(s[0] + gt[c * 8], s[1] + gt[c * 8 + 1], s[2] + gt[c * 8 + 2], s[3] + gt[c * 8 + 3]);
+            row[1] = make_float4(s[4] + gt[c * 8 + 4], s[5] + gt[c * 8 + 5], s[6] + gt[c * 8 + 6], 0.f);
         }
-        __syncthreads();
-        for (int r = 0; r < 8; ++r) {
-            const int i = threadIdx.x + 256 * r, xi = i / W, c = i % W;
-            Ht[((long long)b * L + x0 + xi) * W + c] = __float2bfloat16(tile[xi][c]);
-        }
-        __syncthreads();
+    }
+    if (!ok && threadIdx.x == 0) {
+        atomicOr(a.err, 1);
+        mbar_wait(&full, 0);               // copies still in flight land before the memory is released
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 128);
     }
 }
 
@@ -198,6 +369,27 @@ __global__ void k_proj_fwd(const bf16* __restrict__ Ht, const bf16* __restrict__
         y[((long long)b * COUT + j) * L + xx] = xin[((long long)b * CIN + j) * L + xx] + acc[j];
 }
 
+// dP[c][i] and dp[c] from k_layer's partial rows [n][W][8]; block: 32 of the 512 columns,
+// 8 row lanes; blockIdx.y splits the rows
+__global__ void __launch_bounds__(256) k_lift_sum(const float* __restrict__ part, int n, float* __restrict__ dP,
+                                                  float* __restrict__ dp) {
+    __shared__ float red[8][32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
+    float s = 0.f;
+#pragma unroll 4
+    for (int r = blockIdx.y * 8 + wp; r < n; r += 8 * gridDim.y) s += part[(long long)r * (W * 8) + col];
+    red[wp][lane] = s;
+    __syncthreads();
+    if (wp == 0) {
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t += red[i][lane];
+        const int c = col >> 3, i = col & 7;
+        if (i < CIN) atomicAdd(&dP[c * CIN + i], t);
+        else if (i == CIN) atomicAdd(&dp[c], t);
+    }
+}
+
 // ---- loss and backward ---------------------------------------------------
 // loss = sum_i w_(sample of i) (y_i - t_i)^2 / n  (w = 1 without sample weights)
 __global__ void k_loss(const float* __restrict__ y, const float* __restrict__ t, const float* __restrict__ w,
@@ -221,95 +413,83 @@ __global__ void k_loss(const float* __restrict__ y, const float* __restrict__ t,
     }
 }
 
-// dH4 = Q^T dy (the last layer has no activation, so this is dZ of layer 3) -> dZc, dZt; bias grad
-__global__ void k_proj_bwd(const float* __restrict__ dy, const bf16* __restrict__ Qw, int B, int L,
-                           bf16* __restrict__ dZc, bf16* __restrict__ dZt, float* __restrict__ db) {
+// dH4 = Q^T dy (the last layer has no activation, so this is dZ of layer 3) -> dZc, dZt;
+// dQ[j][c] = sum_(b,x) dy[b][j][x] h[b][x][c], dq[j] = sum dy[b][j][x]; the bias gradient
+// is Q^T dq.  A block takes 256 bins of one sample: a thread per bin for dZ, then a lane
+// per channel pair and a warp per 32 bins for the sums.
+__global__ void __launch_bounds__(256) k_proj_bwd(const float* __restrict__ dy, const bf16* __restrict__ Qw,
+                                                  const bf16* __restrict__ Ht, int B, int L, bf16* __restrict__ dZc,
+                                                  bf16* __restrict__ dZt, float* __restrict__ db,
+                                                  float* __restrict__ dQ, float* __restrict__ dq) {
     __shared__ float sQ[COUT * W];
-    __shared__ float sdb[W];
-    for (int i = threadIdx.x; i < COUT * W; i += blockDim.x) sQ[i] = __bfloat162float(Qw[i]);
-    for (int i = threadIdx.x; i < W; i += blockDim.x) sdb[i] = 0.f;
-    __syncthreads();
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const bool live = idx < (long long)B * L;
+    __shared__ float4 sd[256];
+    __shared__ float red[8][COUT * W];
+    __shared__ float rq[8][COUT];
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5, b = blockIdx.y, x = blockIdx.x * 256 + t;
+    for (int i = t; i < COUT * W; i += 256) sQ[i] = __bfloat162float(Qw[i]);
+    const bool live = x < L;
     float d[COUT] = {0.f, 0.f, 0.f, 0.f};
-    int b = 0, xx = 0;
     if (live) {
-        b = (int)(idx / L);
-        xx = (int)(idx % L);
 #pragma unroll
-        for (int j = 0; j < COUT; ++j) d[j] = dy[((long long)b * COUT + j) * L + xx];
+        for (int j = 0; j < COUT; ++j) d[j] = dy[((long long)b * COUT + j) * L + x];
     }
-    uint4 pack[W / 8];
-    bf16* gp = reinterpret_cast<bf16*>(pack);
+    sd[t] = make_float4(d[0], d[1], d[2], d[3]);
+    __syncthreads();
+    if (live) {
+        uint4* dst = reinterpret_cast<uint4*>(dZt + ((long long)b * L + x) * W);
 #pragma unroll
-    for (int c = 0; c < W; ++c) {
-        float g = 0.f;
+        for (int c0 = 0; c0 < W; c0 += 8) {
+            uint4 pack;
+            bf16* gp = reinterpret_cast<bf16*>(&pack);
 #pragma unroll
-        for (int j = 0; j < COUT; ++j) g = fmaf(sQ[j * W + c], d[j], g);
-        gp[c] = __float2bfloat16(g);
-        if (live) dZc[((long long)c * B + b) * L + xx] = gp[c];
-        float s = g;
+            for (int i = 0; i < 8; ++i) {
+                float g = 0.f;
+#pragma unroll
+                for (int j = 0; j < COUT; ++j) g = fmaf(sQ[j * W + c0 + i], d[j], g);
+                gp[i] = __float2bfloat16(g);
+                dZc[((long long)(c0 + i) * B + b) * L + x] = gp[i];
+            }
+            dst[c0 / 8] = pack;
+        }
+    }
+    // a lane's channels 2 lane, 2 lane + 1 over the warp's 32 bins
+    float acc[2 * COUT] = {};
+    const int xw = blockIdx.x * 256 + wp * 32, rows = min(32, L - xw);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(Ht + ((long long)b * L + xw) * W) + lane;
+#pragma unroll 8
+    for (int r = 0; r < rows; ++r) {
+        const __nv_bfloat162 v = h[r * (W / 2)];
+        const float h0 = __low2float(v), h1 = __high2float(v);
+        const float4 e = sd[wp * 32 + r];
+        acc[0] = fmaf(e.x, h0, acc[0]); acc[1] = fmaf(e.x, h1, acc[1]);
+        acc[2] = fmaf(e.y, h0, acc[2]); acc[3] = fmaf(e.y, h1, acc[3]);
+        acc[4] = fmaf(e.z, h0, acc[4]); acc[5] = fmaf(e.z, h1, acc[5]);
+        acc[6] = fmaf(e.w, h0, acc[6]); acc[7] = fmaf(e.w, h1, acc[7]);
+    }
+#pragma unroll
+    for (int j = 0; j < COUT; ++j) {
+        red[wp][j * W + 2 * lane] = acc[2 * j];
+        red[wp][j * W + 2 * lane + 1] = acc[2 * j + 1];
+        float s = d[j];
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&sdb[c], s);
-    }
-    if (live) {
-        uint4* dst = reinterpret_cast<uint4*>(dZt + idx * W);
-#pragma unroll
-        for (int j = 0; j < W / 8; ++j) dst[j] = pack[j];
+        if (lane == 0) rq[wp][j] = s;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < W; i += blockDim.x) atomicAdd(&db[i], sdb[i]);
-}
-
-// dQ[j][c] = sum_(b,x) dy[b][j][x] h[b][x][c];  dq[j] = sum dy[b][j][x]
-__global__ void k_proj_wgrad(const float* __restrict__ dy, const bf16* __restrict__ Ht, int B, int L, int rows_per_block,
-                             float* __restrict__ dQ, float* __restrict__ dq) {
-    __shared__ float hs[64][W + 1];
-    __shared__ float ds[COUT][64];
-    const int t = threadIdx.x, j = t / W, c = t % W;
-    const long long total = (long long)B * L;
-    const long long r0 = (long long)blockIdx.x * rows_per_block;
-    float acc = 0.f, accq = 0.f;
-    for (long long base = r0; base < r0 + rows_per_block && base < total; base += 64) {
-        for (int r = 0; r < 16; ++r) {
-            const int i = t + 256 * r, row = i / W, cc = i % W;
-            const long long g = base + row;
-            hs[row][cc] = g < total ? __bfloat162float(Ht[g * W + cc]) : 0.f;
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += red[i][t];
+    atomicAdd(&dQ[t], s);
+    if (t < W) {
+        float g = 0.f;
+        for (int j = 0; j < COUT; ++j) {
+            float q = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q += rq[i][j];
+            g = fmaf(sQ[j * W + t], q, g);
+            if (t == 0) atomicAdd(&dq[j], q);
         }
-        {
-            const int jj = t / 64, rr = t % 64;
-            const long long g = base + rr;
-            ds[jj][rr] = g < total ? dy[((g / L) * COUT + jj) * L + (g % L)] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int rr = 0; rr < 64; ++rr) acc = fmaf(ds[j][rr], hs[rr][c], acc);
-        if (c == 0)
-            for (int rr = 0; rr < 64; ++rr) accq += ds[j][rr];
-        __syncthreads();
+        atomicAdd(&db[t], g);
     }
-    atomicAdd(&dQ[j * W + c], acc);
-    if (c == 0) atomicAdd(&dq[j], accq);
-}
-
-// dS[(c,b)][m] = sum_o dT[(o,b)][m] conj(W[c][o][m])
-__global__ void k_mix_bwd_ds(const float* __restrict__ dT, const bf16* __restrict__ Ws, int B, bf16* __restrict__ dS) {
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (idx >= (long long)W * B * MODES) return;
-    const int m = (int)(idx % MODES);
-    const long long t = idx / MODES;
-    const int b = (int)(t % B), c = (int)(t / B);
-    float ar = 0.f, ai = 0.f;
-    for (int o = 0; o < W; ++o) {
-        const float* d = dT + ((long long)o * B + b) * SPEC + 2 * m;
-        const __nv_bfloat162 w = *reinterpret_cast<const __nv_bfloat162*>(Ws + (((long long)c * W + o) * MODES + m) * 2);
-        const float wr = __low2float(w), wi = __high2float(w);
-        ar = fmaf(d[0], wr, fmaf(d[1], wi, ar));
-        ai = fmaf(d[1], wr, fmaf(-d[0], wi, ai));
-    }
-    bf16* o_ = dS + ((long long)c * B + b) * SPEC + 2 * m;
-    o_[0] = __float2bfloat16(ar);
-    o_[1] = __float2bfloat16(ai);
 }
 
 // dW[c][o][m] = sum_b conj(S[(c,b)][m]) dT[(o,b)][m]
@@ -328,91 +508,6 @@ __global__ void k_mix_bwd_dw(const float* __restrict__ dT, const float* __restri
     }
     dW[(((long long)c * W + o) * MODES + m) * 2] = ar;
     dW[(((long long)c * W + o) * MODES + m) * 2 + 1] = ai;
-}
-
-// g = dHs[c][b][x] + dHp[b][x][c]; with Zprev: dZ = g act'(Zprev) -> dZc, dZt, bias grad;
-// without (layer 0): g written back into dHs (the gradient of the lifted input)
-__global__ void k_combine_bwd(float* __restrict__ dHs, const float* __restrict__ dHp, const float* __restrict__ Zprev,
-                              int B, int L, bf16* __restrict__ dZc, bf16* __restrict__ dZt, float* __restrict__ db) {
-    __shared__ float tile[32][W + 1];
-    const int b = blockIdx.y;
-    float bsum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int xt = 0; xt < XT; ++xt) {
-        const int x0 = (blockIdx.x * XT + xt) * 32;
-        if (x0 >= L) break;
-        for (int r = 0; r < 8; ++r) {
-            const int i = threadIdx.x + 256 * r, xi = i / W, c = i % W;
-            tile[xi][c] = dHp[((long long)b * L + x0 + xi) * W + c];
-        }
-        __syncthreads();
-        float gv[8];
-        for (int r = 0; r < 8; ++r) {
-            const int i = threadIdx.x + 256 * r, c = i / 32, xi = i % 32;
-            const long long o = ((long long)c * B + b) * L + x0 + xi;
-            float g = dHs[o] + tile[xi][c];
-            if (Zprev) {
-                g *= gelu_d(Zprev[o]);
-                dZc[o] = __float2bfloat16(g);
-                bsum[r] += g;
-            } else {
-                dHs[o] = g;
-            }
-            gv[r] = g;
-        }
-        __syncthreads();
-        if (Zprev) {
-            for (int r = 0; r < 8; ++r) {
-                const int i = threadIdx.x + 256 * r, c = i / 32, xi = i % 32;
-                tile[xi][c] = gv[r];
-            }
-            __syncthreads();
-            for (int r = 0; r < 8; ++r) {
-                const int i = threadIdx.x + 256 * r, xi = i / W, c = i % W;
-                dZt[((long long)b * L + x0 + xi) * W + c] = __float2bfloat16(tile[xi][c]);
-            }
-            __syncthreads();
-        }
-    }
-    if (Zprev) {
-        // every warp holds channels warp + 8 r (r = 0..7) across its 32 lanes
-        for (int r = 0; r < 8; ++r) {
-            float s = bsum[r];
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if ((threadIdx.x & 31) == 0) atomicAdd(&db[(threadIdx.x >> 5) + 8 * r], s);
-        }
-    }
-}
-
-// dP[c][i] = sum_(b,x) dH0[c][b][x] x[b][i][x];  dp[c] = sum dH0[c][b][x]
-__global__ void k_lift_wgrad(const float* __restrict__ dH0, const float* __restrict__ x, int B, int L,
-                             float* __restrict__ dP, float* __restrict__ dp) {
-    __shared__ float red[CIN + 1][8];
-    const int c = blockIdx.x;
-    const long long total = (long long)B * L;
-    float acc[CIN + 1];
-#pragma unroll
-    for (int i = 0; i <= CIN; ++i) acc[i] = 0.f;
-    for (long long g = blockIdx.y * (long long)blockDim.x + threadIdx.x; g < total;
-         g += (long long)gridDim.y * blockDim.x) {
-        const int b = (int)(g / L), xx = (int)(g % L);
-        const float d = dH0[((long long)c * B + b) * L + xx];
-        acc[CIN] += d;
-#pragma unroll
-        for (int i = 0; i < CIN; ++i) acc[i] = fmaf(d, x[((long long)b * CIN + i) * L + xx], acc[i]);
-    }
-#pragma unroll
-    for (int i = 0; i <= CIN; ++i) {
-        float s = acc[i];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0) red[i][threadIdx.x >> 5] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x <= CIN) {
-        float s = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[threadIdx.x][w];
-        if (threadIdx.x < CIN) atomicAdd(&dP[c * CIN + threadIdx.x], s);
-        else atomicAdd(&dp[c], s);
-    }
 }
 
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
@@ -639,9 +734,13 @@ struct optifax_fno_s {
     bf16 *F = nullptr, *FT = nullptr, *G = nullptr, *GT = nullptr;
     bf16 *Hc[NLAYER + 1] = {}, *Ht[NLAYER + 1] = {};
     float* Z[NLAYER - 1] = {};
-    float* S[NLAYER] = {};
+    float *S[NLAYER] = {}, *dT[NLAYER] = {};    // one allocation each, batch rows [layer][64 B][64]
     bf16 *T = nullptr, *dS = nullptr, *dZc = nullptr, *dZt = nullptr;
-    float *Y1 = nullptr, *Y2 = nullptr, *y = nullptr, *dy = nullptr, *dT = nullptr, *loss = nullptr;
+    float *y = nullptr, *dy = nullptr, *loss = nullptr, *part = nullptr;
+    int* err = nullptr;                       // the device's tensor-core error word
+    // tensor maps of k_layer's operands (all of them this object's buffers) for batch mapB
+    int mapB = 0;
+    CUtensorMap mG, mFT, mT, mDS, mDZ, mH[NLAYER], mWp[NLAYER], mWpT[NLAYER];
 };
 
 namespace {
@@ -659,19 +758,55 @@ int alloc0(P** p, size_t bytes) {
         if (rc_) return rc_;          \
     } while (0)
 
+int fno_maps(optifax_fno_s* f, int B) {
+    if (f->mapB == B) return OPTIFAX_OK;
+    f->mapB = 0;
+    const long long L = f->L, BL = (long long)B * L;
+    for (int l = 1; l < NLAYER; ++l) {
+        f->S[l] = f->S[0] + (long long)l * B * W * SPEC;
+        f->dT[l] = f->dT[0] + (long long)l * B * W * SPEC;
+    }
+    OFX_TRY(ofx_tc::make_map(&f->mG, f->G, L, SPEC, SPEC, 128));
+    OFX_TRY(ofx_tc::make_map(&f->mFT, f->FT, L, SPEC, SPEC, 128));
+    OFX_TRY(ofx_tc::make_map(&f->mT, f->T, (long long)B * W, SPEC, SPEC, 64));
+    OFX_TRY(ofx_tc::make_map(&f->mDS, f->dS, (long long)B * W, SPEC, SPEC, 64));
+    OFX_TRY(ofx_tc::make_map(&f->mDZ, f->dZt, BL, W, W, 128));
+    for (int l = 0; l < NLAYER; ++l) {
+        OFX_TRY(ofx_tc::make_map(&f->mH[l], f->Ht[l], BL, W, W, 128));
+        OFX_TRY(ofx_tc::make_map(&f->mWp[l], f->wb + off_wp(l), W, W, W, 64));
+        OFX_TRY(ofx_tc::make_map(&f->mWpT[l], f->wpt + (long long)l * W * W, W, W, W, 64));
+    }
+    f->mapB = B;
+    return OPTIFAX_OK;
+}
+
+// K splits of the transform products (M = 64 B rows, K = L): enough CTAs to fill the GPU,
+// at least two 64-column steps each (one sample, 4096 bins: 8 splits 8.8 us, 32 splits 5)
+inline int spec_splits(int B, int L) {
+    const int tiles = (W * B + 127) / 128, most = L / 128;
+    const int want = (296 + tiles - 1) / tiles;
+    const int s = want < 8 ? 8 : (want > 32 ? 32 : want);
+    return s < most ? s : (most > 0 ? most : 1);
+}
+
 int fno_forward(optifax_fno_s* f, const float* x, int B, cudaStream_t st) {
     const int L = f->L;
     const long long WB = (long long)W * B, rowsA = WB > 128 ? WB : 128;
+    OFX_TRY(fno_maps(f, B));
+    // the split-K products add into S: one clearing for the four layers
+    if (cudaMemsetAsync(f->S[0], 0, sizeof(float) * NLAYER * WB * SPEC, st) != cudaSuccess) return OPTIFAX_ERR_CUDA;
     k_lift<<<nblk((long long)B * L), 256, 0, st>>>(x, f->wb + OFF_P, f->master + OFF_PB, B, L, f->Hc[0], f->Ht[0]);
     for (int l = 0; l < NLAYER; ++l) {
-        OFX_TRY(optifax_gemm_bf16(f->Hc[l], L, rowsA, f->F, L, SPEC, f->S[l], SPEC, (int)WB, SPEC, L, 8, 0, st));
-        k_mix_fwd<<<nblk(WB * MODES), 256, 0, st>>>(f->S[l], f->wb + off_ws(l), B, f->T);
-        OFX_TRY(optifax_gemm_bf16(f->T, SPEC, rowsA, f->G, SPEC, L, f->Y1, L, (int)WB, L, SPEC, 1, 0, st));
-        OFX_TRY(optifax_gemm_bf16(f->Ht[l], W, (long long)B * L, f->wb + off_wp(l), W, W, f->Y2, W, B * L, W, W, 1,
-                                  0, st));
-        const int act = l < NLAYER - 1;
-        k_combine_fwd<<<dim3((L + 32 * XT - 1) / (32 * XT), B), 256, 0, st>>>(
-            f->Y1, f->Y2, f->master + off_b(l), B, L, act, act ? f->Z[l] : nullptr, f->Hc[l + 1], f->Ht[l + 1]);
+        OFX_TRY(optifax_gemm_bf16(f->Hc[l], L, rowsA, f->F, L, SPEC, f->S[l], SPEC, (int)WB, SPEC, L,
+                                  spec_splits(B, L), 1, st));
+        launch_mix<false>(f->S[l], f->wb + off_ws(l), B, f->T, st);
+        LayerArgs a = {};
+        a.bias = f->master + off_b(l);
+        a.act = l < NLAYER - 1;
+        a.Z = a.act ? f->Z[l] : nullptr;
+        a.Hc = f->Hc[l + 1]; a.Ht = f->Ht[l + 1];
+        a.err = f->err; a.B = B; a.L = L;
+        k_layer<LAYER_FWD><<<dim3((L + 127) / 128, B), 128, LAYER_SMEM, st>>>(f->mG, f->mH[l], f->mT, f->mWp[l], a);
     }
     k_proj_fwd<<<nblk((long long)B * L), 256, 0, st>>>(f->Ht[NLAYER], f->wb + OFF_Q, f->master + OFF_QB, x, B, L,
                                                        f->y);
@@ -681,31 +816,39 @@ int fno_forward(optifax_fno_s* f, const float* x, int B, cudaStream_t st) {
 int fno_backward(optifax_fno_s* f, const float* x, const float* target, const float* sample_w, int B,
                  cudaStream_t st) {
     const int L = f->L;
-    const long long WB = (long long)W * B, rowsA = WB > 128 ? WB : 128, BL = (long long)B * L;
+    const long long WB = (long long)W * B, BL = (long long)B * L;
     if (cudaMemsetAsync(f->grad, 0, sizeof(float) * N_PARAMS, st) != cudaSuccess ||
+        cudaMemsetAsync(f->dT[0], 0, sizeof(float) * NLAYER * WB * SPEC, st) != cudaSuccess ||
         cudaMemsetAsync(f->loss, 0, sizeof(float), st) != cudaSuccess)
         return OPTIFAX_ERR_CUDA;
     const long long ny = BL * COUT;
     k_loss<<<256, 256, 0, st>>>(f->y, target, sample_w, (long long)COUT * L, ny, 1.f / (float)ny, f->dy, f->loss);
-    k_proj_bwd<<<nblk(BL), 256, 0, st>>>(f->dy, f->wb + OFF_Q, B, L, f->dZc, f->dZt, f->grad + off_b(NLAYER - 1));
-    const int rpb = 2048;
-    k_proj_wgrad<<<nblk(BL, rpb), 256, 0, st>>>(f->dy, f->Ht[NLAYER], B, L, rpb, f->grad + OFF_Q, f->grad + OFF_QB);
+    k_proj_bwd<<<dim3((L + 255) / 256, B), 256, 0, st>>>(f->dy, f->wb + OFF_Q, f->Ht[NLAYER], B, L, f->dZc, f->dZt,
+                                                         f->grad + off_b(NLAYER - 1), f->grad + OFF_Q,
+                                                         f->grad + OFF_QB);
     for (int l = NLAYER - 1; l >= 0; --l) {
-        const int splits = (int)((BL + 2047) / 2048);
+        // dWp: K = B L over CTAs of 512 (64 rows of A: half of the tile is padding)
+        const int splits = (int)(BL <= (4096LL << 9) ? (BL + 511) / 512 : 4096);
         OFX_TRY(optifax_gemm_bf16(f->dZc, BL, 128, f->Hc[l], BL, W, f->grad + off_wp(l), W, W, W, (int)BL, splits, 1,
                                   st));
-        OFX_TRY(optifax_gemm_bf16(f->dZc, L, 2 * WB, f->GT, L, SPEC, f->dT, SPEC, (int)WB, SPEC, L, 8, 0, st));
-        k_mix_bwd_ds<<<nblk(WB * MODES), 256, 0, st>>>(f->dT, f->wb + off_ws(l), B, f->dS);
-        k_mix_bwd_dw<<<nblk((long long)W * W * MODES), 256, 0, st>>>(f->dT, f->S[l], B, f->grad + off_ws(l));
-        OFX_TRY(optifax_gemm_bf16(f->dS, SPEC, rowsA, f->FT, SPEC, L, f->Y1, L, (int)WB, L, SPEC, 1, 0, st));
-        OFX_TRY(optifax_gemm_bf16(f->dZt, W, BL, f->wpt + (long long)l * W * W, W, W, f->Y2, W, (int)BL, W, W, 1, 0,
-                                  st));
-        const dim3 cg((L + 32 * XT - 1) / (32 * XT), B);
+        OFX_TRY(optifax_gemm_bf16(f->dZc, L, 2 * WB, f->GT, L, SPEC, f->dT[l], SPEC, (int)WB, SPEC, L,
+                                  spec_splits(B, L), 1, st));
+        launch_mix<true>(f->dT[l], f->wb + off_ws(l), B, f->dS, st);
+        k_mix_bwd_dw<<<nblk((long long)W * W * MODES), 256, 0, st>>>(f->dT[l], f->S[l], B, f->grad + off_ws(l));
+        LayerArgs a = {};
+        a.err = f->err; a.B = B; a.L = L;
+        const dim3 grid((L + 127) / 128, B);
         if (l > 0) {
-            k_combine_bwd<<<cg, 256, 0, st>>>(f->Y1, f->Y2, f->Z[l - 1], B, L, f->dZc, f->dZt, f->grad + off_b(l - 1));
+            a.Z = f->Z[l - 1];
+            a.Hc = f->dZc; a.Ht = f->dZt;
+            a.db = f->grad + off_b(l - 1);
+            k_layer<LAYER_BWD><<<grid, 128, LAYER_SMEM, st>>>(f->mFT, f->mDZ, f->mDS, f->mWpT[l], a);
         } else {
-            k_combine_bwd<<<cg, 256, 0, st>>>(f->Y1, f->Y2, nullptr, B, L, nullptr, nullptr, nullptr);
-            k_lift_wgrad<<<dim3(W, 8), 256, 0, st>>>(f->Y1, x, B, L, f->grad + OFF_P, f->grad + OFF_PB);
+            a.x = x;
+            a.db = f->part;
+            k_layer<LAYER_BWD_IN><<<grid, 128, LAYER_SMEM, st>>>(f->mFT, f->mDZ, f->mDS, f->mWpT[l], a);
+            k_lift_sum<<<dim3(W * 8 / 32, 8), 256, 0, st>>>(f->part, (int)(grid.x * grid.y), f->grad + OFF_P,
+                                                            f->grad + OFF_PB);
         }
     }
     return cudaGetLastError() == cudaSuccess ? OPTIFAX_OK : OPTIFAX_ERR_CUDA;
@@ -713,15 +856,15 @@ int fno_backward(optifax_fno_s* f, const float* x, const float* target, const fl
 
 void fno_free(optifax_fno_s* f) {
     void* ps[] = {f->master, f->grad, f->m, f->v, f->wb, f->wpt, f->F, f->FT, f->G, f->GT, f->T, f->dS, f->dZc,
-                  f->dZt, f->Y1, f->Y2, f->y, f->dy, f->dT, f->loss};
+                  f->dZt, f->y, f->dy, f->loss, f->part};
     for (void* p : ps)
         if (p) cudaFree(p);
     for (int l = 0; l <= NLAYER; ++l) {
         if (f->Hc[l]) cudaFree(f->Hc[l]);
         if (f->Ht[l]) cudaFree(f->Ht[l]);
     }
-    for (int l = 0; l < NLAYER; ++l)
-        if (f->S[l]) cudaFree(f->S[l]);
+    if (f->S[0]) cudaFree(f->S[0]);
+    if (f->dT[0]) cudaFree(f->dT[0]);
     for (int l = 0; l < NLAYER - 1; ++l)
         if (f->Z[l]) cudaFree(f->Z[l]);
     delete f;
@@ -761,17 +904,24 @@ extern "C" int optifax_fno_create(optifax_fno* out, int32_t n_bins, int32_t max_
         A(&f->Ht[l], sizeof(bf16) * BL * W);
     }
     for (int l = 0; l < NLAYER - 1; ++l) A(&f->Z[l], sizeof(float) * WB * L);
-    for (int l = 0; l < NLAYER; ++l) A(&f->S[l], sizeof(float) * WB * SPEC);
+    A(&f->S[0], sizeof(float) * NLAYER * WB * SPEC);
+    A(&f->dT[0], sizeof(float) * NLAYER * WB * SPEC);
+    A(&f->part, sizeof(float) * W * 8 * max_batch * ((L + 127) / 128));
     A(&f->T, sizeof(bf16) * rowsA * SPEC);
     A(&f->dS, sizeof(bf16) * rowsA * SPEC);
     A(&f->dZc, sizeof(bf16) * 2 * WB * L);     // the [o][(b,x)] view is read as 128 rows
     A(&f->dZt, sizeof(bf16) * BL * W);
-    A(&f->Y1, sizeof(float) * WB * L);
-    A(&f->Y2, sizeof(float) * BL * W);
     A(&f->y, sizeof(float) * BL * COUT);
     A(&f->dy, sizeof(float) * BL * COUT);
-    A(&f->dT, sizeof(float) * WB * SPEC);
     A(&f->loss, sizeof(float));
+    if (!rc) {
+        f->err = ofx_tc::error_word();
+        if (!f->err ||
+            cudaFuncSetAttribute(k_layer<LAYER_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_layer<LAYER_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_layer<LAYER_BWD_IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM) != cudaSuccess)
+            rc = OPTIFAX_ERR_CUDA;
+    }
     if (!rc) {
         k_dft_tables<<<nblk((long long)SPEC * L), 256>>>((int)L, f->F, f->FT, f->G, f->GT);
         if (cudaDeviceSynchronize() != cudaSuccess) rc = OPTIFAX_ERR_CUDA;

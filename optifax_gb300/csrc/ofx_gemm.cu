@@ -8,15 +8,13 @@
 // lane per output row).  K can be split over gridDim.z; split partial sums are
 // added into C with atomics.  Every wait is bounded: a timeout sets an error flag
 // (optifax_tc_error) and the kernel releases its tensor memory and returns.
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
 
 #include "../../include/optifax.h"
 #include "ofx_tc.cuh"
+#include "ofx_tmap.cuh"
 
 namespace {
 
@@ -167,37 +165,14 @@ __global__ void __launch_bounds__(128, 1)
     }
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
-std::once_flag g_encode_once;
 bool g_attr_set[64] = {};
 
-PFN_cuTensorMapEncodeTiled_v12000 encoder() {
-    std::call_once(g_encode_once, [] {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    });
-    return g_encode;
-}
-
-// rows x cols BF16 row-major with leading dimension ld (elements); box box_rows x 64
-int make_map(CUtensorMap* m, const void* ptr, long long rows, long long cols, long long ld, int box_rows) {
-    auto enc = encoder();
-    if (!enc) return OPTIFAX_ERR_CUDA;
-    cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-    cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
-    cuuint32_t box[2] = {static_cast<cuuint32_t>(BK), static_cast<cuuint32_t>(box_rows)};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? OPTIFAX_OK : OPTIFAX_ERR_CUDA;
-}
-
 }  // namespace
+
+int* ofx_tc::error_word() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, g_tc_err) == cudaSuccess ? static_cast<int*>(p) : nullptr;
+}
 
 extern "C" int optifax_gemm_bf16(const void* A, int64_t lda, int64_t a_rows, const void* B, int64_t ldb,
                                  int64_t b_rows, float* C, int64_t ldc, int32_t M, int32_t N, int32_t K,
@@ -216,9 +191,9 @@ extern "C" int optifax_gemm_bf16(const void* A, int64_t lda, int64_t a_rows, con
         g_attr_set[dev] = true;
     }
     CUtensorMap ma, mb;
-    int rc = make_map(&ma, A, a_rows, K, lda, BM);
+    int rc = ofx_tc::make_map(&ma, A, a_rows, K, lda, BM);
     if (rc) return rc;
-    rc = make_map(&mb, B, b_rows, K, ldb, BN);
+    rc = ofx_tc::make_map(&mb, B, b_rows, K, ldb, BN);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int kps = (K + splits - 1) / splits;
