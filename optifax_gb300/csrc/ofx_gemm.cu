@@ -131,15 +131,18 @@ __global__ void __launch_bounds__(128, 1)
     }
     __syncthreads();
     if (ok) {
-        const bool vec = !g.atomic && (g.ldc % 4 == 0) && (n0 + BN <= g.N) &&
-                         ((reinterpret_cast<uintptr_t>(g.C) & 15) == 0);
+        const bool vec = (g.ldc % 4 == 0) && (n0 + BN <= g.N) && ((reinterpret_cast<uintptr_t>(g.C) & 15) == 0);
         for (int idx = threadIdx.x; idx < BM * (BN / 4); idx += blockDim.x) {
             const int r = idx / (BN / 4), c4 = (idx % (BN / 4)) * 4;
             const int row = m0 + r;
             if (row >= g.M) continue;
             float* dst = g.C + static_cast<long long>(row) * g.ldc + n0 + c4;
             const float* src = tile + r * LDT + c4;
-            if (vec) {
+            if (vec && g.atomic) {
+                // one 16-byte reduction instead of four: split sums are bound by their atomics
+                asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(src[0]),
+                             "f"(src[1]), "f"(src[2]), "f"(src[3]) : "memory");
+            } else if (vec) {
                 *reinterpret_cast<float4*>(dst) = make_float4(src[0], src[1], src[2], src[3]);
             } else {
 #pragma unroll
