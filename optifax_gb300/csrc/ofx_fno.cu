@@ -35,10 +35,15 @@
 #include <cstring>
 
 #include "../../include/optifax.h"
+#include "ofx_fft.cuh"
 #include "ofx_tc.cuh"
 #include "ofx_tmap.cuh"
 
 typedef __nv_bfloat16 bf16;
+
+using ofx_tc::dep_launch;
+using ofx_tc::dep_wait;
+using ofx_tc::launch_dep;
 
 namespace {
 
@@ -87,33 +92,38 @@ __global__ void k_refresh(const float* __restrict__ master, bf16* wb, bf16* wpt)
 }
 
 // ---- forward -------------------------------------------------------------
-__global__ void k_lift(const float* __restrict__ x, const bf16* __restrict__ Pw, const float* __restrict__ pb, int B,
-                       int L, bf16* __restrict__ Hc, bf16* __restrict__ Ht) {
+// A thread takes one bin and 16 channels; a warp 32 bins of one channel group
+__global__ void __launch_bounds__(256) k_lift(const float* __restrict__ x, const bf16* __restrict__ Pw,
+                                              const float* __restrict__ pb, int B, int L, bf16* __restrict__ Hc,
+                                              bf16* __restrict__ Ht) {
     __shared__ float sP[W * CIN];
     __shared__ float sb[W];
-    for (int i = threadIdx.x; i < W * CIN; i += blockDim.x) sP[i] = __bfloat162float(Pw[i]);
-    for (int i = threadIdx.x; i < W; i += blockDim.x) sb[i] = pb[i];
+    dep_launch();
+    dep_wait();
+    for (int i = threadIdx.x; i < W * CIN; i += 256) sP[i] = __bfloat162float(Pw[i]);
+    for (int i = threadIdx.x; i < W; i += 256) sb[i] = pb[i];
     __syncthreads();
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int c0 = (threadIdx.x >> 6) * 16;
+    const long long idx = blockIdx.x * 64LL + (threadIdx.x & 63);
     if (idx >= (long long)B * L) return;
     const int b = (int)(idx / L), xx = (int)(idx % L);
     float in[CIN];
 #pragma unroll
     for (int i = 0; i < CIN; ++i) in[i] = x[((long long)b * CIN + i) * L + xx];
-    uint4 pack[W / 8];
+    uint4 pack[2];
     bf16* hp = reinterpret_cast<bf16*>(pack);
 #pragma unroll
-    for (int c = 0; c < W; ++c) {
+    for (int j = 0; j < 16; ++j) {
+        const int c = c0 + j;
         float h = sb[c];
 #pragma unroll
         for (int i = 0; i < CIN; ++i) h = fmaf(sP[c * CIN + i], in[i], h);
-        const bf16 hb = __float2bfloat16(h);
-        hp[c] = hb;
-        Hc[((long long)c * B + b) * L + xx] = hb;
+        hp[j] = __float2bfloat16(h);
+        Hc[((long long)c * B + b) * L + xx] = hp[j];
     }
-    uint4* dst = reinterpret_cast<uint4*>(Ht + idx * W);
-#pragma unroll
-    for (int j = 0; j < W / 8; ++j) dst[j] = pack[j];
+    uint4* dst = reinterpret_cast<uint4*>(Ht + idx * W + c0);
+    dst[0] = pack[0];
+    dst[1] = pack[1];
 }
 
 // Channel mixing per mode: out[b][u][m] = sum_v in[(v,b)][m] w (or conj w) with w =
@@ -128,6 +138,8 @@ __global__ void __launch_bounds__(256) k_mix(const float* __restrict__ in, const
     __shared__ float2 red[8][MIXB][MODES];
     const int m = threadIdx.x & 31, wp = threadIdx.x >> 5, u0 = blockIdx.x * U, b0 = blockIdx.y * MIXB;
     float ar[U][MIXB] = {}, ai[U][MIXB] = {};
+    dep_launch();
+    dep_wait();
 #pragma unroll
     for (int i = 0; i < W / 8; ++i) {
         const int v = wp * (W / 8) + i;
@@ -171,8 +183,8 @@ __global__ void __launch_bounds__(256) k_mix(const float* __restrict__ in, const
 template <bool BWD>
 void launch_mix(const float* in, const bf16* Ws, int B, bf16* out, cudaStream_t st) {
     const unsigned groups = (unsigned)((B + MIXB - 1) / MIXB);
-    if (B <= 8) k_mix<BWD, 1><<<dim3(W, groups), 256, 0, st>>>(in, Ws, B, out);
-    else k_mix<BWD, 4><<<dim3(W / 4, groups), 256, 0, st>>>(in, Ws, B, out);
+    if (B <= 8) launch_dep(k_mix<BWD, 1>, dim3(W, groups), dim3(256), 0, st, in, Ws, B, out);
+    else launch_dep(k_mix<BWD, 4>, dim3(W / 4, groups), dim3(256), 0, st, in, Ws, B, out);
 }
 
 // ---- one layer's spatial part ---------------------------------------------
@@ -212,8 +224,11 @@ __global__ void __launch_bounds__(128, 4)
         mbar_init(&accum, 1);
         fence_barrier_init();
     }
-    if (MODE == LAYER_FWD && threadIdx.x < W) s_bias[threadIdx.x] = a.bias[threadIdx.x];
     if (warp == 0) tmem_alloc(&tmem_slot, 128);
+    __syncthreads();   // the next grid may take tensor memory only once this CTA has its own
+    dep_launch();
+    dep_wait();
+    if (MODE == LAYER_FWD && threadIdx.x < W) s_bias[threadIdx.x] = a.bias[threadIdx.x];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -340,33 +355,41 @@ __global__ void __launch_bounds__(128, 4)
     }
 }
 
-// y[b][j][x] = x[b][j][x] + q[j] + sum_c Q[j][c] h[b][x][c]
-__global__ void k_proj_fwd(const bf16* __restrict__ Ht, const bf16* __restrict__ Qw, const float* __restrict__ qb,
-                           const float* __restrict__ xin, int B, int L, float* __restrict__ y) {
+// y[b][j][x] = x[b][j][x] + q[j] + sum_c Q[j][c] h[b][x][c]; four lanes share a bin, 16
+// channels each
+__global__ void __launch_bounds__(256) k_proj_fwd(const bf16* __restrict__ Ht, const bf16* __restrict__ Qw,
+                                                  const float* __restrict__ qb, const float* __restrict__ xin, int B,
+                                                  int L, float* __restrict__ y) {
     __shared__ float sQ[COUT * W];
-    for (int i = threadIdx.x; i < COUT * W; i += blockDim.x) sQ[i] = __bfloat162float(Qw[i]);
+    dep_launch();
+    dep_wait();
+    if (threadIdx.x < COUT * W) sQ[threadIdx.x] = __bfloat162float(Qw[threadIdx.x]);
     __syncthreads();
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (idx >= (long long)B * L) return;
-    const int b = (int)(idx / L), xx = (int)(idx % L);
-    float acc[COUT];
+    const long long idx = blockIdx.x * 64LL + (threadIdx.x >> 2);
+    const int part = threadIdx.x & 3;
+    const bool live = idx < (long long)B * L;
+    const uint4* src = reinterpret_cast<const uint4*>(Ht + (live ? idx : 0) * W + 16 * part);
+    float acc[COUT] = {};
 #pragma unroll
-    for (int j = 0; j < COUT; ++j) acc[j] = qb[j];
-    const uint4* src = reinterpret_cast<const uint4*>(Ht + idx * W);
-#pragma unroll
-    for (int q8 = 0; q8 < W / 8; ++q8) {
+    for (int q8 = 0; q8 < 2; ++q8) {
         const uint4 u = src[q8];
         const bf16* hp = reinterpret_cast<const bf16*>(&u);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const float h = __bfloat162float(hp[e]);
 #pragma unroll
-            for (int j = 0; j < COUT; ++j) acc[j] = fmaf(sQ[j * W + q8 * 8 + e], h, acc[j]);
+            for (int j = 0; j < COUT; ++j) acc[j] = fmaf(sQ[j * W + 16 * part + q8 * 8 + e], h, acc[j]);
         }
     }
 #pragma unroll
-    for (int j = 0; j < COUT; ++j)
-        y[((long long)b * COUT + j) * L + xx] = xin[((long long)b * CIN + j) * L + xx] + acc[j];
+    for (int j = 0; j < COUT; ++j) {
+        acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 1);
+        acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 2);
+    }
+    if (!live) return;
+    const int b = (int)(idx / L), xx = (int)(idx % L);
+    const float v = part == 0 ? acc[0] : (part == 1 ? acc[1] : (part == 2 ? acc[2] : acc[3]));   // output j = part
+    y[((long long)b * COUT + part) * L + xx] = xin[((long long)b * CIN + part) * L + xx] + (v + qb[part]);
 }
 
 // dP[c][i] and dp[c] from k_layer's partial rows [n][W][8]; block: 32 of the 512 columns,
@@ -376,6 +399,8 @@ __global__ void __launch_bounds__(256) k_lift_sum(const float* __restrict__ part
     __shared__ float red[8][32];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
     float s = 0.f;
+    dep_launch();
+    dep_wait();
 #pragma unroll 4
     for (int r = blockIdx.y * 8 + wp; r < n; r += 8 * gridDim.y) s += part[(long long)r * (W * 8) + col];
     red[wp][lane] = s;
@@ -397,6 +422,8 @@ __global__ void k_loss(const float* __restrict__ y, const float* __restrict__ t,
                        float* __restrict__ loss) {
     __shared__ float red[32];
     float part = 0.f;
+    dep_launch();
+    dep_wait();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float d = y[i] - t[i];
         const float wi = w ? w[i / per_sample] : 1.f;
@@ -426,6 +453,8 @@ __global__ void __launch_bounds__(256) k_proj_bwd(const float* __restrict__ dy, 
     __shared__ float red[8][COUT * W];
     __shared__ float rq[8][COUT];
     const int t = threadIdx.x, lane = t & 31, wp = t >> 5, b = blockIdx.y, x = blockIdx.x * 256 + t;
+    dep_launch();
+    dep_wait();
     for (int i = t; i < COUT * W; i += 256) sQ[i] = __bfloat162float(Qw[i]);
     const bool live = x < L;
     float d[COUT] = {0.f, 0.f, 0.f, 0.f};
@@ -494,6 +523,8 @@ __global__ void __launch_bounds__(256) k_proj_bwd(const float* __restrict__ dy, 
 
 // dW[c][o][m] = sum_b conj(S[(c,b)][m]) dT[(o,b)][m]
 __global__ void k_mix_bwd_dw(const float* __restrict__ dT, const float* __restrict__ S, int B, float* __restrict__ dW) {
+    dep_launch();
+    dep_wait();
     const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (idx >= (long long)W * W * MODES) return;
     const int m = (int)(idx % MODES);
@@ -580,6 +611,8 @@ __global__ void k_ff_step(const float* __restrict__ y, const float* __restrict__
     __shared__ double red[32];
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     double e = 0.0;
+    dep_launch();
+    dep_wait();
     if (k < N) {
         float2 X = make_float2(0.f, 0.f);
         if (y) {
@@ -632,50 +665,94 @@ __device__ __forceinline__ int env_bin(const EnvBand& b, int N, int L, int j, bo
     return k < 0 ? k + N : k;
 }
 
-// in-place radix-2 DIT FFT of L points in shared memory (input already in
-// bit-reversed order); sign +1: exp(+2 pi i ...), -1: exp(-2 pi i ...)
-__device__ void smem_fft(float2* sm, int L, float sign) {
-    for (int len = 2; len <= L; len <<= 1) {
-        const int half = len >> 1;
-        for (int b = threadIdx.x; b < L / 2; b += blockDim.x) {
-            const int grp = b / half, j = b - grp * half;
-            const int i0 = grp * len + j, i1 = i0 + half;
-            float sn, cs;
-            sincospif(sign * 2.f * (float)j / (float)len, &sn, &cs);
-            const float2 u = sm[i0], v0 = sm[i1];
-            const float2 v = make_float2(v0.x * cs - v0.y * sn, v0.x * sn + v0.y * cs);
-            sm[i0] = make_float2(u.x + v.x, u.y + v.y);
-            sm[i1] = make_float2(u.x - v.x, u.y - v.y);
-        }
-        __syncthreads();
+constexpr int ENV_MAX = 4096, ENV_T = 512;
+
+// Slot of point m: the strided passes and the last pass's bit-reversed scatter spread
+// over the banks
+__device__ __forceinline__ int env_slot(int m) { return m ^ ((m >> 4) & 15); }
+
+// Quarter period of exp(-2 pi i m / L)
+__device__ __forceinline__ void env_table(float2* quad, int L) {
+    for (int i = threadIdx.x; i < (L + 3) / 4; i += ENV_T) {
+        float sn, cs;
+        sincospif(-2.f * (float)i / (float)L, &sn, &cs);
+        quad[i] = make_float2(cs, sn);
     }
+}
+__device__ __forceinline__ float2 env_tw(const float2* quad, int logL, int m) {
+    if (logL < 2) return make_float2(1.f, 0.f);              // L = 2 has the factor 1 only
+    const float2 w = quad[m & ((1 << (logL - 2)) - 1)];
+    const int k = m >> (logL - 2);                           // times (-i)^k
+    const float2 u = (k & 1) ? make_float2(w.y, -w.x) : w;
+    return (k & 2) ? make_float2(-u.x, -u.y) : u;
+}
+
+// One decimation-in-frequency pass of radix R over blocks of 2^logB points; the last
+// pass leaves frequency k in slot k.
+template <int R>
+__device__ void env_pass(float2* sm, const float2* quad, int logL, int logB) {
+    const int L = 1 << logL, LR = (1 << logB) / R, b = threadIdx.x;   // L / R <= ENV_T
+    const bool live = b < L / R, last = LR == 1;
+    const int off = b & (LR - 1), base = (b - off) * R + off;
+    float2 v[R];
+    if (live) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = sm[env_slot(base + q * LR)];
+        ofx::dftp<R>(v);
+    }
+    if (last) __syncthreads();
+    if (live) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            const int r = ofx::brev4(q, ofx::ilog2(R));
+            if (last) sm[env_slot(__brev((unsigned)(base + q)) >> (32 - logL))] = v[q];
+            else sm[env_slot(base + q * LR)] = q ? ofx::cmul(v[q], env_tw(quad, logL, (off * r) << (logL - logB))) : v[q];
+        }
+    }
+    __syncthreads();
+}
+
+// exp(-2 pi i j k / L) transform of the 2^logL points at env_slot(j), in place and in
+// natural order, by ENV_T threads.  Radix 8 with one shared-memory table: the previous
+// radix-2 form called sincospi in each of the L/2 log2(L) butterflies (25 us at 4096).
+__device__ void env_fft(float2* sm, const float2* quad, int logL) {
+    __syncthreads();
+    int logB = logL;
+    for (; logB >= 3; logB -= 3) env_pass<8>(sm, quad, logL, logB);
+    if (logB == 2) env_pass<4>(sm, quad, logL, logB);
+    if (logB == 1) env_pass<2>(sm, quad, logL, logB);
 }
 
 // grid (spectra, 2 bands): envelopes -> channels 0/1 (pump / pump_scale), 2/3
 // (signal / sigma), 4 log10(sigma / pump_scale), 5 j / L
-__global__ void k_ff_encode_env(const float2* __restrict__ Y, long long ystride, int N, int L, int logL, EnvBand bp,
+__global__ void __launch_bounds__(ENV_T) k_ff_encode_env(const float2* __restrict__ Y, long long ystride, int N, int L, int logL, EnvBand bp,
                                 EnvBand bs, float pump_scale, const float* __restrict__ sigma_in,
                                 float* __restrict__ x, int nch, float* __restrict__ sigma_out) {
-    __shared__ float2 sm[4096];
+    __shared__ float2 sm[ENV_MAX];
+    __shared__ float2 quad[ENV_MAX / 4];
     __shared__ float red[32];
     __shared__ float s_sig;
     const int p = blockIdx.x, band = blockIdx.y;
     const EnvBand bd = band ? bs : bp;
     const float2* y = Y + p * ystride;
-    for (int j = threadIdx.x; j < L; j += blockDim.x) {
+    dep_launch();
+    env_table(quad, L);
+    dep_wait();
+    // exp(+...): real and imaginary parts exchanged before and after
+    for (int j = threadIdx.x; j < L; j += ENV_T) {
         bool in;
         const int k = env_bin(bd, N, L, j, &in);
-        sm[__brev((unsigned)j) >> (32 - logL)] = in ? y[k] : make_float2(0.f, 0.f);
+        const float2 u = in ? y[k] : make_float2(0.f, 0.f);
+        sm[env_slot(j)] = make_float2(u.y, u.x);
     }
-    __syncthreads();
-    smem_fft(sm, L, 1.f);
+    env_fft(sm, quad, logL);
     float scale = 1.f / pump_scale, sg = 1.f;
     if (band == 1) {
         if (sigma_in) {
             if (threadIdx.x == 0) s_sig = sigma_in[p];
         } else {
             float acc = 0.f;
-            for (int j = threadIdx.x; j < L; j += blockDim.x) acc = fmaf(sm[j].x, sm[j].x, fmaf(sm[j].y, sm[j].y, acc));
+            for (int j = threadIdx.x; j < L; j += ENV_T) acc = fmaf(sm[j].x, sm[j].x, fmaf(sm[j].y, sm[j].y, acc));
             for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
             if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
             __syncthreads();
@@ -695,9 +772,10 @@ __global__ void k_ff_encode_env(const float2* __restrict__ Y, long long ystride,
     }
     float* xo = x + (long long)p * nch * L;
     const float lg = log10f(sg / pump_scale);
-    for (int j = threadIdx.x; j < L; j += blockDim.x) {
-        xo[(2 * band) * L + j] = sm[j].x * scale;
-        xo[(2 * band + 1) * L + j] = sm[j].y * scale;
+    for (int j = threadIdx.x; j < L; j += ENV_T) {
+        const float2 u = sm[env_slot(j)];
+        xo[(2 * band) * L + j] = u.y * scale;
+        xo[(2 * band + 1) * L + j] = u.x * scale;
         if (band == 1 && nch > 4) {
             xo[4 * L + j] = lg;
             xo[5 * L + j] = (float)j / (float)L;
@@ -705,21 +783,40 @@ __global__ void k_ff_encode_env(const float2* __restrict__ Y, long long ystride,
     }
 }
 
-// grid (2 bands): network output envelopes -> band bins of X (X zeroed by the host)
-__global__ void k_ff_decode_env(const float* __restrict__ y, const float* __restrict__ sigma, int N, int L, int logL,
-                                EnvBand bp, EnvBand bs, float pump_scale, float2* __restrict__ X) {
-    __shared__ float2 sm[4096];
+// Blocks 0 and 1: network output envelopes -> the band bins of X; the others clear the
+// bins outside both bands, ENV_T each
+__global__ void __launch_bounds__(ENV_T)
+    k_ff_decode_env(const float* __restrict__ y, const float* __restrict__ sigma, int N, int L, int logL, EnvBand bp,
+                    EnvBand bs, float pump_scale, float2* __restrict__ X) {
+    __shared__ float2 sm[ENV_MAX];
+    __shared__ float2 quad[ENV_MAX / 4];
+    dep_launch();
+    if (blockIdx.x >= 2) {
+        dep_wait();
+        const int k = (blockIdx.x - 2) * ENV_T + threadIdx.x;
+        bool in = k >= N;
+        for (const EnvBand& b : {bp, bs}) {
+            int o = k - b.kc;
+            if (o < 0) o += N;
+            if (o >= N - L / 2) o -= N;
+            in = in || (o >= b.lo && o < b.hi);
+        }
+        if (!in) X[k] = make_float2(0.f, 0.f);
+        return;
+    }
     const int band = blockIdx.x;
     const EnvBand bd = band ? bs : bp;
-    for (int j = threadIdx.x; j < L; j += blockDim.x)
-        sm[__brev((unsigned)j) >> (32 - logL)] = make_float2(y[(2 * band) * L + j], y[(2 * band + 1) * L + j]);
-    __syncthreads();
-    smem_fft(sm, L, -1.f);
+    env_table(quad, L);
+    dep_wait();
+    for (int j = threadIdx.x; j < L; j += ENV_T)
+        sm[env_slot(j)] = make_float2(y[(2 * band) * L + j], y[(2 * band + 1) * L + j]);
+    env_fft(sm, quad, logL);
     const float scale = (band ? sigma[0] : pump_scale) / (float)L;
-    for (int j = threadIdx.x; j < L; j += blockDim.x) {
+    for (int j = threadIdx.x; j < L; j += ENV_T) {
         bool in;
         const int k = env_bin(bd, N, L, j, &in);
-        if (in) X[k] = make_float2(sm[j].x * scale, sm[j].y * scale);
+        const float2 u = sm[env_slot(j)];
+        if (in) X[k] = make_float2(u.x * scale, u.y * scale);
     }
 }
 
@@ -789,13 +886,14 @@ inline int spec_splits(int B, int L) {
     return s < most ? s : (most > 0 ? most : 1);
 }
 
-int fno_forward(optifax_fno_s* f, const float* x, int B, cudaStream_t st) {
+int fno_forward(optifax_fno_s* f, const float* x, float* y, int B, cudaStream_t st) {
     const int L = f->L;
     const long long WB = (long long)W * B, rowsA = WB > 128 ? WB : 128;
     OFX_TRY(fno_maps(f, B));
     // the split-K products add into S: one clearing for the four layers
     if (cudaMemsetAsync(f->S[0], 0, sizeof(float) * NLAYER * WB * SPEC, st) != cudaSuccess) return OPTIFAX_ERR_CUDA;
-    k_lift<<<nblk((long long)B * L), 256, 0, st>>>(x, f->wb + OFF_P, f->master + OFF_PB, B, L, f->Hc[0], f->Ht[0]);
+    launch_dep(k_lift, dim3(nblk((long long)B * L, 64)), dim3(256), 0, st, x, f->wb + OFF_P, f->master + OFF_PB, B, L,
+               f->Hc[0], f->Ht[0]);
     for (int l = 0; l < NLAYER; ++l) {
         OFX_TRY(optifax_gemm_bf16(f->Hc[l], L, rowsA, f->F, L, SPEC, f->S[l], SPEC, (int)WB, SPEC, L,
                                   spec_splits(B, L), 1, st));
@@ -806,10 +904,11 @@ int fno_forward(optifax_fno_s* f, const float* x, int B, cudaStream_t st) {
         a.Z = a.act ? f->Z[l] : nullptr;
         a.Hc = f->Hc[l + 1]; a.Ht = f->Ht[l + 1];
         a.err = f->err; a.B = B; a.L = L;
-        k_layer<LAYER_FWD><<<dim3((L + 127) / 128, B), 128, LAYER_SMEM, st>>>(f->mG, f->mH[l], f->mT, f->mWp[l], a);
+        launch_dep(k_layer<LAYER_FWD>, dim3((L + 127) / 128, B), dim3(128), LAYER_SMEM, st, f->mG, f->mH[l], f->mT,
+                   f->mWp[l], a);
     }
-    k_proj_fwd<<<nblk((long long)B * L), 256, 0, st>>>(f->Ht[NLAYER], f->wb + OFF_Q, f->master + OFF_QB, x, B, L,
-                                                       f->y);
+    launch_dep(k_proj_fwd, dim3(nblk((long long)B * L, 64)), dim3(256), 0, st, f->Ht[NLAYER], f->wb + OFF_Q,
+               f->master + OFF_QB, x, B, L, y);
     return cudaGetLastError() == cudaSuccess ? OPTIFAX_OK : OPTIFAX_ERR_CUDA;
 }
 
@@ -822,10 +921,10 @@ int fno_backward(optifax_fno_s* f, const float* x, const float* target, const fl
         cudaMemsetAsync(f->loss, 0, sizeof(float), st) != cudaSuccess)
         return OPTIFAX_ERR_CUDA;
     const long long ny = BL * COUT;
-    k_loss<<<256, 256, 0, st>>>(f->y, target, sample_w, (long long)COUT * L, ny, 1.f / (float)ny, f->dy, f->loss);
-    k_proj_bwd<<<dim3((L + 255) / 256, B), 256, 0, st>>>(f->dy, f->wb + OFF_Q, f->Ht[NLAYER], B, L, f->dZc, f->dZt,
-                                                         f->grad + off_b(NLAYER - 1), f->grad + OFF_Q,
-                                                         f->grad + OFF_QB);
+    launch_dep(k_loss, dim3(256), dim3(256), 0, st, f->y, target, sample_w, (long long)COUT * L, ny, 1.f / (float)ny,
+               f->dy, f->loss);
+    launch_dep(k_proj_bwd, dim3((L + 255) / 256, B), dim3(256), 0, st, f->dy, f->wb + OFF_Q, f->Ht[NLAYER], B, L, f->dZc,
+               f->dZt, f->grad + off_b(NLAYER - 1), f->grad + OFF_Q, f->grad + OFF_QB);
     for (int l = NLAYER - 1; l >= 0; --l) {
         // dWp: K = B L over CTAs of 512 (64 rows of A: half of the tile is padding)
         const int splits = (int)(BL <= (4096LL << 9) ? (BL + 511) / 512 : 4096);
@@ -834,7 +933,8 @@ int fno_backward(optifax_fno_s* f, const float* x, const float* target, const fl
         OFX_TRY(optifax_gemm_bf16(f->dZc, L, 2 * WB, f->GT, L, SPEC, f->dT[l], SPEC, (int)WB, SPEC, L,
                                   spec_splits(B, L), 1, st));
         launch_mix<true>(f->dT[l], f->wb + off_ws(l), B, f->dS, st);
-        k_mix_bwd_dw<<<nblk((long long)W * W * MODES), 256, 0, st>>>(f->dT[l], f->S[l], B, f->grad + off_ws(l));
+        launch_dep(k_mix_bwd_dw, dim3(nblk((long long)W * W * MODES)), dim3(256), 0, st, f->dT[l], f->S[l], B,
+                   f->grad + off_ws(l));
         LayerArgs a = {};
         a.err = f->err; a.B = B; a.L = L;
         const dim3 grid((L + 127) / 128, B);
@@ -842,13 +942,13 @@ int fno_backward(optifax_fno_s* f, const float* x, const float* target, const fl
             a.Z = f->Z[l - 1];
             a.Hc = f->dZc; a.Ht = f->dZt;
             a.db = f->grad + off_b(l - 1);
-            k_layer<LAYER_BWD><<<grid, 128, LAYER_SMEM, st>>>(f->mFT, f->mDZ, f->mDS, f->mWpT[l], a);
+            launch_dep(k_layer<LAYER_BWD>, grid, dim3(128), LAYER_SMEM, st, f->mFT, f->mDZ, f->mDS, f->mWpT[l], a);
         } else {
             a.x = x;
             a.db = f->part;
-            k_layer<LAYER_BWD_IN><<<grid, 128, LAYER_SMEM, st>>>(f->mFT, f->mDZ, f->mDS, f->mWpT[l], a);
-            k_lift_sum<<<dim3(W * 8 / 32, 8), 256, 0, st>>>(f->part, (int)(grid.x * grid.y), f->grad + OFF_P,
-                                                            f->grad + OFF_PB);
+            launch_dep(k_layer<LAYER_BWD_IN>, grid, dim3(128), LAYER_SMEM, st, f->mFT, f->mDZ, f->mDS, f->mWpT[l], a);
+            launch_dep(k_lift_sum, dim3(W * 8 / 32, 8), dim3(256), 0, st, f->part, (int)(grid.x * grid.y),
+                       f->grad + OFF_P, f->grad + OFF_PB);
         }
     }
     return cudaGetLastError() == cudaSuccess ? OPTIFAX_OK : OPTIFAX_ERR_CUDA;
@@ -967,9 +1067,12 @@ extern "C" int optifax_fno_forward(optifax_fno f, const float* x, float* y, int3
     if (!f) return OPTIFAX_ERR_NULL_HANDLE;
     if (!x || batch < 1 || batch > f->maxB) return OPTIFAX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    OFX_TRY(fno_forward(f, x, batch, st));
-    if (y && cudaMemcpyAsync(y, f->y, sizeof(float) * (size_t)batch * COUT * f->L, cudaMemcpyDeviceToDevice, st) !=
-                 cudaSuccess)
+    // the network reads x to its end: an output that lies over the input is written last
+    const size_t nx = (size_t)batch * CIN * f->L, ny = (size_t)batch * COUT * f->L;
+    const bool apart = y && (y + ny <= x || x + nx <= y);
+    OFX_TRY(fno_forward(f, x, apart ? y : f->y, batch, st));
+    if (y && !apart &&
+        cudaMemcpyAsync(y, f->y, sizeof(float) * ny, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
         return OPTIFAX_ERR_CUDA;
     return OPTIFAX_OK;
 }
@@ -979,7 +1082,7 @@ extern "C" int optifax_fno_backward(optifax_fno f, const float* x, const float* 
     if (!f) return OPTIFAX_ERR_NULL_HANDLE;
     if (!x || !target || batch < 1 || batch > f->maxB) return OPTIFAX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    OFX_TRY(fno_forward(f, x, batch, st));
+    OFX_TRY(fno_forward(f, x, f->y, batch, st));
     OFX_TRY(fno_backward(f, x, target, sample_w, batch, st));
     if (loss && cudaMemcpyAsync(loss, f->loss, sizeof(float), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
         return OPTIFAX_ERR_CUDA;
@@ -1031,11 +1134,10 @@ extern "C" int optifax_ff_step(const float* y, const float* sigma, const void* X
         return OPTIFAX_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (energy && cudaMemsetAsync(energy, 0, sizeof(double), st) != cudaSuccess) return OPTIFAX_ERR_CUDA;
-    k_ff_step<<<nblk(n_points), 256, 0, st>>>(y, sigma, static_cast<const float2*>(X_in),
-                                              static_cast<const float2*>(feedback), static_cast<const float2*>(pump),
-                                              static_cast<const float2*>(lin), tally_w, n_points, k0, n_bins, split,
-                                              pump_scale, static_cast<float2*>(X_out), static_cast<float2*>(Y_next),
-                                              energy);
+    launch_dep(k_ff_step, dim3(nblk(n_points)), dim3(256), 0, st, y, sigma, static_cast<const float2*>(X_in),
+               static_cast<const float2*>(feedback), static_cast<const float2*>(pump), static_cast<const float2*>(lin),
+               tally_w, (int)n_points, (int)k0, (int)n_bins, (int)split, pump_scale, static_cast<float2*>(X_out),
+               static_cast<float2*>(Y_next), energy);
     return cudaGetLastError() == cudaSuccess ? OPTIFAX_OK : OPTIFAX_ERR_CUDA;
 }
 
@@ -1065,9 +1167,9 @@ extern "C" int optifax_ff_encode_env(const void* spectra, int64_t stride, int32_
         return OPTIFAX_ERR_INVALID_ARGUMENT;
     int rc = env_args(n_points, n_bins, band, &bp, &bs, &logL);
     if (rc) return rc;
-    k_ff_encode_env<<<dim3(n_spectra, 2), 512, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const float2*>(spectra), stride, n_points, n_bins, logL, bp, bs, pump_scale, sigma_in, x,
-        n_channels, sigma_out);
+    launch_dep(k_ff_encode_env, dim3(n_spectra, 2), dim3(ENV_T), 0, static_cast<cudaStream_t>(stream),
+               static_cast<const float2*>(spectra), (long long)stride, (int)n_points, (int)n_bins, logL, bp, bs,
+               pump_scale, sigma_in, x, (int)n_channels, sigma_out);
     return cudaGetLastError() == cudaSuccess ? OPTIFAX_OK : OPTIFAX_ERR_CUDA;
 }
 
@@ -1079,8 +1181,7 @@ extern "C" int optifax_ff_decode_env(const float* y, const float* sigma, int32_t
     int rc = env_args(n_points, n_bins, band, &bp, &bs, &logL);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (cudaMemsetAsync(X_out, 0, sizeof(float2) * (size_t)n_points, st) != cudaSuccess) return OPTIFAX_ERR_CUDA;
-    k_ff_decode_env<<<2, 512, 0, st>>>(y, sigma, n_points, n_bins, logL, bp, bs, pump_scale,
-                                       static_cast<float2*>(X_out));
+    launch_dep(k_ff_decode_env, dim3(2 + nblk(n_points, ENV_T)), dim3(ENV_T), 0, st, y, sigma, (int)n_points,
+               (int)n_bins, logL, bp, bs, pump_scale, static_cast<float2*>(X_out));
     return cudaGetLastError() == cudaSuccess ? OPTIFAX_OK : OPTIFAX_ERR_CUDA;
 }

@@ -69,6 +69,8 @@ __global__ void __launch_bounds__(128, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    dep_launch();
+    dep_wait();
 
     int issued = 0;
     if (threadIdx.x == 0) {
@@ -207,8 +209,9 @@ extern "C" int optifax_gemm_bf16(const void* A, int64_t lda, int64_t a_rows, con
         cudaMemset2DAsync(C, static_cast<size_t>(ldc) * 4, 0, static_cast<size_t>(N) * 4, M, st) != cudaSuccess)
         return OPTIFAX_ERR_CUDA;
     dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, nsplit);
-    gemm_bf16_tn<<<grid, 128, SMEM_BYTES, st>>>(ma, mb, g);
-    return cudaGetLastError() == cudaSuccess ? OPTIFAX_OK : OPTIFAX_ERR_CUDA;
+    return ofx_tc::launch_dep(gemm_bf16_tn, grid, dim3(128), SMEM_BYTES, st, ma, mb, g) == cudaSuccess
+               ? OPTIFAX_OK
+               : OPTIFAX_ERR_CUDA;
 }
 
 extern "C" int optifax_tc_error(int32_t* out, int32_t clear) {

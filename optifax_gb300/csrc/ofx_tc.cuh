@@ -12,6 +12,12 @@ namespace ofx_tc {
 // kernel reports an error instead of hanging.
 constexpr long long kWaitCycles = 4000000000LL;
 
+// Programmatic dependent launch: a kernel launched with the attribute may start before the
+// previous kernel of its stream has ended; dep_wait() returns once that kernel's memory is
+// complete and visible, dep_launch() lets the next one start.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

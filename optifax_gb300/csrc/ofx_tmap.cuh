@@ -39,6 +39,24 @@ inline int make_map(CUtensorMap* m, const void* ptr, long long rows, long long c
     return r == CUDA_SUCCESS ? OPTIFAX_OK : OPTIFAX_ERR_CUDA;
 }
 
+// Launch with programmatic stream serialisation: the kernel's start overlaps the end of
+// the stream's previous kernel (every kernel launched so calls dep_wait before it touches
+// global memory).  The surrogate's forward pass is a chain of 5 us kernels.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dep(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid;
+    lc.blockDim = block;
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, k, KArgs(args)...);
+}
+
 // Device address of the current device's error word (optifax_tc_error), or null
 int* error_word();
 
