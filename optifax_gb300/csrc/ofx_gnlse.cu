@@ -21,7 +21,7 @@
 // dispersion phase B_k z is a 64-bit fixed-point product (exact mod one turn; only
 // the final angle goes
 // through FP32).  FP32 field arithmetic, norms reduced across the CTA in FP64
-// (per-thread partials of 16 modes in FP32), FP64 step control.
+// (per-thread partials of 4 or 8 modes in FP32), FP64 step control.
 //
 // Layout: the CTA's M/P threads hold the spectral state y in registers, P modes each
 // (8, or 4 below 2048 points), in the FFT's bit-reversed slot order (slot s <-> mode
@@ -32,7 +32,10 @@
 // conj(inverse(conj(.))), its ifft (1/n) conj(forward(conj(.))).  The point-wise steps in
 // the time domain work on the registers between the last pass of an inverse and the
 // first pass of the next forward transform, so one shared-memory buffer serves all four.
-// What bounds it: the serial chain of 24 transforms a step on one SM per pulse.
+// Stages 2, 4 and 6 read the rows once for two sums, their own and the next stage's (the
+// error's), which waits in shared memory for its last term: 9 rows read a step, not 26.
+// What bounds it: the serial chain of 24 transforms a step on one SM per pulse (2,500 to
+// 3,500 cycles each at 4096 points).
 #include <cmath>
 #include <cstdint>
 
@@ -50,39 +53,44 @@ __constant__ double kDpC[7] = {0.0, 1.0 / 5, 3.0 / 10, 4.0 / 5, 8.0 / 9, 1.0, 1.
 
 __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
 
-// Sums of two per-thread values over the CTA in FP64; every thread gets them.
-template <int T>
-__device__ __forceinline__ void block_sum2(double a, double b, double* red, double (&out)[2]) {
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    const int t = threadIdx.x;
-    __syncthreads();                       // red may still be read from the previous call
-    if ((t & 31) == 0) {
-        red[2 * (t >> 5)] = a;
-        red[2 * (t >> 5) + 1] = b;
-    }
-    __syncthreads();
-    double s0 = 0.0, s1 = 0.0;
-#pragma unroll 1
-    for (int w = 0; w < T / 32; ++w) {     // fixed order: identical totals in every thread
-        s0 += red[2 * w];
-        s1 += red[2 * w + 1];
-    }
-    out[0] = s0; out[1] = s1;
-}
-
-// Squared norm of a thread's modes: FP32 partial sums (8 terms, relative error below
-// 1e-6), widened once for the FP64 block reduction.  GB300's FP64 pipe is narrow, so
-// per-mode FP64 conversions and adds cost a visible share of the step.
+// Squared norm of a thread's modes: FP32 partial sums (8 terms, relative error below 1e-6)
 template <int P>
-__device__ __forceinline__ double norm2(const float2 (&a)[P]) {
+__device__ __forceinline__ float norm2(const float2 (&a)[P]) {
     float s = 0.f;
 #pragma unroll
     for (int j = 0; j < P; ++j) s = fmaf(a[j].x, a[j].x, fmaf(a[j].y, a[j].y, s));
-    return (double)s;
+    return s;
+}
+
+// Sums of two per-thread values over the CTA in FP64 (part: 2 T floats, red: 8 doubles),
+// for warp 0 alone.  An FP64 instruction of one warp takes 64 cycles of its scheduler's
+// narrow FP64 unit, so the sums are four warps' work, one per scheduler, and every warp
+// reducing its own and adding up all warps' (as this was) took 10,000 cycles.
+template <int T>
+__device__ __forceinline__ void block_sum2(float a, float b, float* part, double* red, double (&out)[2]) {
+    const int t = threadIdx.x;
+    part[t] = a;
+    part[T + t] = b;
+    __syncthreads();
+    if (t < 128) {
+        double x = 0.0, y = 0.0;
+#pragma unroll
+        for (int i = 0; i < T / 128; ++i) {
+            x += (double)part[t + 128 * i];
+            y += (double)part[T + t + 128 * i];
+        }
+        // lanes 0-15 go on with a, 16-31 with b
+        const bool up = t & 16;
+        double z = (up ? y : x) + __shfl_xor_sync(0xffffffffu, up ? x : y, 16);
+#pragma unroll
+        for (int o = 8; o >= 1; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+        if ((t & 15) == 0) red[2 * (t >> 5) + (up ? 1 : 0)] = z;
+    }
+    __syncthreads();
+    if (t < 32) {
+        out[0] = (red[0] + red[2]) + (red[4] + red[6]);
+        out[1] = (red[1] + red[3]) + (red[5] + red[7]);
+    }
 }
 
 // Own modes of stage array j in the global scratch: pairs of modes, [pair][thread]
@@ -142,20 +150,37 @@ __host__ __device__ constexpr float dp_e(int q) {
     }
 }
 
-// acc += sum_q w_q h K[(base + q) % 7] over the compile-time weights w_q (row R of
-// kA, or kE when R < 0), q < NQ
-template <int R, int NQ, int M, int P>
-__device__ __forceinline__ void combine(float2 (&acc)[P], const float2* K, int t, int base, float hz) {
+// a += sum_{q < R - 1} a_Rq h k_q and, with the row after it (R2; the error weights when
+// R2 < 0), b += sum_{q < R - 1} w_q h k_q from one reading of the rows; then both add
+// the k_{R-1} of the registers.  The next stage continues from b.
+template <int R, int R2, int M, int P>
+__device__ __forceinline__ void combine2(float2 (&a)[P], float2 (&b)[P], const float2 (&last)[P], const float2* K,
+                                         int t, int base, float hz) {
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        const float wq = (R >= 0) ? dp_a(R, q) : dp_e(q);
-        if (wq == 0.f) continue;
+    for (int q = 0; q < R; ++q) {
+        const float wa = dp_a(R, q), wb = R2 >= 0 ? dp_a(R2, q) : dp_e(q);
+        if (wa == 0.f && wb == 0.f) continue;
         float2 k[P];
-        load_row<M, P>(K, (base + q) % 7, t, k);
+        if (q < R - 1) load_row<M, P>(K, (base + q) % 7, t, k);
 #pragma unroll
-        for (int j = 0; j < P; ++j) acc[j] = cfma1(k[j], hz * wq, acc[j]);
+        for (int j = 0; j < P; ++j) {
+            const float2 kj = q < R - 1 ? k[j] : last[j];
+            if (wa != 0.f) a[j] = cfma1(kj, hz * wa, a[j]);
+            if (wb != 0.f) b[j] = cfma1(kj, hz * wb, b[j]);
+        }
     }
 }
+
+// What warp 0 decides and the CTA reads.
+struct GCtl {
+    double ny, acc_nyn, acc_err;
+    long long zc, hc, h, side_z, save_z;
+    long long zs[8];                     // the attempt's stage positions, with e^{-alpha z / 2} and its inverse
+    float att[8], iatt[8];
+    float hz, save_att;
+    int save_idx, save_i, attempts, accepted, status, nofailed, side, base, flags;
+};
+enum : int { kStash = 1, kAdvance = 2, kSave = 4, kEnd = 8 };
 
 }  // namespace
 
@@ -168,8 +193,8 @@ struct SmemG {
     static constexpr size_t off_w = off_rw + sizeof(float2) * M;
     static constexpr size_t off_tw = off_w + sizeof(float) * M;
     static constexpr size_t off_td = (off_tw + sizeof(float2) * F::TW + 15) & ~size_t(15);
-    static constexpr size_t off_red = off_td + sizeof(float) * F::TD;
-    static constexpr size_t bytes = off_red + sizeof(double) * 2 * (T / 32);
+    static constexpr size_t off_part = off_td + sizeof(float) * F::TD;             // sum carried to the next stage
+    static constexpr size_t bytes = off_part + sizeof(float2) * M;
 };
 
 template <int M>
@@ -185,7 +210,10 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
     float* w_s = reinterpret_cast<float*>(smem + SM::off_w);
     float2* tw = reinterpret_cast<float2*>(smem + SM::off_tw);
     float* td = reinterpret_cast<float*>(smem + SM::off_td);
-    double* red = reinterpret_cast<double*>(smem + SM::off_red);
+    float4* carry = reinterpret_cast<float4*>(smem + SM::off_part);
+    float* part = reinterpret_cast<float*>(smem);                         // norms: buf between two transforms
+    __shared__ double red[8];
+    __shared__ GCtl ctl;
 
     const int t = threadIdx.x;
     __shared__ GnlseDev sP;
@@ -223,206 +251,302 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
 #pragma unroll
     for (int j = 0; j < P; ++j) y[j] = cscale(conjf2(v[j]), invM);
 
-    long long zc = 0, hc = 0, h = 0, side_z = 0;
-    int save_idx = 0, stage = 0, base = 0;
-    int attempts = 0, accepted = 0, status = 0;
-    bool nofailed = true, new_step = true, side = false;
-    double ny = 0.0, acc_nyn = 0.0, acc_err = 0.0;
-    float hz = 0.f;
     const long long nm1 = P_.n_saves - 1;
     auto save_point = [&](int i) -> long long { return ((long long)i * total + nm1 / 2) / nm1; };
 
-    // save `save_idx` from the spectral state src at position zp: AW e^{Lz}
+    // ---- control: warp 0, all lanes the same values, lane 0 writes ----
+    // The scalar FP64 arithmetic of a step in every warp cost a third of the step (a warp's
+    // FP64 instruction occupies the scheduler's unit for 64 cycles).
+    // Positions and attenuations of the next attempt's stages, one per lane; side: a step to side_z
+    auto prepare = [&](bool side) {
+        const int stage = t < 7 ? t : 6;
+        const long long span = side ? ctl.side_z - ctl.zc : ctl.hc;
+        const long long zs = stage == 0 ? (side ? ctl.side_z : ctl.zc) : ctl.zc + llrint(kDpC[stage] * (double)span);
+        const double zd = (double)zs * unit;
+        const float att = expf((float)(-0.5 * P_.alpha * zd)), iatt = expf((float)(0.5 * P_.alpha * zd));
+        const float hz = (float)((double)span * unit);
+        __syncwarp();
+        if (t < 7) {
+            ctl.zs[t] = zs;
+            ctl.att[t] = att;
+            ctl.iatt[t] = iatt;
+        }
+        if (t == 0) {
+            ctl.hz = hz;
+            ctl.side = side;
+            if (side) {
+                ctl.save_i = ctl.save_idx++;
+                ctl.save_z = zs;
+                ctl.save_att = att;
+            }
+        }
+        __syncwarp();
+    };
+    auto new_step = [&](long long h) {                 // a first attempt with step h
+        h = h > hmax ? hmax : (h < 1 ? 1 : h);
+        long long hc = h;
+        const long long left = total - ctl.zc;
+        if (1.1 * (double)hc >= (double)left) hc = left;                   // stretch to the end
+        __syncwarp();
+        if (t == 0) { ctl.h = h; ctl.hc = hc; ctl.nofailed = 1; }
+        __syncwarp();
+        prepare(false);
+    };
+    auto side_step = [&]() -> bool {                   // the next save point, if inside the accepted step
+        const int i = ctl.save_idx;
+        const long long z = i < P_.n_saves ? save_point(i) : 0;
+        const bool in = i < P_.n_saves && z < ctl.zc + ctl.hc;
+        __syncwarp();
+        if (in) {
+            if (t == 0) ctl.side_z = z;
+            __syncwarp();
+            prepare(true);
+        }
+        return in;
+    };
+    auto advance = [&]() -> int {                      // the accepted step becomes the state
+        const long long hc = ctl.hc, zc = ctl.zc + hc;
+        const double err = ctl.acc_err;
+        int i = ctl.save_idx, flags = kAdvance;
+        if (i < P_.n_saves && save_point(i) == zc) {
+            flags |= kSave;
+            if (t == 0) {
+                ctl.save_i = i;
+                ctl.save_z = zc;
+                ctl.save_att = expf((float)(-0.5 * P_.alpha * (double)zc * unit));
+            }
+            ++i;
+        }
+        const bool nofailed = ctl.nofailed, limit = ctl.attempts >= P_.max_attempts;
+        __syncwarp();
+        if (t == 0) {
+            ctl.zc = zc;
+            ctl.ny = ctl.acc_nyn;
+            ctl.base = (ctl.base + 6) % 7;             // FSAL: k7 becomes the next k1
+            ctl.save_idx = i;
+        }
+        __syncwarp();
+        if (i >= P_.n_saves || zc >= total) return flags | kEnd;
+        // growth after a step with no failure: h / (1.25 (err/rtol)^(1/5)), at most 5 h
+        long long h = hc;
+        if (nofailed) {
+            const float ratio = (float)(err / P_.rtol);
+            const float temp = 1.25f * powf(ratio, 0.2f);
+            h = temp > 0.2f ? (long long)((double)hc / (double)temp) : 5 * hc;
+        }
+        if (limit) {
+            if (t == 0) ctl.status |= OPTIFAX_PULSE_ATTEMPT_LIMIT;
+            return flags | kEnd;
+        }
+        new_step(h);
+        return flags;
+    };
+    auto decide = [&](const double (&s2)[2]) -> int {  // after the last stage of an attempt
+        const double root = sqrt((t & 1) ? s2[1] : s2[0]);
+        const double errn = __shfl_sync(0xffffffffu, root, 0), nyn = __shfl_sync(0xffffffffu, root, 1);
+        const double err = errn / fmax(fmax(ctl.ny, nyn), thr);
+        const bool ok = err <= P_.rtol;
+        const int attempts = ctl.attempts;
+        const long long hc = ctl.hc;
+        const bool nofailed = ctl.nofailed, nan = !isfinite(errn) || !isfinite(nyn);
+        __syncwarp();
+        if (t == 0) {
+            if (P_.trace && attempts < P_.trace_cap) {
+                P_.trace[2 * attempts] = hc;
+                P_.trace[2 * attempts + 1] = ok ? 1 : 0;
+            }
+            ctl.attempts = attempts + 1;
+            if (nan) ctl.status |= OPTIFAX_PULSE_NAN;
+            else if (ok) {
+                ++ctl.accepted;
+                ctl.acc_err = err;
+                ctl.acc_nyn = nyn;
+            }
+        }
+        __syncwarp();
+        if (nan) return kEnd;
+        // a save point inside the step: y_new is stashed, then a step of exactly that length
+        if (ok) return side_step() ? kStash : advance();
+        // a failed step: the first failure scales by max(0.1, 0.8 (rtol/err)^(1/5)),
+        // later ones halve (the factor only scales an integer step: FP32 powf serves)
+        long long next = hc / 2;
+        if (nofailed) {
+            const float errf = (float)err;
+            next = (long long)((double)hc * (double)fmaxf(0.1f, 0.8f * powf((float)P_.rtol / errf, 0.2f)));
+        }
+        if (t == 0) {
+            ctl.nofailed = 0;
+            ctl.hc = next < 1 ? 1 : next;
+        }
+        __syncwarp();
+        if (attempts + 1 >= P_.max_attempts) {
+            if (t == 0) ctl.status |= OPTIFAX_PULSE_ATTEMPT_LIMIT;
+            return kEnd;
+        }
+        prepare(false);
+        return 0;
+    };
+
+    // save ctl.save_i from the spectral state src at position ctl.save_z: AW e^{Lz}
     // (fftshifted, x dT n) and AT = fft(AW e^{Lz})
-    auto do_save = [&](const float2 (&src)[P], long long zp) {
-        const float att = expf((float)(-0.5 * P_.alpha * (double)zp * unit));
+    auto do_save = [&](const float2 (&src)[P]) {
+        const float att = ctl.save_att;
+        const uint64_t zp = (uint64_t)ctl.save_z;
+        const size_t row = (size_t)ctl.save_i * M;
 #pragma unroll
         for (int j = 0; j < P; ++j) {
-            const float2 aw = cscale(cmul(src[j], turn_to_unit(rate_s[j * T + t] * (uint64_t)zp)), att);
+            const float2 aw = cscale(cmul(src[j], turn_to_unit(rate_s[j * T + t] * zp)), att);
             const int k = bitrev(P * t + j, LOG2M);
-            P_.AW_out[(size_t)save_idx * M + ((k + M / 2) & (M - 1))] = cscale(aw, awscale);
+            P_.AW_out[row + ((k + M / 2) & (M - 1))] = cscale(aw, awscale);
             v[j] = conjf2(aw);
         }
         fftp_inverse<M, P>(buf, tw, td, t, v);
 #pragma unroll
-        for (int q = 0; q < P; ++q) P_.AT_out[(size_t)save_idx * M + t + q * T] = conjf2(v[q]);
+        for (int q = 0; q < P; ++q) P_.AT_out[row + t + q * T] = conjf2(v[q]);
         __syncthreads();                   // the next transform writes what others may still read
-        ++save_idx;
     };
-    do_save(y, 0);
+    if (t == 0) {
+        ctl = GCtl{};
+        ctl.att[0] = ctl.iatt[0] = ctl.save_att = 1.f;
+        ctl.save_idx = 1;
+    }
+    __syncthreads();
+    do_save(y);
 
+    int stage = 0, base = 0, side = 0;
     for (;;) {
-        // ---- stage input ys and its position zs ----
-        long long zs = zc;
+        // ---- stage input ys: every second stage reads the rows for itself and the next ----
 #pragma unroll
         for (int j = 0; j < P; ++j) ys[j] = y[j];
-        if (stage > 0) {
-            if (stage == 1 && !side) {
-                if (new_step) {
-                    h = h > hmax ? hmax : (h < 1 ? 1 : h);
-                    hc = h;
-                    if (1.1 * (double)hc >= (double)(total - zc)) hc = total - zc;   // stretch to the end
-                    nofailed = true;
-                    new_step = false;
-                }
-                hz = (float)((double)hc * unit);
-            } else if (stage == 1) {
-                hz = (float)((double)(side_z - zc) * unit);
+        const float hz = ctl.hz;
+        float2 part2[P];                   // the next stage's sum without its last term (stage 6: the error's)
+        if (stage == 1) {
+            float2 k[P];
+            load_row<M, P>(K, base, t, k);
+#pragma unroll
+            for (int j = 0; j < P; ++j) ys[j] = cfma1(k[j], hz * dp_a(1, 0), ys[j]);
+        } else if (stage == 3 || stage == 5) {
+            const float w = hz * (stage == 3 ? dp_a(3, 2) : dp_a(5, 4));
+#pragma unroll
+            for (int i = 0; i < P / 2; ++i) {
+                const float4 c = carry[i * T + t];
+                ys[2 * i] = cfma1(v[2 * i], w, make_float2(c.x, c.y));
+                ys[2 * i + 1] = cfma1(v[2 * i + 1], w, make_float2(c.z, c.w));
             }
-            switch (stage) {
-                case 1: combine<1, 1, M, P>(ys, K, t, base, hz); break;
-                case 2: combine<2, 2, M, P>(ys, K, t, base, hz); break;
-                case 3: combine<3, 3, M, P>(ys, K, t, base, hz); break;
-                case 4: combine<4, 4, M, P>(ys, K, t, base, hz); break;
-                case 5: combine<5, 5, M, P>(ys, K, t, base, hz); break;
-                default: combine<6, 6, M, P>(ys, K, t, base, hz); break;
-            }
-            zs = zc + llrint(kDpC[stage] * (double)(side ? side_z - zc : hc));
+        } else if (stage != 0) {
+#pragma unroll
+            for (int j = 0; j < P; ++j) part2[j] = stage == 6 ? make_float2(0.f, 0.f) : y[j];
+            if (stage == 2) combine2<2, 3, M, P>(ys, part2, v, K, t, base, hz);
+            else if (stage == 4) combine2<4, 5, M, P>(ys, part2, v, K, t, base, hz);
+            else combine2<6, -1, M, P>(ys, part2, v, K, t, base, hz);
+#pragma unroll
+            for (int i = 0; i < P / 2; ++i)
+                carry[i * T + t] = make_float4(part2[2 * i].x, part2[2 * i].y, part2[2 * i + 1].x, part2[2 * i + 1].y);
         }
-        // ---- right-hand side f(zs, ys) (gnlsefib.m:54-66) into v ----
-        {
-            const double zd = (double)zs * unit;
-            const float att = expf((float)(-0.5 * P_.alpha * zd));
-            const float iatt = expf((float)(0.5 * P_.alpha * zd));
-#pragma unroll
-            for (int j = 0; j < P; ++j) {
-                e[j] = turn_to_unit(rate_s[j * T + t] * (uint64_t)zs);       // e^{i B z}
-                v[j] = conjf2(cscale(cmul(ys[j], e[j]), att));
-            }
-            fftp_inverse<M, P>(buf, tw, td, t, v);                            // conj(AT)
-            float2 at[P];
-#pragma unroll
-            for (int q = 0; q < P; ++q) at[q] = conjf2(v[q]);
-            if (raman) {
-#pragma unroll
-                for (int q = 0; q < P; ++q) v[q] = make_float2(at[q].x * at[q].x + at[q].y * at[q].y, 0.f);
-                fftp_forward_regs<M, P>(buf, tw, t, v);                       // forward(|AT|^2)
-#pragma unroll
-                for (int j = 0; j < P; ++j)                                   // conj(ifft(|AT|^2) RW)
-                    v[j] = conjf2(cscale(cmul(conjf2(v[j]), rw_s[j * T + t]), invM));
-                fftp_inverse<M, P>(buf, tw, td, t, v);                        // conj(RS / (dT fR))
-            }
-#pragma unroll
-            for (int q = 0; q < P; ++q) {
-                const float it = at[q].x * at[q].x + at[q].y * at[q].y;
-                const float2 g = raman ? make_float2(fmaf(omfr, it, dtfr * v[q].x), -dtfr * v[q].y)
-                                       : make_float2(it, 0.f);
-                v[q] = conjf2(cmul(at[q], g));                                // conj(Q)
-            }
-            fftp_forward_regs<M, P>(buf, tw, t, v);                           // ifft(Q) = conj(v) / M
-#pragma unroll
-            for (int j = 0; j < P; ++j) {
-                const float2 m = cmul(conjf2(v[j]), conjf2(e[j]));
-                const float s = gam * w_s[j * T + t] * iatt * invM;
-                v[j] = make_float2(-m.y * s, m.x * s);                        // i gamma W M e^{-Lz}
-            }
-        }
-        store_row<M, P>(K, (base + stage) % 7, t, v);
-        if (stage == 0) {
-            // initial step (ode45, NormControl): min(hmax, 0.8 rtol^(1/5) max(||y||, thr) / ||f||)
-            double s2[2];
-            block_sum2<T>(norm2(y), norm2(v), red, s2);
-            ny = sqrt(s2[0]);
-            const double nf = sqrt(s2[1]);
-            if (nf == 0.0) h = hmax;
-            else {
-                double hh = (0.8 * pow(P_.rtol, 0.2)) * fmax(ny, thr) / nf / unit;
-                long long hi = hh >= (double)hmax ? hmax : (long long)hh;
-                h = hi < 1 ? 1 : hi;
-            }
-            stage = 1;
-            continue;
-        }
-        bool finish = false;
-        if (side) {
-            if (stage < 5) { ++stage; continue; }
+        int flags = 0;
+        if (stage == 6 && side) {
             // stages k2..k6 of the step to the save point done: y(side_z) = y + h' sum a_7j k_j
+            do_save(ys);
+            if (t < 32) {
+                const int f = side_step() ? 0 : advance();
+                if (t == 0) {
+                    if (f) ctl.side = 0;
+                    ctl.flags = f;
+                }
+            }
+            __syncthreads();
+            flags = ctl.flags;
+            if (flags & kAdvance) load_row<M, P>(K, 7, t, ys);       // back to the accepted step
+        } else {
+            // ---- right-hand side f(zs, ys) (gnlsefib.m:54-66) into v ----
+            {
+                const uint64_t zs = (uint64_t)ctl.zs[stage];
+                const float att = ctl.att[stage], iatt = ctl.iatt[stage];
 #pragma unroll
-            for (int j = 0; j < P; ++j) ys[j] = y[j];
-            combine<6, 6, M, P>(ys, K, t, base, hz);
-            do_save(ys, side_z);
-            if (save_idx < P_.n_saves && save_point(save_idx) < zc + hc) {
-                side_z = save_point(save_idx);
+                for (int j = 0; j < P; ++j) {
+                    e[j] = turn_to_unit(rate_s[j * T + t] * zs);              // e^{i B z}
+                    v[j] = conjf2(cscale(cmul(ys[j], e[j]), att));
+                }
+                fftp_inverse<M, P>(buf, tw, td, t, v);                        // conj(AT)
+                float2 at[P];
+#pragma unroll
+                for (int q = 0; q < P; ++q) at[q] = conjf2(v[q]);
+                if (raman) {
+#pragma unroll
+                    for (int q = 0; q < P; ++q) v[q] = make_float2(at[q].x * at[q].x + at[q].y * at[q].y, 0.f);
+                    fftp_forward_regs<M, P>(buf, tw, t, v);                   // forward(|AT|^2)
+#pragma unroll
+                    for (int j = 0; j < P; ++j)                               // conj(ifft(|AT|^2) RW)
+                        v[j] = conjf2(cscale(cmul(conjf2(v[j]), rw_s[j * T + t]), invM));
+                    fftp_inverse<M, P>(buf, tw, td, t, v);                    // conj(RS / (dT fR))
+                }
+#pragma unroll
+                for (int q = 0; q < P; ++q) {
+                    const float it = at[q].x * at[q].x + at[q].y * at[q].y;
+                    const float2 g = raman ? make_float2(fmaf(omfr, it, dtfr * v[q].x), -dtfr * v[q].y)
+                                           : make_float2(it, 0.f);
+                    v[q] = conjf2(cmul(at[q], g));                            // conj(Q)
+                }
+                fftp_forward_regs<M, P>(buf, tw, t, v);                       // ifft(Q) = conj(v) / M
+#pragma unroll
+                for (int j = 0; j < P; ++j) {
+                    const float2 m = cmul(conjf2(v[j]), conjf2(e[j]));
+                    const float s = gam * w_s[j * T + t] * iatt * invM;
+                    v[j] = make_float2(-m.y * s, m.x * s);                    // i gamma W M e^{-Lz}
+                }
+            }
+            if (stage != 5) store_row<M, P>(K, (base + stage) % 7, t, v);     // k6 stays in registers
+            if (stage > 0 && stage < 6) { ++stage; continue; }
+            double s2[2];
+            __syncthreads();                   // buf is free for the norms
+            if (stage == 0) {
+                // initial step (ode45, NormControl): min(hmax, 0.8 rtol^(1/5) max(||y||, thr) / ||f||)
+                block_sum2<T>(norm2(y), norm2(v), part, red, s2);
+                if (t < 32) {
+                    const double ny = sqrt(s2[0]), nf = sqrt(s2[1]);
+                    long long h = hmax;
+                    if (nf != 0.0) {
+                        const double hh = (0.8 * pow(P_.rtol, 0.2)) * fmax(ny, thr) / nf / unit;
+                        const long long hi = hh >= (double)hmax ? hmax : (long long)hh;
+                        h = hi < 1 ? 1 : hi;
+                    }
+                    if (t == 0) ctl.ny = ny;
+                    new_step(h);
+                }
+                __syncthreads();
                 stage = 1;
                 continue;
             }
-            // back to the accepted step: y_new from the stash row
-            load_row<M, P>(K, 7, t, ys);
-            side = false;
-            finish = true;
-        } else {
-            if (stage < 6) { ++stage; continue; }
-
             // ---- stage 6 done: ys = y_new, error estimate and decision ----
             float2 ev[P];
 #pragma unroll
-            for (int j = 0; j < P; ++j) ev[j] = make_float2(0.f, 0.f);
-            combine<-1, 7, M, P>(ev, K, t, base, hz);
-            double s2[2];
-            block_sum2<T>(norm2(ev), norm2(ys), red, s2);
-            const double errn = sqrt(s2[0]), nyn = sqrt(s2[1]);
-            const double err = errn / fmax(fmax(ny, nyn), thr);
-            const bool ok = err <= P_.rtol;
-            if (t == 0 && P_.trace && attempts < P_.trace_cap) {
-                P_.trace[2 * attempts] = hc;
-                P_.trace[2 * attempts + 1] = ok ? 1 : 0;
+            for (int i = 0; i < P / 2; ++i) {
+                const float4 c = carry[i * T + t];
+                ev[2 * i] = cfma1(v[2 * i], hz * dp_e(6), make_float2(c.x, c.y));
+                ev[2 * i + 1] = cfma1(v[2 * i + 1], hz * dp_e(6), make_float2(c.z, c.w));
             }
-            ++attempts;
-            if (!isfinite(errn) || !isfinite(nyn)) { status |= OPTIFAX_PULSE_NAN; break; }
-            if (ok) {
-                ++accepted;
-                acc_err = err;
-                acc_nyn = nyn;
-                if (save_idx < P_.n_saves && save_point(save_idx) < zc + hc) {
-                    // a save point inside the step: stash y_new, then a step of exactly that length
-                    store_row<M, P>(K, 7, t, ys);
-                    side = true;
-                    side_z = save_point(save_idx);
-                    stage = 1;
-                    continue;
-                }
-                finish = true;
-            } else {
-                // a failed step: the first failure scales by max(0.1, 0.8 (rtol/err)^(1/5)),
-                // later ones halve (the factor only scales an integer step: FP32 powf serves)
-                if (nofailed) {
-                    nofailed = false;
-                    const float errf = (float)err;
-                    const double fac = (double)fmaxf(0.1f, 0.8f * powf((float)P_.rtol / errf, 0.2f));
-                    const long long hi = (long long)((double)hc * fac);
-                    hc = hi < 1 ? 1 : hi;
-                } else {
-                    hc = hc / 2 < 1 ? 1 : hc / 2;
-                }
-                if (attempts >= P_.max_attempts) { status |= OPTIFAX_PULSE_ATTEMPT_LIMIT; break; }
-                stage = 1;
-                continue;
+            block_sum2<T>(norm2(ev), norm2(ys), part, red, s2);
+            if (t < 32) {
+                const int f = decide(s2);
+                if (t == 0) ctl.flags = f;
             }
+            __syncthreads();
+            flags = ctl.flags;
+            if (flags & kStash) store_row<M, P>(K, 7, t, ys);
         }
-        if (finish) {
-            zc += hc;
+        if (flags & kAdvance) {
+            base = ctl.base;
 #pragma unroll
             for (int j = 0; j < P; ++j) y[j] = ys[j];
-            ny = acc_nyn;
-            base = (base + 6) % 7;                          // FSAL: k7 becomes the next k1
-            if (save_idx < P_.n_saves && save_point(save_idx) == zc) do_save(y, zc);
-            if (save_idx >= P_.n_saves || zc >= total) break;
-            // growth after a step with no failure: h / (1.25 (err/rtol)^(1/5)), at most 5 h
-            if (nofailed) {
-                const float ratio = (float)(acc_err / P_.rtol);
-                const float temp = 1.25f * powf(ratio, 0.2f);
-                h = temp > 0.2f ? (long long)((double)hc / (double)temp) : 5 * hc;
-            } else {
-                h = hc;
-            }
-            new_step = true;
-            if (attempts >= P_.max_attempts) { status |= OPTIFAX_PULSE_ATTEMPT_LIMIT; break; }
-            stage = 1;
+            if (flags & kSave) do_save(y);
         }
+        if (flags & kEnd) break;
+        side = ctl.side;
+        stage = 1;
     }
     if (t == 0 && P_.stats) {
         optifax_gnlse_stats st;
-        st.attempts = attempts; st.accepted = accepted; st.status = status; st.reserved = 0;
+        st.attempts = ctl.attempts; st.accepted = ctl.accepted; st.status = ctl.status; st.reserved = 0;
         *P_.stats = st;
     }
 }
