@@ -174,7 +174,8 @@ __device__ __forceinline__ void combine2(float2 (&a)[P], float2 (&b)[P], const f
 // What warp 0 decides and the CTA reads.
 struct GCtl {
     double ny, acc_nyn, acc_err;
-    long long zc, hc, h, side_z, save_z;
+    long long zc, hc, side_z, save_z;
+    long long next_z;                    // position of save point save_idx (past the end: none left)
     long long zs[8];                     // the attempt's stage positions, with e^{-alpha z / 2} and its inverse
     float att[8], iatt[8];
     float hz, save_att;
@@ -225,7 +226,8 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
     const double unit = P_.length / (double)(1ll << kZBits);
     const long long total = 1ll << kZBits;
     const long long hmax = total / 10;
-    const double thr = P_.atol / P_.rtol;
+    const double thr = P_.atol / P_.rtol, half_loss = 0.5 * P_.alpha;
+    const float rtolf = (float)P_.rtol;
     constexpr float invM = 1.0f / (float)M;
     const float gam = (float)P_.gamma, omfr = (float)(1.0 - P_.fr), dtfr = (float)(P_.dT * P_.fr);
     const float awscale = (float)(P_.dT * (double)M);
@@ -252,7 +254,9 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
     for (int j = 0; j < P; ++j) y[j] = cscale(conjf2(v[j]), invM);
 
     const long long nm1 = P_.n_saves - 1;
-    auto save_point = [&](int i) -> long long { return ((long long)i * total + nm1 / 2) / nm1; };
+    auto save_point = [&](int i) -> long long {
+        return i < P_.n_saves ? ((long long)i * total + nm1 / 2) / nm1 : total + 1;
+    };
 
     // ---- control: warp 0, all lanes the same values, lane 0 writes ----
     // The scalar FP64 arithmetic of a step in every warp cost a third of the step (a warp's
@@ -263,7 +267,7 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
         const long long span = side ? ctl.side_z - ctl.zc : ctl.hc;
         const long long zs = stage == 0 ? (side ? ctl.side_z : ctl.zc) : ctl.zc + llrint(kDpC[stage] * (double)span);
         const double zd = (double)zs * unit;
-        const float att = expf((float)(-0.5 * P_.alpha * zd)), iatt = expf((float)(0.5 * P_.alpha * zd));
+        const float loss = (float)(half_loss * zd), att = expf(-loss), iatt = expf(loss);
         const float hz = (float)((double)span * unit);
         __syncwarp();
         if (t < 7) {
@@ -275,7 +279,10 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
             ctl.hz = hz;
             ctl.side = side;
             if (side) {
-                ctl.save_i = ctl.save_idx++;
+                const int i = ctl.save_idx;
+                ctl.save_i = i;
+                ctl.save_idx = i + 1;
+                ctl.next_z = save_point(i + 1);
                 ctl.save_z = zs;
                 ctl.save_att = att;
             }
@@ -288,14 +295,13 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
         const long long left = total - ctl.zc;
         if (1.1 * (double)hc >= (double)left) hc = left;                   // stretch to the end
         __syncwarp();
-        if (t == 0) { ctl.h = h; ctl.hc = hc; ctl.nofailed = 1; }
+        if (t == 0) { ctl.hc = hc; ctl.nofailed = 1; }
         __syncwarp();
         prepare(false);
     };
     auto side_step = [&]() -> bool {                   // the next save point, if inside the accepted step
-        const int i = ctl.save_idx;
-        const long long z = i < P_.n_saves ? save_point(i) : 0;
-        const bool in = i < P_.n_saves && z < ctl.zc + ctl.hc;
+        const long long z = ctl.next_z;
+        const bool in = z < ctl.zc + ctl.hc;
         __syncwarp();
         if (in) {
             if (t == 0) ctl.side_z = z;
@@ -307,32 +313,30 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
     auto advance = [&]() -> int {                      // the accepted step becomes the state
         const long long hc = ctl.hc, zc = ctl.zc + hc;
         const double err = ctl.acc_err;
-        int i = ctl.save_idx, flags = kAdvance;
-        if (i < P_.n_saves && save_point(i) == zc) {
-            flags |= kSave;
-            if (t == 0) {
-                ctl.save_i = i;
-                ctl.save_z = zc;
-                ctl.save_att = expf((float)(-0.5 * P_.alpha * (double)zc * unit));
-            }
-            ++i;
-        }
+        const bool save = ctl.next_z == zc;
+        const int i = ctl.save_idx + (save ? 1 : 0), flags = save ? kAdvance | kSave : kAdvance;
         const bool nofailed = ctl.nofailed, limit = ctl.attempts >= P_.max_attempts;
         __syncwarp();
         if (t == 0) {
             ctl.zc = zc;
             ctl.ny = ctl.acc_nyn;
             ctl.base = (ctl.base + 6) % 7;             // FSAL: k7 becomes the next k1
-            ctl.save_idx = i;
+            if (save) {
+                ctl.save_i = i - 1;
+                ctl.save_z = zc;
+                ctl.save_att = expf(-(float)(half_loss * ((double)zc * unit)));
+                ctl.save_idx = i;
+                ctl.next_z = save_point(i);
+            }
         }
         __syncwarp();
         if (i >= P_.n_saves || zc >= total) return flags | kEnd;
-        // growth after a step with no failure: h / (1.25 (err/rtol)^(1/5)), at most 5 h
+        // growth after a step with no failure: h / (1.25 (err/rtol)^(1/5)), at most 5 h (the
+        // factor only scales an integer step: FP32 serves)
         long long h = hc;
         if (nofailed) {
-            const float ratio = (float)(err / P_.rtol);
-            const float temp = 1.25f * powf(ratio, 0.2f);
-            h = temp > 0.2f ? (long long)((double)hc / (double)temp) : 5 * hc;
+            const float temp = 1.25f * powf((float)err / rtolf, 0.2f);
+            h = temp > 0.2f ? (long long)((double)hc * (double)(1.0f / temp)) : 5 * hc;
         }
         if (limit) {
             if (t == 0) ctl.status |= OPTIFAX_PULSE_ATTEMPT_LIMIT;
@@ -371,8 +375,7 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
         // later ones halve (the factor only scales an integer step: FP32 powf serves)
         long long next = hc / 2;
         if (nofailed) {
-            const float errf = (float)err;
-            next = (long long)((double)hc * (double)fmaxf(0.1f, 0.8f * powf((float)P_.rtol / errf, 0.2f)));
+            next = (long long)((double)hc * (double)fmaxf(0.1f, 0.8f * powf(rtolf / (float)err, 0.2f)));
         }
         if (t == 0) {
             ctl.nofailed = 0;
@@ -409,6 +412,7 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
         ctl = GCtl{};
         ctl.att[0] = ctl.iatt[0] = ctl.save_att = 1.f;
         ctl.save_idx = 1;
+        ctl.next_z = save_point(1);
     }
     __syncthreads();
     do_save(y);
@@ -464,7 +468,7 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
                 const float att = ctl.att[stage], iatt = ctl.iatt[stage];
 #pragma unroll
                 for (int j = 0; j < P; ++j) {
-                    e[j] = turn_to_unit(rate_s[j * T + t] * zs);              // e^{i B z}
+                    if (stage != 6) e[j] = turn_to_unit(rate_s[j * T + t] * zs);   // e^{i B z}; stage 5's position
                     v[j] = conjf2(cscale(cmul(ys[j], e[j]), att));
                 }
                 fftp_inverse<M, P>(buf, tw, td, t, v);                        // conj(AT)
