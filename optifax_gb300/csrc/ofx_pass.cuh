@@ -231,6 +231,7 @@ __device__ __forceinline__ float rcp_fast(float x) {
 // square root costs more than the rest of a point's stage arithmetic.
 struct Bounds {
     float qhi, qlo0, qlo1;
+    Bounds() = default;
     __device__ Bounds(float scale, float hi, float lo) {
         const float is2 = 1.f / (scale * scale), l = lo > 0.f ? lo * lo * is2 : -1.f;
         qhi = hi > 0.f && lo > 0.f ? hi * hi * is2 * (1.f - 1e-5f) : -1.f;      // -1: always the exact classes
@@ -354,7 +355,11 @@ struct Xch {
 // wait on L2 beside 200 KB of shared memory).
 struct RunState {
     double tally[4], prev_tally;
-    int n_acc, n_rej, tot_att, tot_acc, tot_rej, steady, stop, slots;
+    int n_acc, n_rej, tot_att, tot_acc, tot_rej, steady, stop, slots, trips_done;
+    // where registers are short: the next attempt's z-phasors and G sample, the classes' bounds
+    float2 z[3];
+    float g;
+    Bounds bounds;
 };
 
 template <int M, int METHOD, int C>
@@ -557,20 +562,42 @@ __device__ __forceinline__ void lanes_inv(float2 (&v)[NV], int l) {
     }
 }
 
-// Inner twiddles W_C^{j ka} of a lane's values (SPLIT), with their reciprocals' d
+// Inner twiddles W_C^{j ka} of a lane's values (SPLIT), with their reciprocals' d: in
+// registers, or, for two lanes of 8 values, the constants of the 16-point DFT by a select
+// (at 4096 points per CTA 512 threads leave 128 registers, of which the table held 24:
+// half of what that kernel spilled, and beside 220 KB of shared memory a spill is an L2
+// access).
 template <int M, int C>
 struct Inner {
-    float2 w[Xch<M, C>::SPLIT ? kPoints<M> : 1];
-    float d[Xch<M, C>::SPLIT ? kPoints<M> : 1];
+    static constexpr int P = kPoints<M>, LANES = Xch<M, C>::LANES;
+    static constexpr bool SPLIT = Xch<M, C>::SPLIT, CONST = SPLIT && LANES == 2 && P == 8;
+    float2 w[SPLIT && !CONST ? P : 1];
+    float d[SPLIT && !CONST ? P : 1];
     __device__ __forceinline__ void fill(const Twiddle* quad, int t) {
-        if constexpr (Xch<M, C>::SPLIT) {
-            constexpr int P = kPoints<M>;
+        if constexpr (SPLIT && !CONST) {
 #pragma unroll
             for (int r = 0; r < P; ++r) {
-                const Twiddle a = quad_tw<M>(quad, ((t % Xch<M, C>::LANES) * brev4(r, ilog2(P))) * (M / C) % M);
+                const Twiddle a = quad_tw<M>(quad, ((t % LANES) * brev4(r, ilog2(P))) * (M / C) % M);
                 w[r] = make_float2(a.c, a.s);
                 d[r] = a.d;
             }
+        }
+    }
+    // v times the twiddle of value r of lane l, and v over it
+    __device__ __forceinline__ float2 mul(float2 v, int r, int l) const {
+        if constexpr (CONST) {
+            const float2 u = rot_fwd(v, brev4(r, 3));
+            return l ? u : v;
+        } else {
+            return cmul(v, w[r]);
+        }
+    }
+    __device__ __forceinline__ float2 div(float2 v, int r, int l) const {
+        if constexpr (CONST) {
+            const float2 u = rot_inv(v, brev4(r, 3));
+            return l ? u : v;
+        } else {
+            return mul_recip(v, w[r], d[r]);
         }
     }
 };
@@ -596,7 +623,7 @@ __device__ __forceinline__ void exchange_fwd(const float2* g, float2* bufx, uint
         for (int i = 0; i < P; ++i) v[i] = g[swz((i * XC::LANES + l) * XC::COLS + col)];
         dftp<P>(v);
 #pragma unroll
-        for (int r = 1; r < P; ++r) v[r] = cmul(v[r], in.w[r]);
+        for (int r = 1; r < P; ++r) v[r] = in.mul(v[r], r, l);
         lanes_fwd<XC::LANES, P>(v, l);
 #pragma unroll
         for (int r = 0; r < P; ++r) {
@@ -663,7 +690,7 @@ __device__ __forceinline__ void exchange_inv(const float2* g, float2* bufx, uint
         }
         lanes_inv<XC::LANES, P>(v, l);
 #pragma unroll
-        for (int r = 1; r < P; ++r) v[r] = mul_recip(v[r], in.w[r], in.d[r]);
+        for (int r = 1; r < P; ++r) v[r] = in.div(v[r], r, l);
         dftp_inv<P>(v);
         const bool ends = HALO && (col < 2 || col >= XC::COLS - 2);
 #pragma unroll
@@ -896,6 +923,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     if (t == 0) {
         sP = pulses[p];
         *run = RunState{};
+        run->bounds = Bounds(METHOD != OPTIFAX_RK23 ? 50.f : 200.f, sP.max_err, sP.min_err);
     }
     __syncthreads();
     const PulseDev& P_ = sP;
@@ -934,7 +962,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
         bar_arm(bar_e, kBytesE);
         bar_arm(bar_e + 8, kBytesE);
     }
-    uint32_t ph_a = 0, ph_x = 0, ph_e = 0;        // phase parities: A, B to D, end values (bit per parity)
+    uint32_t ph_x = 0, ph_e = 0;      // phase parities: B to D, end values (bit per parity); A: the attempt's
     // per-thread tables as vectors of four (or two) values: [j / 4][t][j % 4]
     auto at4 = [&](int j) { return ((j >> 2) * T + t) * 4 + (j & 3); };
     auto at2 = [&](int j) { return ((j >> 1) * T + t) * 2 + (j & 1); };
@@ -982,7 +1010,8 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     const Hot hot_ = load_hot();
     auto hot = [&]() -> Hot { if constexpr (tight) return load_hot(); else return hot_; };
     const int max_attempts = cfg.max_attempts_mul * (P_.S + 16) + 64;
-    const Bounds bounds(heun ? 50.f : 200.f, P_.max_err, P_.min_err);
+    const Bounds bounds_ = tight ? Bounds{} : Bounds(heun ? 50.f : 200.f, P_.max_err, P_.min_err);
+    auto bounds = [&]() -> Bounds { if constexpr (tight) return run->bounds; else return bounds_; };
     // what the caller asked for beyond the field, as one register (tested per attempt)
     constexpr int kForced = 1, kTrace = 2, kSteps = 4, kAp = 8;
     const int opts = (P_.forced && P_.n_forced > 0 ? kForced : 0) | (P_.trace ? kTrace : 0) |
@@ -996,7 +1025,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     float k = nee ? 1.f : 0.f, stepprev = 4.f, stepmod = 4.f;
     unsigned q = 0;                          // accumulated dispersion position (sum of stepmod)
     int s_cached = -1;                       // stepmod of the cached per-mode D - 1
-    int attempt = 0, status = 0, par = 0, trip = 0, trips_done = 0, gatt = 0;
+    int attempt = 0, status = 0, par = 0, trip = 0, gatt = 0;         // gatt: attempts of all trips
 
     // neighbours' drive values at the thread's ends; hv: the halo point's drive (end threads)
     auto edges = [&](const Pair (&nl)[H], float2 hv, float2& L, float2& R) {
@@ -1028,14 +1057,27 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     };
 
     // z-phasors of an attempt's stages and its G sample, made ahead (before the
-    // transforms of the previous step) and keyed by the position and the step
+    // transforms of the previous step; ready: valid for the next attempt).  Where registers
+    // are short warp 0 makes them, and they wait in shared memory.
+    bool ready = false;                      // (where they are short; else keyed by position and step)
     float zk = -1.f, zs = -1.f, gval = 0.f;
     float2 z0 = make_float2(0.f, 0.f), z1 = z0, z2 = z0;
-    auto prepare = [&](float kp, float sm) {
+    auto phasors = [&](float kp, float sm) {
         if constexpr (heun) zphases(P_.tau_z4, t, kp, kp + sm, 0.f, z0, z1, z2);
         else zphases(P_.tau_z4, t, kp + 0.5f * sm, kp + 0.75f * sm, kp + sm, z0, z1, z2);
         gval = hot().G[(int)kp];
-        zk = kp; zs = sm;
+    };
+    auto prepare = [&](float kp, float sm) {
+        if constexpr (tight) {
+            ready = true;
+            if (t < 32) {
+                phasors(kp, sm);
+                if (t == 0) { run->z[0] = z0; run->z[1] = z1; run->z[2] = z2; run->g = gval; }
+            }
+        } else {
+            phasors(kp, sm);
+            zk = kp; zs = sm;
+        }
     };
 
     Pair k1r[H];      // RK23: K1 (first stage, FSAL) between attempts
@@ -1069,7 +1111,17 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                 // z of the first stage in steps and index of G (G33(k) is 1-based in NEE_CPU.m)
                 const float kpos = nee ? k - 1.f : k;
                 bool accepted = false;
-                if (kpos != zk || stepmod != zs) prepare(kpos, stepmod);
+                if constexpr (tight) {
+                    if (ready) {
+                        z0 = run->z[0]; z1 = run->z[1]; gval = run->g;
+                        if constexpr (!heun) z2 = run->z[2];
+                    } else {
+                        phasors(kpos, stepmod);
+                    }
+                    ready = false;
+                } else if (kpos != zk || stepmod != zs) {
+                    prepare(kpos, stepmod);
+                }
                 const float hg = (stepmod * hot().h) * gval, cs = hot().cs;
                 Pair ev[H];                                    // E, then E behind the absorber
                 Pair dv[H];                                    // its error difference
@@ -1135,7 +1187,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
 #pragma unroll
                     for (int j = 0; j < H; ++j) dv[j] = pair_fma(k4[j], -1.f / 8.f, pp[j]);   // = E - A1
                 }
-                const int bits = classify_all<H, nee>(bounds, P_, heun ? 50.f : 200.f, dv, ev);
+                const int bits = classify_all<H, nee>(bounds(), P_, heun ? 50.f : 200.f, dv, ev);
                 // E behind the absorber: into the FFT buffer, or the columns' buffer
                 {
                     float2 o[P];
@@ -1161,8 +1213,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     }
                 }
 
-                int fl = combine_flags<T / 32, C>(bits, red, bar_a, ph_a, kBytesA, dead, gatt, t, c, cfg);
-                ph_a ^= 1;
+                int fl = combine_flags<T / 32, C>(bits, red, bar_a, gatt & 1, kBytesA, dead, gatt, t, c, cfg);
                 if (fl & kDead) { status |= OPTIFAX_PULSE_TIMEOUT; goto done; }
                 if ((opts & kForced) && gatt < P_.n_forced) fl = (P_.forced[gatt] & 3) | (fl & 4);
                 if (fl & 4) trip_status |= OPTIFAX_PULSE_NAN;
@@ -1372,8 +1423,8 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
             }
         }
         status |= trip_status;
-        trips_done = trip + 1;
         if (t == 0) {
+            run->trips_done = trip + 1;
             if (rec && P_.fb && P_.trips) {
                 optifax_trip_record tr;
                 tr.attempts = attempt; tr.accepted = run->n_acc; tr.rejected = run->n_rej; tr.status = trip_status;
@@ -1406,7 +1457,7 @@ done:
         optifax_pulse_stats st;
         st.attempts = run->tot_att; st.accepted = run->tot_acc; st.rejected = run->tot_rej; st.status = status;
         st.z_steps = (long long)q; st.k_final = k; st.stepmod_final = stepmod; st.n_chunks = P_.nchunks;
-        st.reserved[0] = trips_done; st.reserved[1] = st.reserved[2] = 0;
+        st.reserved[0] = run->trips_done; st.reserved[1] = st.reserved[2] = 0;
         *P_.stats = st;
     }
     if constexpr (C > 1) cg::this_cluster().sync();      // no CTA leaves while a peer may still read its memory
