@@ -589,7 +589,7 @@ struct Inner {
             const float2 u = rot_fwd(v, brev4(r, 3));
             return l ? u : v;
         } else {
-            return cmul(v, w[r]);
+            return cmul(w[r], v);
         }
     }
     __device__ __forceinline__ float2 div(float2 v, int r, int l) const {
