@@ -96,7 +96,11 @@ struct SmemX {
     // E and increment of every segment's 4 halo points; field and carrier of the end threads' two
     static constexpr size_t off_bar = off_halo + (C > 1 ? sizeof(cplx) * 16 * C : 0);
     static constexpr size_t off_red = off_bar + sizeof(uint64_t) * 4;
-    static constexpr size_t bytes = off_red + sizeof(int) * (2 * SH::NW + 2 * 16 + 4);
+    // absorber factors of the threads that have one (a quarter of them: the absorber spans
+    // [6/16, 10/16] of the window in every variant): [point][thread]
+    static constexpr int SLOTS = SH::T / 4 + 2;
+    static constexpr size_t off_abc = (off_red + sizeof(int) * (2 * SH::NW + 2 * 16 + 4) + 15) & ~size_t(15);
+    static constexpr size_t bytes = off_abc + sizeof(typename Num<R>::real) * SH::P * SLOTS;
     static_assert(bytes <= 232448 - 288, "shared memory of one CTA");
 };
 
@@ -320,8 +324,10 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
     cplx* halo_d = halo_e + 4 * C;
     int* red = reinterpret_cast<int*>(smem + SM::off_red);
     int* dead = red + 2 * NW + 2 * 16;
+    real* abc_s = reinterpret_cast<real*>(smem + SM::off_abc);
     __shared__ PulseX sP;
     __shared__ cplx w16[8];
+    __shared__ int slots;
 
     const int t = threadIdx.x;
     const int c = (C > 1) ? (int)cg::this_cluster().block_rank() : 0;
@@ -330,6 +336,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
     if (t == 0) {
         sP = pulses[p];
         *dead = 0;
+        slots = 0;
     }
     if (t < 8) w16[t] = wn[(size_t)t * (N / 16)];
     __syncthreads();
@@ -410,13 +417,23 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
         return 1.0 - 1.0 / (g * g);
     };
     cplx a[P], cph[P];
-    bool absorbs = false;              // whether a point of this thread lies in the absorber
 #pragma unroll
     for (int j = 0; j < P; ++j) {
         a[j] = X::from(Pd.E_in[i0 + j]);
         cph[j] = carrier(i0 + j);
-        const double f = absorber(i0 + j);
-        if (f != 1.0) absorbs = true;
+    }
+    // The absorber's factors, kept: an FP64 cosh and a division per point in every attempt
+    // cost the threads that have some 2 to 13 us (us per attempt, recomputed and kept: FP64
+    // 2^12 points 30.4 and 28.4, 2^16 213 and 203; float-float 2^14 20.2 and 17.5, 2^16 87
+    // and 74).  The FP64 kernel of 2048 points per CTA is the exception (107 and 116).
+    constexpr bool kKeep = !(std::is_same<R, double>::value && M == 2048);
+    int absorb = -1;
+    if (i0 + P > 6 * (N / 16) && i0 <= 10 * (N / 16) && cfg.abc_mode != ABC_NONE) {
+        absorb = kKeep ? atomicAdd(&slots, 1) : 0;
+        if constexpr (kKeep) {
+#pragma unroll 1
+            for (int j = 0; j < P; ++j) abc_s[j * SM::SLOTS + absorb] = X::rfrom(absorber(i0 + j));
+        }
     }
     // the end threads' two halo points: hs[0..1] field, hs[2..3] carrier
     cplx* hs = halo_e + 8 * C + 4 * (2 * seg + (rend ? 1 : 0));
@@ -548,9 +565,10 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
                 // pct = 100 |E - A1| / (|E| + 1) (OPO_CUDA_BATCH_XTAL.cu:325-349; NEE_CPU.m:73-79)
                 bits = classify_points<R, NEE, P>(e, d2, a1, bounds, maxE, minE);
             }
-            if (absorbs) {
+            if (absorb >= 0) {
 #pragma unroll
-                for (int j = 0; j < P; ++j) e[j] = X::scale(e[j], X::rfrom(absorber(i0 + j)));
+                for (int j = 0; j < P; ++j)
+                    e[j] = X::scale(e[j], kKeep ? abc_s[j * SM::SLOTS + absorb] : X::rfrom(absorber(i0 + j)));
             }
             fft.store_own(C > 1 ? bufG : bufX, e);
             if constexpr (C > 1) {
