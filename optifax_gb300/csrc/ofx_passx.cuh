@@ -328,6 +328,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
     __shared__ PulseX sP;
     __shared__ cplx w16[8];
     __shared__ int slots;
+    __shared__ unsigned long long grid_last[3];
 
     const int t = threadIdx.x;
     const int c = (C > 1) ? (int)cg::this_cluster().block_rank() : 0;
@@ -337,6 +338,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
         sP = pulses[p];
         *dead = 0;
         slots = 0;
+        for (int i = 0; i < 3; ++i) grid_last[i] = 0;
     }
     if (t < 8) w16[t] = wn[(size_t)t * (N / 16)];
     __syncthreads();
@@ -577,7 +579,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
                     for (int j = 0; j < P; ++j) push_halo_x(halo_e, seg, P * tin + j, e[j], bar_a);
                 }
             }
-            int fl = combine_flags<NW, C>(bits, red, bar_a, ph_a, kBytesA, dead, attempt, t, c, cfg);
+            int fl = combine_flags<NW, C>(bits, red, bar_a, ph_a, kBytesA, dead, grid_last, attempt, t, c, cfg);
             ph_a ^= 1;
             if (fl & kDead) { status |= OPTIFAX_PULSE_TIMEOUT; goto done; }
             if (fl & 4) status |= OPTIFAX_PULSE_NAN;
