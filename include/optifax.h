@@ -15,8 +15,8 @@
  * (NULL = legacy default stream) and returns before the work completes.
  * Functions return OPTIFAX_OK or an optifax_status code; they never abort.
  * A handle may be used by one host thread at a time.  Its calls may go to
- * different streams: the handle's device scratch (descriptors, exchange
- * buffers, stage rows) is shared by its calls, so a call on another stream than
+ * different streams: the handle's device scratch (descriptors, cavity
+ * rows, stage rows) is shared by its calls, so a call on another stream than
  * the previous call's waits on the GPU until the previous call's work is done.
  * Independent concurrent work takes one handle per stream.  Calls on a handle
  * are not for CUDA stream capture (descriptors are staged from host memory and
@@ -186,8 +186,9 @@ int optifax_opo_mex_batch(optifax_handle h,
  * (unlike the reference, whose batch shares one schedule).  `pulses` is a
  * HOST array of n_pulses descriptors holding device pointers.  stats
  * (optional) is a DEVICE array of n_pulses entries.  cta_points selects the
- * points held per CTA (512..4096, 0 = automatic); a pulse of N points runs on
- * a cluster of N / cta_points CTAs.
+ * points held per CTA (512..4096); a pulse of N points runs on a cluster of
+ * N / cta_points CTAs.  0 = automatic: the most CTAs per pulse at which the GPU
+ * holds every cluster of the call at once, 4096 points per CTA where it does not.
  */
 int optifax_propagate(optifax_handle h, const optifax_pulse* pulses, int32_t n_pulses,
                       int32_t method, int32_t variant, int32_t cta_points,
@@ -197,7 +198,7 @@ int optifax_propagate(optifax_handle h, const optifax_pulse* pulses, int32_t n_p
  * The same batch as optifax_propagate recorded once into a CUDA graph and then
  * replayed: the graph holds one persistent grid per (cta_points, cluster) group,
  * forked and joined as optifax_propagate launches them, with its own descriptors
- * and exchange scratch (no host staging on replay).  The pulses' device pointers
+ * and cavity scratch (no host staging on replay).  The pulses' device pointers
  * (inputs, outputs, stats) are fixed at capture: every replay reads the inputs'
  * current contents and rewrites the outputs.  No counterpart in the reference,
  * whose batch shares one cuFFT plan and one step.  The graph uses the handle's

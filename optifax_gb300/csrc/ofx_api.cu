@@ -183,8 +183,8 @@ int resident_clusters(optifax_context* h, const KernelEntry& ke) {
 //   1  half the CTAs
 //   2  4096 points per CTA (one CTA up to 4096 points): the least SM time per attempt
 // One pulse, us per attempt (GB300, 2 W, 30 um poling), at spread 2 -> 1 -> 0:
-//   2048: 4.2 -> 4.2 -> 3.3    4096: 6.5 -> 4.2 -> 3.5    8192: 9.4 -> 6.1 -> 4.4
-//   16384: 9.8 -> 5.9 -> 5.0   32768: 10.5 -> 10.5 -> (2048 points per CTA)
+//   2048: 4.1 -> 4.3 -> 3.3    4096: 6.4 -> 4.2 -> 3.4    8192: 9.3 -> 6.0 -> 4.3
+//   16384: 9.8 -> 5.8 -> 5.0   32768: 10.3 -> 10.3 -> 6.7
 // SM time per attempt goes the other way (4096: 6.5, 17, 28 SM us), so the wider
 // spreads serve calls that leave SMs idle otherwise.
 int spread_points(int N, int spread) {
