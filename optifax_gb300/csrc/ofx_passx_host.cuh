@@ -75,7 +75,8 @@ inline cudaError_t xattributes(const XKernel<R>& k) {
 // bound these kernels, so a pulse takes as many SMs as a cluster allows: 512 points per
 // CTA up to 2^13 points, then n / 16 (one pulse, us per attempt, GB300, FP64 at 1024 and
 // 512 points per CTA: 2^10 38 and 26, 2^12 48 and 30, 2^13 53 and 33; float-float at 2^13
-// 19 and 16).  Several pulses on one schedule run at once, so they take 1024 points per
+// 19 and 16; measured before the absorber's factors were kept, now 24, 28, 30 and 12.5 at
+// 512).  Several pulses on one schedule run at once, so they take 1024 points per
 // CTA (float-float: 512 up to 2^12 points) where the wider shape's clusters do not all
 // fit the GPU.
 template <typename R>

@@ -41,7 +41,8 @@ inline int make_map(CUtensorMap* m, const void* ptr, long long rows, long long c
 
 // Launch with programmatic stream serialisation: the kernel's start overlaps the end of
 // the stream's previous kernel (every kernel launched so calls dep_wait before it touches
-// global memory).  The surrogate's forward pass is a chain of 5 us kernels.
+// global memory).  The surrogate's forward pass is a chain of 14 kernels of 5 us: 100 us for
+// one sample by plain launches, 64 so (with the wider lift and projection).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dep(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t lc = {};
