@@ -127,64 +127,69 @@ __global__ void __launch_bounds__(256) k_lift(const float* __restrict__ x, const
 }
 
 // Channel mixing per mode: out[b][u][m] = sum_v in[(v,b)][m] w (or conj w) with w =
-// Ws[v][u][m] (forward, u = o) or Ws[u][v][m] conjugated (backward, u = c).  One block
-// per (u, group of samples); its 32 lanes are the modes and its 8 warps take 8 v each, so
-// the weights are read once per sample group in whole rows and a sum is 8 steps deep
-// (a thread per output walked 64 dependent steps: 17 us for one sample or 32).
-constexpr int MIXB = 4;           // samples per block
-template <bool BWD, int U>        // U outputs per block share its reads of `in`
+// Ws[v][u][m] (forward, u = o) or Ws[u][v][m] conjugated (backward, u = c).  The sum is
+// rounded to BF16 for a whole row of the next product, so its order is part of the result:
+// one FP32 accumulator pair per output, v = 0..63 in turn (in eight partial sums a last
+// bit before the rounding moved elements of small batches' gradients by up to 1e-3).
+// What cost time in that order were its loads, one dependent step after the other, so a
+// block of U outputs and MB samples first copies its rows of `in` and its weights to shared
+// memory, all copies in flight at once; then a warp per (output, sample), lane = mode,
+// runs the 64 steps.
+template <int U, int MB>
+struct Mix {
+    static constexpr int IN = W * MB * SPEC;                              // floats: [v][sample][2 m]
+    static constexpr size_t smem = sizeof(float) * IN + sizeof(__nv_bfloat162) * W * U * MODES;
+};
+template <bool BWD, int U, int MB>
 __global__ void __launch_bounds__(256) k_mix(const float* __restrict__ in, const bf16* __restrict__ Ws, int B,
                                              bf16* __restrict__ out) {
-    __shared__ float2 red[8][MIXB][MODES];
-    const int m = threadIdx.x & 31, wp = threadIdx.x >> 5, u0 = blockIdx.x * U, b0 = blockIdx.y * MIXB;
-    float ar[U][MIXB] = {}, ai[U][MIXB] = {};
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float* s_in = reinterpret_cast<float*>(smem_raw);
+    __nv_bfloat162* s_w = reinterpret_cast<__nv_bfloat162*>(s_in + Mix<U, MB>::IN);      // [v][output][mode]
+    const int u0 = blockIdx.x * U, b0 = blockIdx.y * MB, n = min(MB, B - b0);
     dep_launch();
     dep_wait();
-#pragma unroll
-    for (int i = 0; i < W / 8; ++i) {
-        const int v = wp * (W / 8) + i;
-        float2 s[MIXB];
-#pragma unroll
-        for (int k = 0; k < MIXB; ++k)
-            s[k] = b0 + k < B ? *reinterpret_cast<const float2*>(in + ((long long)v * B + b0 + k) * SPEC + 2 * m)
-                              : make_float2(0.f, 0.f);
-#pragma unroll
-        for (int q = 0; q < U; ++q) {
-            const long long wi = BWD ? ((long long)(u0 + q) * W + v) : ((long long)v * W + u0 + q);
-            const __nv_bfloat162 w = *reinterpret_cast<const __nv_bfloat162*>(Ws + (wi * MODES + m) * 2);
-            const float wr = __low2float(w), wj = BWD ? -__high2float(w) : __high2float(w);
-#pragma unroll
-            for (int k = 0; k < MIXB; ++k) {
-                ar[q][k] = fmaf(s[k].x, wr, fmaf(-s[k].y, wj, ar[q][k]));
-                ai[q][k] = fmaf(s[k].x, wj, fmaf(s[k].y, wr, ai[q][k]));
-            }
+    for (int i = threadIdx.x; i < W * MB * (SPEC / 4); i += 256) {
+        const int row = i / (SPEC / 4), c4 = 4 * (i % (SPEC / 4)), v = row / MB, k = row % MB;
+        if (k < n) ofx_tc::cp_async16(s_in + row * SPEC + c4, in + ((long long)v * B + b0 + k) * SPEC + c4);
+    }
+    for (int i = threadIdx.x; i < W * U * (MODES / 4); i += 256) {
+        const int row = i / (MODES / 4), m4 = 4 * (i % (MODES / 4)), v = row / U, q = row % U;
+        const long long wi = BWD ? ((long long)(u0 + q) * W + v) : ((long long)v * W + u0 + q);
+        ofx_tc::cp_async16(s_w + row * MODES + m4, Ws + (wi * MODES + m4) * 2);
+    }
+    ofx_tc::cp_async_wait();
+    __syncthreads();
+    const int m = threadIdx.x & 31, q = (threadIdx.x >> 5) % U, k = (threadIdx.x >> 5) / U;
+    if (k >= n) return;
+    float ar = 0.f, ai = 0.f;
+#pragma unroll 8
+    for (int v = 0; v < W; ++v) {
+        const float2 s = *reinterpret_cast<const float2*>(s_in + (v * MB + k) * SPEC + 2 * m);
+        const __nv_bfloat162 w = s_w[(v * U + q) * MODES + m];
+        const float wr = __low2float(w), wi = __high2float(w);
+        if (BWD) {
+            ar = fmaf(s.x, wr, fmaf(s.y, wi, ar));
+            ai = fmaf(s.y, wr, fmaf(-s.x, wi, ai));
+        } else {
+            ar = fmaf(s.x, wr, fmaf(-s.y, wi, ar));
+            ai = fmaf(s.x, wi, fmaf(s.y, wr, ai));
         }
     }
-#pragma unroll
-    for (int q = 0; q < U; ++q) {
-        if (q) __syncthreads();
-#pragma unroll
-        for (int k = 0; k < MIXB; ++k) red[wp][k][m] = make_float2(ar[q][k], ai[q][k]);
-        __syncthreads();
-        if (wp < MIXB && b0 + wp < B) {
-            float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                s.x += red[i][wp][m].x;
-                s.y += red[i][wp][m].y;
-            }
-            *reinterpret_cast<__nv_bfloat162*>(out + ((long long)(b0 + wp) * W + u0 + q) * SPEC + 2 * m) =
-                __floats2bfloat162_rn(s.x, s.y);
-        }
-    }
+    *reinterpret_cast<__nv_bfloat162*>(out + ((long long)(b0 + k) * W + u0 + q) * SPEC + 2 * m) =
+        __floats2bfloat162_rn(ar, ai);
 }
-// one output per block up to 8 samples (64 blocks a group), four above, where the groups
-// fill the GPU and reading `in` once per output is what costs
+// One output and one sample per block up to 8 samples (64 blocks a sample, 24 KB each);
+// above, where the blocks fill the GPU and reading `in` once per output is what costs, four
+// outputs and two samples (64 KB, so a third of the reads)
+constexpr int MIXU = 4, MIXB = 2;
 template <bool BWD>
 void launch_mix(const float* in, const bf16* Ws, int B, bf16* out, cudaStream_t st) {
-    const unsigned groups = (unsigned)((B + MIXB - 1) / MIXB);
-    if (B <= 8) launch_dep(k_mix<BWD, 1>, dim3(W, groups), dim3(256), 0, st, in, Ws, B, out);
-    else launch_dep(k_mix<BWD, 4>, dim3(W / 4, groups), dim3(256), 0, st, in, Ws, B, out);
+    if (B <= 8)
+        launch_dep(k_mix<BWD, 1, 1>, dim3(W, B), dim3(256), Mix<1, 1>::smem, st, in, Ws, B, out);
+    else
+        launch_dep(k_mix<BWD, MIXU, MIXB>, dim3(W / MIXU, (B + MIXB - 1) / MIXB), dim3(256), Mix<MIXU, MIXB>::smem, st,
+                   in, Ws, B, out);
 }
 
 // ---- one layer's spatial part ---------------------------------------------
@@ -217,7 +222,7 @@ __global__ void __launch_bounds__(128, 4)
     __shared__ __align__(8) uint64_t full, accum;
     __shared__ uint32_t tmem_slot;
     __shared__ float s_bias[W];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
     const int b = blockIdx.y, x0 = blockIdx.x * 128;
     if (threadIdx.x == 0) {
         mbar_init(&full, 1);
@@ -884,15 +889,10 @@ int fno_maps(optifax_fno_s* f, int B) {
     return OPTIFAX_OK;
 }
 
-// K splits of the transform products (M = 64 B rows, K = L): enough CTAs to fill the GPU,
-// at least two 64-column steps each (one sample, 4096 bins: 8 splits 8.8 us, 32 splits 5;
-// 32 samples: 10 us with 16)
-inline int spec_splits(int B, int L) {
-    const int tiles = (W * B + 127) / 128, most = L / 128;
-    const int want = (296 + tiles - 1) / tiles;
-    const int s = want < 8 ? 8 : (want > 32 ? 32 : want);
-    return s < most ? s : (most > 0 ? most : 1);
-}
+// K splits of the transform products (M = 64 B rows, K = L).  Their FP32 sums are rounded
+// to BF16 behind the mixing, so the number is part of the result and the same for every
+// batch.
+constexpr int SPEC_SPLITS = 8;
 
 int fno_forward(optifax_fno_s* f, const float* x, float* y, int B, cudaStream_t st) {
     const int L = f->L;
@@ -904,7 +904,7 @@ int fno_forward(optifax_fno_s* f, const float* x, float* y, int B, cudaStream_t 
                f->Hc[0], f->Ht[0]);
     for (int l = 0; l < NLAYER; ++l) {
         OFX_TRY(optifax_gemm_bf16(f->Hc[l], L, rowsA, f->F, L, SPEC, f->S[l], SPEC, (int)WB, SPEC, L,
-                                  spec_splits(B, L), 1, st));
+                                  SPEC_SPLITS, 1, st));
         launch_mix<false>(f->S[l], f->wb + off_ws(l), B, f->T, st);
         LayerArgs a = {};
         a.bias = f->master + off_b(l);
@@ -939,7 +939,7 @@ int fno_backward(optifax_fno_s* f, const float* x, const float* target, const fl
         OFX_TRY(optifax_gemm_bf16(f->dZc, BL, 128, f->Hc[l], BL, W, f->grad + off_wp(l), W, W, W, (int)BL, splits, 1,
                                   st));
         OFX_TRY(optifax_gemm_bf16(f->dZc, L, 2 * WB, f->GT, L, SPEC, f->dT[l], SPEC, (int)WB, SPEC, L,
-                                  spec_splits(B, L), 1, st));
+                                  SPEC_SPLITS, 1, st));
         launch_mix<true>(f->dT[l], f->wb + off_ws(l), B, f->dS, st);
         launch_dep(k_mix_bwd_dw, dim3(nblk((long long)W * W * MODES)), dim3(256), 0, st, f->dT[l], f->S[l], B,
                    f->grad + off_ws(l));
@@ -1027,7 +1027,11 @@ extern "C" int optifax_fno_create(optifax_fno* out, int32_t n_bins, int32_t max_
         if (!f->err ||
             cudaFuncSetAttribute(k_layer<LAYER_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM) != cudaSuccess ||
             cudaFuncSetAttribute(k_layer<LAYER_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_layer<LAYER_BWD_IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM) != cudaSuccess)
+            cudaFuncSetAttribute(k_layer<LAYER_BWD_IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_mix<false, MIXU, MIXB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)Mix<MIXU, MIXB>::smem) != cudaSuccess ||
+            cudaFuncSetAttribute(k_mix<true, MIXU, MIXB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)Mix<MIXU, MIXB>::smem) != cudaSuccess)
             rc = OPTIFAX_ERR_CUDA;
     }
     if (!rc) {
