@@ -360,48 +360,38 @@ __global__ void __launch_bounds__(128, 4)
     }
 }
 
-// y[b][j][x] = x[b][j][x] + q[j] + sum_c Q[j][c] h[b][x][c]; four lanes share a bin, 16
-// channels each.  The four weights of a channel are one 16-byte read, the lanes' channels
-// apart by a pad (4-byte reads, two lanes to a bank: 13.5 us at 32 samples of 4096 bins)
+// y[b][j][x] = x[b][j][x] + (q[j] + sum_c Q[j][c] h[b][x][c]), c in turn: the loss's
+// gradient is a difference of y that is rounded to BF16.  Four lanes share a bin, one output
+// each; they read the same 16 bytes of its row, and of the weights 16 bytes each, four banks
+// apart.
 __global__ void __launch_bounds__(256) k_proj_fwd(const bf16* __restrict__ Ht, const bf16* __restrict__ Qw,
                                                   const float* __restrict__ qb, const float* __restrict__ xin, int B,
                                                   int L, float* __restrict__ y) {
-    __shared__ __align__(16) float sQ[COUT * (W + 4)];
+    constexpr int LDQ = W + 4;
+    __shared__ __align__(16) float sQ[COUT * LDQ];
     dep_launch();
     dep_wait();
-    if (threadIdx.x < COUT * W) {
-        const int j = threadIdx.x / W, c = threadIdx.x % W;
-        sQ[COUT * (c + c / 16) + j] = __bfloat162float(Qw[threadIdx.x]);
-    }
+    if (threadIdx.x < COUT * W) sQ[threadIdx.x / W * LDQ + threadIdx.x % W] = __bfloat162float(Qw[threadIdx.x]);
     __syncthreads();
     const long long idx = blockIdx.x * 64LL + (threadIdx.x >> 2);
-    const int part = threadIdx.x & 3;
-    const bool live = idx < (long long)B * L;
-    const uint4* src = reinterpret_cast<const uint4*>(Ht + (live ? idx : 0) * W + 16 * part);
-    float acc[COUT] = {};
+    const int j = threadIdx.x & 3;
+    if (idx >= (long long)B * L) return;
+    const uint4* src = reinterpret_cast<const uint4*>(Ht + idx * W);
+    uint4 u[W / 8];
 #pragma unroll
-    for (int q8 = 0; q8 < 2; ++q8) {
-        const uint4 u = src[q8];
-        const bf16* hp = reinterpret_cast<const bf16*>(&u);
+    for (int i = 0; i < W / 8; ++i) u[i] = src[i];
+    float acc = qb[j];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const float h = __bfloat162float(hp[e]);
-            const float4 q = *reinterpret_cast<const float4*>(sQ + COUT * (17 * part + q8 * 8 + e));
-            acc[0] = fmaf(q.x, h, acc[0]);
-            acc[1] = fmaf(q.y, h, acc[1]);
-            acc[2] = fmaf(q.z, h, acc[2]);
-            acc[3] = fmaf(q.w, h, acc[3]);
-        }
+    for (int c = 0; c < W; c += 4) {
+        const float4 q = *reinterpret_cast<const float4*>(sQ + j * LDQ + c);
+        const bf16* hp = reinterpret_cast<const bf16*>(&u[c / 8]) + c % 8;
+        acc = fmaf(q.x, __bfloat162float(hp[0]), acc);
+        acc = fmaf(q.y, __bfloat162float(hp[1]), acc);
+        acc = fmaf(q.z, __bfloat162float(hp[2]), acc);
+        acc = fmaf(q.w, __bfloat162float(hp[3]), acc);
     }
-#pragma unroll
-    for (int j = 0; j < COUT; ++j) {
-        acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 1);
-        acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 2);
-    }
-    if (!live) return;
     const int b = (int)(idx / L), xx = (int)(idx % L);
-    const float v = part == 0 ? acc[0] : (part == 1 ? acc[1] : (part == 2 ? acc[2] : acc[3]));   // output j = part
-    y[((long long)b * COUT + part) * L + xx] = xin[((long long)b * CIN + part) * L + xx] + (v + qb[part]);
+    y[((long long)b * COUT + j) * L + xx] = xin[((long long)b * CIN + j) * L + xx] + acc;
 }
 
 // dP[c][i] and dp[c] from k_layer's partial rows [n][W][8]; block: 32 of the 512 columns,

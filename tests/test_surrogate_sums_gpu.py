@@ -1,4 +1,5 @@
-"""The channel mixing sums its 64 terms in channel order, one FP32 sum per output.  Marked gpu.
+"""The channel mixing and the projection sum their 64 terms in channel order, one FP32 sum
+per output.  Marked gpu.
 
 Its sums are rounded to BF16 for a whole row of the next product, so another order of the
 same terms is another result: a last bit before the rounding becomes 2^-8 of a mode.  The
@@ -90,3 +91,23 @@ def test_backward_mixing_in_channel_order(B):
     want = _bf16(_in_order(dz, w)).astype(np.float64) * (B * L)
     got = _layer(g.cpu().numpy(), 2)[2]
     assert np.array_equal(got.astype(np.float64), want)
+
+
+@pytest.mark.parametrize("L_,B", [(128, 1), (192, 3), (4096, 2)])
+def test_projection_in_channel_order(L_, B):
+    """q, then Q_c h_c for c in turn, then the input: the output feeds the BF16 gradients of the loss."""
+    from optifax_gb300.surrogate import FNO
+    rng = np.random.default_rng(L_ + B)
+    p = np.zeros(fo.N_PARAMS, dtype=np.float32)
+    h = _bf16(rng.normal(size=W))
+    _layer(p, 3)[2][:] = h
+    Q = _bf16(rng.normal(size=(fo.COUT, W)))
+    p[fo.OFF_Q:fo.OFF_QB] = Q.ravel()
+    p[fo.OFF_QB:] = rng.normal(size=fo.COUT)
+    x = rng.normal(size=(B, fo.CIN, L_)).astype(np.float32)
+    net = FNO(n_bins=L_, max_batch=B, params=p)
+    y = net.forward(torch.from_numpy(x).to(net.dev)).cpu().numpy()
+    acc = p[fo.OFF_QB:].copy()
+    for c in range(W):
+        acc = (Q[:, c].astype(np.float64) * h[c] + acc.astype(np.float64)).astype(np.float32)
+    assert np.array_equal(y, x[:, :fo.COUT] + acc[None, :, None])
