@@ -350,6 +350,7 @@ int enqueue_groups(optifax_context* h, const std::vector<Group>& groups, int met
         cfg.max_attempts_mul = 64;
         cfg.grid_sync = grid_sync;
         cfg.clusters = (int)g.d.size();
+        cfg.wait = kWait;
         cudaStream_t ls = st;
         if (gi > 0) {
             ls = side[gi - 1];

@@ -175,6 +175,7 @@ extern "C" int optifax_propagate_noalloc(const optifax_pulse* pulse, int32_t var
     cfg.guard = vc.guard;
     cfg.shared_sched = 0;
     cfg.max_attempts_mul = 64;
+    cfg.wait = kWait;
     FftTables tabs;
     tabs.quad = reinterpret_cast<const Twiddle*>(base + kOffQuad);
     tabs.low = reinterpret_cast<const Twiddle*>(base + (N == 8192 ? kOffLow8k : kOffLow16k));

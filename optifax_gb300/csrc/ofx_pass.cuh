@@ -92,7 +92,9 @@ struct KernelCfg {
     int max_attempts_mul;
     unsigned long long* grid_sync;   // shared schedule: 3 words, zero before the launch
     int clusters;        // of the launch
+    int wait;            // limit of a bounded wait, in looks at an mbarrier (about 4 us each)
 };
+constexpr int kWait = 1 << 19;       // about 2 s
 
 // Kernel flavours: the MEX Heun and RK23 schedules (OPTIFAX_HEUN, OPTIFAX_RK23) and
 // the Heun schedule with NEE_CPU.m step control, a separate instantiation so the
@@ -356,7 +358,7 @@ struct Xch {
 struct RunState {
     double tally[4], prev_tally;
     unsigned long long grid_last[3];      // shared schedules: the grid's words after their last round
-    int n_acc, n_rej, tot_att, tot_acc, tot_rej, steady, stop, slots, trips_done;
+    int n_acc, n_rej, tot_att, tot_acc, tot_rej, steady, stop, slots, trips_done, status, trip_status;
     // where registers are short: the next attempt's z-phasors and G sample, the classes' bounds
     float2 z[3];
     float g;
@@ -388,7 +390,7 @@ struct Smem {
     // and, for a segment's two end threads, the field and the carrier of their halo points
     static constexpr size_t off_bar = off_halo + (C > 1 ? sizeof(float2) * (8 + 8) * C : 0);
     static constexpr size_t off_red = off_bar + sizeof(uint64_t) * 6;
-    static constexpr size_t off_dred = off_red + sizeof(int) * (2 * NW + 2 * 16 + 4);   // warp and CTA flags, dead, grid flags
+    static constexpr size_t off_dred = off_red + sizeof(int) * (2 * NW + 2 * 16 + 8);   // warp and CTA flags, grid flags, waits that ran out
     static constexpr size_t off_run = ((off_dred + 15) & ~size_t(15)) + sizeof(double) * (NW * 4 + 2 * 16 * 4);
     static constexpr size_t bytes = off_run + sizeof(RunState);
     static_assert(bytes <= 232448 - 288, "shared memory of one CTA");
@@ -451,17 +453,105 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
                  " selp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0;
 }
-// Bounded wait (about 2 s); after a wait that ran out the CTA's flag makes every later
-// one return at once, and the pass ends at its next block barrier.
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, volatile int* dead) {
-    if (bar_try(bar, parity)) return;
-    const long long t0 = clock64();
+
+// Waits that run out.  dead[0]: a wait of this CTA ran out.  dead[kBars]: the cluster
+// barriers of rejected steps and tallies so far; dead[kTold]: the number of the barrier at
+// which a peer, whose wait ran out, leaves (0: none).
+//  - A wait of steps B to E that ran out only sets dead[0]: the attempt goes on with what is
+//    there (every branch depends on agreed flags alone), and the next attempt's flags, of
+//    which dead[0] is one, end the pass in the whole cluster.
+//  - The wait for the flags themselves (step A) is lost for all threads of a CTA or for none
+//    (verdict_lost).  A CTA that loses it tells its peers the number of its last cluster
+//    barrier; they are there or still run, so none has left.
+//  - That barrier may pair with a peer's barrier of a rejected step or of the tallies.  The
+//    word is visible behind it, in every CTA, so nobody sends anything any more.  (A word of
+//    a later barrier may come in there too; it is another number.)
+//  - A CTA that knows of a wait that ran out then stays for 2^20 cycles (peers' stores in
+//    flight land in microseconds) and reports it.
+//  - An mbarrier is armed again only after a phase of it that completed.
+constexpr int kTold = 3, kBars = 4, kOut = 5, kVerdict = 6;
+// whether the phase completed
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* dead, int limit) {
     while (!bar_try(bar, parity)) {
-        if (*dead) return;
-        if (clock64() - t0 > 4000000000LL) {
-            *dead = 1;
-            return;
+        if (--limit < 0 || dead[0]) {
+            dead[0] = 1;
+            return false;
         }
+    }
+    return true;
+}
+// the same, then thread 0 arms the next phase
+__device__ __forceinline__ void bar_next(uint32_t bar, uint32_t parity, int bytes, volatile int* dead, int limit,
+                                         int t) {
+    if (bar_wait(bar, parity, dead, limit) && t == 0) bar_arm(bar, bytes);
+}
+// Where a thread's patience ran out: whether the phase is lost, the same for all T threads of
+// the CTA without a barrier between them.  The threads count themselves in dead[kOut], and
+// the last of all T looks once more and writes the verdict (1 complete, 2 lost).  A thread
+// that finds the phase complete while the count is below T goes on, counted or not: whoever
+// counts last looks later, and finds it complete too.
+template <int T>
+__device__ __noinline__ bool verdict_lost(uint32_t bar, uint32_t parity, volatile int* dead) {
+    int verdict = 0;
+    if (atomicAdd((int*)dead + kOut, 1) == T - 1) dead[kVerdict] = bar_try(bar, parity) ? 1 : 2;
+    while (!verdict) {
+        const bool done = bar_try(bar, parity);
+        verdict = dead[kVerdict];
+        if (!verdict && done && dead[kOut] < T) verdict = 1;
+    }
+    if (verdict == 2) dead[0] = 1;
+    else if (atomicSub((int*)dead + kOut, 1) == 1) dead[kVerdict] = 0;      // none left: for the next phase
+    return verdict == 2;
+}
+// The wait for the flags.  (A block-wide OR behind an ordinary wait took clusters 5 to 8 %:
+// 4096 points on 8 CTAs 3.3 -> 3.5 us an attempt; the verdict's code inlined 2 %.)
+template <int T>
+__device__ __forceinline__ bool flags_lost(uint32_t bar, uint32_t parity, volatile int* dead, int limit) {
+    do {
+        if (bar_try(bar, parity)) return false;
+    } while (--limit >= 0 && !dead[kTold]);
+    return verdict_lost<T>(bar, parity, dead);
+}
+// before and behind a cluster barrier that may pair with a peer's last one
+__device__ __forceinline__ void count_bar(int* dead, int t) {
+    if (t == 0) ++dead[kBars];
+}
+__device__ __forceinline__ bool peer_gone(const volatile int* dead) {
+    return dead[kTold] != 0 && dead[kTold] == dead[kBars];
+}
+// The two parts around the last cluster barrier.  Thread and rank are read again here: kept to
+// the end of the pass they cost the 4096-point kernels registers that they do not have.
+template <int C>
+__device__ __forceinline__ int2 whoami() {
+    int t, c = 0;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    if constexpr (C > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(c));
+    return make_int2(t, c);
+}
+// before: the word to the peers, where a wait ran out; returns whether the barrier is to be
+// left out, as the last one met a peer's last
+template <int C>
+__device__ __forceinline__ bool last_word(int* dead) {
+    __syncthreads();
+    if constexpr (C > 1) {
+        if (dead[0] | dead[kTold]) {
+            if (peer_gone(dead)) return true;
+            const int2 me = whoami<C>();
+            if (me.x < C && me.x != me.y) *cg::this_cluster().map_shared_rank(dead + kTold, me.x) = dead[kBars] + 1;
+        }
+    }
+    return false;
+}
+// behind: if a wait of the cluster ran out, the status says so
+template <int C>
+__device__ __forceinline__ void end_lost(const volatile int* dead, optifax_pulse_stats* stats) {
+    if (!(dead[0] | dead[kTold])) return;
+    if (C > 1)
+        for (const long long t0 = clock64(); clock64() - t0 < (1 << 20);) {}
+    const int2 me = whoami<C>();
+    if (me.x == 0 && me.y == 0 && stats) {
+        *stats = optifax_pulse_stats{};
+        stats->status = OPTIFAX_PULSE_TIMEOUT;
     }
 }
 
@@ -761,7 +851,7 @@ __device__ __forceinline__ void push_inverse(float2* bufg, uint32_t g, uint32_t 
 // OR of the error flags over the pulse: one slot per warp, then (clusters) one per CTA.
 // Double buffered by attempt.  The barrier inside also publishes what the threads
 // stored before it (stage output, pushed columns).
-constexpr int kDead = 8;          // a bounded wait ran out
+constexpr int kDead = 8;          // a bounded wait ran out: the same in every thread of the CTA
 
 // The same over every pulse of a shared schedule (a cooperative launch).  One 64-bit word
 // per attempt, three in turn, counts the clusters that have arrived and, per flag, those
@@ -772,8 +862,8 @@ constexpr int kDead = 8;          // a bounded wait ran out
 // accesses do (a word is used again only once every CTA has read its last round).  Six
 // pulses of 2048 points, us per attempt: 4.1 with release and acquire accesses and cleared
 // words, 3.65 so; one pulse alone 3.35.
-__device__ __forceinline__ int combine_grid(int f, int* slot, unsigned long long* last, int attempt, int t, int c,
-                                            const KernelCfg& cfg) {
+__device__ __forceinline__ int combine_grid(int f, int* slot, unsigned long long* last, int* dead, int attempt, int t,
+                                            int c, const KernelCfg& cfg) {
     const int i = attempt % 3;
     unsigned long long* w = cfg.grid_sync + i;
     if (t == 0) {
@@ -784,13 +874,14 @@ __device__ __forceinline__ int combine_grid(int f, int* slot, unsigned long long
             asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(w), "l"(v) : "memory");
         }
         last += i;
-        const unsigned t0 = (unsigned)(clock64() >> 12);
+        int limit = 16 * cfg.wait;         // a look takes 0.2 us or more
         unsigned long long v;
         for (;;) {
             asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
             v -= *last;
             if ((int)(v & 0xffffu) == cfg.clusters) break;
-            if ((unsigned)(clock64() >> 12) - t0 > 1000000u) {           // 2 s
+            if (--limit < 0) {
+                *dead = 1;
                 f |= kDead;
                 break;
             }
@@ -807,6 +898,7 @@ __device__ __forceinline__ int combine_flags(int bits, int* red, uint32_t bar, u
                                              unsigned long long* last, int attempt, int t, int c, const KernelCfg& cfg) {
     const int par = attempt & 1;
     int* wf = red + par * NW;
+    if (C > 1 && *(volatile int*)dead) bits |= kDead;
     const int w = __reduce_or_sync(0xffffffffu, bits);
     if ((t & 31) == 0) wf[t >> 5] = w;
     __syncthreads();
@@ -822,20 +914,22 @@ __device__ __forceinline__ int combine_flags(int bits, int* red, uint32_t bar, u
         for (int i = 0; i < NW; ++i) f |= wf[i];
     }
     if constexpr (C > 1) {
-        const int lost = *(volatile int*)dead;       // written before the barrier: the same for every thread
         int* cl = red + 2 * NW + par * 16;
         if (t < C && t != c) {
             const uint32_t src = smem_u32(cl + c), dst = cluster_addr(src, t);
             st_async(dst, f, dst + (bar - src));
         }
-        bar_wait(bar, parity, dead);
+        if (flags_lost<32 * NW>(bar, parity, dead, cfg.wait)) return kDead;
         if (t == 0) bar_arm(bar, bytes);
 #pragma unroll
         for (int r = 0; r < C; ++r)
             if (r != c) f |= cl[r];
-        f = lost ? kDead : (f & 7);
+        if (f & kDead) {
+            if (t == 0) *dead = 1;
+            return kDead;
+        }
     }
-    if (cfg.shared_sched) f = combine_grid(f, red + 2 * NW + 2 * 16 + 1, last, attempt, t, c, cfg);
+    if (cfg.shared_sched) f = combine_grid(f, red + 2 * NW + 2 * 16 + 1, last, dead, attempt, t, c, cfg);
     return f;
 }
 
@@ -929,6 +1023,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     __shared__ PulseDev sP;
     if (t == 0) {
         sP = pulses[p];
+        dead[0] = dead[kTold] = dead[kBars] = dead[kOut] = dead[kVerdict] = 0;
         *run = RunState{};
         run->bounds = Bounds(METHOD != OPTIFAX_RK23 ? 50.f : 200.f, sP.max_err, sP.min_err);
     }
@@ -959,7 +1054,6 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     const uint32_t bars = smem_u32(smem + SM::off_bar);
     const uint32_t bar_a = bars, bar_b = bars + 8, bar_c = bars + 16, bar_d = bars + 24, bar_e = bars + 32;
     if (C > 1 && t == 0) {
-        *dead = 0;
         for (int i = 0; i < 6; ++i) bar_init(bars + 8 * i);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         bar_arm(bar_a, kBytesA);
@@ -1016,7 +1110,6 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     auto load_hot = [&] { return Hot{P_.h, P_.c_shock, P_.sel, (float)P_.S, P_.nchunks, P_.G, P_.fb != nullptr}; };
     const Hot hot_ = load_hot();
     auto hot = [&]() -> Hot { if constexpr (tight) return load_hot(); else return hot_; };
-    const int max_attempts = cfg.max_attempts_mul * (P_.S + 16) + 64;
     const Bounds bounds_ = tight ? Bounds{} : Bounds(heun ? 50.f : 200.f, P_.max_err, P_.min_err);
     auto bounds = [&]() -> Bounds { if constexpr (tight) return run->bounds; else return bounds_; };
     // what the caller asked for beyond the field, as one register (tested per attempt)
@@ -1025,14 +1118,13 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                      (!nee && (P_.stepmods || P_.smt) ? kSteps : 0) | (P_.Ap ? kAp : 0);
     constexpr float invN = 1.0f / (float)N;
     const int guard = cfg.guard;
-    const int n_trips = P_.n_trips > 0 ? P_.n_trips : 1;
     const bool rec = (c == 0 && t == 0);
     const uint32_t x_addr = smem_u32(bufX), g_addr = smem_u32(bufG);
 
     float k = nee ? 1.f : 0.f, stepprev = 4.f, stepmod = 4.f;
     unsigned q = 0;                          // accumulated dispersion position (sum of stepmod)
     int s_cached = -1;                       // stepmod of the cached per-mode D - 1
-    int attempt = 0, status = 0, par = 0, trip = 0, gatt = 0;         // gatt: attempts of all trips
+    int par = 0, gatt = 0;                   // gatt: attempts of all trips
 
     // neighbours' drive values at the thread's ends; hv: the halo point's drive (end threads)
     auto edges = [&](const Pair (&nl)[H], float2 hv, float2& L, float2& R) {
@@ -1055,8 +1147,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
         } else if constexpr (C > 1) {
             if (lend || rend) {
                 const uint32_t b = bar_e + 8 * ep;
-                bar_wait(b, (ph_e >> ep) & 1, dead);
-                if (t == 0) bar_arm(b, kBytesE);
+                bar_next(b, (ph_e >> ep) & 1, kBytesE, dead, cfg.wait, t);
                 (lend ? L : R) = ends[(ep * C + seg) * 2 + (lend ? 0 : 1)];
             }
             ph_e ^= 1u << ep;
@@ -1088,10 +1179,9 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     };
 
     Pair k1r[H];      // RK23: K1 (first stage, FSAL) between attempts
-    for (trip = 0; trip < n_trips; ++trip) {
+    do {
         k = nee ? 1.f : 0.f; stepprev = 4.f; stepmod = 4.f; q = 0;
-        attempt = 0;
-        int trip_status = 0;
+        int limit = gatt + cfg.max_attempts_mul * (P_.S + 16) + 64;     // of this trip's attempts
         if constexpr (!heun) {
             // initial K1 at k = 0 with stepmod = 4 (OPO_CUDA_ODE23.cu:432-438)
             const float hg = (stepmod * hot().h) * hot().G[0], cs = hot().cs;
@@ -1113,7 +1203,10 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
             if (!nee) stepmod = stepprev;
             const float cend = (float)(chunk + 1) * hot().sel;
             while (more(k, cend)) {
-                if (attempt >= max_attempts) { status |= OPTIFAX_PULSE_ATTEMPT_LIMIT; goto done; }
+                if (gatt >= limit) {
+                    if (t == 0) run->status |= OPTIFAX_PULSE_ATTEMPT_LIMIT;
+                    goto done;
+                }
                 const int krec = (int)k;
                 // z of the first stage in steps and index of G (G33(k) is 1-based in NEE_CPU.m)
                 const float kpos = nee ? k - 1.f : k;
@@ -1222,9 +1315,9 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
 
                 int fl = combine_flags<T / 32, C>(bits, red, bar_a, gatt & 1, kBytesA, dead, run->grid_last, gatt, t,
                                                   c, cfg);
-                if (fl & kDead) { status |= OPTIFAX_PULSE_TIMEOUT; goto done; }
+                if (fl & kDead) goto done;
                 if ((opts & kForced) && gatt < P_.n_forced) fl = (P_.forced[gatt] & 3) | (fl & 4);
-                if (fl & 4) trip_status |= OPTIFAX_PULSE_NAN;
+                if ((fl & 4) && t == 0) run->trip_status |= OPTIFAX_PULSE_NAN;
 
                 if ((fl & 1) && stepmod > 1.f && (nee || (k - stepmod) > 0.f)) {
                     // ---- reject: A0 unchanged; MEX: k moves back by one in net (the loop
@@ -1234,8 +1327,6 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                         P_.trace[3 * gatt + 2] = fl & 7;
                     }
                     if (t == 0) ++run->n_rej;
-                    // the next attempt's flags and halos must not overtake this one's
-                    if constexpr (C > 1) cg::this_cluster().sync();
                     if (!nee) k = k - stepmod;
                     stepmod = stepmod - 1.f;
                     stepprev = stepmod;
@@ -1250,6 +1341,12 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                         edges(nl, make_float2(0.f, 0.f), L, R);
                         k_all<H>(nl, L, R, hg1, cs, k1r);
                     }
+                    // the next attempt's flags and halos must not overtake this one's
+                    if constexpr (C > 1) {
+                        count_bar(dead, t);
+                        cg::this_cluster().sync();
+                        if (peer_gone(dead)) limit = 0;
+                    }
                 } else {
                     // ---- accept ----
                     if ((opts & kTrace) && rec && gatt < P_.trace_cap) {
@@ -1261,7 +1358,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     const int s_used = (int)stepmod;
                     if ((opts & kSteps) && rec && krec < P_.stepmods_limit && krec < P_.S) {
                         if (P_.stepmods) P_.stepmods[krec] = (float)s_used;
-                        if (P_.smt) P_.smt[(size_t)trip * P_.S + krec] = (float)s_used;
+                        if (P_.smt) P_.smt[(size_t)run->trips_done * P_.S + krec] = (float)s_used;
                     }
                     // step control (OPO_CUDA_BATCH_XTAL.cu:487-506; ODE23 :519-538 doubles;
                     // NEE_CPU.m:77-83: grow below minErr, clamp only at the crystal end)
@@ -1325,8 +1422,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     }
                     if constexpr (C > 1) {
                         if constexpr (XC_::LOCAL) __syncthreads();
-                        bar_wait(bar_b, ph_x, dead);
-                        if (t == 0) bar_arm(bar_b, kAll);
+                        bar_next(bar_b, ph_x, kAll, dead, cfg.wait, t);
                     }
                     float2 v[P];
                     fftp_forward<M, P>(bufX, tw_s, t, v);
@@ -1380,7 +1476,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
 #pragma unroll 1
                             for (int i = 0; i < P_.n_esd; ++i)
                                 P_.esd[(size_t)i * N + kk] += P_.esd_w[(size_t)i * N + kk] * x2;
-                            if (P_.hist) P_.hist[(size_t)trip * N + kk] = X;
+                            if (P_.hist) P_.hist[(size_t)run->trips_done * N + kk] = X;
                             xsp[kk] = cadd(cmul(X, P_.fb[kk]), P_.pump[kk]);
                         }
 #pragma unroll
@@ -1390,13 +1486,11 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     if constexpr (C > 1) {
                         push_inverse<M, C>(bufG, g_addr, bar_c, v, t, c);
                         if constexpr (XC_::LOCAL) __syncthreads();
-                        bar_wait(bar_c, ph_x, dead);
-                        if (t == 0) bar_arm(bar_c, kAll);
+                        bar_next(bar_c, ph_x, kAll, dead, cfg.wait, t);
                         exchange_inv<M, C, HALO>(bufG, bufX, smem_u32(halo_d), bar_d, xtw_s, xtd_s, inner, t, c, invN);
                         __syncthreads();
                         if (HALO && (lend || rend)) {
-                            bar_wait(bar_d, ph_x, dead);
-                            if (t == 0) bar_arm(bar_d, kBytesD);
+                            bar_next(bar_d, ph_x, kBytesD, dead, cfg.wait, t);
                             const float2 d1 = halo_d[4 * seg + (lend ? 1 : 2)];
                             const float2 d2 = halo_d[4 * seg + (lend ? 0 : 3)];
                             hs[0] = cav ? d1 : cadd(hs[0], d1);
@@ -1419,43 +1513,43 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                     }
                     if (cav) {
                         double tally[4];
-                        reduce_tallies<M, C>(part, tally, dred, t, c, trip & 1);
+                        count_bar(dead, t);
+                        reduce_tallies<M, C>(part, tally, dred, t, c, run->trips_done & 1);
                         if (t == 0)
                             for (int i = 0; i < 4; ++i) run->tally[i] = tally[i];
                     }
                     q = qn;
                 }
-                ++attempt;
                 ++gatt;
                 if (!nee || accepted) k = k + stepmod;
             }
         }
-        status |= trip_status;
         if (t == 0) {
-            run->trips_done = trip + 1;
+            const int trip = run->trips_done, attempts = gatt - run->tot_att;
+            run->status |= run->trip_status;
             if (rec && P_.fb && P_.trips) {
                 optifax_trip_record tr;
-                tr.attempts = attempt; tr.accepted = run->n_acc; tr.rejected = run->n_rej; tr.status = trip_status;
+                tr.attempts = attempts; tr.accepted = run->n_acc; tr.rejected = run->n_rej; tr.status = run->trip_status;
                 for (int i = 0; i < 4; ++i) tr.tally[i] = run->tally[i];
                 P_.trips[trip] = tr;
             }
-            run->tot_att += attempt; run->tot_acc += run->n_acc; run->tot_rej += run->n_rej;
-            run->n_acc = run->n_rej = 0;
+            run->tot_att = gatt; run->tot_acc += run->n_acc; run->tot_rej += run->n_rej;
+            run->n_acc = run->n_rej = run->trip_status = 0;
             // steady state of a cavity: the totals are the same in every CTA of the cluster
             const double cur = run->tally[P_.steady_tally & 3];
             const bool flat = trip > 0 && cur != 0.0 &&
                               fabs(cur - run->prev_tally) <= (double)P_.steady_tol * fabs(cur);
             run->steady = flat ? run->steady + 1 : 0;
             run->prev_tally = cur;
-            run->stop = P_.fb && P_.steady_trips > 0 && run->steady >= P_.steady_trips;
+            run->stop = trip + 1 >= P_.n_trips || (P_.fb && P_.steady_trips > 0 && run->steady >= P_.steady_trips) ||
+                        (C > 1 && peer_gone(dead));
+            run->trips_done = trip + 1;
             for (int i = 0; i < 4; ++i) run->tally[i] = 0.0;
         }
-        if (n_trips > 1) {
-            __syncthreads();
-            if (run->stop) break;
-        }
-    }
+        __syncthreads();
+    } while (!run->stop);
 done:
+    const bool gone = last_word<C>(dead);
 #pragma unroll
     for (int j = 0; j < H; ++j) {
         P_.A_out[i0 + j] = make_float2(a[j].re.x, a[j].im.x);
@@ -1463,12 +1557,15 @@ done:
     }
     if (rec && P_.stats) {
         optifax_pulse_stats st;
-        st.attempts = run->tot_att; st.accepted = run->tot_acc; st.rejected = run->tot_rej; st.status = status;
+        st.attempts = run->tot_att; st.accepted = run->tot_acc; st.rejected = run->tot_rej; st.status = run->status;
         st.z_steps = (long long)q; st.k_final = k; st.stepmod_final = stepmod; st.n_chunks = P_.nchunks;
         st.reserved[0] = run->trips_done; st.reserved[1] = st.reserved[2] = 0;
         *P_.stats = st;
     }
-    if constexpr (C > 1) cg::this_cluster().sync();      // no CTA leaves while a peer may still read its memory
+    if constexpr (C > 1) {
+        if (!gone) cg::this_cluster().sync();        // no CTA leaves while a peer may still read its memory
+    }
+    end_lost<C>(dead, P_.stats);
 }
 
 }  // namespace ofx

@@ -99,7 +99,7 @@ struct SmemX {
     // absorber factors of the threads that have one (a quarter of them: the absorber spans
     // [6/16, 10/16] of the window in every variant): [point][thread]
     static constexpr int SLOTS = SH::T / 4 + 2;
-    static constexpr size_t off_abc = (off_red + sizeof(int) * (2 * SH::NW + 2 * 16 + 4) + 15) & ~size_t(15);
+    static constexpr size_t off_abc = (off_red + sizeof(int) * (2 * SH::NW + 2 * 16 + 8) + 15) & ~size_t(15);
     static constexpr size_t bytes = off_abc + sizeof(typename Num<R>::real) * SH::P * SLOTS;
     static_assert(bytes <= 232448 - 288, "shared memory of one CTA");
 };
@@ -336,7 +336,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
     const cplx* __restrict__ wn = tabs.wn;
     if (t == 0) {
         sP = pulses[p];
-        *dead = 0;
+        dead[0] = dead[kTold] = dead[kBars] = dead[kOut] = dead[kVerdict] = 0;
         slots = 0;
         for (int i = 0; i < 3; ++i) grid_last[i] = 0;
     }
@@ -581,7 +581,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
             }
             int fl = combine_flags<NW, C>(bits, red, bar_a, ph_a, kBytesA, dead, grid_last, attempt, t, c, cfg);
             ph_a ^= 1;
-            if (fl & kDead) { status |= OPTIFAX_PULSE_TIMEOUT; goto done; }
+            if (fl & kDead) goto done;
             if (fl & 4) status |= OPTIFAX_PULSE_NAN;
 
             if ((fl & 1) && stepmod > 1.0 && (NEE || (k - stepmod) > 0.0)) {
@@ -591,7 +591,11 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
                 }
                 ++n_rej;
                 // the next attempt's flags and halos must not overtake this one's
-                if constexpr (C > 1) cg::this_cluster().sync();
+                if constexpr (C > 1) {
+                    count_bar(dead, t);
+                    cg::this_cluster().sync();
+                    if (peer_gone(dead)) goto done;
+                }
                 if (!NEE) k = k - stepmod;
                 stepmod = stepmod - 1.0;
                 stepprev = stepmod;
@@ -673,8 +677,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
                 }
                 if constexpr (C > 1) {
                     if constexpr (LOCAL) __syncthreads();
-                    bar_wait(bar_b, ph_x, dead);
-                    if (t == 0) bar_arm(bar_b, kAll);
+                    bar_next(bar_b, ph_x, kAll, dead, cfg.wait, t);
                 }
                 fft.forward(v);
 #pragma unroll
@@ -691,8 +694,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
                         push(bufG, m / COLS, swzx<P>(c * COLS + m % COLS), v[i], bar_c);
                     }
                     if constexpr (LOCAL) __syncthreads();
-                    bar_wait(bar_c, ph_x, dead);
-                    if (t == 0) bar_arm(bar_c, kAll);
+                    bar_next(bar_c, ph_x, kAll, dead, cfg.wait, t);
                     // undo the twiddles, inverse C-point DFTs -> own points
                     if constexpr (SH::SPLIT) {
                         const int l = t % SH::LANES, col = t / SH::LANES;
@@ -738,8 +740,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
                     }
                     __syncthreads();
                     if (lend || rend) {
-                        bar_wait(bar_d, ph_x, dead);
-                        if (t == 0) bar_arm(bar_d, kBytesD);
+                        bar_next(bar_d, ph_x, kBytesD, dead, cfg.wait, t);
                         hs[0] = halo_d[4 * seg + (lend ? 1 : 2)];
                         hs[1] = halo_d[4 * seg + (lend ? 0 : 3)];
                     }
@@ -758,6 +759,7 @@ passx_kernel(const PulseX* __restrict__ pulses, XTables<R> tabs, KernelCfg cfg) 
         }
     }
 done:
+    const bool gone = last_word<C>(dead);
 #pragma unroll
     for (int j = 0; j < P; ++j) Pd.A_out[i0 + j] = X::to_d(a[j]);
     if (rec && Pd.stats) {
@@ -767,7 +769,10 @@ done:
         st.reserved[0] = 1; st.reserved[1] = st.reserved[2] = 0;
         *Pd.stats = st;
     }
-    if constexpr (C > 1) cg::this_cluster().sync();      // no CTA leaves while a peer may still write its memory
+    if constexpr (C > 1) {
+        if (!gone) cg::this_cluster().sync();        // no CTA leaves while a peer may still write its memory
+    }
+    end_lost<C>(dead, Pd.stats);
 }
 
 }  // namespace ofx

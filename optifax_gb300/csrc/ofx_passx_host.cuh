@@ -196,6 +196,7 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
     cfg.max_attempts_mul = 64;
     cfg.grid_sync = w.flags;
     cfg.clusters = B;
+    cfg.wait = kWait;
     XTables<R> tabs;
     tabs.wn = w.tab;
     cudaLaunchConfig_t lc = {};
