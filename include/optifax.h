@@ -64,7 +64,8 @@ typedef enum {
 /* Per-pulse status bits returned in optifax_pulse_stats.status. */
 #define OPTIFAX_PULSE_NAN           0x1  /* a non-finite field value was produced */
 #define OPTIFAX_PULSE_ATTEMPT_LIMIT 0x2  /* the step-attempt safety limit was reached */
-#define OPTIFAX_PULSE_TIMEOUT       0x4  /* a wait inside a cluster ran out (about 2 s); the field is not valid */
+#define OPTIFAX_PULSE_TIMEOUT       0x4  /* a wait inside a cluster or between the clusters of a shared schedule ran out
+                                            (about 2 s): the field is NaN, the other outputs are not complete */
 
 typedef struct {
     int32_t attempts;       /* step attempts (accepted + rejected) */
@@ -170,7 +171,8 @@ const char* optifax_last_error(optifax_handle h);
  * Outputs: A_out (plhs[0], N x B), Ap_out (plhs[1]), stepmods_out (plhs[2]);
  * the outputs may alias the inputs.  As in the reference, all pulses of the
  * batch share one adaptive step schedule (error flags are OR-ed over the
- * batch): for n_pulses > 1 the batch runs as one cooperative launch.
+ * batch): for n_pulses > 1 the batch runs as one cooperative launch.  There are no
+ * statistics here: where a wait ran out (OPTIFAX_PULSE_TIMEOUT elsewhere), A_out is NaN.
  */
 int optifax_opo_mex_batch(optifax_handle h,
                           const void* E, const float* alpha_w, const float* G,
@@ -268,7 +270,8 @@ int optifax_propagate_noalloc(const optifax_pulse* pulse, int32_t variant,
  * flags | 8 if accepted}; stats_host (optional, HOST).  Variant ODE23 is not
  * offered; NEE follows NEE_CPU.m for grids up to 2^14 points (the snapshot
  * outputs are not produced by this entry).  Calls on one device are serialised
- * internally, and each call waits for its stream before returning.
+ * internally, and each call waits for its stream before returning; a wait of the
+ * pass that ran out (OPTIFAX_PULSE_TIMEOUT) returns OPTIFAX_ERR_CUDA.
  */
 int optifax_propagate_fp64(int32_t n_points, int32_t n_pulses, int32_t n_steps,
                            const double* E_in, double* A_out, const double* alpha,

@@ -32,7 +32,7 @@ struct optifax_context {
     size_t xs_cap = 0;                   // in complex values
     std::vector<cudaStream_t> side;      // streams for concurrent launch groups
     std::vector<cudaEvent_t> ev;         // fork/join events
-    unsigned long long* d_grid_sync = nullptr;   // shared schedules: 3 words
+    unsigned long long* d_grid_sync = nullptr;   // shared schedules: 4 words
     ofx::GnlseDev* d_gnlse_desc = nullptr;   // GNLSE: descriptors and stage scratch
     size_t gnlse_desc_cap = 0;
     float2* d_gnlse_k = nullptr;

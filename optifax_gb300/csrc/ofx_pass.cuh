@@ -90,7 +90,7 @@ struct KernelCfg {
     int guard;           // XTAL/BATCH_OP: ceil chunk count and k < Nsteps loop guard
     int shared_sched;    // 1: OR the error flags over every pulse of the launch (grid barrier)
     int max_attempts_mul;
-    unsigned long long* grid_sync;   // shared schedule: 3 words, zero before the launch
+    unsigned long long* grid_sync;   // shared schedule: 4 words, zero before the launch; the last: a wait ran out
     int clusters;        // of the launch
     int wait;            // limit of a bounded wait, in looks at an mbarrier (about 4 us each)
 };
@@ -542,16 +542,25 @@ __device__ __forceinline__ bool last_word(int* dead) {
     }
     return false;
 }
-// behind: if a wait of the cluster ran out, the status says so
-template <int C>
-__device__ __forceinline__ void end_lost(const volatile int* dead, optifax_pulse_stats* stats) {
+// behind: if a wait of the cluster ran out, the field is NaN (the one sign that a caller without
+// a status has) and the status says so
+template <int M, int C, typename V>
+__device__ __forceinline__ void end_lost(const volatile int* dead, V* out, optifax_pulse_stats* stats, const KernelCfg& cfg) {
     if (!(dead[0] | dead[kTold])) return;
+    __syncthreads();                   // behind the stores of the field
     if (C > 1)
         for (const long long t0 = clock64(); clock64() - t0 < (1 << 20);) {}
     const int2 me = whoami<C>();
-    if (me.x == 0 && me.y == 0 && stats) {
-        *stats = optifax_pulse_stats{};
-        stats->status = OPTIFAX_PULSE_TIMEOUT;
+    V nan;
+    nan.x = nan.y = __int_as_float(0x7fc00000);
+#pragma unroll 1
+    for (int i = me.x; i < M; i += blockDim.x) out[me.y * M + i] = nan;
+    if (me.x == 0 && me.y == 0) {
+        if (cfg.shared_sched) atomicOr(cfg.grid_sync + 3, 1ull);
+        if (stats) {
+            *stats = optifax_pulse_stats{};
+            stats->status = OPTIFAX_PULSE_TIMEOUT;
+        }
     }
 }
 
@@ -1565,7 +1574,7 @@ done:
     if constexpr (C > 1) {
         if (!gone) cg::this_cluster().sync();        // no CTA leaves while a peer may still read its memory
     }
-    end_lost<C>(dead, P_.stats);
+    end_lost<M, C>(dead, P_.A_out, P_.stats, cfg);
 }
 
 }  // namespace ofx

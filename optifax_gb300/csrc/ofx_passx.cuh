@@ -772,7 +772,7 @@ done:
     if constexpr (C > 1) {
         if (!gone) cg::this_cluster().sync();        // no CTA leaves while a peer may still write its memory
     }
-    end_lost<C>(dead, Pd.stats);
+    end_lost<M, C>(dead, Pd.A_out, Pd.stats, cfg);
 }
 
 }  // namespace ofx

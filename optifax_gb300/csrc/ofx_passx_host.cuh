@@ -94,6 +94,12 @@ inline const XKernel<R>* xchoose(const std::vector<XKernel<R>>& kernels, int n, 
     return wide;
 }
 
+// What a call reads back: the schedule's statistics and the shared schedule's words
+struct XReport {
+    optifax_pulse_stats stats;
+    unsigned long long sync[4];
+};
+
 template <typename R>
 struct XWork {
     int n_tab = 0;
@@ -104,8 +110,7 @@ struct XWork {
     size_t desc_n = 0;
     int* trace = nullptr;
     size_t trace_n = 0;
-    optifax_pulse_stats* stats = nullptr;
-    unsigned long long* flags = nullptr;
+    XReport* report = nullptr;
 };
 
 template <typename T>
@@ -154,10 +159,8 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
     size_t tn = w.trace_n * 3 * sizeof(int);
     if (tcap && (rc = grow_dev(&w.trace, &tn, 3 * sizeof(int) * tcap))) return rc;
     if (tcap) w.trace_n = tn / (3 * sizeof(int));
-    size_t sb = w.stats ? sizeof(optifax_pulse_stats) : 0;
-    if ((rc = grow_dev(&w.stats, &sb, sizeof(optifax_pulse_stats)))) return rc;
-    size_t fb = w.flags ? 4 * sizeof(*w.flags) : 0;
-    if ((rc = grow_dev(&w.flags, &fb, 4 * sizeof(*w.flags)))) return rc;
+    size_t rb = w.report ? sizeof(XReport) : 0;
+    if ((rc = grow_dev(&w.report, &rb, sizeof(XReport)))) return rc;
 
     std::vector<PulseX> d((size_t)B);
     int nchunks = (int)((double)S / sel);
@@ -172,7 +175,7 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
         x.G = G + (g_per_pulse ? (size_t)b * S : 0);
         x.trace = (b == 0 && tcap) ? w.trace : nullptr;
         x.trace_cap = (b == 0) ? (int)tcap : 0;
-        x.stats = (b == 0) ? w.stats : nullptr;
+        x.stats = (b == 0) ? &w.report->stats : nullptr;
         x.ztab = reinterpret_cast<cplx*>(w.ztab) + (size_t)b * zcap;
         x.zcap = zcap;
         x.tau_theta = turns_fixed((long double)w0 * (long double)dt);
@@ -183,8 +186,7 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
         x.N = n; x.S = S; x.nchunks = nchunks;
     }
     if (cudaMemcpyAsync(w.desc, d.data(), sizeof(PulseX) * (size_t)B, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemsetAsync(w.flags, 0, 4 * sizeof(*w.flags), st) != cudaSuccess ||
-        cudaMemsetAsync(w.stats, 0, sizeof(optifax_pulse_stats), st) != cudaSuccess)
+        cudaMemsetAsync(w.report, 0, sizeof(XReport), st) != cudaSuccess)
         return OPTIFAX_ERR_CUDA;
     if (xattributes(*ke) != cudaSuccess) return OPTIFAX_ERR_CUDA;
     KernelCfg cfg;
@@ -194,7 +196,7 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
     cfg.guard = vc.guard;
     cfg.shared_sched = B > 1 ? 1 : 0;
     cfg.max_attempts_mul = 64;
-    cfg.grid_sync = w.flags;
+    cfg.grid_sync = w.report->sync;
     cfg.clusters = B;
     cfg.wait = kWait;
     XTables<R> tabs;
@@ -218,17 +220,19 @@ int passx_run(const std::vector<XKernel<R>>& kernels, XWork<R>& w, int n, int B,
     lc.numAttrs = na;
     const PulseX* dd = w.desc;
     if (cudaLaunchKernelEx(&lc, ke->fn, dd, tabs, cfg) != cudaSuccess) return OPTIFAX_ERR_CUDA;
-    optifax_pulse_stats hs;
-    if (cudaMemcpyAsync(&hs, w.stats, sizeof(hs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    XReport report;
+    if (cudaMemcpyAsync(&report, w.report, sizeof(report), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return OPTIFAX_ERR_CUDA;
+    const optifax_pulse_stats& hs = report.stats;
     if (tcap) {
         const size_t nt = (size_t)(hs.attempts < trace_cap ? hs.attempts : trace_cap);
         if (nt && cudaMemcpy(trace_host, w.trace, 3 * sizeof(int) * nt, cudaMemcpyDeviceToHost) != cudaSuccess)
             return OPTIFAX_ERR_CUDA;
     }
     if (stats_host) *stats_host = hs;
-    return OPTIFAX_OK;
+    // a wait of this or another pulse of the schedule ran out: its field is NaN
+    return (hs.status & OPTIFAX_PULSE_TIMEOUT) || report.sync[3] ? OPTIFAX_ERR_CUDA : OPTIFAX_OK;
 }
 
 }  // namespace ofx

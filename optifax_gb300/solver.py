@@ -364,11 +364,15 @@ def autotune(n_points_list=(4096, 8192, 16384, 32768, 65536), crystal_length=0.1
 
 
 def decode_stats(stats: torch.Tensor) -> List[dict]:
-    """Decode the (n, 12) int32 stats tensor into optifax_pulse_stats dicts."""
+    """Decode the (n, 12) int32 stats tensor into optifax_pulse_stats dicts.  Raises
+    OptifaxError where a wait of a pass ran out (PULSE_TIMEOUT: its field is NaN)."""
     raw = stats.cpu().numpy()
     out = []
     for row in raw:
         b = row.tobytes()
         s = nat.OptifaxPulseStats.from_buffer_copy(b)
         out.append({f: getattr(s, f) for f, _ in nat.OptifaxPulseStats._fields_ if f != "reserved"})
+    late = [i for i, s in enumerate(out) if s["status"] & nat.PULSE_TIMEOUT]
+    if late:
+        raise nat.OptifaxError(f"a wait inside the crystal pass ran out (pulses {late}); their fields are not valid")
     return out

@@ -1,5 +1,6 @@
 """The crystal pass's bounded waits, run out by a short limit and something that nobody sends
-(wait_kernels.cu): every CTA of the cluster agrees, the status says so, the GPU stays usable.  Marked gpu.
+(wait_kernels.cu): every CTA of the cluster agrees, the field is NaN, the status says so, the
+GPU stays usable.  Marked gpu.
 """
 import ctypes
 import os
@@ -27,22 +28,23 @@ def lib(tmp_path_factory):
 
 
 def _pass(lib, kind, clusters, expected):
+    from optifax_gb300 import _native as nat
     status = (ctypes.c_int * clusters)()
     flag = ctypes.c_int()
     out = np.ones(2 * POINTS[kind] * clusters, dtype=np.float32)
     rc = lib.wait_pass(kind, clusters, expected, SHORT, status, out.ctypes.data_as(ctypes.c_void_p),
                        ctypes.byref(flag))
     assert rc == 0
-    return [s & 4 for s in status], out
+    return [s & nat.PULSE_TIMEOUT for s in status], out, flag.value
 
 
 @pytest.mark.parametrize("kind", range(5))
 @pytest.mark.parametrize("clusters", [1, 3])
 def test_schedule_that_expects_one_cluster_more(lib, kind, clusters):
-    status, _ = _pass(lib, kind, clusters, clusters + 1)
-    assert all(status)
-    status, out = _pass(lib, kind, clusters, clusters)                 # and the next launch runs
-    assert not any(status) and not out.any()
+    status, out, flag = _pass(lib, kind, clusters, clusters + 1)
+    assert all(status) and np.isnan(out).all() and flag == 1
+    status, out, flag = _pass(lib, kind, clusters, clusters)           # and the next launch runs
+    assert not any(status) and not out.any() and flag == 0
 
 
 def test_flags_agree_across_a_cluster(lib):

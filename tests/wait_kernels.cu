@@ -136,6 +136,7 @@ __global__ void __cluster_dims__(2) flag_kernel(int what, KernelCfg cfg, int* ou
     int f = 0;
     if (!(what == 1 && c == 1))
         f = combine_flags<kNW, 2>(t == 5 ? 1 + c : 0, red, bar, 0, 4, dead, last, 0, t, c, cfg);
+    __shared__ float2 nowhere[2];
     bool gone = false;
     if (!(f & kDead)) {
         count_bar(dead, t);
@@ -143,7 +144,7 @@ __global__ void __cluster_dims__(2) flag_kernel(int what, KernelCfg cfg, int* ou
         gone = peer_gone(dead);
     }
     if (!last_word<2>(dead)) cg::this_cluster().sync();
-    end_lost<2>(dead, nullptr);
+    end_lost<1, 2, float2>(dead, nowhere, nullptr, cfg);
     out[c * kT + t] = f | (gone ? 64 : 0) | ((dead[0] | dead[kTold]) ? 128 : 0);
 }
 
