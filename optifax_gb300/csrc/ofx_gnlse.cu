@@ -331,12 +331,11 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
         }
         __syncwarp();
         if (i >= P_.n_saves || zc >= total) return flags | kEnd;
-        // growth after a step with no failure: h / (1.25 (err/rtol)^(1/5)), at most 5 h (the
-        // factor only scales an integer step: FP32 serves)
+        // growth after a step with no failure: h / (1.25 (err/rtol)^(1/5)), at most 5 h
         long long h = hc;
         if (nofailed) {
-            const float temp = 1.25f * powf((float)err / rtolf, 0.2f);
-            h = temp > 0.2f ? (long long)((double)hc * (double)(1.0f / temp)) : 5 * hc;
+            const float temp = 1.25f * powf((float)(err / P_.rtol), 0.2f);
+            h = temp > 0.2f ? (long long)((double)hc / (double)temp) : 5 * hc;
         }
         if (limit) {
             if (t == 0) ctl.status |= OPTIFAX_PULSE_ATTEMPT_LIMIT;
