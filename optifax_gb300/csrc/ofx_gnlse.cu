@@ -418,30 +418,36 @@ gnlse_kernel(const GnlseDev* __restrict__ pulses, const Twiddle* __restrict__ qu
 
     int stage = 0, base = 0, side = 0;
     for (;;) {
-        // ---- stage input ys: every second stage reads the rows for itself and the next ----
-#pragma unroll
-        for (int j = 0; j < P; ++j) ys[j] = y[j];
+        // ---- stage input ys: every second stage reads the rows for itself and the next.  The
+        // weighted rows are summed by themselves and y is added last: one rounding at y's size
+        // (fields at 4096 points and 1 to 10 kW against FP64 on the same steps: 3.0e-7 with the rows
+        // added to y one after the other, 2.6e-7 so) ----
         const float hz = ctl.hz;
         float2 part2[P];                   // the next stage's sum without its last term (stage 6: the error's)
         if (stage == 1) {
             float2 k[P];
             load_row<M, P>(K, base, t, k);
 #pragma unroll
-            for (int j = 0; j < P; ++j) ys[j] = cfma1(k[j], hz * dp_a(1, 0), ys[j]);
+            for (int j = 0; j < P; ++j) ys[j] = cfma1(k[j], hz * dp_a(1, 0), y[j]);
         } else if (stage == 3 || stage == 5) {
             const float w = hz * (stage == 3 ? dp_a(3, 2) : dp_a(5, 4));
 #pragma unroll
             for (int i = 0; i < P / 2; ++i) {
                 const float4 c = carry[i * T + t];
-                ys[2 * i] = cfma1(v[2 * i], w, make_float2(c.x, c.y));
-                ys[2 * i + 1] = cfma1(v[2 * i + 1], w, make_float2(c.z, c.w));
+                ys[2 * i] = add2(y[2 * i], cfma1(v[2 * i], w, make_float2(c.x, c.y)));
+                ys[2 * i + 1] = add2(y[2 * i + 1], cfma1(v[2 * i + 1], w, make_float2(c.z, c.w)));
             }
-        } else if (stage != 0) {
+        } else if (stage == 0) {
 #pragma unroll
-            for (int j = 0; j < P; ++j) part2[j] = stage == 6 ? make_float2(0.f, 0.f) : y[j];
+            for (int j = 0; j < P; ++j) ys[j] = y[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < P; ++j) ys[j] = part2[j] = make_float2(0.f, 0.f);
             if (stage == 2) combine2<2, 3, M, P>(ys, part2, v, K, t, base, hz);
             else if (stage == 4) combine2<4, 5, M, P>(ys, part2, v, K, t, base, hz);
             else combine2<6, -1, M, P>(ys, part2, v, K, t, base, hz);
+#pragma unroll
+            for (int j = 0; j < P; ++j) ys[j] = add2(y[j], ys[j]);
 #pragma unroll
             for (int i = 0; i < P / 2; ++i)
                 carry[i * T + t] = make_float4(part2[2 * i].x, part2[2 * i].y, part2[2 * i + 1].x, part2[2 * i + 1].y);
