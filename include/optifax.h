@@ -153,6 +153,12 @@ typedef struct {
  * tables and the pulse-descriptor staging buffers (device workspace). */
 int optifax_create(optifax_handle* out, int device);
 int optifax_destroy(optifax_handle h);
+/* Points per CTA (512..4096, a power of two) of the handle's later calls and pulses that
+ * bring no choice of their own: optifax_opo_mex_batch, and optifax_propagate, its graphs
+ * and optifax_opo_run with cta_points 0.  0, the default: the library's rule (see
+ * optifax_propagate).  With a choice of the caller's the shapes, and so a result's
+ * bits, depend on nothing else than the call itself; 4096 takes the least SM time. */
+int optifax_set_cta_points(optifax_handle h, int32_t cta_points);
 const char* optifax_status_string(int status);
 /* Human-readable detail of the last failure on this handle. */
 const char* optifax_last_error(optifax_handle h);
@@ -189,8 +195,15 @@ int optifax_opo_mex_batch(optifax_handle h,
  * HOST array of n_pulses descriptors holding device pointers.  stats
  * (optional) is a DEVICE array of n_pulses entries.  cta_points selects the
  * points held per CTA (512..4096); a pulse of N points runs on a cluster of
- * N / cta_points CTAs.  0 = automatic: the most CTAs per pulse at which the GPU
- * holds every cluster of the call at once, 4096 points per CTA where it does not.
+ * N / cta_points CTAs.  0 = the library's rule.  It has three levels, one for the
+ * whole call: (0) 512 points per CTA for grids of 2048 and 4096 points, 1024 for 8192
+ * and 16384, 2048 for 32768; (1) twice as many (2048 points: one CTA); (2) 4096, or one
+ * CTA for smaller grids.  512, 1024 and 65536 points have one level.  The first level is
+ * taken at which the GPU holds at once every cluster of this call and of as many such
+ * calls as there are handles on the device.  Shapes differ in rounding, so by the rule
+ * a pulse's last bits depend on the other pulses of its call and on the number of
+ * handles; a choice of the caller's (here, per pulse, or optifax_set_cta_points) fixes
+ * them.  Programs that share the GPU with other processes do well to choose 4096.
  */
 int optifax_propagate(optifax_handle h, const optifax_pulse* pulses, int32_t n_pulses,
                       int32_t method, int32_t variant, int32_t cta_points,

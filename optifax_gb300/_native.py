@@ -22,7 +22,7 @@ EXPORTS = ["optifax_create", "optifax_destroy", "optifax_status_string", "optifa
            "optifax_ff_encode", "optifax_ff_step",
            "optifax_ff_encode_env", "optifax_ff_decode_env", "optifax_setup_work_bytes", "optifax_setup_pulses",
            "optifax_gnlse", "optifax_fno_set_grads", "optifax_propagate_graph", "optifax_graph_launch",
-           "optifax_graph_kernels", "optifax_graph_destroy"]
+           "optifax_graph_kernels", "optifax_graph_destroy", "optifax_set_cta_points"]
 
 _lib = None
 
@@ -71,6 +71,8 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
     lib.optifax_create.restype = ctypes.c_int
     lib.optifax_destroy.argtypes = [vp]
     lib.optifax_destroy.restype = ctypes.c_int
+    lib.optifax_set_cta_points.argtypes = [vp, ctypes.c_int32]
+    lib.optifax_set_cta_points.restype = ctypes.c_int
     lib.optifax_status_string.argtypes = [ctypes.c_int]
     lib.optifax_status_string.restype = ctypes.c_char_p
     lib.optifax_last_error.argtypes = [vp]
@@ -184,6 +186,10 @@ class Context:
         check(self.lib.optifax_create(ctypes.byref(h), int(device)), None, "optifax_create")
         self.handle = h
         self.device = device
+
+    def set_cta_points(self, cta_points: int):
+        """Points per CTA of this handle's calls and pulses without a choice of their own (0: the rule's)."""
+        check(self.lib.optifax_set_cta_points(self.handle, int(cta_points)), self.handle, "optifax_set_cta_points")
 
     def close(self):
         if getattr(self, "handle", None):

@@ -27,3 +27,7 @@ def test_a_wait_that_ran_out_raises():
 def test_other_status_bits_are_returned():
     got = sv.decode_stats(_stats(0, nat.PULSE_NAN, nat.PULSE_ATTEMPT_LIMIT))
     assert [g["status"] for g in got] == [0, 1, 2] and got[0]["attempts"] == 7
+
+
+def test_choice_of_points_needs_a_handle():
+    assert nat.load().optifax_set_cta_points(None, 0) == 5
