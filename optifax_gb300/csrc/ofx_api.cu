@@ -182,18 +182,20 @@ int resident_clusters(optifax_context* h, const KernelEntry& ke) {
 
 // Points per CTA of a grid of N points that carries no choice of the caller, by spread:
 //   0  the shortest time per attempt of one pulse
-//   1  half the CTAs
+//   1  half the CTAs; at 2048 points one CTA (two of 1024 points are slower and twice the SMs)
 //   2  4096 points per CTA (one CTA up to 4096 points): the least SM time per attempt
 // One pulse, us per attempt (GB300, 2 W, 30 um poling), at spread 2 -> 1 -> 0:
-//   2048: 4.1 -> 4.3 -> 3.3    4096: 6.4 -> 4.2 -> 3.4    8192: 9.3 -> 6.0 -> 4.3
-//   16384: 9.8 -> 5.8 -> 5.0   32768: 10.3 -> 10.3 -> 6.7
-// SM time per attempt goes the other way (4096: 6.5, 17, 28 SM us), so the wider
+//            2048 (1024 x 2)       4096          8192              16384             32768
+//   Heun  3.8 (4.0)  -> 3.0   6.5 4.2 3.3   9.1 5.9 4.2   9.6 5.7 4.9    9.9  9.9 6.8
+//   RK23  4.8 (4.6)  -> 3.5   7.6  -  3.6  10.3 6.6 4.5  10.8 8.9 5.2
+//   NEE   3.7 (3.9)  -> 2.9   6.4  -  3.2   9.1 5.9 4.2   9.6 5.7 4.7
+// SM time per attempt goes the other way (4096: 6.5, 17, 26 SM us), so the wider
 // spreads serve calls that leave SMs idle otherwise.
 int spread_points(int N, int spread) {
     const int narrow = N <= 4096 ? N : 4096;
     if (N <= 1024 || N > 32768 || spread >= 2) return narrow;
     const int wide = N <= 4096 ? 512 : N == 32768 ? 2048 : 1024;
-    return spread == 0 ? wide : (2 * wide < narrow ? 2 * wide : narrow);
+    return spread == 0 ? wide : (N > 2048 && 2 * wide < narrow ? 2 * wide : narrow);
 }
 
 // One pulse of a call before its group is known
