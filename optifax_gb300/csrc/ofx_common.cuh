@@ -30,7 +30,6 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
 __device__ __forceinline__ float2 cfma1(float2 a, float s, float2 b) { return fma2(a, dup2(s), b); }
 
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
@@ -39,7 +38,6 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.y, b.x, -a.x * b.y));
 }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
-__device__ __forceinline__ float cabsf2(float2 a) { return hypotf(a.x, a.y); }
 
 // A phase in turns held as an unsigned 64-bit fixed-point fraction
 // (2^64 == one turn).  Products of a per-unit phase with an integer position

@@ -20,13 +20,11 @@ namespace {
 
 const std::vector<XKernel<double>>& fp64_kernels() {
     static const std::vector<XKernel<double>> v = {
-        xkernel<double, 512, 1, false>(), xkernel<double, 1024, 1, false>(), xkernel<double, 512, 2, false>(),
-        xkernel<double, 512, 4, false>(), xkernel<double, 512, 8, false>(), xkernel<double, 512, 16, false>(),
-        xkernel<double, 1024, 2, false>(), xkernel<double, 1024, 4, false>(), xkernel<double, 1024, 8, false>(),
+        xkernel<double, 512, 1, false>(), xkernel<double, 512, 2, false>(), xkernel<double, 512, 4, false>(),
+        xkernel<double, 512, 8, false>(), xkernel<double, 512, 16, false>(), xkernel<double, 1024, 8, false>(),
         xkernel<double, 1024, 16, false>(), xkernel<double, 2048, 16, false>(), xkernel<double, 4096, 16, false>(),
-        xkernel<double, 512, 1, true>(), xkernel<double, 1024, 1, true>(), xkernel<double, 512, 2, true>(),
-        xkernel<double, 512, 4, true>(), xkernel<double, 512, 8, true>(), xkernel<double, 512, 16, true>(),
-        xkernel<double, 1024, 2, true>(), xkernel<double, 1024, 4, true>(), xkernel<double, 1024, 8, true>(),
+        xkernel<double, 512, 1, true>(), xkernel<double, 512, 2, true>(), xkernel<double, 512, 4, true>(),
+        xkernel<double, 512, 8, true>(), xkernel<double, 512, 16, true>(), xkernel<double, 1024, 8, true>(),
         xkernel<double, 1024, 16, true>(),
     };
     return v;

@@ -11,6 +11,5 @@ void register_kernels_heun_small(std::vector<KernelEntry>& v) {
     v.push_back(kernel_entry<512, 2, OPTIFAX_HEUN>());
     v.push_back(kernel_entry<512, 4, OPTIFAX_HEUN>());
     v.push_back(kernel_entry<512, 8, OPTIFAX_HEUN>());
-    v.push_back(kernel_entry<512, 16, OPTIFAX_HEUN>(true));
 }
 }  // namespace ofx

@@ -46,23 +46,6 @@ __device__ __forceinline__ ff ff_add(ff a, ff b) {
     const ff s = ff_two_sum(a.hi, b.hi);
     return ff_quick(s.hi, s.lo + (a.lo + b.lo));
 }
-__device__ __forceinline__ ff ff_neg(ff a) { return ff{-a.hi, -a.lo}; }
-__device__ __forceinline__ ff ff_sub(ff a, ff b) { return ff_add(a, ff_neg(b)); }
-__device__ __forceinline__ ff ff_mul(ff a, ff b) {
-    const float p = a.hi * b.hi;
-    const float e = fmaf(a.hi, b.hi, -p);
-    return ff_quick(p, fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, e)));
-}
-// a*b + c*d with one final normalisation
-__device__ __forceinline__ ff ff_dot2(ff a, ff b, ff c, ff d) {
-    const float p = a.hi * b.hi, q = c.hi * d.hi;
-    const float ep = fmaf(a.hi, b.hi, -p), eq = fmaf(c.hi, d.hi, -q);
-    const ff s = ff_two_sum(p, q);
-    float t = s.lo + (ep + eq);
-    t = fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, t));
-    t = fmaf(c.hi, d.lo, fmaf(c.lo, d.hi, t));
-    return ff_quick(s.hi, t);
-}
 // scaling by an exact power of two (0.5, 2): exact
 __device__ __forceinline__ ff ff_pow2(ff a, float s) { return ff{a.hi * s, a.lo * s}; }
 __device__ __forceinline__ ff ff_from(double x) {
@@ -97,15 +80,11 @@ template <> struct Num<double> {
     }
     static __device__ __forceinline__ cplx scale(cplx a, real s) { return make_double2(a.x * s, a.y * s); }
     static __device__ __forceinline__ cplx pow2(cplx a, double s) { return make_double2(a.x * s, a.y * s); }
-    static __device__ __forceinline__ cplx conj(cplx a) { return make_double2(a.x, -a.y); }
     static __device__ __forceinline__ cplx mul_i(cplx a) { return make_double2(-a.y, a.x); }       // i a
     static __device__ __forceinline__ cplx mul_mi(cplx a) { return make_double2(a.y, -a.x); }      // -i a
     static __device__ __forceinline__ real rfrom(double x) { return x; }
     static __device__ __forceinline__ cplx from(double2 v) { return v; }
     static __device__ __forceinline__ double2 to_d(cplx v) { return v; }
-    static __device__ __forceinline__ real norm2(cplx a) { return a.x * a.x + a.y * a.y; }
-    static __device__ __forceinline__ real radd(real a, real b) { return a + b; }
-    static __device__ __forceinline__ real rmul(real a, real b) { return a * b; }
     static __device__ __forceinline__ bool finite(cplx a) { return isfinite(a.x) && isfinite(a.y); }
     static __device__ __forceinline__ real triple(real a) { return 3.0 * a; }
     // n - i c d
@@ -197,15 +176,11 @@ template <> struct Num<ff> {
         const float f = (float)s;
         return cff{a.rh * f, a.ih * f, a.rl * f, a.il * f};
     }
-    static __device__ __forceinline__ cplx conj(cplx a) { return cff{a.rh, -a.ih, a.rl, -a.il}; }
     static __device__ __forceinline__ cplx mul_i(cplx a) { return cff{-a.ih, a.rh, -a.il, a.rl}; }
     static __device__ __forceinline__ cplx mul_mi(cplx a) { return cff{a.ih, -a.rh, a.il, -a.rl}; }
     static __device__ __forceinline__ real rfrom(double x) { return ff_from(x); }
     static __device__ __forceinline__ cplx from(double2 v) { return make(ff_from(v.x), ff_from(v.y)); }
     static __device__ __forceinline__ double2 to_d(cplx v) { return make_double2(ff_d(re(v)), ff_d(im(v))); }
-    static __device__ __forceinline__ real norm2(cplx a) { return ff_dot2(re(a), re(a), im(a), im(a)); }
-    static __device__ __forceinline__ real radd(real a, real b) { return ff_add(a, b); }
-    static __device__ __forceinline__ real rmul(real a, real b) { return ff_mul(a, b); }
     static __device__ __forceinline__ bool finite(cplx a) { return isfinite(a.rh) && isfinite(a.ih); }
     static __device__ __forceinline__ real triple(real a) { return ff_add(a, ff_pow2(a, 2.f)); }
     static __device__ __forceinline__ cplx sub_i(cplx n, cplx d, real c) { return sub(n, mul_i(scale(d, c))); }

@@ -343,7 +343,6 @@ struct Xch {
     static constexpr int COLS = M / C;
     static constexpr bool SPLIT = COLS < T;
     static constexpr int LANES = SPLIT ? T / COLS : 1;
-    static constexpr int XT = T;                             // every thread takes part
     static constexpr int PER = SPLIT ? 1 : COLS / T;
     static constexpr int NV = SPLIT ? P : PER * (C - 1);     // outer twiddles per thread
     // own parts of the exchange by plain stores and a block barrier (clusters of up to
@@ -380,10 +379,10 @@ struct Smem {
     // [6/16, 10/16] of the window in every variant), P each
     static constexpr size_t off_tw = off_abc + sizeof(float) * P * (T / 4 + 2);
     static constexpr size_t off_td = (off_tw + sizeof(float2) * F::TW + 15) & ~size_t(15);
-    // exchange twiddles W_N^{n2 k1} and their d: [value][XT]
+    // exchange twiddles W_N^{n2 k1} and their d: [value][T]
     static constexpr size_t off_xtw = (off_td + sizeof(float) * F::TD + 15) & ~size_t(15);
-    static constexpr size_t off_xtd = off_xtw + (C > 1 ? sizeof(float2) * XC::NV * XC::XT : 0);
-    static constexpr size_t off_edge = (off_xtd + (C > 1 ? sizeof(float) * XC::NV * XC::XT : 0) + 15) & ~size_t(15);
+    static constexpr size_t off_xtd = off_xtw + (C > 1 ? sizeof(float2) * XC::NV * T : 0);
+    static constexpr size_t off_edge = (off_xtd + (C > 1 ? sizeof(float) * XC::NV * T : 0) + 15) & ~size_t(15);
     static constexpr size_t off_halo = off_edge + sizeof(float2) * 4 * NW;           // [parity][first, last][warp]
     // Heun: E and increment of the 4 halo points of every segment; RK23: the neighbours'
     // end values [parity][segment][left, right]
@@ -714,7 +713,6 @@ template <int M, int C>
 __device__ __forceinline__ void exchange_fwd(const float2* g, float2* bufx, uint32_t x, uint32_t bar, const float2* xtw,
                                              const Inner<M, C>& in, int t, int c) {
     using XC = Xch<M, C>;
-    if (t >= XC::XT) return;
     if constexpr (XC::SPLIT) {
         constexpr int P = XC::P;
         const int l = t % XC::LANES, col = t / XC::LANES;
@@ -727,7 +725,7 @@ __device__ __forceinline__ void exchange_fwd(const float2* g, float2* bufx, uint
         lanes_fwd<XC::LANES, P>(v, l);
 #pragma unroll
         for (int r = 0; r < P; ++r) {
-            const float2 o[1] = {cmul(v[r], xtw[r * XC::XT + t])};
+            const float2 o[1] = {cmul(v[r], xtw[r * XC::T + t])};
             push_block<1, XC::LOCAL>(bufx, x, bar, outer_k1<M, C>(r, t), c * XC::COLS + col, o, c);
         }
     } else {
@@ -743,7 +741,7 @@ __device__ __forceinline__ void exchange_fwd(const float2* g, float2* bufx, uint
         for (int u = 0; u < XC::PER; ++u) {
             dftp<C>(v[u]);
 #pragma unroll
-            for (int r = 1; r < C; ++r) v[u][r] = cmul(v[u][r], xtw[(u * (C - 1) + r - 1) * XC::XT + t]);
+            for (int r = 1; r < C; ++r) v[u][r] = cmul(v[u][r], xtw[(u * (C - 1) + r - 1) * XC::T + t]);
         }
 #pragma unroll
         for (int r = 0; r < C; ++r) {
@@ -778,7 +776,6 @@ template <int M, int C, bool HALO>
 __device__ __forceinline__ void exchange_inv(const float2* g, float2* bufx, uint32_t halo, uint32_t bar, const float2* xtw,
                                              const float* xtd, const Inner<M, C>& in, int t, int c, float invN) {
     using XC = Xch<M, C>;
-    if (t >= XC::XT) return;
     if constexpr (XC::SPLIT) {
         constexpr int P = XC::P;
         const int l = t % XC::LANES, col = t / XC::LANES;
@@ -786,7 +783,7 @@ __device__ __forceinline__ void exchange_inv(const float2* g, float2* bufx, uint
 #pragma unroll
         for (int r = 0; r < P; ++r) {
             v[r] = g[swz(outer_k1<M, C>(r, t) * XC::COLS + col)];
-            v[r] = mul_recip(v[r], xtw[r * XC::XT + t], xtd[r * XC::XT + t]);
+            v[r] = mul_recip(v[r], xtw[r * XC::T + t], xtd[r * XC::T + t]);
         }
         lanes_inv<XC::LANES, P>(v, l);
 #pragma unroll
@@ -815,7 +812,7 @@ __device__ __forceinline__ void exchange_inv(const float2* g, float2* bufx, uint
             w[0] = v[u][0];
 #pragma unroll
             for (int r = 1; r < C; ++r) {               // register r of the inverse DFT holds k1 = bitrev(r)
-                const int i = (u * (C - 1) + r - 1) * XC::XT + t;
+                const int i = (u * (C - 1) + r - 1) * XC::T + t;
                 w[r] = mul_recip(v[u][brev4(r, ilog2(C))], xtw[i], xtd[i]);
             }
             dftp_inv<C>(w);
@@ -1043,14 +1040,12 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     fft_tables<M, P>(tw_s, td_s, tabs.quad, t);
     if constexpr (C > 1) {
         using XC = Xch<M, C>;
-        if (t < XC::XT) {
 #pragma unroll 1
-            for (int i = 0; i < XC::NV; ++i) {
-                const int n2 = c * XC::COLS + (XC::SPLIT ? t / XC::LANES : t * XC::PER + i / (C - 1));
-                const float2 w = twn_val<M, C>(tabs.quad, tabs.low, n2 * outer_k1<M, C>(i, t));
-                xtw_s[i * XC::XT + t] = w;
-                xtd_s[i * XC::XT + t] = inv_norm2_m1(w);
-            }
+        for (int i = 0; i < XC::NV; ++i) {
+            const int n2 = c * XC::COLS + (XC::SPLIT ? t / XC::LANES : t * XC::PER + i / (C - 1));
+            const float2 w = twn_val<M, C>(tabs.quad, tabs.low, n2 * outer_k1<M, C>(i, t));
+            xtw_s[i * XC::T + t] = w;
+            xtd_s[i * XC::T + t] = inv_norm2_m1(w);
         }
     }
     Inner<M, C> inner;

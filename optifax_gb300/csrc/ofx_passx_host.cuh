@@ -76,9 +76,9 @@ inline cudaError_t xattributes(const XKernel<R>& k) {
 // CTA up to 2^13 points, then n / 16 (one pulse, us per attempt, GB300, FP64 at 1024 and
 // 512 points per CTA: 2^10 38 and 26, 2^12 48 and 30, 2^13 53 and 33; float-float at 2^13
 // 19 and 16; measured before the absorber's factors were kept, now 24, 28, 30 and 12.5 at
-// 512).  Several pulses on one schedule run at once, so they take 1024 points per
-// CTA (float-float: 512 up to 2^12 points) where the wider shape's clusters do not all
-// fit the GPU.
+// 512).  Several pulses on one schedule run at once: at 2^13 points the GPU holds 14 of
+// them at 512 points per CTA and one more at 1024 (below, it holds as many at 512 as a
+// call may have; above, there is one shape).
 template <typename R>
 inline const XKernel<R>* xchoose(const std::vector<XKernel<R>>& kernels, int n, int B, bool nee) {
     auto find = [&](int m) -> const XKernel<R>* {
@@ -87,11 +87,9 @@ inline const XKernel<R>* xchoose(const std::vector<XKernel<R>>& kernels, int n, 
             if (k.M == m && k.C == n / m && k.nee == nee) return &k;
         return nullptr;
     };
-    const XKernel<R>* narrow = find(n < 1024 || (std::is_same<R, ff>::value && n <= 4096) ? 512 : 1024);
     const XKernel<R>* wide = find(512);
-    if (!narrow || !wide) return narrow;
-    if (wide != narrow && B > 1 && (xattributes(*wide) != cudaSuccess || B > xresident(*wide))) return narrow;
-    return wide;
+    if (n != 8192 || B == 1 || !wide) return wide;
+    return xattributes(*wide) != cudaSuccess || B > xresident(*wide) ? find(1024) : wide;
 }
 
 // What a call reads back: the schedule's statistics and the shared schedule's words
