@@ -357,7 +357,7 @@ struct Xch {
 struct RunState {
     double tally[4], prev_tally;
     unsigned long long grid_last[3];      // shared schedules: the grid's words after their last round
-    int n_acc, n_rej, tot_att, tot_acc, tot_rej, steady, stop, slots, trips_done, status, trip_status;
+    int n_acc, n_rej, tot_att, tot_acc, tot_rej, steady, stop, slots, trips_done, status;
     // where registers are short: the next attempt's z-phasors and G sample, the classes' bounds
     float2 z[3];
     float g;
@@ -1185,6 +1185,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
     Pair k1r[H];      // RK23: K1 (first stage, FSAL) between attempts
     do {
         k = nee ? 1.f : 0.f; stepprev = 4.f; stepmod = 4.f; q = 0;
+        int trip_status = 0;
         int limit = gatt + cfg.max_attempts_mul * (P_.S + 16) + 64;     // of this trip's attempts
         if constexpr (!heun) {
             // initial K1 at k = 0 with stepmod = 4 (OPO_CUDA_ODE23.cu:432-438)
@@ -1321,7 +1322,7 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
                                                   c, cfg);
                 if (fl & kDead) goto done;
                 if ((opts & kForced) && gatt < P_.n_forced) fl = (P_.forced[gatt] & 3) | (fl & 4);
-                if ((fl & 4) && t == 0) run->trip_status |= OPTIFAX_PULSE_NAN;
+                if (fl & 4) trip_status |= OPTIFAX_PULSE_NAN;
 
                 if ((fl & 1) && stepmod > 1.f && (nee || (k - stepmod) > 0.f)) {
                     // ---- reject: A0 unchanged; MEX: k moves back by one in net (the loop
@@ -1530,15 +1531,15 @@ pass_kernel(const PulseDev* __restrict__ pulses, FftTables tabs, KernelCfg cfg) 
         }
         if (t == 0) {
             const int trip = run->trips_done, attempts = gatt - run->tot_att;
-            run->status |= run->trip_status;
+            run->status |= trip_status;
             if (rec && P_.fb && P_.trips) {
                 optifax_trip_record tr;
-                tr.attempts = attempts; tr.accepted = run->n_acc; tr.rejected = run->n_rej; tr.status = run->trip_status;
+                tr.attempts = attempts; tr.accepted = run->n_acc; tr.rejected = run->n_rej; tr.status = trip_status;
                 for (int i = 0; i < 4; ++i) tr.tally[i] = run->tally[i];
                 P_.trips[trip] = tr;
             }
             run->tot_att = gatt; run->tot_acc += run->n_acc; run->tot_rej += run->n_rej;
-            run->n_acc = run->n_rej = run->trip_status = 0;
+            run->n_acc = run->n_rej = 0;
             // steady state of a cavity: the totals are the same in every CTA of the cluster
             const double cur = run->tally[P_.steady_tally & 3];
             const bool flat = trip > 0 && cur != 0.0 &&
