@@ -30,9 +30,11 @@ WORKLOAD = ("SPOPO round trips: N=2^14 over 12 ps, 5 mm MgO:PPLN 30 um, sech2 10
             "10% OC, signal-band feedback, delay 0, noise seed 1")
 
 
-# DRAM bytes per OPO round trip of pass_kernel<4096, 4, HEUN>: ncu dram__bytes_read.sum
-# (1,914,112) + dram__bytes_write.sum (159,232) of the bench's timed 10-trip launch
-TRAFFIC_PER_TRIP = (1914112 + 159232) / 10.0
+# DRAM bytes of one launch of pass_kernel<1024, 16, HEUN> on this workload: ncu
+# dram__bytes_read.sum of a two-trip launch behind a 256 MB write (dram__bytes_write.sum 0);
+# 1.1 to 1.9 MB for one trip and 2.0 to 2.4 MB for two, so the launch's inputs and tables, not
+# a cost per trip
+TRAFFIC_PER_LAUNCH = 1988864.0
 
 
 def _spec():
@@ -938,7 +940,8 @@ def main():
     if rank == 0 and world == 1 and not args.no_sweep:
         sweep_line = sweep_record(1, 1, cpu_kw={"n_sample": 16, "fraction": 0.01})
 
-    M = args.cta_points or N // 16          # the library's choice for one pulse of this size
+    # the library's choice for one pulse
+    M = args.cta_points or (N if N <= 1024 else 512 if N <= 4096 else 1024 if N <= 16384 else max(N // 16, 2048))
     if rank == 0:
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K, "warmup": W,
@@ -954,10 +957,10 @@ def main():
                        "attempts_timed": attempts,
                        "l2": "flushed (256 MB write) before the timed launch; the field stays on-chip by design"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": TRAFFIC_PER_TRIP * K,
-                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the timed "
-                                           "launch at 10 trips (2.07 MB, four-CTA kernel), per trip x trips: the field stays "
-                                           "on chip, so real DRAM traffic is tables and per-step G reads",
+                         "frac": achieved / peak, "traffic": TRAFFIC_PER_LAUNCH,
+                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of a two-trip launch of "
+                                           "the timed kernel (1.99 MB + 0; 1.1 to 1.9 MB for one trip): the field stays "
+                                           "on chip, so a launch reads its inputs and tables and little per trip",
                          "peak_kind": peak_kind,
                          "algorithmic": "16 B per grid point per step attempt",
                          "compute_tflops": flops_per_launch / (t_max / 1000.0) / 1e12},

@@ -213,7 +213,7 @@ int optifax_propagate(optifax_handle h, const optifax_pulse* pulses, int32_t n_p
  * The same batch as optifax_propagate recorded once into a CUDA graph and then
  * replayed: the graph holds one persistent grid per (cta_points, cluster) group,
  * forked and joined as optifax_propagate launches them, with its own descriptors
- * and cavity scratch (no host staging on replay).  The pulses' device pointers
+ * (no host staging on replay; passes need no scratch).  The pulses' device pointers
  * (inputs, outputs, stats) are fixed at capture: every replay reads the inputs'
  * current contents and rewrites the outputs.  No counterpart in the reference,
  * whose batch shares one cuFFT plan and one step.  The graph uses the handle's

@@ -411,8 +411,7 @@ __device__ __forceinline__ Tp* remote(Tp* p, int rank) {
 }
 
 // 32-bit shared::cluster addressing: `mapa` turns a local shared address into the
-// same offset in CTA `rank` of the cluster (half the registers of generic pointers;
-// clusters of up to 4 -- with 8 the generic stores measured faster)
+// same offset in CTA `rank` of the cluster (half the registers of generic pointers)
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
