@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(256) k_lift(const float* __restrict__ x, const
 // What cost time in that order were its loads, one dependent step after the other, so a
 // block of U outputs and MB samples first copies its rows of `in` and its weights to shared
 // memory, all copies in flight at once; then a warp per (output, sample), lane = mode,
-// runs the 64 steps.
+// runs the 64 steps (32 samples: 6.8 us cold, 14 in eight partial sums from global memory).
 template <int U, int MB>
 struct Mix {
     static constexpr int IN = W * MB * SPEC;                              // floats: [v][sample][2 m]
@@ -363,7 +363,8 @@ __global__ void __launch_bounds__(128, 4)
 // y[b][j][x] = x[b][j][x] + (q[j] + sum_c Q[j][c] h[b][x][c]), c in turn: the loss's
 // gradient is a difference of y that is rounded to BF16.  Four lanes share a bin, one output
 // each; they read the same 16 bytes of its row, and of the weights 16 bytes each, four banks
-// apart.
+// apart (32 samples of 4096 bins: 14.0 us cold, waiting on its loads; 10.5 with 16 channels a
+// lane, whose sums had another order).
 __global__ void __launch_bounds__(256) k_proj_fwd(const bf16* __restrict__ Ht, const bf16* __restrict__ Qw,
                                                   const float* __restrict__ qb, const float* __restrict__ xin, int B,
                                                   int L, float* __restrict__ y) {
